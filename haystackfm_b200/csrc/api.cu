@@ -27,6 +27,8 @@
 #include "hfm_internal.h"
 #include "resolve.cuh"
 #include "search.cuh"
+#include "smem.cuh"
+#include "trie.cuh"
 
 namespace hfm {
 
@@ -96,8 +98,8 @@ struct DevBuf {
 };
 
 struct Counters {                    // device-side counters, one block per handle
-  unsigned long long iv_used, hit_used, touches, steps, seg_used;
-  uint32_t n_ovf, still_ovf, walk_err, queue, queue2, n_mid, n_wrp, queue3, seg_queue, merge_queue, fix_queue, _pad;
+  unsigned long long iv_used, hit_used, touches, steps, n_units;
+  uint32_t n_ovf, still_ovf, walk_err, queue, queue2, n_mid, n_wrp, queue3, n_long, trie_queue, n_left, _pad;
 };
 
 struct FmDev {
@@ -123,8 +125,8 @@ struct hfm_index {
   DevBuf q, qoff, counts, nhits, niv, ivoff, status, ovf, ivpool, hitpool, seg_row, seg_off, pos_base, seg_base,
       scan_tmp, out_pairs, ref_bounds, hit_start, hit_count, hit_base, hits, npos_scan, work, cwork, ctr,
       mivpool, bswork, memwork, hkeys, hslot, hflags, huid, urow, ulen, uoff, uout, blockmap, blockmap2, ovf2, ovf3,
-      lflag, lpos, sids, lids, ucount, ubase, uread, uk, ubits, uexit, ust, ucoff, ucnt, segpool, fxe, fxc, fxx,
-      fxo, fxn, npos, loc_pairs, okeys, oids, otemp;
+      lflag, lpos, sids, lids, ucount, ubase, uread, uk, nslot, slot_base, slot_hits, npos, loc_pairs, okeys, oids,
+      otemp, trie_nodes, trie_left, trie_resume;
   uint32_t flags = 0;
   uint32_t seg_len = 512;  // SMEM reads longer than 2 * seg_len take the segmented sweep
   uint32_t queue_chunk = 1;       // reads a per-thread kernel takes from its queue per atomic
@@ -135,7 +137,6 @@ struct hfm_index {
                           // candidate lists; 3 global 1024-entry lists
   int num_sms = 0;
   uint64_t iv_cap = 0, miv_cap = 0, hit_cap = 0;   // pool capacities in elements (uint2 / BIv / hit)
-  uint64_t seg_cap = 0;                            // segment candidate pool capacity (Cand)
   Counters* h_ctr = nullptr;        // pinned
   uint32_t timeout_ms = 0;          // host-side deadline of every wait on the stream (0: none)
   std::vector<void*> orphans;       // result blocks of calls that timed out (freed once the stream drains)
@@ -174,8 +175,9 @@ static int build_device_fm(const HostFm& h, FmDev& f, cudaStream_t s) {
   const uint64_t width = h.encoding == 0 ? h.num_planes : L;
   // Decode the reference records (compacted lanes, u32 superblock count + u16 delta per
   // lane) into whole per-symbol counts and 4 symbol-code bitplanes, then re-encode them as
-  // the device records: whole counts (wide) or counts from the start of the device
-  // superblock of 1024 records, which fit a u16 (narrow).
+  // the device records: whole counts (wide; brought to row 32 on the device, k_wide_records)
+  // or counts from the start of the device superblock of 1024 records, which fit a u16
+  // (narrow).
   auto decode = [&](uint64_t b, uint32_t cnt[16], uint64_t planes[4]) {
     const uint8_t* r = h.block_data + b * h.block_stride;
     uint64_t words[16] = {0};
@@ -251,6 +253,10 @@ static int build_device_fm(const HostFm& h, FmDev& f, cudaStream_t s) {
     if (k == 4 && !h.has_lookup) continue;
     RET(upload(*bufs[k], srcs[k], sizes[k], s));
     f.nbytes[k] = sizes[k];
+  }
+  if (fmt == OCC_WIDE) {
+    k_wide_records<<<(unsigned)((nblk + 255) / 256), 256, 0, s>>>(f.occ.as<uint4>(), (uint32_t)nblk);
+    CK(cudaGetLastError());
   }
   CK(cudaStreamSynchronize(s));      // host vectors die at return
   DevFm& d = f.d;
@@ -328,10 +334,11 @@ static constexpr uint32_t BS_SET_CAP = 64;     // fast-path interval-set capacit
 static constexpr uint32_t BS_WARP_SET_CAP = 8192;   // long-tail pass, per warp
 static constexpr uint32_t MEM_SET_CAP = FAST_SET_CAP;   // fast-path interval-set capacity (SMEM / MEM)
 static constexpr uint32_t MEM_WARP_SET_CAP = 8192;  // long-tail pass, per warp
-static constexpr int MEM_KC = 32;              // fast-path candidate capacity (thread-local)
-static constexpr uint32_t MID_CAND_CAP = 1024;  // candidate list of the per-thread rerun (global memory)
+static constexpr int MEM_KC = 32;              // hit list of fast-pass variant 2 (thread-local)
+static constexpr uint32_t MID_HIT_CAP = 1024;  // hit list of the per-thread rerun (global memory)
 static constexpr uint32_t MID_THREADS_PER_SM = 256;
-static constexpr uint32_t FAST_CAND_CAP = 1024;  // global candidate list of fast-pass variant 3
+static constexpr uint32_t FAST_HIT_CAP = 1024;   // hit list of fast-pass variant 3 (global memory)
+static constexpr uint64_t MEM_SET_BYTES = 2ull * MEM_SET_CAP * 12;   // the two interval sets of a thread
 static constexpr int MEMS_PLAIN = 4;             // mems_variant of the plain one-thread-per-read launch
 
 // Backward search for a batch.  with_ivs = false: counts only.
@@ -597,6 +604,27 @@ static int prefix_order(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff
   return HFM_OK;
 }
 
+// How k_trie runs a batch of nq reads: resident warps and reads per warp.  A warp's nodes
+// are shared by its reads, so groups are as large as the batch allows while every resident
+// warp still has one; beyond that a whole number of rounds keeps the last one full.
+static constexpr size_t TRIE_SMEM = TRIE_WARPS * sizeof(TrieShared);
+static int trie_plan(hfm_index* x, uint32_t nq, uint32_t& blocks, uint32_t& group) {
+  int bpsm = 0;
+  for (auto k : {k_trie<false>, k_trie<true>})
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRIE_SMEM));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_trie<false>, TRIE_WARPS * 32, TRIE_SMEM));
+  const uint64_t warps = (uint64_t)std::max(1, bpsm) * x->num_sms * TRIE_WARPS;
+  const uint64_t rounds = std::max<uint64_t>(1, (nq + warps * 32 - 1) / (warps * 32));
+  group = (uint32_t)std::max<uint64_t>(1, (nq + warps * rounds - 1) / (warps * rounds));
+  const uint64_t groups = (nq + group - 1) / group;
+  blocks = (uint32_t)std::max<uint64_t>(1, (std::min(warps, groups) + TRIE_WARPS - 1) / TRIE_WARPS);
+  RET(x->trie_nodes.ensure((size_t)blocks * TRIE_WARPS * TRIE_NODE_BYTES));
+  RET(x->trie_left.ensure((size_t)nq * 4 + 4));
+  RET(x->trie_resume.ensure((size_t)nq * 4 + 4));
+  return HFM_OK;
+}
+static constexpr uint32_t TRIE_SORT_GROUP = 4;   // groups of this many reads or more are formed by prefix
+
 static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff, uint32_t nq, uint32_t min_len,
                        uint32_t mode, const uint32_t* h_bounds, uint32_t nb, uint32_t cap, hfm_dev_mems* out,
                        const hfm_sched* sc = nullptr) {
@@ -619,7 +647,14 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
   if (n_warp && !order) return set_error(HFM_E_ARG, "sched.n_warp needs sched.d_order");
   begin_stats(x);
   uint32_t launches = 0, other = 0;
-  if (!order && x->read_order == 1 && x->threads_per_read == 1 && x->mems_variant != MEMS_PLAIN && nq > 1) {
+  // IUPAC texts: the first sweep of the reads in one piece is shared by the reads of a warp
+  // (k_trie).  A per-read work log needs every read's own work.
+  const bool trie = x->fwd.fmt == OCC_WIDE && x->mems_variant == 3 && x->threads_per_read == 1 && !wlog && min_len > 0 &&
+                    nq > n_warp;
+  uint32_t tblocks = 0, tgroup = 0;
+  if (trie) RET(trie_plan(x, nq - n_warp, tblocks, tgroup));
+  if (!order && x->threads_per_read == 1 && x->mems_variant != MEMS_PLAIN && nq > 1 &&
+      (x->read_order == 1 || (trie && tgroup >= TRIE_SORT_GROUP))) {
     RET(prefix_order(x, d_q, d_qoff, nq, order, other));
     own_order = true;
   }
@@ -637,77 +672,76 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
   bool counting = x->count_work || wlog;
   RET(x->ref_bounds.ensure((size_t)nb * 4 + 4));
   if (nb) CK(cudaMemcpyAsync(x->ref_bounds.p, h_bounds, (size_t)nb * 4, cudaMemcpyHostToDevice, x->stream));
-  RET(x->hit_start.ensure((size_t)nq * 8 + 8)); RET(x->hit_count.ensure((size_t)nq * 4 + 4));
   RET(x->status.ensure((size_t)nq * 4 + 4)); RET(x->ovf.ensure((size_t)nq * 4 + 4));
   if (x->miv_cap < (uint64_t)nq * 24 + 4096) x->miv_cap = (uint64_t)nq * 24 + 4096;     // BIv = 16 B
   if (x->hit_cap < (uint64_t)nq * 24 + 4096) x->hit_cap = (uint64_t)nq * 24 + 4096;   // hit = 32 B
   MemsParams P{min_len, mode, cap, nb ? 1u : 0u};
   const FmDev& Fw = x->fwd; const FmDev& Rv = x->rev;
   // persistent fast pass: one wave of resident threads, MEM_SET_CAP intervals per set.
-  // Variant 2: 8 resident blocks of 128 threads per SM with a 32-entry candidate list in
-  // local memory; variant 3 (default): 8 blocks per SM with a 1024-entry list per thread
-  // in global memory, so reads up to ~10 kbp finish in this pass.  The kernels are
-  // specialised for the index's Occ record format (narrow or wide).
+  // Variant 2: hit lists of 32 entries in local memory; variant 3 (default): 1024 entries per
+  // thread in global memory, and long reads cut into segments.  The kernels are specialised
+  // for the index's Occ record format (narrow or wide).
   int variant = x->mems_variant;
   int bpsm = 0;
   const uint32_t fmt = Fw.fmt;
   WITH_FMT(fmt, {
-    if (variant == 3) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_mems<false, 32, 0, 8, FM>, 128, 0));
-    else CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_mems<false, 32, MEM_KC, 8, FM>, 128, 0));
+    if (variant == 2) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_smem<false, 32, MEM_KC, 8, FM>, 128, 0));
+    else CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_smem<false, 32, 0, 8, FM>, 128, 0));
   });
   const uint64_t full_threads = (uint64_t)std::max(1, bpsm) * x->num_sms * 128;
-  uint64_t threads = std::min<uint64_t>(full_threads, ((uint64_t)nq + 127) / 128 * 128);
-  // Long reads (SMEM mode with global candidate lists) take the segmented sweep: the
-  // fast pass gets the other reads, in the same relative order.
+  // Reads longer than 2 * seg_len (variant 3) are searched as segments; the fast pass gets
+  // the other reads whole, in the same relative order.
   const uint32_t* fast_ids = order ? order + n_warp : nullptr;
   uint32_t n_fast = nq - n_warp, n_long = 0;
-  uint64_t n_units = 0;
-  if (mode == 0 && variant == 3 && n_fast > 0 && min_len > 0) {
+  uint64_t n_units = 0, n_slots = nq;
+  const uint64_t* slot_base = nullptr;
+  if (variant == 3 && n_fast > 0 && min_len > 0) {
+    CK(cudaMemsetAsync(x->ctr.p, 0, sizeof(Counters), x->stream));
+    RET(x->nslot.ensure((size_t)nq * 4 + 4));
+    if (n_warp) CK(cudaMemsetAsync(x->nslot.p, 0, (size_t)nq * 4, x->stream));
     RET(x->lflag.ensure((size_t)n_fast * 4 + 4));
-    RET(x->lpos.ensure(((size_t)n_fast + 1) * 8));
-    k_long_flags<<<(n_fast + 255) / 256, 256, 0, x->stream>>>(fast_ids, n_fast, d_qoff, 2 * x->seg_len,
-                                                              x->lflag.as<uint32_t>());
+    k_long_reads<<<(n_fast + 255) / 256, 256, 0, x->stream>>>(fast_ids, n_fast, d_qoff, x->seg_len, x->lflag.as<uint32_t>(),
+                                                              x->nslot.as<uint32_t>(), &dctr(x)->n_long, &dctr(x)->n_units);
     other++;
     CK(cudaGetLastError());
-    RET(scan(x, x->lflag.as<uint32_t>(), 1, n_fast, x->lpos.as<uint64_t>(), other));
-    uint64_t nl = 0;
-    RET(read_u64(x, x->lpos.as<uint64_t>() + n_fast, nl));
-    n_long = (uint32_t)nl;
+    RET(read_ctr(x));
+    n_long = x->h_ctr->n_long;
+    n_units = x->h_ctr->n_units;
     if (n_long) {
+      RET(x->lpos.ensure(((size_t)n_fast + 1) * 8));
       RET(x->sids.ensure((size_t)n_fast * 4 + 4));
       RET(x->lids.ensure((size_t)n_long * 4 + 4));
       RET(x->ucount.ensure((size_t)n_long * 4 + 4));
+      RET(x->ubase.ensure(((size_t)n_long + 1) * 8));
+      RET(x->uread.ensure(n_units * 4)); RET(x->uk.ensure(n_units * 4));
+      RET(x->slot_base.ensure(((size_t)nq + 1) * 8));
+      if (n_warp)                              // routed reads keep one slot each
+        k_fill_listed<<<(n_warp + 255) / 256, 256, 0, x->stream>>>(order, n_warp, x->nslot.as<uint32_t>(), 1u);
+      RET(scan(x, x->lflag.as<uint32_t>(), 1, n_fast, x->lpos.as<uint64_t>(), other));
       k_split_ids<<<(n_fast + 255) / 256, 256, 0, x->stream>>>(fast_ids, n_fast, x->lflag.as<uint32_t>(),
                                                                x->lpos.as<uint64_t>(), x->sids.as<uint32_t>(),
                                                                x->lids.as<uint32_t>(), x->ucount.as<uint32_t>(), d_qoff,
                                                                x->seg_len);
-      other++;
-      CK(cudaGetLastError());
-      RET(x->ubase.ensure(((size_t)n_long + 1) * 8));
       RET(scan(x, x->ucount.as<uint32_t>(), 1, n_long, x->ubase.as<uint64_t>(), other));
-      RET(read_u64(x, x->ubase.as<uint64_t>() + n_long, n_units));
-      RET(x->uread.ensure(n_units * 4)); RET(x->uk.ensure(n_units * 4));
-      RET(x->ubits.ensure(n_units * (x->seg_len / 32) * 4)); RET(x->uexit.ensure(n_units * 4));
-      RET(x->ust.ensure(n_units * 4)); RET(x->ucoff.ensure(n_units * 8)); RET(x->ucnt.ensure(n_units * 4));
-      RET(x->fxe.ensure(n_units * 4)); RET(x->fxc.ensure(n_units * 4)); RET(x->fxx.ensure(n_units * 4));
-      RET(x->fxo.ensure(n_units * 8)); RET(x->fxn.ensure(n_units * 4));
       k_unit_fill<<<(n_long + 255) / 256, 256, 0, x->stream>>>(x->lids.as<uint32_t>(), n_long, x->ubase.as<uint64_t>(),
                                                                x->uread.as<uint32_t>(), x->uk.as<uint32_t>());
-      other++;
+      RET(scan(x, x->nslot.as<uint32_t>(), 1, nq, x->slot_base.as<uint64_t>(), other));
+      other += n_warp ? 3 : 2;
       CK(cudaGetLastError());
+      slot_base = x->slot_base.as<uint64_t>();
       fast_ids = x->sids.as<uint32_t>();
       n_fast -= n_long;
-      x->seg_cap = std::max<uint64_t>(x->seg_cap, n_units * 24 + 65536);
-      threads = std::max<uint64_t>(threads, std::min<uint64_t>(full_threads, (n_units + 127) / 128 * 128));
+      n_slots = (uint64_t)nq - n_long + n_units;
+      if (n_slots >= 0xFFFFFFFFull) return set_error(HFM_E_ARG, "too many read segments in one call");
     }
   }
+  const uint64_t threads = std::min<uint64_t>(full_threads, (n_units + n_fast + 127) / 128 * 128);
+  RET(x->hit_start.ensure(n_slots * 8 + 8)); RET(x->hit_count.ensure(n_slots * 4 + 4));
   const bool plain = variant == MEMS_PLAIN;
   if (plain && (order || n_warp)) return set_error(HFM_E_ARG, "the plain launch takes no schedule");
   if (!plain) {
-    RET(x->memwork.ensure(std::max<uint64_t>(threads, 32) * 4 * MEM_SET_CAP * 16));
-    // variant 3: candidate lists in global memory (FAST_CAND_CAP per thread), so long reads
-    // stay on the fast pass instead of overflowing a 32-entry local list
-    if (variant == 3) RET(x->cwork.ensure((size_t)std::max<uint64_t>(threads, 128) * FAST_CAND_CAP * sizeof(Cand)));
+    RET(x->memwork.ensure(std::max<uint64_t>(threads, 128) * MEM_SET_BYTES));
+    if (variant == 3) RET(x->cwork.ensure((size_t)std::max<uint64_t>(threads, 128) * FAST_HIT_CAP * 32));
   } else if (nq) {
     // plain launch, count pass: every read's MemHits and positions counted by a full
     // search, read back and prefix-summed to size the outputs before the write pass
@@ -721,16 +755,16 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       if (counting)
         k_mems_plain<true, 0, FM><<<(nq + 127) / 128, 128, 0, x->stream>>>(
             Fw.d, Rv.d, Fw.compat.as<uint16_t>(), Rv.compat.as<uint16_t>(), d_q, d_qoff, P, nq, none, none, oc,
-            x->npos.as<uint32_t>(), &dctr(x)->seg_used);
+            x->npos.as<uint32_t>(), &dctr(x)->n_units);
       else
         k_mems_plain<false, 0, FM><<<(nq + 127) / 128, 128, 0, x->stream>>>(
             Fw.d, Rv.d, Fw.compat.as<uint16_t>(), Rv.compat.as<uint16_t>(), d_q, d_qoff, P, nq, none, none, oc,
-            x->npos.as<uint32_t>(), &dctr(x)->seg_used);
+            x->npos.as<uint32_t>(), &dctr(x)->n_units);
     });
     launches++;
     CK(cudaGetLastError());
     RET(read_ctr(x));
-    const uint64_t ivs_need = x->h_ctr->seg_used;
+    const uint64_t ivs_need = x->h_ctr->n_units;   // the count pass leaves its pool need there
     x->stats.occ_touches += x->h_ctr->touches;
     RET(x->hit_base.ensure(((size_t)nq + 1) * 8));
     RET(scan(x, x->hit_count.as<uint32_t>(), 1, nq, x->hit_base.as<uint64_t>(), other));
@@ -742,10 +776,10 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
   bool done = false;
   for (int attempt = 0; attempt < 8 && !done; attempt++) {
     RET(x->mivpool.ensure(x->miv_cap * 16)); x->miv_cap = x->mivpool.cap / 16;
-    if (n_long) { RET(x->segpool.ensure(x->seg_cap * sizeof(Cand))); x->seg_cap = x->segpool.cap / sizeof(Cand); }
     RET(x->hitpool.ensure(x->hit_cap * 32)); x->hit_cap = x->hitpool.cap / 32;
     CK(cudaMemsetAsync(x->ctr.p, 0, sizeof(Counters), x->stream));
     if (wlog && nq) CK(cudaMemsetAsync(wlog, 0, (size_t)nq * 16, x->stream));
+    if (!plain && nq) CK(cudaMemsetAsync(x->status.p, 0, (size_t)nq * 4, x->stream));
     Pool ivp{x->mivpool.p, &dctr(x)->iv_used, x->miv_cap}, hp{x->hitpool.p, &dctr(x)->hit_used, x->hit_cap};
     MemsOut o{x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), x->status.as<uint32_t>(),
               x->ovf.as<uint32_t>(), &dctr(x)->n_ovf, &dctr(x)->touches};
@@ -759,11 +793,11 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
         if (counting)
           k_mems_plain<true, 1, FM><<<(nq + 127) / 128, 128, 0, x->stream>>>(
               Fw.d, Rv.d, Fw.compat.as<uint16_t>(), Rv.compat.as<uint16_t>(), d_q, d_qoff, P, nq, ivp, hp, o,
-              x->npos.as<uint32_t>(), &dctr(x)->seg_used);
+              x->npos.as<uint32_t>(), &dctr(x)->n_units);
         else
           k_mems_plain<false, 1, FM><<<(nq + 127) / 128, 128, 0, x->stream>>>(
               Fw.d, Rv.d, Fw.compat.as<uint16_t>(), Rv.compat.as<uint16_t>(), d_q, d_qoff, P, nq, ivp, hp, o,
-              x->npos.as<uint32_t>(), &dctr(x)->seg_used);
+              x->npos.as<uint32_t>(), &dctr(x)->n_units);
       });
       launches++;
       CK(cudaGetLastError());
@@ -771,71 +805,39 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       x->k_search_rec = true;
     }
     if (!plain && (n_fast > 0 || n_long > 0)) cudaEventRecord(x->evk[0], x->stream);
-    if (!plain && n_fast > 0 && n_long == 0) {     // with long reads, k_mems_seg runs the short reads too
-      MemsWork W{x->memwork.as<BIv>(), MEM_SET_CAP, variant == 3 ? x->cwork.as<Cand>() : nullptr,
-                 variant == 3 ? FAST_CAND_CAP : 0u, &dctr(x)->queue, fast_ids, n_fast, &dctr(x)->still_ovf, 0u, wlog};
-      W.chunk = x->queue_chunk;
-      unsigned grid = (unsigned)(threads / 128);
-      if (x->memwork.cap < (size_t)grid * 128 * 4 * MEM_SET_CAP * 16) return set_error(HFM_E_ARG, "internal: work area too small");
-      if (variant == 3 && x->cwork.cap < (size_t)grid * 128 * FAST_CAND_CAP * sizeof(Cand))
-        return set_error(HFM_E_ARG, "internal: candidate area too small");
+    if (!plain && (n_fast > 0 || n_long > 0)) {
+      MemsWork W{};
+      W.sets = x->memwork.as<BIv>(); W.set_cap = MEM_SET_CAP;
+      W.hits = variant == 3 ? x->cwork.as<uint4>() : nullptr; W.hit_cap = variant == 3 ? FAST_HIT_CAP : 0u;
+      W.queue = &dctr(x)->queue; W.still_ovf = &dctr(x)->still_ovf; W.work_log = wlog; W.chunk = x->queue_chunk;
+      SmemJobs J{};
+      J.unit_read = x->uread.as<uint32_t>(); J.unit_k = x->uk.as<uint32_t>(); J.seg_len = x->seg_len;
+      J.n_units = (uint32_t)n_units; J.ids = fast_ids; J.n_ids = n_fast; J.slot_base = slot_base;
+      const unsigned grid = (unsigned)(threads / 128);
+      if (x->memwork.cap < (size_t)grid * 128 * MEM_SET_BYTES) return set_error(HFM_E_ARG, "internal: work area too small");
+      if (variant == 3 && x->cwork.cap < (size_t)grid * 128 * FAST_HIT_CAP * 32)
+        return set_error(HFM_E_ARG, "internal: hit list area too small");
+      if (trie && n_fast > 0) {
+        TrieWork T{x->trie_nodes.as<uint4>(), &dctr(x)->trie_queue, tgroup, x->trie_left.as<uint32_t>(), &dctr(x)->n_left,
+                   x->trie_resume.as<uint32_t>()};
+        auto run = [&](auto kern) {
+          kern<<<tblocks, TRIE_WARPS * 32, TRIE_SMEM, x->stream>>>(Fw.d, Rv.d, Rv.compat.as<uint16_t>(), d_q, d_qoff, P, hp, o,
+                                                                  T, J);
+        };
+        if (counting) run(k_trie<true>); else run(k_trie<false>);
+        launches++;
+        CK(cudaGetLastError());
+        J.ids = T.left; J.n_ids_dev = T.n_left; J.resume = T.resume;
+      }
       WITH_FMT(fmt, {
-        if (counting && variant == 3)
-          k_mems<true, 32, 0, 5, FM><<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(),
-                                                                  Rv.compat.as<uint16_t>(), d_q, d_qoff, P, ivp, hp, o, W);
-        else if (counting)
-          k_mems<true, 32, MEM_KC, 5, FM><<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(),
-                                                                       Rv.compat.as<uint16_t>(), d_q, d_qoff, P, ivp, hp,
-                                                                       o, W);
-        else if (variant == 3)
-          k_mems<false, 32, 0, 8, FM><<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(),
-                                                                   Rv.compat.as<uint16_t>(), d_q, d_qoff, P, ivp, hp, o, W);
-        else
-          k_mems<false, 32, MEM_KC, 8, FM><<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(),
-                                                                        Rv.compat.as<uint16_t>(), d_q, d_qoff, P, ivp, hp,
-                                                                        o, W);
+        auto go = [&](auto kern) {
+          kern<<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(), Rv.compat.as<uint16_t>(), d_q, d_qoff, P,
+                                            hp, o, W, J);
+        };
+        if (variant == 3) { if (counting) go(k_smem<true, 32, 0, 5, FM>); else go(k_smem<false, 32, 0, 8, FM>); }
+        else { if (counting) go(k_smem<true, 32, MEM_KC, 5, FM>); else go(k_smem<false, 32, MEM_KC, 8, FM>); }
       });
       launches++;
-      CK(cudaGetLastError());
-    }
-    if (n_long > 0) {
-      // segmented sweep of the long reads, then the merge along each read's true chain
-      SegWork G{x->seg_len, x->seg_len / 32, x->uread.as<uint32_t>(), x->uk.as<uint32_t>(), (uint32_t)n_units, x->ubits.as<uint32_t>(),
-                x->uexit.as<uint32_t>(), x->ust.as<uint32_t>(), x->ucoff.as<uint64_t>(), x->ucnt.as<uint32_t>(),
-                x->segpool.as<Cand>(), &dctr(x)->seg_used, x->seg_cap, fast_ids, n_fast, x->lids.as<uint32_t>(),
-                x->ubase.as<uint64_t>(), n_long, &dctr(x)->merge_queue, &dctr(x)->touches, x->fxe.as<uint32_t>(),
-                x->fxc.as<uint32_t>(), x->fxx.as<uint32_t>(), x->fxo.as<uint64_t>(), x->fxn.as<uint32_t>()};
-      MemsWork W{x->memwork.as<BIv>(), MEM_SET_CAP, x->cwork.as<Cand>(), FAST_CAND_CAP, &dctr(x)->seg_queue, nullptr,
-                 0u, &dctr(x)->still_ovf, 0u, wlog};
-      W.chunk = x->queue_chunk;
-      MemsWork Wf = W;
-      Wf.queue = &dctr(x)->fix_queue;
-      uint64_t ts = std::min<uint64_t>(threads / 128 * 128, (n_units + n_fast + 127) / 128 * 128);
-      uint64_t tmg = std::min<uint64_t>(threads / 128 * 128, ((uint64_t)n_long + 127) / 128 * 128);
-      unsigned gs = (unsigned)std::max<uint64_t>(1, ts / 128), gm = (unsigned)std::max<uint64_t>(1, tmg / 128);
-      if (x->memwork.cap < (size_t)gs * 128 * 4 * MEM_SET_CAP * 16 || x->cwork.cap < (size_t)gs * 128 * FAST_CAND_CAP * sizeof(Cand))
-        return set_error(HFM_E_ARG, "internal: work area too small");
-      WITH_FMT(fmt, {
-        if (counting) {
-          k_mems_seg<true, 32, 5, FM><<<gs, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(),
-                                                                 Rv.compat.as<uint16_t>(), d_q, d_qoff, P, ivp, hp, o, W, G);
-          k_mems_fix<true, 32, 5, FM><<<gs, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(),
-                                                                 Rv.compat.as<uint16_t>(), d_q, d_qoff, P, ivp, Wf, G);
-          k_mems_merge<true, 32, 5, FM><<<gm, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(),
-                                                                   Rv.compat.as<uint16_t>(), d_q, d_qoff, P, ivp, hp, o,
-                                                                   W, G);
-        } else {
-          k_mems_seg<false, 32, 8, FM><<<gs, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(),
-                                                                  Rv.compat.as<uint16_t>(), d_q, d_qoff, P, ivp, hp, o, W,
-                                                                  G);
-          k_mems_fix<false, 32, 8, FM><<<gs, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(),
-                                                                  Rv.compat.as<uint16_t>(), d_q, d_qoff, P, ivp, Wf, G);
-          k_mems_merge<false, 32, 8, FM><<<gm, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(),
-                                                                    Rv.compat.as<uint16_t>(), d_q, d_qoff, P, ivp, hp, o,
-                                                                    W, G);
-        }
-      });
-      launches += 3;
       CK(cudaGetLastError());
     }
     if (!plain && (n_fast > 0 || n_long > 0)) {
@@ -847,13 +849,13 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
     const uint32_t* wlist = x->ovf.as<uint32_t>();
     if (n_ovf) {
       x->stats.fallback_reads += n_ovf;
-      // Reads that outgrew only the 32-entry candidate list (long reads) rerun on the
-      // per-thread kernel with a MID_CAND_CAP-entry list in global memory; set overflows,
-      // reads the schedule routed, and middle-tier overflows go to the warp-per-read kernel.
+      // Reads that outgrew only a 32-entry hit list (variant 2) rerun on the per-thread kernel
+      // with MID_HIT_CAP entries in global memory; set overflows, reads the schedule routed,
+      // and what still overflows go to the warp-per-read kernel.
       RET(x->ovf2.ensure((size_t)nq * 4 + 4));
       RET(x->ovf3.ensure((size_t)nq * 4 + 4));
       CK(cudaMemsetAsync(&dctr(x)->n_mid, 0, 12, x->stream));
-      k_split_ovf<<<(n_ovf + 255) / 256, 256, 0, x->stream>>>(x->ovf.as<uint32_t>(), n_ovf, n_warp,
+      k_split_ovf<<<(n_ovf + 255) / 256, 256, 0, x->stream>>>(x->ovf.as<uint32_t>(), n_ovf, variant == 2 ? n_warp : n_ovf,
                                                               x->status.as<uint32_t>(), x->ovf3.as<uint32_t>(),
                                                               &dctr(x)->n_mid, x->ovf2.as<uint32_t>(), &dctr(x)->n_wrp);
       other++;
@@ -865,22 +867,23 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
                                           threads / 128 * 128});
         tm = std::max<uint64_t>(tm, 128);
         unsigned grid = (unsigned)(tm / 128);
-        if (x->memwork.cap < (size_t)grid * 128 * 4 * MEM_SET_CAP * 16) return set_error(HFM_E_ARG, "internal: work area too small");
-        RET(x->cwork.ensure((size_t)grid * 128 * MID_CAND_CAP * sizeof(Cand)));
-        MemsWork W{x->memwork.as<BIv>(), MEM_SET_CAP, x->cwork.as<Cand>(), MID_CAND_CAP, &dctr(x)->queue3,
-                   x->ovf3.as<uint32_t>(), n_mid, &dctr(x)->still_ovf, 0u, wlog};
+        if (x->memwork.cap < (size_t)grid * 128 * MEM_SET_BYTES) return set_error(HFM_E_ARG, "internal: work area too small");
+        RET(x->cwork.ensure((size_t)grid * 128 * MID_HIT_CAP * 32));
+        MemsWork W{};
+        W.sets = x->memwork.as<BIv>(); W.set_cap = MEM_SET_CAP; W.hits = x->cwork.as<uint4>(); W.hit_cap = MID_HIT_CAP;
+        W.queue = &dctr(x)->queue3; W.still_ovf = &dctr(x)->still_ovf; W.work_log = wlog;
+        SmemJobs J{};
+        J.ids = x->ovf3.as<uint32_t>(); J.n_ids = n_mid; J.slot_base = slot_base;
+        CK(cudaMemsetAsync(x->status.p, 0, (size_t)nq * 4, x->stream));
         MemsOut o2 = o;
         o2.ovf_list = x->ovf2.as<uint32_t>();
         o2.n_ovf = &dctr(x)->n_wrp;
         WITH_FMT(fmt, {
-          if (counting)
-            k_mems<true, 32, 0, 5, FM><<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(),
-                                                                    Rv.compat.as<uint16_t>(), d_q, d_qoff, P, ivp, hp, o2,
-                                                                    W);
-          else
-            k_mems<false, 32, 0, 8, FM><<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(),
-                                                                     Rv.compat.as<uint16_t>(), d_q, d_qoff, P, ivp, hp, o2,
-                                                                     W);
+          auto go = [&](auto kern) {
+            kern<<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(), Rv.compat.as<uint16_t>(), d_q, d_qoff,
+                                              P, hp, o2, W, J);
+          };
+          if (counting) go(k_smem<true, 32, 0, 5, FM>); else go(k_smem<false, 32, 0, 8, FM>);
         });
         launches++;
         CK(cudaGetLastError());
@@ -894,17 +897,18 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       // sub-warp pass over every read (threads_per_read 4, 8 or 16): one read per group of
       // G lanes with the fast pass's set and candidate capacities; reads that outgrow them
       // go on to the warp tier below
-      const uint64_t per_group = (uint64_t)MEM_SET_CAP * 4 * 16 + (uint64_t)FAST_CAND_CAP * sizeof(Cand);
+      const uint64_t per_group = (uint64_t)MEM_SET_CAP * 2 * 16 + (uint64_t)FAST_HIT_CAP * sizeof(Cand);
       const uint64_t groups = std::min<uint64_t>({(uint64_t)n_ovf, (uint64_t)x->num_sms * (2048 / G),
                                                   std::max<uint64_t>(128 / G, (8ull << 30) / per_group)});
       const unsigned grid = (unsigned)((groups * G + 127) / 128);
-      RET(x->work.ensure((size_t)grid * (128 / G) * MEM_SET_CAP * 4 * 16));
-      RET(x->cwork.ensure((size_t)grid * (128 / G) * FAST_CAND_CAP * sizeof(Cand)));
+      RET(x->work.ensure((size_t)grid * (128 / G) * MEM_SET_CAP * 2 * 16));
+      RET(x->cwork.ensure((size_t)grid * (128 / G) * FAST_HIT_CAP * sizeof(Cand)));
       RET(x->ovf3.ensure((size_t)nq * 4 + 4));
       CK(cudaMemsetAsync(&dctr(x)->n_mid, 0, 4, x->stream));
       CK(cudaMemsetAsync(&dctr(x)->queue2, 0, 4, x->stream));
-      MemsWork W{x->work.as<BIv>(), MEM_SET_CAP, x->cwork.as<Cand>(), FAST_CAND_CAP, &dctr(x)->queue2, wlist,
-                 n_ovf, &dctr(x)->still_ovf, 0u, wlog};
+      MemsWork W{};
+      W.sets = x->work.as<BIv>(); W.set_cap = MEM_SET_CAP; W.cands = x->cwork.as<Cand>(); W.cand_cap = FAST_HIT_CAP;
+      W.queue = &dctr(x)->queue2; W.ids = wlist; W.n = n_ovf; W.still_ovf = &dctr(x)->still_ovf; W.work_log = wlog;
       MemsOut o3 = o;
       o3.ovf_list = x->ovf3.as<uint32_t>();
       o3.n_ovf = &dctr(x)->n_mid;
@@ -922,20 +926,22 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       wlist = x->ovf3.as<uint32_t>();
     }
     if (n_ovf) {
-      // long tail: one warp per overflowed read, 4 sets and a candidate list per warp,
+      // long tail: one warp per overflowed read, two sets and a candidate list per warp,
       // growing 4x until every read fits
       uint32_t set_cap = MEM_WARP_SET_CAP, cand_cap = 1024;
       while (true) {
-        uint64_t per_warp = (uint64_t)set_cap * 4 * 16 + (uint64_t)cand_cap * sizeof(Cand);
+        uint64_t per_warp = (uint64_t)set_cap * 2 * 16 + (uint64_t)cand_cap * sizeof(Cand);
         uint64_t warps = std::min<uint64_t>({(uint64_t)n_ovf, (uint64_t)x->num_sms * 16,
                                              std::max<uint64_t>(4, (2ull << 30) / per_warp)});
         unsigned grid = (unsigned)((warps + 3) / 4);
-        RET(x->work.ensure((size_t)grid * 4 * set_cap * 4 * 16));
+        RET(x->work.ensure((size_t)grid * 4 * set_cap * 2 * 16));
         RET(x->cwork.ensure((size_t)grid * 4 * cand_cap * sizeof(Cand)));
         CK(cudaMemsetAsync(&dctr(x)->still_ovf, 0, 4, x->stream));
         CK(cudaMemsetAsync(&dctr(x)->queue2, 0, 4, x->stream));
-        MemsWork W{x->work.as<BIv>(), set_cap, x->cwork.as<Cand>(), cand_cap, &dctr(x)->queue2, wlist,
-                   n_ovf, &dctr(x)->still_ovf, 1u, wlog};
+        MemsWork W{};
+        W.sets = x->work.as<BIv>(); W.set_cap = set_cap; W.cands = x->cwork.as<Cand>(); W.cand_cap = cand_cap;
+        W.queue = &dctr(x)->queue2; W.ids = wlist; W.n = n_ovf; W.still_ovf = &dctr(x)->still_ovf; W.rerun = 1u;
+        W.work_log = wlog; W.slot_base = slot_base;
         if (counting)
           k_mems_warp<true><<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(), Rv.compat.as<uint16_t>(),
                                                         d_q, d_qoff, P, ivp, hp, o, W);
@@ -950,24 +956,28 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
         set_cap *= 4; cand_cap *= 4;
       }
     }
-    if (x->h_ctr->iv_used <= x->miv_cap && x->h_ctr->hit_used <= x->hit_cap &&
-        (n_long == 0 || x->h_ctr->seg_used <= x->seg_cap)) { done = true; break; }
+    if (x->h_ctr->iv_used <= x->miv_cap && x->h_ctr->hit_used <= x->hit_cap) { done = true; break; }
     x->miv_cap = std::max(x->miv_cap, (uint64_t)(x->h_ctr->iv_used * 3 / 2 + 4096));
     x->hit_cap = std::max(x->hit_cap, (uint64_t)(x->h_ctr->hit_used * 3 / 2 + 4096));
-    if (n_long) x->seg_cap = std::max(x->seg_cap, (uint64_t)(x->h_ctr->seg_used * 3 / 2 + 65536));
   }
   if (!done) return set_error(HFM_E_OVERFLOW, "MEM pools did not converge");
   x->stats.occ_touches += x->h_ctr->touches;
-  // CSR of hits, then positions
+  // CSR of hits (over the slots, then per read), then positions
   RET(x->hit_base.ensure(((size_t)nq + 1) * 8));
-  RET(scan(x, x->hit_count.as<uint32_t>(), 1, nq, x->hit_base.as<uint64_t>(), other));
+  if (slot_base) RET(x->slot_hits.ensure((n_slots + 1) * 8));
+  uint64_t* slot_hits = slot_base ? x->slot_hits.as<uint64_t>() : x->hit_base.as<uint64_t>();
+  RET(scan(x, x->hit_count.as<uint32_t>(), 1, n_slots, slot_hits, other));
   uint64_t nh = 0;
-  RET(read_u64(x, x->hit_base.as<uint64_t>() + nq, nh));
+  RET(read_u64(x, slot_hits + n_slots, nh));
   RET(x->hits.ensure(nh * 32 + 32));
   if (nq) {
-    k_gather_hits<<<(nq + 255) / 256, 256, 0, x->stream>>>(x->hitpool.as<uint4>(), x->hit_start.as<uint64_t>(),
-                                                          x->hit_count.as<uint32_t>(), x->hit_base.as<uint64_t>(), nq,
-                                                          x->hits.as<uint4>());
+    if (slot_base) {
+      k_slot_to_read<<<(nq + 256) / 256, 256, 0, x->stream>>>(slot_hits, slot_base, nq, x->hit_base.as<uint64_t>());
+      other++;
+    }
+    k_gather_hits<<<(unsigned)((n_slots + 255) / 256), 256, 0, x->stream>>>(
+        x->hitpool.as<uint4>(), x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), slot_hits, (uint32_t)n_slots,
+        x->hits.as<uint4>());
     other++;
     CK(cudaGetLastError());
   }
@@ -1041,6 +1051,7 @@ struct FixedChain {
   uint64_t upos_cap;           // distinct positions (rows walked once by the deduplicated resolve)
   GraphTotals* d_tot; GraphTotals* h_tot;     // device / pinned host
   uint64_t threads;            // resident threads of the persistent kernels
+  bool trie; uint32_t tblocks, tgroup;        // k_trie's plan
   uint32_t warp_cap = MEM_WARP_SET_CAP, warp_cands = 1024;   // warp tier: intervals per set, candidates
 };
 
@@ -1058,39 +1069,37 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
   };
   const uint64_t hcap = x->hit_cap, pcap = c.pos_cap, upcap = std::min(c.upos_cap, c.pos_cap);
   if (hcap >= 0xFFFFFFFFull) return set_error(HFM_E_ARG, "MemHit capacity above 2^32");
+  const bool seg = c.P.min_len > 0;
+  const uint64_t ucap = c.max_bases / x->seg_len + nq + 1;    // segments of the long reads
+  const uint64_t scap = seg ? nq + ucap : nq;                 // result slots
+  if (scap >= 0xFFFFFFFFull) return set_error(HFM_E_ARG, "read segment capacity above 2^32");
   // work buffers
-  RET(x->hit_start.ensure((size_t)nq * 8 + 8)); RET(x->hit_count.ensure((size_t)nq * 4 + 4));
+  RET(x->hit_start.ensure(scap * 8 + 8)); RET(x->hit_count.ensure(scap * 4 + 4));
   RET(x->status.ensure((size_t)nq * 4 + 4)); RET(x->ovf.ensure((size_t)nq * 4 + 4));
-  RET(x->ovf2.ensure((size_t)nq * 4 + 4)); RET(x->ovf3.ensure((size_t)nq * 4 + 4));
   RET(x->mivpool.ensure(x->miv_cap * 16)); RET(x->hitpool.ensure(hcap * 32));
   if (!launch) {                     // occupancy queried outside the capture
     int bpsm = 0;
-    WITH_FMT(fmt, { CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_mems<false, 32, 0, 8, FM>, 128, 0)); });
+    WITH_FMT(fmt, { CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_smem<false, 32, 0, 8, FM>, 128, 0)); });
     c.threads = (uint64_t)std::max(1, bpsm) * x->num_sms * 128;
+    c.trie = fmt == OCC_WIDE && x->mems_variant == 3 && x->threads_per_read == 1 && seg;
+    if (c.trie) RET(trie_plan(x, nq, c.tblocks, c.tgroup));
   }
   const uint64_t threads = c.threads;
-  RET(x->memwork.ensure(threads * 4 * MEM_SET_CAP * 16));
-  RET(x->cwork.ensure((size_t)threads * FAST_CAND_CAP * sizeof(Cand)));
-  const bool seg = c.P.mode == 0 && c.P.min_len > 0;
-  const uint64_t ucap = c.max_bases / x->seg_len + nq + 1;    // segments of the long reads
+  RET(x->memwork.ensure(threads * MEM_SET_BYTES));
   if (seg) {
     RET(x->lflag.ensure((size_t)nq * 4 + 4)); RET(x->lpos.ensure(((size_t)nq + 1) * 8));
     RET(x->sids.ensure((size_t)nq * 4 + 4)); RET(x->lids.ensure((size_t)nq * 4 + 4));
     RET(x->ucount.ensure((size_t)nq * 4 + 4)); RET(x->ubase.ensure(((size_t)nq + 1) * 8));
     RET(x->uread.ensure(ucap * 4)); RET(x->uk.ensure(ucap * 4));
-    RET(x->ubits.ensure(ucap * (x->seg_len / 32) * 4)); RET(x->uexit.ensure(ucap * 4));
-    RET(x->ust.ensure(ucap * 4)); RET(x->ucoff.ensure(ucap * 8)); RET(x->ucnt.ensure(ucap * 4));
-    RET(x->fxe.ensure(ucap * 4)); RET(x->fxc.ensure(ucap * 4)); RET(x->fxx.ensure(ucap * 4));
-    RET(x->fxo.ensure(ucap * 8)); RET(x->fxn.ensure(ucap * 4));
-    x->seg_cap = std::max<uint64_t>(x->seg_cap, ucap * 24 + 65536);
-    RET(x->segpool.ensure(x->seg_cap * sizeof(Cand)));
+    RET(x->nslot.ensure((size_t)nq * 4 + 4)); RET(x->slot_base.ensure(((size_t)nq + 1) * 8));
+    RET(x->slot_hits.ensure((scap + 1) * 8));
   }
   // warp tier: up to 16 warps per SM, at most 2 GB of sets
-  const uint64_t per_warp = (uint64_t)c.warp_cap * 4 * 16;
+  const uint64_t per_warp = (uint64_t)c.warp_cap * 2 * 16;
   const uint64_t wwarps = std::max<uint64_t>(4, std::min<uint64_t>((uint64_t)x->num_sms * 8, (2ull << 30) / per_warp));
   const uint32_t wgrid = (uint32_t)((wwarps + 3) / 4);
   RET(x->work.ensure((size_t)wgrid * 4 * per_warp));
-  RET(x->cwork.ensure(std::max<size_t>((size_t)threads * FAST_CAND_CAP, (size_t)wgrid * 4 * c.warp_cands) * sizeof(Cand)));
+  RET(x->cwork.ensure(std::max<size_t>((size_t)threads * FAST_HIT_CAP * 32, (size_t)wgrid * 4 * c.warp_cands * sizeof(Cand))));
   RET(x->hit_base.ensure(((size_t)nq + 1) * 8));
   RET(x->hits.ensure((hcap + 1) * 32));
   RET(x->npos_scan.ensure((hcap + 1) * 8));
@@ -1116,14 +1125,20 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
   if (launch) CK(cudaMemsetAsync(x->ctr.p, 0, sizeof(Counters), x->stream));
   // the prefix queue order (read_order 1), inside the captured work like the rest
   const uint32_t* ord = nullptr;
-  if (x->read_order == 1 && x->threads_per_read == 1 && nq > 1) RET(prefix_order(x, c.d_q, c.d_qoff, nq, ord, dummy, launch));
-  // search: long reads cut into segments, every read through the segment queue
+  if (x->threads_per_read == 1 && nq > 1 && (x->read_order == 1 || (c.trie && c.tgroup >= TRIE_SORT_GROUP)))
+    RET(prefix_order(x, c.d_q, c.d_qoff, nq, ord, dummy, launch));
+  // search: long reads cut into segments, the others whole, in one launch
+  const uint64_t* slot_base = seg ? x->slot_base.as<uint64_t>() : nullptr;
+  SmemJobs J{};
+  J.ids = ord; J.n_ids = nq; J.slot_base = slot_base;
   if (seg) {
     if (launch) {
-      k_long_flags<<<(nq + 255) / 256, 256, 0, x->stream>>>(ord, nq, c.d_qoff, 2 * x->seg_len, x->lflag.as<uint32_t>());
+      k_long_reads<<<(nq + 255) / 256, 256, 0, x->stream>>>(ord, nq, c.d_qoff, x->seg_len, x->lflag.as<uint32_t>(),
+                                                            x->nslot.as<uint32_t>(), &dc->n_long, &dc->n_units);
       CK(cudaGetLastError());
     }
     RET(SCAN(x->lflag.as<uint32_t>(), 1, nq, x->lpos.as<uint64_t>()));
+    RET(SCAN(x->nslot.as<uint32_t>(), 1, nq, x->slot_base.as<uint64_t>()));
     if (launch) {
       CK(cudaMemsetAsync(x->ucount.p, 0, (size_t)nq * 4, x->stream));
       k_split_ids<<<(nq + 255) / 256, 256, 0, x->stream>>>(ord, nq, x->lflag.as<uint32_t>(), x->lpos.as<uint64_t>(),
@@ -1133,70 +1148,49 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
     }
     RET(SCAN(x->ucount.as<uint32_t>(), 1, nq, x->ubase.as<uint64_t>()));   // ubase[nq] = segments
     const uint64_t* n_long_dev = x->lpos.as<uint64_t>() + nq;
-    const uint64_t* n_units_dev = x->ubase.as<uint64_t>() + nq;
     if (launch) {
       k_unit_fill<<<(nq + 255) / 256, 256, 0, x->stream>>>(x->lids.as<uint32_t>(), nq, x->ubase.as<uint64_t>(),
                                                            x->uread.as<uint32_t>(), x->uk.as<uint32_t>(), n_long_dev);
       CK(cudaGetLastError());
-      SegWork G{x->seg_len, x->seg_len / 32, x->uread.as<uint32_t>(), x->uk.as<uint32_t>(), 0u, x->ubits.as<uint32_t>(),
-                x->uexit.as<uint32_t>(), x->ust.as<uint32_t>(), x->ucoff.as<uint64_t>(), x->ucnt.as<uint32_t>(),
-                x->segpool.as<Cand>(), &dc->seg_used, x->seg_cap, x->sids.as<uint32_t>(), 0u, x->lids.as<uint32_t>(),
-                x->ubase.as<uint64_t>(), 0u, &dc->merge_queue, &dc->touches, x->fxe.as<uint32_t>(),
-                x->fxc.as<uint32_t>(), x->fxx.as<uint32_t>(), x->fxo.as<uint64_t>(), x->fxn.as<uint32_t>(),
-                n_units_dev, n_long_dev, nq};
-      MemsWork W{x->memwork.as<BIv>(), MEM_SET_CAP, x->cwork.as<Cand>(), FAST_CAND_CAP, &dc->seg_queue, nullptr,
-                 0u, &dc->still_ovf, 0u, nullptr, nullptr};
-      W.chunk = x->queue_chunk;
-      MemsWork Wf = W;
-      Wf.queue = &dc->fix_queue;
-      const unsigned g = (unsigned)(threads / 128);
-      WITH_FMT(fmt, {
-        k_mems_seg<false, 32, 8, FM><<<g, 128, 0, x->stream>>>(Fw.d, Rv.d, cfw, crv, c.d_q, c.d_qoff, P, ivp, hp, o, W, G);
-        k_mems_fix<false, 32, 8, FM><<<g, 128, 0, x->stream>>>(Fw.d, Rv.d, cfw, crv, c.d_q, c.d_qoff, P, ivp, Wf, G);
-        k_mems_merge<false, 32, 8, FM><<<g, 128, 0, x->stream>>>(Fw.d, Rv.d, cfw, crv, c.d_q, c.d_qoff, P, ivp, hp, o, W,
-                                                                 G);
-      });
-      CK(cudaGetLastError());
     }
-  } else if (launch) {
-    MemsWork W{x->memwork.as<BIv>(), MEM_SET_CAP, x->cwork.as<Cand>(), FAST_CAND_CAP, &dc->queue, ord, nq,
-               &dc->still_ovf, 0u, nullptr, nullptr};
-    W.chunk = x->queue_chunk;
-    WITH_FMT(fmt, {
-      k_mems<false, 32, 0, 8, FM><<<(unsigned)(threads / 128), 128, 0, x->stream>>>(Fw.d, Rv.d, cfw, crv, c.d_q,
-                                                                                    c.d_qoff, P, ivp, hp, o, W);
-    });
-    CK(cudaGetLastError());
+    J.unit_read = x->uread.as<uint32_t>(); J.unit_k = x->uk.as<uint32_t>(); J.seg_len = x->seg_len;
+    J.n_units_dev = x->ubase.as<uint64_t>() + nq; J.n_long_dev = n_long_dev;
+    J.ids = x->sids.as<uint32_t>();
   }
-  // overflow tiers, over the device lists: a per-thread rerun with a 1024-entry candidate
-  // list, then one warp per read with sets of MEM_WARP_SET_CAP intervals
   if (launch) {
-    k_split_ovf<<<(nq + 255) / 256, 256, 0, x->stream>>>(x->ovf.as<uint32_t>(), nq, 0u, x->status.as<uint32_t>(),
-                                                         x->ovf3.as<uint32_t>(), &dc->n_mid, x->ovf2.as<uint32_t>(),
-                                                         &dc->n_wrp, &dc->n_ovf);
-    CK(cudaGetLastError());
-    const uint64_t tm = std::max<uint64_t>(128, std::min<uint64_t>((uint64_t)x->num_sms * MID_THREADS_PER_SM, threads));
-    MemsWork Wm{x->memwork.as<BIv>(), MEM_SET_CAP, x->cwork.as<Cand>(), MID_CAND_CAP, &dc->queue3, x->ovf3.as<uint32_t>(),
-                0u, &dc->still_ovf, 0u, nullptr, &dc->n_mid};
-    MemsOut o2 = o;
-    o2.ovf_list = x->ovf2.as<uint32_t>();
-    o2.n_ovf = &dc->n_wrp;
+    CK(cudaMemsetAsync(x->status.p, 0, (size_t)nq * 4, x->stream));
+    CK(cudaMemsetAsync(x->hit_count.p, 0, scap * 4, x->stream));        // slots past the count stay empty
+    MemsWork W{};
+    W.sets = x->memwork.as<BIv>(); W.set_cap = MEM_SET_CAP; W.hits = x->cwork.as<uint4>(); W.hit_cap = FAST_HIT_CAP;
+    W.queue = &dc->queue; W.still_ovf = &dc->still_ovf; W.chunk = x->queue_chunk;
+    if (c.trie) {
+      TrieWork T{x->trie_nodes.as<uint4>(), &dc->trie_queue, c.tgroup, x->trie_left.as<uint32_t>(), &dc->n_left,
+                 x->trie_resume.as<uint32_t>()};
+      k_trie<false><<<c.tblocks, TRIE_WARPS * 32, TRIE_SMEM, x->stream>>>(Fw.d, Rv.d, crv, c.d_q, c.d_qoff, P, hp, o, T, J);
+      CK(cudaGetLastError());
+      J.ids = T.left; J.n_ids_dev = T.n_left; J.resume = T.resume;
+    }
     WITH_FMT(fmt, {
-      k_mems<false, 32, 0, 8, FM><<<(unsigned)(tm / 128), 128, 0, x->stream>>>(Fw.d, Rv.d, cfw, crv, c.d_q, c.d_qoff, P,
-                                                                                ivp, hp, o2, Wm);
+      k_smem<false, 32, 0, 8, FM><<<(unsigned)(threads / 128), 128, 0, x->stream>>>(Fw.d, Rv.d, cfw, crv, c.d_q, c.d_qoff,
+                                                                                    P, hp, o, W, J);
     });
-    MemsWork Ww{x->work.as<BIv>(), c.warp_cap, x->cwork.as<Cand>(), c.warp_cands, &dc->queue2, x->ovf2.as<uint32_t>(), 0u,
-                &dc->still_ovf, 1u, nullptr, &dc->n_wrp};
+    // reads that outgrew their sets or hit list: one warp per read, over the device list
+    MemsWork Ww{};
+    Ww.sets = x->work.as<BIv>(); Ww.set_cap = c.warp_cap; Ww.cands = x->cwork.as<Cand>(); Ww.cand_cap = c.warp_cands;
+    Ww.queue = &dc->queue2; Ww.ids = x->ovf.as<uint32_t>(); Ww.still_ovf = &dc->still_ovf; Ww.rerun = 1u;
+    Ww.n_dev = &dc->n_ovf; Ww.slot_base = slot_base;
     k_mems_warp<false><<<wgrid, 128, 0, x->stream>>>(Fw.d, Rv.d, cfw, crv, c.d_q, c.d_qoff, P, ivp, hp, o, Ww);
     CK(cudaGetLastError());
   }
   // CSR of MemHits (hits past the count stay zero, so their position counts add nothing)
-  RET(SCAN(x->hit_count.as<uint32_t>(), 1, nq, x->hit_base.as<uint64_t>()));
+  uint64_t* slot_hits = seg ? x->slot_hits.as<uint64_t>() : x->hit_base.as<uint64_t>();
+  RET(SCAN(x->hit_count.as<uint32_t>(), 1, scap, slot_hits));
   if (launch) {
+    if (seg) k_slot_to_read<<<(nq + 256) / 256, 256, 0, x->stream>>>(slot_hits, slot_base, nq, x->hit_base.as<uint64_t>());
     CK(cudaMemsetAsync(x->hits.p, 0, (hcap + 1) * 32, x->stream));
-    k_gather_hits<<<(nq + 255) / 256, 256, 0, x->stream>>>(x->hitpool.as<uint4>(), x->hit_start.as<uint64_t>(),
-                                                          x->hit_count.as<uint32_t>(), x->hit_base.as<uint64_t>(), nq,
-                                                          x->hits.as<uint4>());
+    k_gather_hits<<<(unsigned)((scap + 255) / 256), 256, 0, x->stream>>>(
+        x->hitpool.as<uint4>(), x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), slot_hits, (uint32_t)scap,
+        x->hits.as<uint4>());
     CK(cudaGetLastError());
   }
   RET(SCAN(x->hits.as<uint32_t>() + 5, 8, hcap, x->npos_scan.as<uint64_t>()));
@@ -1557,6 +1551,29 @@ int hfm_index_load(const uint8_t* bytes, size_t len, int kind, const hfm_opts* o
 // ---------------------------------------------------------------------------
 static constexpr uint32_t LAYOUT_VERSION = 1;
 
+// Wide records as the blob holds them: counts before row 0 of the record and whole planes
+// (k_wide_records is the way back).
+static void blob_wide_records(uint8_t* rec, uint64_t n) {
+  auto work = [rec](uint64_t b0, uint64_t b1) {
+    for (uint64_t b = b0; b < b1; b++) {
+      uint32_t r[24], o[24];
+      std::memcpy(r, rec + b * 96, 96);
+      for (int c = 0; c < 16; c++) {
+        uint32_t m = ~0u;
+        for (int p = 0; p < 4; p++) m &= ((c >> p) & 1) ? r[16 + p] : ~r[16 + p];
+        o[c] = r[c] - (uint32_t)__builtin_popcount(m);
+      }
+      for (int p = 0; p < 4; p++) { o[16 + 2 * p] = r[16 + p]; o[17 + 2 * p] = r[20 + p]; }
+      std::memcpy(rec + b * 96, o, 96);
+    }
+  };
+  const unsigned nt = n < (1u << 16) ? 1 : std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
+  std::vector<std::thread> th;
+  const uint64_t per = (n + nt - 1) / nt;
+  for (unsigned t = 0; t < nt; t++) if (t * per < n) th.emplace_back(work, t * per, std::min<uint64_t>(n, (t + 1) * per));
+  for (auto& x : th) x.join();
+}
+
 int hfm_index_export_layout(hfm_index* x, uint8_t** bytes_out, uint64_t* len_out) {
   if (!x || !bytes_out || !len_out) return set_error(HFM_E_ARG, "NULL argument");
   *bytes_out = nullptr; *len_out = 0;
@@ -1590,6 +1607,7 @@ int hfm_index_export_layout(hfm_index* x, uint8_t** bytes_out, uint64_t* len_out
       if (f.nbytes[b]) {
         cudaError_t e = cudaMemcpy(w, bufs[b]->p, f.nbytes[b], cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) { std::free(out); cudaGetLastError(); return set_error(HFM_E_CUDA, "layout copy failed"); }
+        if (b == 0 && f.fmt == OCC_WIDE) blob_wide_records(w, f.nbytes[b] / (OCC_WIDE_U4 * 16));
       }
       w += f.nbytes[b];
     }
@@ -1663,6 +1681,10 @@ int hfm_index_load_layout(const uint8_t* bytes, uint64_t len, const hfm_opts* op
       RET(upload(*bufs[b], bytes + D.at[b], D.nb[b], x->stream));
       f.nbytes[b] = D.nb[b];
     }
+    if (D.d.fmt == OCC_WIDE && D.d.num_blocks) {
+      k_wide_records<<<(D.d.num_blocks + 255) / 256, 256, 0, x->stream>>>(f.occ.as<uint4>(), D.d.num_blocks);
+      CK(cudaGetLastError());
+    }
     f.d = D.d;
     f.d.occ = f.occ.as<uint4>(); f.d.sb = f.sb.as<uint32_t>(); f.d.ssa = f.ssa.as<uint4>();
     f.d.sa_vals = f.sa_vals.as<uint32_t>(); f.d.seq_bounds = f.bounds.as<uint32_t>();
@@ -1687,9 +1709,8 @@ int hfm_index_device_bytes(const hfm_index* x, uint64_t* index_bytes, uint64_t* 
       &x->hit_start, &x->hit_count, &x->hit_base, &x->hits, &x->npos_scan, &x->work, &x->cwork, &x->ctr,
       &x->mivpool, &x->bswork, &x->memwork, &x->hkeys, &x->hslot, &x->hflags, &x->huid, &x->urow, &x->ulen,
       &x->uoff, &x->uout, &x->blockmap, &x->blockmap2, &x->ovf2, &x->ovf3, &x->lflag, &x->lpos, &x->sids,
-      &x->lids, &x->ucount, &x->ubase, &x->uread, &x->uk, &x->ubits, &x->uexit, &x->ust, &x->ucoff, &x->ucnt,
-      &x->segpool, &x->fxe, &x->fxc, &x->fxx, &x->fxo, &x->fxn, &x->npos, &x->iota, &x->loc_pairs,
-      &x->okeys, &x->oids, &x->otemp};
+      &x->lids, &x->ucount, &x->ubase, &x->uread, &x->uk, &x->nslot, &x->slot_base, &x->slot_hits, &x->npos,
+      &x->iota, &x->loc_pairs, &x->okeys, &x->oids, &x->otemp, &x->trie_nodes, &x->trie_left, &x->trie_resume};
   uint64_t a = 0, b = 0;
   if (!x->shared_index) for (const DevBuf* d : idx_bufs) a += d->cap;
   for (const DevBuf* d : work_bufs) b += d->cap;
@@ -1714,9 +1735,9 @@ void hfm_index_free(hfm_index* x) {
                     &x->hit_base, &x->hits, &x->npos_scan, &x->work, &x->cwork, &x->ctr, &x->mivpool, &x->bswork, &x->memwork,
                     &x->hkeys, &x->hslot, &x->hflags, &x->huid, &x->urow, &x->ulen, &x->uoff, &x->uout,
                     &x->blockmap, &x->blockmap2, &x->ovf2, &x->ovf3, &x->lflag, &x->lpos, &x->sids, &x->lids,
-                    &x->ucount, &x->ubase, &x->uread, &x->uk, &x->ubits, &x->uexit, &x->ust, &x->ucoff, &x->ucnt,
-                    &x->segpool, &x->fxe, &x->fxc, &x->fxx, &x->fxo, &x->fxn, &x->npos, &x->iota, &x->loc_pairs,
-                    &x->okeys, &x->oids, &x->otemp})
+                    &x->ucount, &x->ubase, &x->uread, &x->uk, &x->nslot, &x->slot_base, &x->slot_hits, &x->npos,
+                    &x->iota, &x->loc_pairs, &x->okeys, &x->oids, &x->otemp, &x->trie_nodes, &x->trie_left,
+                    &x->trie_resume})
     b->release();
   for (auto& e : x->ev) if (e) cudaEventDestroy(e);
   for (auto& e : x->evk) if (e) cudaEventDestroy(e);
@@ -2004,7 +2025,6 @@ extern "C" int hfm_mems_graph_create(hfm_index* x, const uint8_t* d_q, const uin
   if (sh->mems_variant == MEMS_PLAIN) sh->mems_variant = 3;
   sh->miv_cap = std::max<uint64_t>(x->miv_cap, (uint64_t)nq * 24 + 4096);
   sh->hit_cap = std::max<uint64_t>(x->hit_cap, (uint64_t)nq * 24 + 4096);
-  sh->seg_cap = x->seg_cap;
   CK(cudaMallocHost((void**)&g->h_bases, 512));
   RET(g->tot.ensure(2 * sizeof(GraphTotals)));
   RET(sh->ref_bounds.ensure((size_t)nb * 4 + 4));
@@ -2046,7 +2066,7 @@ extern "C" int hfm_mems_graph_launch(hfm_graph* g, hfm_dev_mems* out, uint32_t* 
     const GraphTotals& t = *c.h_tot;
     if (k.walk_err) return set_error(HFM_E_WALK, "LF walk exceeded sample_rate steps: index inconsistent");
     reason = (k.iv_used > x->miv_cap ? HFM_GRAPH_INTERVALS : 0u) | (k.hit_used > x->hit_cap ? HFM_GRAPH_HITS : 0u) |
-             (k.seg_used > x->seg_cap ? HFM_GRAPH_SEGMENTS : 0u) | (k.still_ovf ? HFM_GRAPH_WARP_SETS : 0u) |
+             (k.still_ovf ? HFM_GRAPH_WARP_SETS : 0u) |
              (t.ovf ? HFM_GRAPH_POSITIONS : 0u);
     if (reason & HFM_GRAPH_WARP_SETS) {       // the next capture gets larger warp-tier sets
       c.warp_cap = std::min<uint32_t>(c.warp_cap * 4, 1u << 22);

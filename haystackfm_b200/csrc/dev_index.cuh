@@ -3,8 +3,13 @@
 //
 // Device layout (built once by hfm_index_load from the reference's bincode records):
 //   occ   : one record per 64 BWT rows, two formats:
-//             wide   (96 B, any text): 16 x u32 counts of every code before the record, then
-//                    4 x u64 planes of the rows' 4-bit codes (three 32-byte sectors);
+//             wide   (96 B, any text): 16 x u32 counts of every code before the record's row
+//                    32, then the four planes of its rows' 4-bit codes, u32 each, of rows
+//                    0..31 and of rows 32..63 (three 32-byte sectors).  A count at any row
+//                    is the one at row 32 plus the rows between (or minus them, for rows
+//                    0..31), so half the planes are loaded, masked and counted: the 16 counts
+//                    of a border are 16 popcounts of 32 bits instead of 32 of them, and
+//                    popcounts (16 lanes a cycle) bound the search on IUPAC texts;
 //             narrow (32 B, texts of codes 0..4 only — ExactDna and ACGT-only IUPAC texts):
 //                    4 x u16 counts of codes 1..4 from the start of the record's superblock
 //                    (1,024 records = 65,536 rows) to the record, then 3 x u64 planes (one
@@ -15,8 +20,8 @@
 //   ssa   : one 16-byte record per 64 rows: u64 "row is sampled" bits + u32 count of
 //           sampled rows before the word (SampledSuffixArray, src/suffix_array/mod.rs:54-63).
 //   sa_vals, seq_boundaries, lookup intervals: as in the reference.
-// rank(c, i) = count[(i-1)/64][c] (+ sb[(i-1)/65536][c], narrow) + popc(rows of code c <=
-// (i-1)%64), identical to OccTable::rank (src/occ/mod.rs:330-363), whose records instead
+// Narrow: rank(c, i) = count[(i-1)/64][c] + sb[(i-1)/65536][c] + popc(rows of code c <=
+// (i-1)%64); both are identical to OccTable::rank (src/occ/mod.rs:330-363), whose records instead
 // hold compacted lanes with a u32 superblock count and a u16 delta per lane
 // (src/occ/mod.rs:144).  Wide records keep whole counts: on IUPAC texts an extension emits
 // many intervals, and each would otherwise need one more dependent load for its superblock
@@ -73,76 +78,105 @@ __device__ __forceinline__ uint32_t sel4(uint4 x, uint32_t i) {
 // One record with the rows of a border selected.  A border i (0 <= i <= text_len) is the
 // position between BWT rows i-1 and i: the record of row i-1, rows 0..(i-1)%64 selected
 // (border 0: record 0 with no row selected; its counts and superblock entry are 0).
-template <uint32_t FMT>
-struct Border {
-  uint4 a, b, c, d, e, f;  // wide: a..d = counts, e, f = planes; narrow: a = counts + p0, b = p1, p2
-  uint64_t low;            // selected rows
-  uint32_t sbi, i;         // superblock (narrow), the border itself
+template <uint32_t FMT> struct Border;
 
-  __device__ __forceinline__ uint64_t plane(int k) const {
-    if (FMT == OCC_WIDE) return k == 0 ? u2to64(e.x, e.y) : k == 1 ? u2to64(e.z, e.w) : k == 2 ? u2to64(f.x, f.y)
-                                                                                                  : u2to64(f.z, f.w);
-    return k == 0 ? u2to64(a.z, a.w) : k == 1 ? u2to64(b.x, b.y) : k == 2 ? u2to64(b.z, b.w) : 0ull;
+template <>
+struct Border<OCC_WIDE> {
+  uint4 a, b, c, d;        // counts before row 32
+  uint4 w;                 // the four planes of the half that holds the border
+  uint32_t m, sg;          // rows between row 32 and the border; 1 after row 32, ~0 before it
+
+  // the rows of `w` counted for a border x rows (0..64) into the record
+  __device__ __forceinline__ void select(uint32_t x) {
+    const uint32_t k = x & 31;
+    m = x >= 64 ? ~0u : x >= 32 ? (1u << k) - 1u : ~0u << k;
+    sg = x >= 32 ? 1u : ~0u;
   }
   // rows of code s among the selected ones (s a compile-time constant after unrolling)
-  __device__ __forceinline__ uint64_t eq(int s) const {
-    uint64_t m = low & ((s & 1) ? plane(0) : ~plane(0)) & ((s & 2) ? plane(1) : ~plane(1)) &
-                 ((s & 4) ? plane(2) : ~plane(2));
-    if (FMT == OCC_WIDE) m &= (s & 8) ? plane(3) : ~plane(3);
-    return m;
+  __device__ __forceinline__ uint32_t eq(int s) const {
+    return m & ((s & 1) ? w.x : ~w.x) & ((s & 2) ? w.y : ~w.y) & ((s & 4) ? w.z : ~w.z) & ((s & 8) ? w.w : ~w.w);
   }
-  // wide: count of code s before the record; narrow (s in 1..4): from the superblock start
   __device__ __forceinline__ uint32_t delta(int s) const {
-    if (FMT == OCC_WIDE) {
-      const uint4 w = s < 4 ? a : s < 8 ? b : s < 12 ? c : d;
-      return sel4(w, (uint32_t)s & 3);
-    }
+    const uint4 v = s < 4 ? a : s < 8 ? b : s < 12 ? c : d;
+    return sel4(v, (uint32_t)s & 3);
+  }
+  // rank of code s at the border
+  __device__ __forceinline__ uint32_t local(int s) const { return delta(s) + (uint32_t)__popc(eq(s)) * sg; }
+};
+
+template <>
+struct Border<OCC_NARROW> {
+  uint4 a, b;              // a = deltas + plane 0, b = planes 1, 2
+  uint64_t low;            // selected rows
+  uint32_t sbi, i;         // superblock, the border itself
+
+  __device__ __forceinline__ uint64_t plane(int k) const {
+    return k == 0 ? u2to64(a.z, a.w) : k == 1 ? u2to64(b.x, b.y) : u2to64(b.z, b.w);
+  }
+  __device__ __forceinline__ uint64_t eq(int s) const {
+    return low & ((s & 1) ? plane(0) : ~plane(0)) & ((s & 2) ? plane(1) : ~plane(1)) & ((s & 4) ? plane(2) : ~plane(2));
+  }
+  // count of code s (1..4) from the superblock start to the record
+  __device__ __forceinline__ uint32_t delta(int s) const {
     const uint32_t w = s <= 2 ? a.x : a.y;
     return ((s - 1) & 1) ? (w >> 16) : (w & 0xFFFFu);
   }
-  // wide: rank of code s at the border; narrow: rank within the superblock
+  // rank of code s within the superblock
   __device__ __forceinline__ uint32_t local(int s) const { return delta(s) + (uint32_t)__popcll(eq(s)); }
 };
 
-template <uint32_t FMT>
-__device__ __forceinline__ Border<FMT> load_border(const DevFm& F, uint32_t i) {
+template <uint32_t FMT, class FM>
+__device__ __forceinline__ Border<FMT> load_border(const FM& F, uint32_t i) {
   Border<FMT> r;
-  uint32_t pos = i ? i - 1 : 0u, blk = pos >> 6;
-  r.low = i ? (2ull << (pos & 63)) - 1ull : 0ull;        // rows 0..pos%64 (pos%64 = 63: all)
-  r.sbi = blk >> SB_BLOCK_SHIFT;
-  r.i = i;
-  if (FMT == OCC_WIDE) {
+  const uint32_t pos = i ? i - 1 : 0u, blk = pos >> 6;
+  if constexpr (FMT == OCC_WIDE) {
     const uint4* p = F.occ + (size_t)blk * OCC_WIDE_U4;
-    r.a = __ldg(p); r.b = __ldg(p + 1); r.c = __ldg(p + 2); r.d = __ldg(p + 3); r.e = __ldg(p + 4); r.f = __ldg(p + 5);
+    const uint32_t x = i ? (pos & 63) + 1u : 0u;
+    r.a = __ldg(p); r.b = __ldg(p + 1); r.c = __ldg(p + 2); r.d = __ldg(p + 3);
+    r.w = __ldg(p + (x >= 32 ? 5 : 4));
+    r.select(x);
   } else {
+    r.low = i ? (2ull << (pos & 63)) - 1ull : 0ull;        // rows 0..pos%64 (pos%64 = 63: all)
+    r.sbi = blk >> SB_BLOCK_SHIFT;
+    r.i = i;
     const uint4* p = F.occ + (size_t)blk * OCC_NARROW_U4;
-    r.a = __ldg(p); r.b = __ldg(p + 1); r.c = make_uint4(0, 0, 0, 0); r.d = r.c; r.e = r.c; r.f = r.c;
+    r.a = __ldg(p); r.b = __ldg(p + 1);
   }
   return r;
 }
 
-__device__ __forceinline__ uint32_t sb_count(const DevFm& F, uint32_t sbi, uint32_t s) {
+// The selected rows of a wide border split by code: m[s] for s = 0..15.
+__device__ __forceinline__ void wide_masks(const uint4& w, uint32_t sel, uint32_t m[16]) {
+  uint32_t q[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) q[k] = sel & ((k & 1) ? w.x : ~w.x) & ((k & 2) ? w.y : ~w.y);
+#pragma unroll
+  for (int s = 0; s < 16; s++) m[s] = q[s & 3] & ((s & 4) ? w.z : ~w.z) & ((s & 8) ? w.w : ~w.w);
+}
+
+// Ranks of all 16 codes at a wide border.
+__device__ __forceinline__ void wide_ranks(const Border<OCC_WIDE>& B, uint32_t r[16]) {
+  uint32_t m[16];
+  wide_masks(B.w, B.m, m);
+#pragma unroll
+  for (int s = 0; s < 16; s++) r[s] = B.delta(s) + (uint32_t)__popc(m[s]) * B.sg;
+}
+
+template <class FM>
+__device__ __forceinline__ uint32_t sb_count(const FM& F, uint32_t sbi, uint32_t s) {
   return __ldg(F.sb + (size_t)sbi * 16 + s);
 }
 
-// Absolute rank of code s at a border (occ(s, i)).
-template <uint32_t FMT>
-__device__ __forceinline__ uint32_t border_rank(const DevFm& F, const Border<FMT>& B, int s) {
-  if constexpr (FMT == OCC_NARROW) {
-    if (s == 0) {
-      uint32_t t = 0;
+// Absolute rank of code s at a border of an ACGT text (occ(s, i)).
+template <class FM>
+__device__ __forceinline__ uint32_t border_rank(const FM& F, const Border<OCC_NARROW>& B, int s) {
+  if (s == 0) {
+    uint32_t t = 0;
 #pragma unroll
-      for (int c = 1; c <= 4; c++) t += sb_count(F, B.sbi, c) + B.local(c);
-      return B.i - t;
-    }
-    return sb_count(F, B.sbi, s) + B.local(s);
-  } else {
-    const uint64_t sel0 = (s & 1) ? 0ull : ~0ull, sel1 = (s & 2) ? 0ull : ~0ull;
-    const uint64_t sel2 = (s & 4) ? 0ull : ~0ull, sel3 = (s & 8) ? 0ull : ~0ull;
-    const uint64_t m = B.low & (B.plane(0) ^ sel0) & (B.plane(1) ^ sel1) & (B.plane(2) ^ sel2) & (B.plane(3) ^ sel3);
-    const uint4 w = s < 4 ? B.a : s < 8 ? B.b : s < 12 ? B.c : B.d;
-    return sel4(w, (uint32_t)s & 3) + (uint32_t)__popcll(m);
+    for (int c = 1; c <= 4; c++) t += sb_count(F, B.sbi, c) + B.local(c);
+    return B.i - t;
   }
+  return sb_count(F, B.sbi, s) + B.local(s);
 }
 
 // The interval [lo, hi) of the BWT split by symbol: calls f(s, d, r, sbi) for every code s
@@ -150,8 +184,8 @@ __device__ __forceinline__ uint32_t border_rank(const DevFm& F, const Border<FMT
 // border's count r: occ(s, lo) = r (wide) or sb_count(F, sbi, s) + r (narrow; one
 // L2-resident load, made only for the codes the caller keeps).  `last` = the highest code
 // the caller needs.
-template <uint32_t FMT, class Fn>
-__device__ __forceinline__ void split_by_symbol(const DevFm& F, uint32_t lo, uint32_t hi, uint32_t last, Fn&& f) {
+template <uint32_t FMT, class FM, class Fn>
+__device__ __forceinline__ void split_by_symbol(const FM& F, uint32_t lo, uint32_t hi, uint32_t last, Fn&& f) {
   if constexpr (FMT == OCC_NARROW) {
     const Border<FMT> L = load_border<FMT>(F, lo), H = load_border<FMT>(F, hi);
     const bool same_sb = L.sbi == H.sbi;
@@ -169,33 +203,10 @@ __device__ __forceinline__ void split_by_symbol(const DevFm& F, uint32_t lo, uin
 #pragma unroll
     for (int s = 0; s <= 4; s++) f(s, d[s], r[s], L.sbi);
   } else {
-    // Wide records: the 16 masks of each border by a split tree over its planes, then the
-    // counts; groups of codes past `last` are not formed.
     const Border<FMT> L = load_border<FMT>(F, lo), H = load_border<FMT>(F, hi);
     uint32_t rl[16], rh[16];
-    {
-      uint64_t m[16];
-      m[0] = L.low;
-#pragma unroll
-      for (int p = 3; p >= 0; --p) {
-        const int cnt = 1 << (3 - p);
-        const uint64_t pv = L.plane(p);
-#pragma unroll
-        for (int k = cnt - 1; k >= 0; --k) { uint64_t v = m[k]; m[2 * k + 1] = v & pv; m[2 * k] = v & ~pv; }
-      }
-#pragma unroll
-      for (int t = 0; t < 16; t++) rl[t] = L.delta(t) + (uint32_t)__popcll(m[t]);
-      m[0] = H.low;
-#pragma unroll
-      for (int p = 3; p >= 0; --p) {
-        const int cnt = 1 << (3 - p);
-        const uint64_t pv = H.plane(p);
-#pragma unroll
-        for (int k = cnt - 1; k >= 0; --k) { uint64_t v = m[k]; m[2 * k + 1] = v & pv; m[2 * k] = v & ~pv; }
-      }
-#pragma unroll
-      for (int t = 0; t < 16; t++) rh[t] = H.delta(t) + (uint32_t)__popcll(m[t]);
-    }
+    wide_ranks(L, rl);
+    wide_ranks(H, rh);
 #pragma unroll
     for (int t = 0; t < 16; t++) {
       if ((uint32_t)t > last) break;
@@ -206,31 +217,37 @@ __device__ __forceinline__ void split_by_symbol(const DevFm& F, uint32_t lo, uin
 
 // The code of BWT row `row` and its rank at that row (LF step of a one-row interval,
 // lane_and_mask_bitplane + rank_at_lane, src/occ/mod.rs:434-480).
-template <uint32_t FMT>
-__device__ __forceinline__ void row_code_rank(const DevFm& F, uint32_t row, uint32_t& code, uint32_t& rank) {
-  Border<FMT> B = load_border<FMT>(F, row + 1);     // the record of `row`, rows 0..row%64
+template <uint32_t FMT, class FM>
+__device__ __forceinline__ void row_code_rank(const FM& F, uint32_t row, uint32_t& code, uint32_t& rank) {
   const uint32_t off = row & 63;
-  uint32_t c = (uint32_t)((B.plane(0) >> off) & 1) | ((uint32_t)((B.plane(1) >> off) & 1) << 1) |
-               ((uint32_t)((B.plane(2) >> off) & 1) << 2);
-  if (FMT == OCC_WIDE) c |= (uint32_t)((B.plane(3) >> off) & 1) << 3;
-  B.low >>= 1;                                         // rows before `row` only
-  B.i = row;
-  code = c;
-  uint32_t r;
-  if (FMT == OCC_WIDE) {
-    uint64_t m = B.low & ((c & 1) ? B.plane(0) : ~B.plane(0)) & ((c & 2) ? B.plane(1) : ~B.plane(1)) &
-                 ((c & 4) ? B.plane(2) : ~B.plane(2)) & ((c & 8) ? B.plane(3) : ~B.plane(3));
-    const uint4 w = c < 4 ? B.a : c < 8 ? B.b : c < 12 ? B.c : B.d;
-    r = sel4(w, c & 3) + (uint32_t)__popcll(m);
-  } else if (c == 0) {
-    r = border_rank<FMT>(F, B, 0);
+  if constexpr (FMT == OCC_WIDE) {
+    // the half of `row` and its one count: 20 of the record's 96 bytes
+    const uint4* p = F.occ + (size_t)(row >> 6) * OCC_WIDE_U4;
+    Border<FMT> B;
+    B.w = __ldg(p + (off >= 32 ? 5 : 4));
+    B.select(off);
+    const uint32_t k = off & 31;
+    const uint32_t c = ((B.w.x >> k) & 1) | ((B.w.y >> k) & 1) << 1 | ((B.w.z >> k) & 1) << 2 | ((B.w.w >> k) & 1) << 3;
+    const uint32_t m = B.m & ((c & 1) ? B.w.x : ~B.w.x) & ((c & 2) ? B.w.y : ~B.w.y) & ((c & 4) ? B.w.z : ~B.w.z) &
+                       ((c & 8) ? B.w.w : ~B.w.w);
+    code = c;
+    rank = __ldg(reinterpret_cast<const uint32_t*>(p) + c) + (uint32_t)__popc(m) * B.sg;
   } else {
-    uint64_t m = B.low & ((c & 1) ? B.plane(0) : ~B.plane(0)) & ((c & 2) ? B.plane(1) : ~B.plane(1)) &
-                 ((c & 4) ? B.plane(2) : ~B.plane(2));
-    uint32_t w = c <= 2 ? B.a.x : B.a.y;
-    r = sb_count(F, B.sbi, c) + (((c - 1) & 1) ? (w >> 16) : (w & 0xFFFFu)) + (uint32_t)__popcll(m);
+    Border<FMT> B = load_border<FMT>(F, row + 1);     // the record of `row`, rows 0..row%64
+    const uint32_t c = (uint32_t)((B.plane(0) >> off) & 1) | ((uint32_t)((B.plane(1) >> off) & 1) << 1) |
+                       ((uint32_t)((B.plane(2) >> off) & 1) << 2);
+    B.low >>= 1;                                         // rows before `row` only
+    B.i = row;
+    code = c;
+    if (c == 0) {
+      rank = border_rank(F, B, 0);
+    } else {
+      const uint64_t m = B.low & ((c & 1) ? B.plane(0) : ~B.plane(0)) & ((c & 2) ? B.plane(1) : ~B.plane(1)) &
+                         ((c & 4) ? B.plane(2) : ~B.plane(2));
+      const uint32_t w = c <= 2 ? B.a.x : B.a.y;
+      rank = sb_count(F, B.sbi, c) + (((c - 1) & 1) ? (w >> 16) : (w & 0xFFFFu)) + (uint32_t)__popcll(m);
+    }
   }
-  rank = r;
 }
 
 // Rank of every symbol code at border i (counts of code s in bwt[0..i)), absent codes 0.
@@ -238,7 +255,7 @@ __device__ __forceinline__ void row_code_rank(const DevFm& F, uint32_t row, uint
 template <uint32_t FMT>
 __device__ __forceinline__ void sym_ranks_t(const DevFm& F, uint32_t i, uint32_t r[16]) {
   const Border<FMT> B = load_border<FMT>(F, i);
-  if (FMT == OCC_NARROW) {
+  if constexpr (FMT == OCC_NARROW) {
     uint32_t t = 0;
 #pragma unroll
     for (int s = 1; s <= 4; s++) { r[s] = sb_count(F, B.sbi, s) + B.local(s); t += r[s]; }
@@ -246,8 +263,7 @@ __device__ __forceinline__ void sym_ranks_t(const DevFm& F, uint32_t i, uint32_t
 #pragma unroll
     for (int s = 5; s < 16; s++) r[s] = 0;
   } else {
-#pragma unroll
-    for (int s = 0; s < 16; s++) r[s] = B.local(s);
+    wide_ranks(B, r);
   }
 }
 
@@ -285,6 +301,25 @@ __device__ __forceinline__ uint32_t upper_bound_u32(const uint32_t* b, uint32_t 
   uint32_t lo = 0, hi = n;
   while (lo < hi) { uint32_t mid = (lo + hi) >> 1; if (b[mid] <= p) lo = mid + 1; else hi = mid; }
   return lo;
+}
+
+// The wide record between its form in the device-layout blob (counts before row 0, planes
+// as u64) and its form on the device.
+__global__ void k_wide_records(uint4* __restrict__ occ, uint32_t nblk) {
+  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= nblk) return;
+  uint4* p = occ + (size_t)b * OCC_WIDE_U4;
+  Border<OCC_WIDE> B;
+  B.a = p[0]; B.b = p[1]; B.c = p[2]; B.d = p[3];
+  const uint4 e = p[4], f = p[5];
+  B.w = make_uint4(e.x, e.z, f.x, f.z);
+  B.m = ~0u; B.sg = 1u;
+  uint32_t r[16];
+  wide_ranks(B, r);
+#pragma unroll
+  for (int k = 0; k < 4; k++) p[k] = make_uint4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
+  p[4] = B.w;
+  p[5] = make_uint4(e.y, e.w, f.y, f.w);
 }
 
 }  // namespace hfm

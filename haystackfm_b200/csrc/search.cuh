@@ -7,12 +7,12 @@
 // not from spreading one read over a warp.  Interval sets live in per-thread slices of a
 // global work area, interleaved across the 32 lanes of a warp (element i of every lane is
 // one contiguous run: 128 B per u32 plane of the SMEM sets, 256 B per uint2 of the backward
-// search sets) with a fixed capacity; a read whose set, candidate list or output outgrows
-// it is queued for a fallback pass with much larger slices (a per-thread rerun for long
-// candidate lists, then one warp per read).  There is therefore no cap on interval-set
-// size, as in the reference CPU (src/fm_index/query.rs:248-274,
-// src/fm_index/smem.rs:332-357).  SMEM reads longer than 2 * seg_len are swept in
-// segments whose pivot chains are merged (below), so no single read is a long serial chain.
+// search sets) with a fixed capacity; a read whose set, hit list or output outgrows it is
+// queued for a fallback pass with much larger slices (a per-thread rerun for long hit
+// lists, then one warp per read).  There is therefore no cap on interval-set size, as in
+// the reference CPU (src/fm_index/query.rs:248-274, src/fm_index/smem.rs:332-357).  The
+// per-thread SMEM kernel is in smem.cuh; this file has the sets, the plain launch and the
+// lane-group kernels.
 #pragma once
 #include <type_traits>
 #include "dev_index.cuh"
@@ -536,41 +536,13 @@ __device__ uint32_t mems_sweep(const DevFm& Fw, const DevFm& Rv, const SmemFm& S
   return sink.nc;
 }
 
-template <bool COUNT_TOUCH, uint32_t FMT, class SR>
-__device__ uint32_t mems_one(const DevFm& Fw, const DevFm& Rv, const SmemFm& Sf, const SmemFm& Sr,
-                             const uint8_t* q, uint32_t n, const MemsParams& P, const SR& curr, const SR& nxt,
-                             const SR& wa, const SR& wb, uint32_t set_cap, Cand* cands, uint32_t cand_cap,
-                             Pool& ivpool, uint32_t& st, uint64_t& touches) {
-  CandSink<SR> sink{cands, 0, cand_cap, &ivpool, &st, set_cap};
-  return mems_sweep<COUNT_TOUCH, FMT>(Fw, Rv, Sf, Sr, q, n, P, curr, nxt, wa, wb, set_cap, sink, st, touches);
-}
-
 // Sort candidates by (qs, qe) (stable), drop duplicates, keep the containment-maximal ones
 // (find_smems, src/fm_index/smem.rs:84-103).  Returns the survivors compacted in place.
-template <bool LONG_LISTS = false>
 __device__ __forceinline__ uint32_t finalize_smems(Cand* c, uint32_t n) {
-  if (LONG_LISTS && n > 128) {
-    // Shell sort (Ciura's gaps) for the long lists of long reads.  Candidates with equal
-    // (qs, qe) name the same pattern, so the same count and interval set: which of them
-    // the dedup below keeps does not matter, and the sort need not be stable.
-    const uint32_t gaps[8] = {701, 301, 132, 57, 23, 10, 4, 1};
-    for (int gi = 0; gi < 8; gi++) {
-      uint32_t g = gaps[gi];
-      if (g >= n) continue;
-      for (uint32_t i = g; i < n; i++) {
-        Cand t = c[i];
-        uint64_t k = ((uint64_t)t.qs << 32) | t.qe;
-        uint32_t j = i;
-        while (j >= g && ((((uint64_t)c[j - g].qs) << 32) | c[j - g].qe) > k) { c[j] = c[j - g]; j -= g; }
-        c[j] = t;
-      }
-    }
-  } else {
-    for (uint32_t i = 1; i < n; i++) {         // insertion sort
-      Cand t = c[i]; uint32_t j = i;
-      while (j > 0 && (c[j - 1].qs > t.qs || (c[j - 1].qs == t.qs && c[j - 1].qe > t.qe))) { c[j] = c[j - 1]; j--; }
-      c[j] = t;
-    }
+  for (uint32_t i = 1; i < n; i++) {           // insertion sort
+    Cand t = c[i]; uint32_t j = i;
+    while (j > 0 && (c[j - 1].qs > t.qs || (c[j - 1].qs == t.qs && c[j - 1].qe > t.qe))) { c[j] = c[j - 1]; j--; }
+    c[j] = t;
   }
   uint32_t w = 0;
   for (uint32_t i = 0; i < n; i++)
@@ -619,16 +591,18 @@ __device__ __forceinline__ bool write_hits(Cand* c, uint32_t n, const MemsParams
 }
 
 struct MemsWork {
-  BIv* sets; uint32_t set_cap;        // 4 sets per thread
-  Cand* cands; uint32_t cand_cap;     // contiguous per thread (fallback pass); nullptr: local
+  BIv* sets; uint32_t set_cap;        // two sets per thread (per lane group)
+  Cand* cands; uint32_t cand_cap;     // lane-group kernels: candidate list per group
+  uint4* hits; uint32_t hit_cap;      // per-thread kernel: hit list per thread (two uint4 a hit)
   unsigned int* queue;
-  const uint32_t* ids; uint32_t n;    // reads to process, in queue order (ids == nullptr: 0..n-1)
+  const uint32_t* ids; uint32_t n;    // lane-group kernels: reads to process, in queue order
   uint32_t* still_ovf;
   uint32_t rerun;                     // 1: a rerun of overflowed reads (counted in still_ovf)
   uint32_t* work_log;                 // COUNT_TOUCH only: 4 u32 per read, [0] += Occ touches, [3] |= 1 on overflow
-                                      // (the warp-per-read kernel also sets bit 1)
+                                      // (the lane-group kernels also set bit 1)
   const uint32_t* n_dev;              // when set, the number of reads is read here (graph-captured chains)
   uint32_t chunk;                     // queue entries taken per atomic (0 or 1: one)
+  const uint64_t* slot_base;          // first result slot of each read (nullptr: slot = read)
   __device__ __forceinline__ uint32_t count() const { return n_dev ? *n_dev : n; }
   __device__ __forceinline__ uint32_t step() const { return chunk > 1 ? chunk : 1u; }
 };
@@ -646,58 +620,6 @@ __global__ void k_split_ovf(const uint32_t* __restrict__ list, uint32_t n, uint3
   if (k < first_warp || (status[i] & ST_SET_OVF)) wrp[atomicAdd(n_wrp, 1u)] = i;
   else mid[atomicAdd(n_mid, 1u)] = i;
 }
-
-template <bool COUNT_TOUCH, int STRIDE, int KC, int MINB, uint32_t FMT>
-__global__ void __launch_bounds__(128, MINB) k_mems(DevFm Fw, DevFm Rv, const uint16_t* __restrict__ compat_fw,
-                                             const uint16_t* __restrict__ compat_rv, const uint8_t* __restrict__ q,
-                                             const uint64_t* __restrict__ qoff, MemsParams P, Pool ivpool,
-                                             Pool hitpool, MemsOut out, MemsWork W) {
-  __shared__ SmemFm Sf, Sr;
-  smem_fm_init(Sf, Fw, compat_fw);
-  smem_fm_init(Sr, Rv, compat_rv);
-  __syncthreads();
-  const uint32_t SCAP = STRIDE == 32 ? FAST_SET_CAP : W.set_cap;
-  using SR = SetRef<BIv, STRIDE>;
-  SR s0 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 0), s1 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 1);
-  SR s2 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 2), s3 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 3);
-  Cand local_c[KC > 0 ? KC : 1];
-  Cand* cands = local_c;
-  uint32_t cand_cap = KC;
-  if (KC == 0) {
-    uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    cands = W.cands + tid * W.cand_cap;
-    cand_cap = W.cand_cap;
-  }
-  uint64_t touches = 0;
-  uint32_t i;
-  const uint32_t nreads = W.count(), chunk = W.step();
-  QueueCursor qc;
-  while (next_read_chunked(W.queue, nreads, W.ids, chunk, qc, i)) {
-    uint32_t st = ST_OK;
-    uint64_t o = qoff[i];
-    uint64_t t0 = touches;
-    uint32_t nc = mems_one<COUNT_TOUCH, FMT>(Fw, Rv, Sf, Sr, q + o, (uint32_t)(qoff[i + 1] - o), P, s0, s1, s2, s3,
-                                        SCAP, cands, cand_cap, ivpool, st, touches);
-    uint64_t hs = 0; uint32_t hc = 0;
-    if (nc != ~0u) {
-      if (P.mode == 0) nc = finalize_smems(cands, nc);
-      if (!write_hits(cands, nc, P, ivpool, hitpool, hs, hc)) st |= ST_POOL_OVF;
-    }
-    if (st) { hs = 0; hc = 0; }
-    out.hit_start[i] = hs; out.hit_count[i] = hc; out.status[i] = st;
-    bool ovf = st & (ST_SET_OVF | ST_CAND_OVF);
-    if (COUNT_TOUCH && W.work_log) {
-      W.work_log[4 * (size_t)i] += (uint32_t)(touches - t0);
-      if (ovf) W.work_log[4 * (size_t)i + 3] |= 1u;
-    }
-    if (ovf) {
-      if (W.rerun) atomicAdd(W.still_ovf, 1u);
-      else out.ovf_list[atomicAdd(out.n_ovf, 1u)] = i;
-    }
-  }
-  if (COUNT_TOUCH && touches) atomicAdd(out.touches, (unsigned long long)touches);
-}
-
 
 // =====================================================================================
 // The plain launch: one thread per read over a grid the size of the batch, interval sets
@@ -790,64 +712,38 @@ __global__ void __launch_bounds__(128) k_mems_plain(DevFm Fw, DevFm Rv, const ui
 }
 
 // =====================================================================================
-// Long reads: the SMEM sweep of a read cut into segments.
-//
-// The sweep visits a chain of pivots, next = max(reach(pivot), pivot + 1), and the next
-// pivot depends only on the read and the current pivot.  k_mems_seg gives one thread to
-// each seg_len-position segment of a long read and sweeps the chain as if a pivot started
-// at the segment's first position, recording the pivots it visits, the first pivot past
-// the segment, and its candidates tagged with their pivots.  k_mems_merge follows the
-// read's true chain across the segments: where it lands on a pivot the segment visited,
-// both chains agree from there to the segment's end, so the segment's candidates from that
-// pivot on are exactly the true chain's; elsewhere the merge sweeps the true chain itself
-// until it meets the segment's chain or leaves the segment.  The candidate set, and so
-// every result, is the one the unsegmented sweep produces; the critical path of a 10 kbp
-// read becomes one segment plus the merge instead of the whole read.
+// Long reads are cut into segments of seg_len positions (smem.cuh): the lists of their
+// segments and of the reads in one piece.
 // =====================================================================================
-constexpr uint32_t SEG_MAX = 4096;   // longest segment (pivot bitmap of SEG_MAX / 32 words)
+constexpr uint32_t SEG_MAX = 4096;   // longest segment
 
-struct SegWork {
-  uint32_t seg_len, seg_words;    // positions per segment (multiple of 32, <= SEG_MAX)
-  const uint32_t* unit_read;      // read of each unit (segment)
-  const uint32_t* unit_k;         // segment index within its read
-  uint32_t n_units;
-  uint32_t* bits;                 // seg_words per unit: pivots the segment's chain visited
-  uint32_t* exit_pivot;           // per unit: first pivot past the segment, ~0u on failure
-  uint32_t* unit_st;              // per unit: status bits of a failed sweep
-  uint64_t* cand_off;             // per unit: first candidate in the unit pool
-  uint32_t* cand_cnt;             // per unit
-  Cand* pool; unsigned long long* pool_used; uint64_t pool_cap;
-  const uint32_t* short_ids;      // k_mems_seg also runs these whole reads after the segments
-  uint32_t n_short;
-  const uint32_t* long_ids;       // merge: long reads, in queue order
-  const uint64_t* unit_base;      // merge: first unit of each long read (n_long + 1)
-  uint32_t n_long;
-  unsigned int* merge_queue;
-  unsigned long long* touches;
-  // fix-up pass: segment j swept again from the previous segment's exit pivot (the true
-  // chain's entry whenever the previous segment's chain met the true one)
-  uint32_t* fx_entry;             // entry pivot used, ~0u when not computed
-  uint32_t* fx_conv;              // pivot where it met the segment's chain, ~0u if it did not
-  uint32_t* fx_exit;              // first pivot past the segment when it did not meet it
-  uint64_t* fx_off;               // its own candidates (pivots before fx_conv) in the pool
-  uint32_t* fx_cnt;
-  // when set (graph-captured chains), the counts are read here: units = *n_units_dev,
-  // long reads = *n_long_dev, short reads = n_fast - *n_long_dev
-  const uint64_t* n_units_dev;
-  const uint64_t* n_long_dev;
-  uint32_t n_fast;
-  __device__ __forceinline__ uint32_t units() const { return n_units_dev ? (uint32_t)*n_units_dev : n_units; }
-  __device__ __forceinline__ uint32_t longs() const { return n_long_dev ? (uint32_t)*n_long_dev : n_long; }
-  __device__ __forceinline__ uint32_t shorts() const { return n_long_dev ? n_fast - (uint32_t)*n_long_dev : n_short; }
-};
-
-// flags[k] = 1 when read ids[k] (k itself without ids) is longer than min_len.
-__global__ void k_long_flags(const uint32_t* __restrict__ ids, uint32_t n, const uint64_t* __restrict__ qoff,
-                             uint32_t min_len, uint32_t* __restrict__ flags) {
+// Reads ids[k] (k itself without ids): flags[k] = 1 when the read is longer than
+// 2 * seg_len, nslot[read] = its segments (1 for a read in one piece), and the totals.
+__global__ void k_long_reads(const uint32_t* __restrict__ ids, uint32_t n, const uint64_t* __restrict__ qoff,
+                             uint32_t seg_len, uint32_t* __restrict__ flags, uint32_t* __restrict__ nslot,
+                             uint32_t* __restrict__ n_long, unsigned long long* __restrict__ n_units) {
   uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
-  uint32_t i = ids ? ids[k] : k;
-  flags[k] = (qoff[i + 1] - qoff[i]) > min_len ? 1u : 0u;
+  const uint32_t i = ids ? ids[k] : k;
+  const uint64_t len = qoff[i + 1] - qoff[i];
+  const bool is_long = len > 2 * (uint64_t)seg_len;
+  const uint32_t segs = is_long ? (uint32_t)((len + seg_len - 1) / seg_len) : 1u;
+  flags[k] = is_long ? 1u : 0u;
+  nslot[i] = segs;
+  if (is_long) { atomicAdd(n_long, 1u); atomicAdd(n_units, (unsigned long long)segs); }
+}
+
+// out[list[k]] = v.
+__global__ void k_fill_listed(const uint32_t* __restrict__ list, uint32_t n, uint32_t* __restrict__ out, uint32_t v) {
+  uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n) out[list[k]] = v;
+}
+
+// hit_base[i] = first hit of read i = first hit of its first slot (i <= n).
+__global__ void k_slot_to_read(const uint64_t* __restrict__ slot_hits, const uint64_t* __restrict__ slot_base, uint32_t n,
+                               uint64_t* __restrict__ hit_base) {
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i <= n) hit_base[i] = slot_hits[slot_base[i]];
 }
 
 // Stable split of ids by flag (lpos = exclusive scan of flags).
@@ -877,240 +773,6 @@ __global__ void k_unit_fill(const uint32_t* __restrict__ long_ids, uint32_t n_lo
   for (uint64_t u = b; u < e; u++) { unit_read[u] = long_ids[r]; unit_k[u] = (uint32_t)(u - b); }
 }
 
-// One persistent queue over the segments of the long reads followed by the whole short
-// reads of the batch (the longest jobs first; the short reads fill the tail).
-template <bool COUNT_TOUCH, int STRIDE, int MINB, uint32_t FMT>
-__global__ void __launch_bounds__(128, MINB) k_mems_seg(DevFm Fw, DevFm Rv, const uint16_t* __restrict__ compat_fw,
-                                                 const uint16_t* __restrict__ compat_rv, const uint8_t* __restrict__ q,
-                                                 const uint64_t* __restrict__ qoff, MemsParams P, Pool ivpool,
-                                                 Pool hitpool, MemsOut out, MemsWork W, SegWork G) {
-  __shared__ SmemFm Sf, Sr;
-  smem_fm_init(Sf, Fw, compat_fw);
-  smem_fm_init(Sr, Rv, compat_rv);
-  __syncthreads();
-  const uint32_t SCAP = STRIDE == 32 ? FAST_SET_CAP : W.set_cap;
-  using SR = SetRef<BIv, STRIDE>;
-  SR s0 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 0), s1 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 1);
-  SR s2 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 2), s3 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 3);
-  uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  Cand* cands = W.cands + tid * W.cand_cap;
-  uint64_t touches = 0;
-  const uint32_t n_units = G.units();
-  const uint32_t njobs = n_units + G.shorts();
-  uint32_t u;
-  const uint32_t chunk = W.step();
-  QueueCursor qc;
-  while (next_read_chunked(W.queue, njobs, nullptr, chunk, qc, u)) {
-    const bool unit = u < n_units;
-    uint32_t i, s, e;
-    uint32_t* bits = nullptr;
-    if (unit) i = G.unit_read[u];
-    else i = G.short_ids[u - n_units];
-    uint64_t o = qoff[i];
-    uint32_t n = (uint32_t)(qoff[i + 1] - o);
-    if (unit) {
-      s = G.unit_k[u] * G.seg_len;
-      e = min(n, s + G.seg_len);
-      bits = G.bits + (size_t)u * G.seg_words;
-      for (uint32_t w = 0; w < G.seg_words; w++) bits[w] = 0;
-    } else {
-      s = 0;
-      e = n;
-    }
-    uint32_t st = ST_OK;
-    uint64_t t0 = touches;
-    CandSink<SR> sink{cands, 0, W.cand_cap, &ivpool, &st, SCAP};
-    uint32_t p = s;
-    while (p < e) {
-      if (unit) { uint32_t d = p - s; bits[d >> 5] |= 1u << (d & 31); }
-      p = smem_pivot<COUNT_TOUCH, FMT>(Fw, Rv, Sf, Sr, q + o, n, p, P, s0, s1, s2, s3, SCAP, st, touches, sink);
-      if (p == ~0u) break;
-    }
-    uint32_t nc = sink.nc;
-    if (unit) {
-      if (p != ~0u && nc) {
-        unsigned long long off = atomicAdd(G.pool_used, (unsigned long long)nc);
-        if (off + nc > G.pool_cap) { st |= ST_POOL_OVF; p = ~0u; }
-        else {
-          for (uint32_t c = 0; c < nc; c++) G.pool[off + c] = cands[c];
-          G.cand_off[u] = off;
-        }
-      }
-      if (p == ~0u || nc == 0) G.cand_off[u] = 0;
-      G.cand_cnt[u] = p == ~0u ? 0u : nc;
-      G.exit_pivot[u] = p;
-      G.unit_st[u] = st;
-      if (COUNT_TOUCH && W.work_log) atomicAdd(W.work_log + 4 * (size_t)i, (uint32_t)(touches - t0));
-    } else {
-      // a whole short read: the same sweep as the fast pass, then its hits
-      uint64_t hs = 0; uint32_t hc = 0;
-      if (p != ~0u) {
-        nc = finalize_smems(cands, nc);
-        if (!write_hits(cands, nc, P, ivpool, hitpool, hs, hc)) st |= ST_POOL_OVF;
-      }
-      if (st) { hs = 0; hc = 0; }
-      out.hit_start[i] = hs; out.hit_count[i] = hc; out.status[i] = st;
-      bool ovf = st & (ST_SET_OVF | ST_CAND_OVF);
-      if (COUNT_TOUCH && W.work_log) {
-        W.work_log[4 * (size_t)i] += (uint32_t)(touches - t0);
-        if (ovf) W.work_log[4 * (size_t)i + 3] |= 1u;
-      }
-      if (ovf) out.ovf_list[atomicAdd(out.n_ovf, 1u)] = i;
-    }
-  }
-  if (COUNT_TOUCH && touches) atomicAdd(G.touches, (unsigned long long)touches);
-}
-
-// Fix-up pass, one thread per segment after the first: sweeps from the previous segment's
-// exit pivot until the chain meets this segment's chain (usually within a few pivots), so
-// the merge below only has to check that the entry it assumed is the true one.
-template <bool COUNT_TOUCH, int STRIDE, int MINB, uint32_t FMT>
-__global__ void __launch_bounds__(128, MINB) k_mems_fix(DevFm Fw, DevFm Rv, const uint16_t* __restrict__ compat_fw,
-                                                 const uint16_t* __restrict__ compat_rv, const uint8_t* __restrict__ q,
-                                                 const uint64_t* __restrict__ qoff, MemsParams P, Pool ivpool,
-                                                 MemsWork W, SegWork G) {
-  __shared__ SmemFm Sf, Sr;
-  smem_fm_init(Sf, Fw, compat_fw);
-  smem_fm_init(Sr, Rv, compat_rv);
-  __syncthreads();
-  const uint32_t SCAP = STRIDE == 32 ? FAST_SET_CAP : W.set_cap;
-  using SR = SetRef<BIv, STRIDE>;
-  SR s0 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 0), s1 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 1);
-  SR s2 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 2), s3 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 3);
-  uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  Cand* cands = W.cands + tid * W.cand_cap;
-  uint64_t touches = 0;
-  uint32_t u;
-  const uint32_t n_units = G.units();
-  while (next_read(W.queue, n_units, nullptr, u)) {
-    uint32_t i = G.unit_read[u], k = G.unit_k[u];
-    G.fx_entry[u] = ~0u; G.fx_conv[u] = ~0u; G.fx_exit[u] = ~0u; G.fx_off[u] = 0; G.fx_cnt[u] = 0;
-    if (k == 0 || G.exit_pivot[u - 1] == ~0u || G.exit_pivot[u] == ~0u) continue;
-    uint64_t o = qoff[i];
-    uint32_t n = (uint32_t)(qoff[i + 1] - o);
-    uint32_t s = k * G.seg_len, e = min(n, s + G.seg_len);
-    uint32_t entry = G.exit_pivot[u - 1];
-    if (entry >= e) { G.fx_entry[u] = entry; G.fx_exit[u] = entry; continue; }
-    const uint32_t* bits = G.bits + (size_t)u * G.seg_words;
-    uint32_t st = ST_OK;
-    uint64_t t0 = touches;
-    CandSink<SR> sink{cands, 0, W.cand_cap, &ivpool, &st, SCAP};
-    uint32_t p = entry;
-    while (p < e && !((bits[(p - s) >> 5] >> ((p - s) & 31)) & 1u)) {
-      p = smem_pivot<COUNT_TOUCH, FMT>(Fw, Rv, Sf, Sr, q + o, n, p, P, s0, s1, s2, s3, SCAP, st, touches, sink);
-      if (p == ~0u) break;
-    }
-    if (COUNT_TOUCH && W.work_log) atomicAdd(W.work_log + 4 * (size_t)i, (uint32_t)(touches - t0));
-    if (p == ~0u) continue;                       // the merge sweeps this segment itself
-    uint32_t nc = sink.nc;
-    if (nc) {
-      unsigned long long off = atomicAdd(G.pool_used, (unsigned long long)nc);
-      if (off + nc > G.pool_cap) continue;        // pool exhausted: counted, regrown by the host
-      for (uint32_t c = 0; c < nc; c++) G.pool[off + c] = cands[c];
-      G.fx_off[u] = off;
-      G.fx_cnt[u] = nc;
-    }
-    if (p < e) { G.fx_conv[u] = p; G.fx_exit[u] = G.exit_pivot[u]; }
-    else G.fx_exit[u] = p;
-    G.fx_entry[u] = entry;
-  }
-  if (COUNT_TOUCH && touches) atomicAdd(G.touches, (unsigned long long)touches);
-}
-
-template <bool COUNT_TOUCH, int STRIDE, int MINB, uint32_t FMT>
-__global__ void __launch_bounds__(128, MINB) k_mems_merge(DevFm Fw, DevFm Rv, const uint16_t* __restrict__ compat_fw,
-                                                   const uint16_t* __restrict__ compat_rv,
-                                                   const uint8_t* __restrict__ q, const uint64_t* __restrict__ qoff,
-                                                   MemsParams P, Pool ivpool, Pool hitpool, MemsOut out, MemsWork W,
-                                                   SegWork G) {
-  __shared__ SmemFm Sf, Sr;
-  smem_fm_init(Sf, Fw, compat_fw);
-  smem_fm_init(Sr, Rv, compat_rv);
-  __syncthreads();
-  const uint32_t SCAP = STRIDE == 32 ? FAST_SET_CAP : W.set_cap;
-  using SR = SetRef<BIv, STRIDE>;
-  SR s0 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 0), s1 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 1);
-  SR s2 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 2), s3 = thread_set<BIv, STRIDE>(W.sets, SCAP, 4, 3);
-  uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  Cand* cands = W.cands + tid * W.cand_cap;
-  uint64_t touches = 0;
-  uint32_t r;
-  const uint32_t n_long = G.longs();
-  while (next_read(G.merge_queue, n_long, nullptr, r)) {
-    uint32_t i = G.long_ids[r];
-    uint64_t o = qoff[i];
-    uint32_t n = (uint32_t)(qoff[i + 1] - o);
-    uint64_t u0 = G.unit_base[r], u1 = G.unit_base[r + 1];
-    uint32_t st = ST_OK;
-    uint64_t t0 = touches;
-    CandSink<SR> sink{cands, 0, W.cand_cap, &ivpool, &st, SCAP};
-    bool fail = false;
-    uint32_t t = 0;                                   // the true chain's next pivot
-    for (uint64_t u = u0; u < u1 && !fail; u++) {
-      uint32_t s = (uint32_t)(u - u0) * G.seg_len, e = min(n, s + G.seg_len);
-      if (t >= e) continue;                           // the chain jumps over this segment
-      if (G.exit_pivot[u] == ~0u) { st |= G.unit_st[u]; fail = true; break; }
-      if (u > u0 && G.fx_entry[u] == t) {             // the fix-up pass started where the chain enters
-        const Cand* fx = G.pool + G.fx_off[u];
-        uint32_t fcnt = G.fx_cnt[u];
-        for (uint32_t c = 0; c < fcnt && !fail; c++) {
-          if (sink.nc >= sink.cap) { st |= ST_CAND_OVF; fail = true; break; }
-          cands[sink.nc++] = fx[c];
-        }
-        if (fail) break;
-        uint32_t cv = G.fx_conv[u];
-        if (cv != ~0u) {
-          const Cand* src = G.pool + G.cand_off[u];
-          uint32_t cnt = G.cand_cnt[u];
-          for (uint32_t c = 0; c < cnt; c++) {
-            Cand cd = src[c];
-            if (cd.pivot < cv) continue;
-            if (sink.nc >= sink.cap) { st |= ST_CAND_OVF; fail = true; break; }
-            cands[sink.nc++] = cd;
-          }
-          t = G.exit_pivot[u];
-        } else {
-          t = G.fx_exit[u];
-        }
-        continue;
-      }
-      uint32_t p = t;
-      const uint32_t* bits = G.bits + u * G.seg_words;
-      while (p < e && !((bits[(p - s) >> 5] >> ((p - s) & 31)) & 1u)) {
-        p = smem_pivot<COUNT_TOUCH, FMT>(Fw, Rv, Sf, Sr, q + o, n, p, P, s0, s1, s2, s3, SCAP, st, touches, sink);
-        if (p == ~0u) { fail = true; break; }
-      }
-      if (fail) break;
-      if (p < e) {                                    // met the segment's chain at p
-        const Cand* src = G.pool + G.cand_off[u];
-        uint32_t cnt = G.cand_cnt[u];
-        for (uint32_t c = 0; c < cnt; c++) {
-          Cand cd = src[c];
-          if (cd.pivot < p) continue;
-          if (sink.nc >= sink.cap) { st |= ST_CAND_OVF; fail = true; break; }
-          cands[sink.nc++] = cd;
-        }
-        t = G.exit_pivot[u];
-      } else {
-        t = p;
-      }
-    }
-    uint64_t hs = 0; uint32_t hc = 0;
-    if (!fail) {
-      uint32_t nc = P.mode == 0 ? finalize_smems<true>(cands, sink.nc) : sink.nc;
-      if (!write_hits(cands, nc, P, ivpool, hitpool, hs, hc)) st |= ST_POOL_OVF;
-    }
-    if (st) { hs = 0; hc = 0; }
-    out.hit_start[i] = hs; out.hit_count[i] = hc; out.status[i] = st;
-    bool ovf = st & (ST_SET_OVF | ST_CAND_OVF);
-    if (COUNT_TOUCH && W.work_log) {
-      atomicAdd(W.work_log + 4 * (size_t)i, (uint32_t)(touches - t0));
-      if (ovf) atomicOr(W.work_log + 4 * (size_t)i + 3, 1u);
-    }
-    if (ovf) out.ovf_list[atomicAdd(out.n_ovf, 1u)] = i;
-  }
-  if (COUNT_TOUCH && touches) atomicAdd(out.touches, (unsigned long long)touches);
-}
 }  // namespace hfm
 
 // =====================================================================================
@@ -1338,124 +1000,72 @@ __device__ uint32_t warp_extend_set(const DevFm& X, const SmemFm& S, uint32_t ma
   return nout;
 }
 
-template <int DIR, bool COUNT_TOUCH, int G = 32>
-__device__ bool warp_any_extend(const DevFm& X, const SmemFm& S, uint32_t mask, const BIv* in, uint32_t nin,
-                                uint64_t& touches) {
-  const int lane = threadIdx.x & (G - 1);
-  bool any = false;
-  for (uint32_t b = 0; b < nin && !any; b += G) {
-    uint32_t i = b + lane;
-    BIv iv = i < nin ? in[i] : BIv{0, 0, 0, 0};
-    uint32_t a = DIR == 0 ? iv.rlo : iv.flo, e = DIR == 0 ? iv.rhi : iv.fhi;
-    uint32_t rl[16], rh[16];
-    sym_ranks(X, S, a, rl);
-    sym_ranks(X, S, e, rh);
-    if (COUNT_TOUCH && i < nin) touches += (a != 0) + (e != 0);
-    bool mine = false;
-#pragma unroll
-    for (int s = 0; s < 16; s++) mine |= i < nin && ((mask >> s) & 1) && rh[s] != rl[s];
-    any = __any_sync(grp_mask<G>(), mine);
-  }
-  return any;
-}
-
-// Candidate search of one read by a group of G lanes; control flow is group-uniform.
+// The search of one read (window, forward, next: smem.cuh) by a group of G lanes; control
+// flow is group-uniform.
 template <bool COUNT_TOUCH, int G = 32>
 __device__ uint32_t warp_mems_one(const DevFm& Fw, const DevFm& Rv, const SmemFm& Sf, const SmemFm& Sr,
-                                  const uint8_t* q, uint32_t n, const MemsParams& P, BIv* curr, BIv* nxt, BIv* wa,
-                                  BIv* wb, uint32_t set_cap, Cand* cands, uint32_t cand_cap, Pool& ivpool,
+                                  const uint8_t* q, uint32_t n, const MemsParams& P, BIv* cur, BIv* alt,
+                                  uint32_t set_cap, Cand* cands, uint32_t cand_cap, Pool& ivpool,
                                   uint32_t& st, uint64_t& touches) {
   const int lane = threadIdx.x & (G - 1);
   const uint32_t gm = grp_mask<G>();
   uint32_t nc = 0;
   if (n == 0 || P.min_len == 0) return 0;
-  const BIv full = {0, Fw.text_len, 0, Fw.text_len};
+  uint32_t ncur = 0, cov;
   bool ovf = false;
-  auto qmask = [&](const SmemFm& S, uint8_t c) -> uint32_t { return c < 16 ? S.compat_mask[c] : 0u; };
-  auto emit = [&](uint32_t qs, uint32_t qe, uint32_t count, const BIv* ivs, uint32_t niv) -> bool {
-    if (nc >= cand_cap) { st |= ST_CAND_OVF; return false; }
-    uint64_t off = 0;
-    if (lane == 0) off = thread_reserve(ivpool, niv);
-    off = __shfl_sync(gm, off, 0, G);
-    if (off == ~0ull) { st |= ST_POOL_OVF; return false; }
-    BIv* dst = (BIv*)ivpool.base + off;
-    for (uint32_t k = lane; k < niv; k += G) dst[k] = ivs[k];
-    if (lane == 0) cands[nc] = Cand{qs, qe, count, niv, off};
-    nc++;
+  auto reset = [&]() {
     __syncwarp(gm);
+    if (lane == 0) cur[0] = BIv{0, Fw.text_len, 0, Fw.text_len};
+    __syncwarp(gm);
+    ncur = 1;
+  };
+  // one step; false, with the set as it was, when nothing extends (or the set outgrew its area)
+  auto left = [&](uint32_t pos) -> bool {
+    uint32_t m = warp_extend_set<1, COUNT_TOUCH, G>(Fw, Sf, qmask(Sf, q[pos]), cur, ncur, alt, set_cap, cov, ovf, touches);
+    if (ovf || m == 0) return false;
+    BIv* t = cur; cur = alt; alt = t; ncur = m;
     return true;
   };
-  if (P.mode == 1) {
-    for (uint32_t i = 0; i < n; i++) {
-      BIv* c = curr; BIv* x = nxt;
-      if (lane == 0) c[0] = full;
-      __syncwarp(gm);
-      uint32_t ncur = 1, cov = 0, j = i;
-      bool matched = false;
-      while (j < n) {
-        uint32_t ncov;
-        uint32_t nn = warp_extend_set<0, COUNT_TOUCH, G>(Rv, Sr, qmask(Sr, q[j]), c, ncur, x, set_cap, ncov, ovf, touches);
-        if (ovf) { st |= ST_SET_OVF; return ~0u; }
-        if (nn == 0) break;
-        BIv* t = c; c = x; x = t; ncur = nn; cov = ncov; j++; matched = true;
-      }
-      if (!matched || j - i < P.min_len) continue;
-      bool lmax = i == 0 || !warp_any_extend<1, COUNT_TOUCH, G>(Fw, Sf, qmask(Sf, q[i - 1]), c, ncur, touches);
-      if (!lmax) continue;
-      if (!emit(i, j, cov, c, ncur)) return ~0u;
-    }
-    return nc;
-  }
-  uint32_t pivot = 0;
-  while (pivot < n) {
-    BIv* c = curr; BIv* x = nxt;
-    if (lane == 0) x[0] = full;
-    __syncwarp(gm);
-    uint32_t cov;
-    uint32_t ncur = warp_extend_set<0, COUNT_TOUCH, G>(Rv, Sr, qmask(Sr, q[pivot]), x, 1, c, set_cap, cov, ovf, touches);
+  auto right = [&](uint32_t pos) -> bool {
+    uint32_t m = warp_extend_set<0, COUNT_TOUCH, G>(Rv, Sr, qmask(Sr, q[pos]), cur, ncur, alt, set_cap, cov, ovf, touches);
+    if (ovf || m == 0) return false;
+    BIv* t = cur; cur = alt; alt = t; ncur = m;
+    return true;
+  };
+  uint32_t i = 0;
+  while (n - i >= P.min_len) {
+    reset();
+    uint32_t k = i + P.min_len;
+    while (k > i && left(k - 1)) k--;
     if (ovf) { st |= ST_SET_OVF; return ~0u; }
-    if (ncur == 0) { pivot++; continue; }
-    uint32_t j = pivot + 1, reach = pivot + 1;
-    for (;;) {
-      uint32_t end, nn = 0, ncov = 0;
-      bool next_empty, record;
-      if (j == n) { end = n; next_empty = true; record = true; }
-      else {
-        nn = warp_extend_set<0, COUNT_TOUCH, G>(Rv, Sr, qmask(Sr, q[j]), c, ncur, x, set_cap, ncov, ovf, touches);
-        if (ovf) { st |= ST_SET_OVF; return ~0u; }
-        end = j; next_empty = nn == 0; record = ncov != cov;
-      }
-      if (record) {
-        reach = end;
-        const BIv* b = c;
-        uint32_t nb = ncur, start = pivot, bcov = cov;
-        BIv* bufs[2] = {wa, wb};
-        int t = 0;
-        while (start > 0) {
-          uint32_t lcov;
-          uint32_t nl = warp_extend_set<1, COUNT_TOUCH, G>(Fw, Sf, qmask(Sf, q[start - 1]), b, nb, bufs[t], set_cap, lcov, ovf, touches);
-          if (ovf) { st |= ST_SET_OVF; return ~0u; }
-          if (nl == 0) break;
-          b = bufs[t]; nb = nl; bcov = lcov; t ^= 1; start--;
-        }
-        if (end - start >= P.min_len) {
-          bool rmax = end == n ||
-                      (start == pivot ? next_empty : !warp_any_extend<0, COUNT_TOUCH, G>(Rv, Sr, qmask(Sr, q[end]), b, nb, touches));
-          if (rmax && !emit(start, end, bcov, b, nb)) return ~0u;
-        }
-      }
-      if (j == n || nn == 0) break;
-      BIv* tt = c; c = x; x = tt; ncur = nn; cov = ncov; j++;
-    }
-    pivot = max(reach, pivot + 1);
+    if (k > i) { i = k; continue; }
+    uint32_t e = i + P.min_len;
+    while (e < n && right(e)) e++;
+    if (ovf) { st |= ST_SET_OVF; return ~0u; }
+    if (nc >= cand_cap) { st |= ST_CAND_OVF; return ~0u; }
+    uint64_t off = 0;
+    if (lane == 0) off = thread_reserve(ivpool, ncur);
+    off = __shfl_sync(gm, off, 0, G);
+    if (off == ~0ull) { st |= ST_POOL_OVF; return ~0u; }
+    BIv* dst = (BIv*)ivpool.base + off;
+    for (uint32_t c = lane; c < ncur; c += G) dst[c] = cur[c];
+    if (lane == 0) cands[nc] = Cand{i, e, 0u, ncur, off, i, 0u};
+    nc++;
+    if (e == n) break;
+    reset();
+    k = e + 1;
+    while (k > i + 1 && left(k - 1)) k--;
+    if (ovf) { st |= ST_SET_OVF; return ~0u; }
+    i = k;
   }
+  __syncwarp(gm);
   return nc;
 }
 
 // Persistent SMEM / MEM search with one read per group of G lanes (G = 32: the warp tier
 // of reads whose sets outgrew the per-thread kernels; G = 4, 8, 16: the sub-warp
-// candidates of the autotuner).  Group g of the grid owns sets and a candidate list at
-// g * 4 * set_cap / g * cand_cap.
+// candidates of the autotuner).  Group g of the grid owns two sets and a candidate list at
+// g * 2 * set_cap / g * cand_cap.
 template <bool COUNT_TOUCH, int G = 32>
 __global__ void __launch_bounds__(128) k_mems_warp(DevFm Fw, DevFm Rv, const uint16_t* __restrict__ compat_fw,
                                                   const uint16_t* __restrict__ compat_rv, const uint8_t* __restrict__ q,
@@ -1468,7 +1078,7 @@ __global__ void __launch_bounds__(128) k_mems_warp(DevFm Fw, DevFm Rv, const uin
   const int lane = threadIdx.x & (G - 1);
   const uint32_t gm = grp_mask<G>();
   uint64_t grp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
-  BIv* base = W.sets + grp * 4 * W.set_cap;
+  BIv* base = W.sets + grp * 2 * W.set_cap;
   Cand* cands = W.cands + grp * W.cand_cap;
   uint64_t touches = 0;
   for (;;) {
@@ -1481,8 +1091,7 @@ __global__ void __launch_bounds__(128) k_mems_warp(DevFm Fw, DevFm Rv, const uin
     uint64_t o = qoff[i];
     uint64_t t0 = touches;
     uint32_t nc = warp_mems_one<COUNT_TOUCH, G>(Fw, Rv, Sf, Sr, q + o, (uint32_t)(qoff[i + 1] - o), P, base,
-                                                base + W.set_cap, base + 2 * W.set_cap, base + 3 * W.set_cap,
-                                                W.set_cap, cands, W.cand_cap, ivpool, st, touches);
+                                                base + W.set_cap, W.set_cap, cands, W.cand_cap, ivpool, st, touches);
     __syncwarp(gm);
     if (COUNT_TOUCH && W.work_log) {
       uint32_t d = grp_sum<G>((uint32_t)(touches - t0));
@@ -1491,11 +1100,13 @@ __global__ void __launch_bounds__(128) k_mems_warp(DevFm Fw, DevFm Rv, const uin
     if (lane == 0) {
       uint64_t hs = 0; uint32_t hc = 0;
       if (nc != ~0u) {
-        if (P.mode == 0) nc = finalize_smems<true>(cands, nc);
         if (!write_hits(cands, nc, P, ivpool, hitpool, hs, hc)) st |= ST_POOL_OVF;
       }
       if (st) { hs = 0; hc = 0; }
-      out.hit_start[i] = hs; out.hit_count[i] = hc; out.status[i] = st;
+      const uint64_t slot = W.slot_base ? W.slot_base[i] : (uint64_t)i;
+      out.hit_start[slot] = hs; out.hit_count[slot] = hc; out.status[i] = st;
+      if (W.slot_base)
+        for (uint64_t x = slot + 1; x < W.slot_base[i + 1]; x++) out.hit_count[x] = 0;
       if (st & (ST_SET_OVF | ST_CAND_OVF)) {
         if (W.rerun) atomicAdd(W.still_ovf, 1u);
         else out.ovf_list[atomicAdd(out.n_ovf, 1u)] = i;      // on to the warp tier

@@ -1,0 +1,360 @@
+// smem.cuh — SMEM / MEM search, one thread per read or read segment.
+//
+// What is searched for.  "q[s, e) occurs in the text" (each query code matching its
+// compatible text codes) holds for every part of a string that it holds for.  Let LM(e) be
+// the smallest s with q[s, e) occurring.  The candidates that find_smems keeps
+// (src/fm_index/smem.rs:71-222: right-maximal prefixes of every pivot's sweep, extended
+// left maximally, those not contained in another) are exactly the pairs (LM(e), e) with
+// e = n or LM(e + 1) > LM(e): an occurrence of such a pair that is not followed by q[e]
+// makes the coverage drop at e in the sweep of every pivot inside it, so the sweep records
+// it.  find_mems (smem.rs:113-124,250-295: the longest match from every start, kept when it
+// does not extend left) gives the same pairs.  The interval set of a pair is the set of SA
+// intervals of the text strings that match it, whatever the order it was extended in.  So
+// both modes are served by one search that visits only matches of at least min_len:
+//
+//   window  extend left from i + min_len down to i; where the set empties at position t, no
+//           match of min_len starts at or before t: go on with i = t + 1
+//   forward extend right from the window while the set is not empty: q[i, e) is a result
+//   next    extend left from e + 1; the set empties at t: the next result that reaches past
+//           e starts at t + 1 or later
+//
+// A read costs about 2 min_len + its match lengths in steps; the sweep it replaces extended
+// every prefix of every pivot at which the coverage drops (some 15 per pivot) left again.
+// Measured on a B200, 256 Mbp ACGT repeat genome, kernel times of the sweep and of this
+// search: 1M reads of 150 bp 58.4 -> 11.6 ms; 60,000 mixed reads up to 10 kbp 71.2 -> 7.7 ms;
+// 250 of them 37.2 -> 5.2 ms; find_mems of 20,000 ragged reads 25.9 -> 1.9 ms.  Bound by the
+// latency of one dependent record load per step.
+//
+// Segments.  A result belongs to the segment of a long read in which it starts.  A segment's
+// search begins at its first position a: if the window there does not match, everything
+// after it is left-maximal by construction; if it does, its match is a result only when it
+// does not extend left by q[a - 1].  Segments need nothing from one another, so a long read
+// is as many independent jobs.
+//
+// Execution.  All lanes of a warp run the same loop, one extension step per turn, whatever
+// phase their read is in: the step takes its direction, interval and code at run time, so a
+// lane that looks backwards and one that goes forward load and count together.
+#pragma once
+#include "search.cuh"
+
+namespace hfm {
+
+// The jobs of one launch: segments of long reads, then whole reads.  Counts that a
+// graph-captured chain does not know on the host are read on the device.
+struct SmemJobs {
+  const uint32_t* unit_read;      // read of each segment
+  const uint32_t* unit_k;         // its index within the read
+  uint32_t seg_len;
+  uint32_t n_units;
+  const uint64_t* n_units_dev;
+  const uint32_t* ids;            // whole reads (nullptr: 0..n_ids-1)
+  uint32_t n_ids;
+  const uint64_t* n_long_dev;     // when set, n_ids counts the long reads too
+  const uint32_t* n_ids_dev;      // when set, the number of whole reads
+  const uint32_t* resume;         // per whole read: position after a result [0, e) that is already in its slot
+                                  // (k_trie), or RESUME_START; nullptr: every read from its start
+  // Results are written per slot: a read's segments in order (one slot for a read in one
+  // piece).  slot_base[i] = first slot of read i; nullptr: slot i.
+  const uint64_t* slot_base;
+  __device__ __forceinline__ uint32_t units() const { return n_units_dev ? (uint32_t)*n_units_dev : n_units; }
+  __device__ __forceinline__ uint32_t whole() const {
+    return n_ids_dev ? *n_ids_dev : n_long_dev ? n_ids - (uint32_t)*n_long_dev : n_ids;
+  }
+};
+
+constexpr uint32_t RESUME_START = 0xFFFFFFFFu;
+
+// One direction of the index as the step needs it.
+struct FmView { const uint4* occ; const uint32_t* sb; };
+
+// Rows of code s, and of codes s..4, among 64 rows of an ACGT record (codes 0..4; plane 2
+// is set for code 4 alone).
+__device__ __forceinline__ uint64_t acgt_eq(uint32_t s, uint64_t p0, uint64_t p1, uint64_t p2) {
+  const uint64_t x = s == 1 ? p0 & ~p1 : s == 2 ? p1 & ~p0 : p0 & p1;
+  return s == 4 ? p2 : x;
+}
+__device__ __forceinline__ uint64_t acgt_ge(uint32_t s, uint64_t p0, uint64_t p1, uint64_t p2) {
+  const uint64_t x = s == 1 ? p0 | p1 : s == 2 ? p1 : p0 & p1;
+  return s == 4 ? p2 : x | p2;
+}
+__device__ __forceinline__ uint32_t acgt_delta(const uint4& a, uint32_t s) {
+  const uint32_t w = s <= 2 ? a.x : a.y;
+  return (s & 1) ? (w & 0xFFFFu) : (w >> 16);
+}
+// Counts of codes s..4 in the record's deltas.
+__device__ __forceinline__ uint32_t acgt_delta_ge(uint32_t x, uint32_t y, uint32_t s) {
+  uint32_t t = y >> 16;
+  if (s <= 3) t += y & 0xFFFFu;
+  if (s <= 2) t += x >> 16;
+  if (s <= 1) t += x & 0xFFFFu;
+  return t;
+}
+
+// Extends one interval of an ACGT text by one code s (1..4): rows [lo, lo + n) of the
+// extended side become [lo', lo' + n'), `base` (the other side's start) moves past the rows
+// of smaller codes.  The border records are those of the first and the last row, so an
+// interval within 64 rows (every one-row interval) reads one sector.  Returns false, and
+// changes nothing, when no row has the code.
+template <bool COUNT_TOUCH>
+__device__ __forceinline__ bool acgt_step(const FmView& X, const uint32_t* C, uint32_t s, uint32_t& lo, uint32_t& base,
+                                          uint32_t& n, uint64_t& touches) {
+  const uint32_t last = lo + n - 1, bl = lo >> 6, bh = last >> 6;
+  const uint4* pl = X.occ + (size_t)bl * OCC_NARROW_U4;
+  const uint4 a = __ldg(pl), b = __ldg(pl + 1);
+  const uint32_t sbl = __ldg(X.sb + (size_t)(bl >> SB_BLOCK_SHIFT) * 16 + s);
+  uint4 a2 = a, b2 = b;
+  if (bh != bl) {
+    const uint4* ph = X.occ + (size_t)bh * OCC_NARROW_U4;
+    a2 = __ldg(ph); b2 = __ldg(ph + 1);
+  }
+  if (COUNT_TOUCH) touches += bh != bl ? 2 : 1;
+  const uint64_t ml = (1ull << (lo & 63)) - 1ull, mh = (2ull << (last & 63)) - 1ull;
+  const uint64_t p0 = u2to64(a.z, a.w), p1 = u2to64(b.x, b.y), p2 = u2to64(b.z, b.w);
+  const uint64_t h0 = u2to64(a2.z, a2.w), h1 = u2to64(b2.x, b2.y), h2 = u2to64(b2.z, b2.w);
+  const uint32_t rl = acgt_delta(a, s) + (uint32_t)__popcll(acgt_eq(s, p0, p1, p2) & ml);
+  uint32_t d = acgt_delta(a2, s) + (uint32_t)__popcll(acgt_eq(s, h0, h1, h2) & mh) - rl;
+  uint32_t g = acgt_delta_ge(a2.x, a2.y, s) - acgt_delta_ge(a.x, a.y, s) +
+               (uint32_t)__popcll(acgt_ge(s, h0, h1, h2) & mh) - (uint32_t)__popcll(acgt_ge(s, p0, p1, p2) & ml);
+  if ((bh >> SB_BLOCK_SHIFT) != (bl >> SB_BLOCK_SHIFT)) {
+    const uint32_t* q = X.sb + (size_t)(bl >> SB_BLOCK_SHIFT) * 16;
+    const uint32_t* r = X.sb + (size_t)(bh >> SB_BLOCK_SHIFT) * 16;
+    d += __ldg(r + s) - sbl;
+    for (uint32_t t = s; t <= 4; t++) g += __ldg(r + t) - __ldg(q + t);
+  }
+  if (!d) return false;
+  base += n - g;
+  lo = C[s] + sbl + rl;
+  n = d;
+  return true;
+}
+
+// A lane's interval set: one interval in registers, or cnt > 1 of them in `cur` (in any
+// order), with `alt` as the buffer that the next step writes.
+template <class SR>
+struct LaneSet {
+  uint32_t flo, rlo, sz, cnt;
+  SR cur, alt;
+};
+
+// One extension of the whole set by the codes of `mask`, to the left or to the right
+// (extend_multi_right / extend_multi_left, src/fm_index/smem.rs:332-357).  Returns false,
+// and leaves the set as it was, when nothing extends (or, with ovf set, when the set
+// outgrows `cap`).
+template <bool COUNT_TOUCH, uint32_t FMT, class SR>
+__device__ __forceinline__ bool lane_step(const FmView& X, const uint32_t* C, bool left, uint32_t mask,
+                                          LaneSet<SR>& L, uint32_t cap, bool& ovf, uint64_t& touches) {
+  if (FMT == OCC_NARROW && L.cnt == 1 && (mask & (mask - 1)) == 0) {
+    if (!mask) return false;
+    uint32_t lo = left ? L.flo : L.rlo, base = left ? L.rlo : L.flo, n = L.sz;
+    if (!acgt_step<COUNT_TOUCH>(X, C, 31u - (uint32_t)__clz(mask), lo, base, n, touches)) return false;
+    L.flo = left ? lo : base; L.rlo = left ? base : lo; L.sz = n;
+    return true;
+  }
+  if (!mask) return false;
+  const uint32_t top = 31u - (uint32_t)__clz(mask);
+  uint32_t m = 0, f0 = 0, f1 = 0, f2 = 0;              // children; the first one stays in registers
+  auto child = [&](uint32_t lo, uint32_t base, uint32_t d) {
+    const uint32_t fl = left ? lo : base, rl = left ? base : lo;
+    if (m == 0) { f0 = fl; f1 = rl; f2 = d; m = 1; return; }
+    if (m >= cap) { ovf = true; return; }
+    if (m == 1) L.alt[0] = BIv{f0, f0 + f2, f1, f1 + f2};
+    L.alt[m++] = BIv{fl, fl + d, rl, rl + d};
+  };
+  const uint32_t cnt = L.cnt;
+  for (uint32_t k = 0; k < cnt; k++) {
+    uint32_t fl = L.flo, rl = L.rlo, n = L.sz;
+    if (cnt > 1) { const BIv v = L.cur[k]; fl = v.flo; rl = v.rlo; n = v.fhi - v.flo; }
+    const uint32_t lo = left ? fl : rl, base = left ? rl : fl;
+    if (n == 1) {
+      // a one-row interval extends by the code of its row alone: one LF step on one record
+      uint32_t s0, rk;
+      row_code_rank<FMT>(X, lo, s0, rk);
+      if (COUNT_TOUCH) touches += 1;
+      if ((mask >> s0) & 1) child(C[s0] + rk, base, 1u);
+    } else {
+      if (COUNT_TOUCH) touches += (lo != 0) + 1;
+      uint32_t run = 0;
+      // count_smaller_than (src/fm_index/bidir.rs:125-143): the new interval of symbol s on
+      // the other strand starts after every code below s, $ included
+      split_by_symbol<FMT>(X, lo, lo + n, top, [&](int s, uint32_t d, uint32_t r, uint32_t sbi) {
+        if (!ovf && ((mask >> s) & 1) && d)
+          child(C[s] + (FMT == OCC_WIDE ? r : sb_count(X, sbi, s) + r), base + run, d);
+        run += d;
+      });
+    }
+    if (ovf) return false;
+  }
+  if (m == 0) return false;
+  if (m == 1) { L.flo = f0; L.rlo = f1; L.sz = f2; }
+  else { const SR t = L.cur; L.cur = L.alt; L.alt = t; }
+  L.cnt = m;
+  return true;
+}
+
+// Shell sort of an interval set by its forward start (hits of one MEM ascend by it).
+template <class SR>
+__device__ __forceinline__ void sort_set(const SR& a, uint32_t n) {
+  for (uint32_t gap = n / 2; gap > 0; gap /= 2)
+    for (uint32_t i = gap; i < n; i++) {
+      const BIv t = a[i];
+      uint32_t j = i;
+      while (j >= gap) {
+        const BIv v = a[j - gap];
+        if (v.flo <= t.flo) break;
+        a[j] = v;
+        j -= gap;
+      }
+      a[j] = t;
+    }
+}
+
+// Persistent search.  KC > 0: hit lists of KC entries in local memory; KC = 0: W.hit_cap
+// entries per thread in global memory.  A job that outgrows its sets or its list is queued
+// for a later tier (out.ovf_list, once per read).
+template <bool COUNT_TOUCH, int STRIDE, int KC, int MINB, uint32_t FMT>
+__global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const uint16_t* __restrict__ compat_fw,
+                                                   const uint16_t* __restrict__ compat_rv,
+                                                   const uint8_t* __restrict__ q, const uint64_t* __restrict__ qoff,
+                                                   MemsParams P, Pool hitpool, MemsOut out, MemsWork W, SmemJobs J) {
+  __shared__ SmemFm Sf, Sr;
+  smem_fm_init(Sf, Fw, compat_fw);
+  smem_fm_init(Sr, Rv, compat_rv);
+  __syncthreads();
+  const uint32_t SCAP = STRIDE == 32 ? FAST_SET_CAP : W.set_cap;
+  using SR = SetRef<BIv, STRIDE>;
+  LaneSet<SR> L;
+  L.cur = thread_set<BIv, STRIDE>(W.sets, SCAP, 2, 0);
+  L.alt = thread_set<BIv, STRIDE>(W.sets, SCAP, 2, 1);
+  uint4 local_h[KC > 0 ? 2 * KC : 1];
+  uint4* hits = local_h;
+  uint32_t hit_cap = KC;
+  if (KC == 0) {
+    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    hits = W.hits + tid * W.hit_cap * 2;
+    hit_cap = W.hit_cap;
+  }
+  enum : uint32_t { FETCH, WINDOW, BACK, FORWARD, NEXT, LEFT_MAX, DONE };
+  const uint32_t n_units = J.units(), n_jobs = n_units + J.whole(), chunk = W.step(), min_len = P.min_len;
+  const uint32_t sym = Fw.sym_mask;
+  QueueCursor qc;
+  uint64_t touches = 0, t0 = 0;
+  uint32_t ph = FETCH, u = 0, read = 0, st = ST_OK;
+  uint32_t n = 0, i = 0, stop = 0, pos = 0, end = 0, nh = 0;
+  bool first = false;                     // the left-maximality of i is not known yet
+  const uint8_t* p = q;
+  for (;;) {
+    if (ph == FETCH) {
+      if (!next_read_chunked(W.queue, n_jobs, nullptr, chunk, qc, u)) break;
+      const bool unit = u < n_units;
+      read = unit ? J.unit_read[u] : J.ids ? J.ids[u - n_units] : u - n_units;
+      const uint64_t o = qoff[read];
+      n = (uint32_t)(qoff[read + 1] - o);
+      p = q + o;
+      i = unit ? J.unit_k[u] * J.seg_len : 0u;
+      stop = unit ? min(n, i + J.seg_len) : n;
+      first = i > 0;
+      nh = 0; st = ST_OK; t0 = touches;
+      ph = WINDOW;
+      if (!unit && J.resume && J.resume[read] != RESUME_START) {
+        // behind a first result that is already known: its hits lead this read's list
+        end = J.resume[read];
+        const uint64_t slot = J.slot_base ? J.slot_base[read] : (uint64_t)read;
+        const uint4* src = (const uint4*)hitpool.base + out.hit_start[slot] * 2;
+        const uint32_t have = out.hit_count[slot];
+        if (have > hit_cap) { st |= ST_CAND_OVF; ph = DONE; }
+        else {
+          for (uint32_t k = 0; k < 2 * have; k++) hits[k] = src[k];
+          nh = have;
+          if (end == 0) i = 1;
+          else { L.flo = 0; L.rlo = 0; L.sz = Fw.text_len; L.cnt = 1; pos = end; ph = NEXT; }
+        }
+      }
+    }
+    if (ph == WINDOW) {
+      if (min_len == 0 || i >= stop || n - i < min_len) ph = DONE;
+      else {
+        L.flo = 0; L.rlo = 0; L.sz = Fw.text_len; L.cnt = 1;
+        pos = i + min_len - 1;
+        ph = BACK;
+      }
+    }
+    bool matched = false;                 // q[i, end) is a longest match from i
+    if (ph != DONE) {
+      const bool left = ph != FORWARD;
+      const FmView X{left ? Fw.occ : Rv.occ, left ? Fw.sb : Rv.sb};
+      const uint8_t code = p[pos];
+      const uint32_t mask = code < 16 ? (uint32_t)Sf.compat_mask[code] & sym : 0u;
+      bool ovf = false;
+      const bool ok = lane_step<COUNT_TOUCH, FMT>(X, Sf.C, left, mask, L, SCAP, ovf, touches);
+      if (ovf) { st |= ST_SET_OVF; ph = DONE; }
+      else if (ph == BACK) {
+        if (!ok) { i = pos + 1; first = false; ph = WINDOW; }
+        else if (pos > i) pos--;
+        else {
+          pos = i + min_len;
+          if (pos == n) { end = n; matched = true; }
+          else ph = FORWARD;
+        }
+      } else if (ph == FORWARD) {
+        if (ok) pos++;
+        if (!ok || pos == n) { end = pos; matched = true; }
+      } else if (ph == NEXT) {
+        if (!ok) { i = pos + 1; ph = WINDOW; }
+        else if (pos <= i + 1) { i = i + 1; ph = WINDOW; }      // q[i, end] is known not to match
+        else pos--;
+      } else {                                                  // LEFT_MAX: the set is still that of q[i, end)
+        first = false;
+        if (ok) { L.flo = 0; L.rlo = 0; L.sz = Fw.text_len; L.cnt = 1; pos = end; ph = end == n ? DONE : NEXT; }
+        else matched = true;
+      }
+    }
+    if (matched && first) { ph = LEFT_MAX; pos = i - 1; matched = false; }
+    if (matched) {
+      // one hit per interval of the set, ascending by forward start
+      if (nh + L.cnt > hit_cap) { st |= ST_CAND_OVF; ph = DONE; }
+      else {
+        if (L.cnt > 1) sort_set(L.cur, L.cnt);
+        for (uint32_t k = 0; k < L.cnt; k++) {
+          uint32_t fl = L.flo, sz = L.sz;
+          if (L.cnt > 1) { const BIv v = L.cur[k]; fl = v.flo; sz = v.fhi - v.flo; }
+          hits[2 * (nh + k)] = make_uint4(i, end, sz, sz > P.max_hits ? 1u : 0u);
+          hits[2 * (nh + k) + 1] = make_uint4(fl, P.resolve ? min(sz, P.max_hits) : 0u, 0u, 0u);
+        }
+        nh += L.cnt;
+        L.flo = 0; L.rlo = 0; L.sz = Fw.text_len; L.cnt = 1;
+        pos = end;
+        ph = end == n ? DONE : NEXT;
+      }
+    }
+    if (ph == DONE) {
+      uint64_t hs = 0;
+      if (st) nh = 0;
+      if (nh) {
+        hs = thread_reserve(hitpool, nh);
+        if (hs == ~0ull) { st |= ST_POOL_OVF; hs = 0; nh = 0; }
+        else {
+          uint4* dst = (uint4*)hitpool.base + hs * 2;
+          for (uint32_t k = 0; k < 2 * nh; k++) dst[k] = hits[k];
+        }
+      }
+      const bool unit = u < n_units;
+      const uint64_t slot = (J.slot_base ? J.slot_base[read] : (uint64_t)read) + (unit ? J.unit_k[u] : 0u);
+      out.hit_start[slot] = hs; out.hit_count[slot] = nh;
+      if (!unit && J.slot_base)
+        for (uint64_t k = slot + 1; k < J.slot_base[read + 1]; k++) out.hit_count[k] = 0;
+      if (COUNT_TOUCH && W.work_log) {
+        atomicAdd(W.work_log + 4 * (size_t)read, (uint32_t)(touches - t0));
+        if (st & (ST_SET_OVF | ST_CAND_OVF)) atomicOr(W.work_log + 4 * (size_t)read + 3, 1u);
+      }
+      if (st) {
+        const uint32_t before = atomicOr(out.status + read, st);
+        const uint32_t tier = ST_SET_OVF | ST_CAND_OVF;
+        if ((st & tier) && !(before & tier)) out.ovf_list[atomicAdd(out.n_ovf, 1u)] = read;
+      }
+      ph = FETCH;
+    }
+  }
+  if (COUNT_TOUCH && touches) atomicAdd(out.touches, (unsigned long long)touches);
+}
+
+}  // namespace hfm
