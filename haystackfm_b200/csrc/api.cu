@@ -604,21 +604,20 @@ static int prefix_order(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff
   return HFM_OK;
 }
 
-// How k_trie runs a batch of nq reads: resident warps and reads per warp.  A warp's nodes
+// How k_trie runs a batch of nq reads: resident blocks and reads per block.  A block's nodes
 // are shared by its reads, so groups are as large as the batch allows while every resident
-// warp still has one; beyond that a whole number of rounds keeps the last one full.
-static constexpr size_t TRIE_SMEM = TRIE_WARPS * sizeof(TrieShared);
+// block still has one; beyond that a whole number of rounds keeps the last one full.
+static constexpr size_t TRIE_SMEM = sizeof(TrieShared);
 static int trie_plan(hfm_index* x, uint32_t nq, uint32_t& blocks, uint32_t& group) {
   int bpsm = 0;
   for (auto k : {k_trie<false>, k_trie<true>})
     CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRIE_SMEM));
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_trie<false>, TRIE_WARPS * 32, TRIE_SMEM));
-  const uint64_t warps = (uint64_t)std::max(1, bpsm) * x->num_sms * TRIE_WARPS;
-  const uint64_t rounds = std::max<uint64_t>(1, (nq + warps * 32 - 1) / (warps * 32));
-  group = (uint32_t)std::max<uint64_t>(1, (nq + warps * rounds - 1) / (warps * rounds));
-  const uint64_t groups = (nq + group - 1) / group;
-  blocks = (uint32_t)std::max<uint64_t>(1, (std::min(warps, groups) + TRIE_WARPS - 1) / TRIE_WARPS);
-  RET(x->trie_nodes.ensure((size_t)blocks * TRIE_WARPS * TRIE_NODE_BYTES));
+  const uint64_t room = (uint64_t)std::max(1, bpsm) * x->num_sms;
+  const uint64_t rounds = std::max<uint64_t>(1, (nq + room * 32 - 1) / (room * 32));
+  group = (uint32_t)std::max<uint64_t>(1, (nq + room * rounds - 1) / (room * rounds));
+  blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(room, (nq + group - 1) / group));
+  RET(x->trie_nodes.ensure((size_t)blocks * TRIE_NODE_BYTES));
   RET(x->trie_left.ensure((size_t)nq * 4 + 4));
   RET(x->trie_resume.ensure((size_t)nq * 4 + 4));
   return HFM_OK;

@@ -1,4 +1,4 @@
-// trie.cuh — the first forward sweep of up to 32 reads of an IUPAC text by one warp.
+// trie.cuh — the first forward sweep of up to 32 reads of an IUPAC text by one block.
 //
 // On a text with N runs and ambiguity codes a read matches tens of text strings at once,
 // nearly all of them windows that touch an N run: they depend on the read's first or last
@@ -8,9 +8,14 @@
 // nodes, each with the mask of the reads that hold it.  From one position to the next every
 // node is split by symbol once, whatever the number of reads; the child of symbol s keeps
 // the reads whose code there matches s.  A child has one parent and one symbol, so the list
-// never holds an interval twice and no lookup is needed.  The lanes of the warp take a node
-// each, one-row nodes (one LF step on one record) and larger ones (16 counts at both
-// borders) in lists of their own, so that a warp runs one kind at a time.
+// never holds an interval twice and no lookup is needed.  The threads of the block take a
+// node each, one-row nodes (one LF step on one record) and larger ones (16 counts at both
+// borders) in lists of their own, so that a warp runs one kind at a time.  The order of a
+// list is the order in which its warps reserved their places: nothing depends on it.
+//
+// A block, not a warp, per group: reads with an N among their first bases grow a group's
+// list to thousands of nodes, and with one warp to work them off such groups ran on alone
+// for more than half of the kernel (60,000 reads: SMs active 37% of the time).
 //
 // A read that reaches its end with a non-empty set has one result, the whole read.  One
 // whose set empties at position j has the result [0, j) (if it is long enough) and goes on
@@ -18,32 +23,41 @@
 // forward phases there (smem.cuh): the SA intervals of the text strings that match.
 //
 // Measured on a B200, 150 bp reads on the 100 Mbp IUPAC text, kernel times of a thread per
-// read and of this sweep: 200,000 reads by prefix 39.5 -> 12.6 ms, 4,099 reads 16.2 -> 1.3 ms,
-// 64 reads 10.7 -> 0.67 ms (one read a warp: the nodes of a read share the lanes).  Bound by
-// issue: the 16 masks and popcounts of a node's two borders and its children's writes.
+// read, of this sweep with a warp per group, and as it is: 200,000 reads by prefix 39.5 /
+// 12.6 / 12.7 ms, 60,000 reads - / 7.7 / 5.0, 4,099 reads 16.2 / 1.30 / 0.88, 64 reads (one
+// a block: its nodes share the threads) 10.7 / 0.67 / 0.65.  Bound by issue: some 400
+// instructions for 32 larger nodes (the 16 masks and popcounts of two borders, then their
+// children); 30 reads carry about 130 of those and as many one-row nodes a position, where
+// one read alone carries some 35.
 #pragma once
 #include "smem.cuh"
 
 namespace hfm {
 
 constexpr uint32_t TRIE_WARPS = 4;          // warps per block
-constexpr uint32_t TRIE_S1 = 160;           // one-row nodes of a list kept in shared memory
-constexpr uint32_t TRIE_SB = 96;            // larger nodes kept in shared memory
-constexpr uint32_t TRIE_CAP = 8192;         // nodes of one list in all
+constexpr uint32_t TRIE_S1 = 640;           // one-row nodes of a list kept in shared memory
+constexpr uint32_t TRIE_SB = 384;           // larger nodes kept in shared memory
+constexpr uint32_t TRIE_CAP = 16384;        // nodes of one list in all
 constexpr uint32_t TRIE_EMIT = 256;         // intervals of one read's set (more: k_smem takes the read)
-constexpr size_t TRIE_NODE_BYTES = 4ull * TRIE_CAP * 16;   // global node area per warp (two sizes, two buffers)
+constexpr size_t TRIE_NODE_BYTES = 4ull * TRIE_CAP * 16;   // global node area per block (two sizes, two buffers)
 
 struct TrieShared {
   uint4 one[2][TRIE_S1];
   uint4 big[2][TRIE_SB];
-  uint2 set[TRIE_EMIT];
-  uint32_t reads[16];                       // reads whose code matches symbol s
+  uint2 set[TRIE_WARPS][TRIE_EMIT];
+  uint32_t reads[TRIE_WARPS][16];           // reads whose code matches symbol s (a copy per warp)
+  // of the next list: nodes, reads that hold one.  Position j counts in [j % 3] and clears
+  // the one after it, which every thread has read two barriers ago.
+  uint32_t n1[3], nb[3], still[3];
+  uint32_t C[16];
+  uint32_t group;
+  uint16_t compat[16];
 };
 
 struct TrieWork {
-  uint4* nodes;                             // TRIE_NODE_BYTES per warp
+  uint4* nodes;                             // TRIE_NODE_BYTES per block
   unsigned int* queue;
-  uint32_t group;                           // reads per warp, 1..32
+  uint32_t group;                           // reads per block, 1..32
   uint32_t* left; uint32_t* n_left;         // reads that k_smem goes on with
   uint32_t* resume;                         // per read: where, or RESUME_START
 };
@@ -81,22 +95,24 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
                                                              const uint64_t* __restrict__ qoff, MemsParams P,
                                                              Pool hitpool, MemsOut out, TrieWork W, SmemJobs J) {
   extern __shared__ __align__(16) unsigned char trie_smem[];
-  __shared__ uint32_t s_C[16];
-  __shared__ uint16_t s_compat[16];
-  if (threadIdx.x < 16) { s_C[threadIdx.x] = Rv.C[threadIdx.x]; s_compat[threadIdx.x] = compat[threadIdx.x] & Fw.sym_mask; }
-  __syncthreads();
-  const uint32_t lane = threadIdx.x & 31, lt = lane_lt_mask();
-  const uint32_t warp = blockIdx.x * TRIE_WARPS + (threadIdx.x >> 5);
-  TrieShared& S = reinterpret_cast<TrieShared*>(trie_smem)[threadIdx.x >> 5];
-  uint4* g = W.nodes + (size_t)warp * 4 * TRIE_CAP;
+  TrieShared& S = *reinterpret_cast<TrieShared*>(trie_smem);
+  if (threadIdx.x < 16) { S.C[threadIdx.x] = Rv.C[threadIdx.x]; S.compat[threadIdx.x] = compat[threadIdx.x] & Fw.sym_mask; }
+  const uint32_t lane = threadIdx.x & 31, lt = lane_lt_mask(), warp = threadIdx.x >> 5;
+  uint32_t* reads = S.reads[warp];
+  uint2* set = S.set[warp];
+  uint4* g = W.nodes + (size_t)blockIdx.x * 4 * TRIE_CAP;
   const uint32_t n_reads = J.whole(), n_groups = (n_reads + W.group - 1) / W.group;
   const FmView X{Rv.occ, Rv.sb};
   uint64_t touches = 0;
   for (;;) {
-    uint32_t grp = 0;
-    if (lane == 0) grp = atomicAdd(W.queue, 1u);
-    grp = __shfl_sync(0xFFFFFFFFu, grp, 0);
+    if (threadIdx.x == 0) {
+      S.group = atomicAdd(W.queue, 1u);
+      S.n1[0] = S.nb[0] = S.still[0] = 0;
+    }
+    __syncthreads();
+    const uint32_t grp = S.group;
     if (grp >= n_groups) break;
+    // lane r of every warp holds read r of the group
     const uint32_t k = grp * W.group + lane;
     const bool mine = lane < W.group && k < n_reads;
     const uint32_t read = mine ? (J.ids ? J.ids[k] : k) : 0u;
@@ -104,15 +120,30 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
     const uint32_t n = mine ? (uint32_t)(qoff[read + 1] - o) : 0u;
     const uint8_t* p = q + o;
     const uint64_t slot = mine ? (J.slot_base ? J.slot_base[read] : (uint64_t)read) : 0;
-    if (mine) { out.hit_start[slot] = 0; out.hit_count[slot] = 0; }
+    if (mine && warp == 0) { out.hit_start[slot] = 0; out.hit_count[slot] = 0; }
     uint32_t alive = __ballot_sync(0xFFFFFFFFu, mine && n >= P.min_len);      // min_len >= 1 here
 
-    // The result [0, j) of the reads in `who`: one hit per node that holds the read,
-    // ascending by forward start.  Returns the reads whose sets are too large for it.
-    auto emit = [&](uint32_t who, uint32_t j, const NodeList& one, uint32_t n1, const NodeList& big, uint32_t nb) {
-      uint32_t too_large = 0;
+    // Hands the reads in `who` to k_smem: after [0, j), or from the start.
+    auto leave = [&](uint32_t who, uint32_t j) {
+      if (!who) return;
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(W.n_left, (uint32_t)__popc(who));
+      at = __shfl_sync(0xFFFFFFFFu, at, 0);
+      if ((who >> lane) & 1) {
+        W.left[at + __popc(who & lt)] = read;
+        W.resume[read] = j;
+      }
+    };
+    // The result [0, j) of the reads in `who`, a warp per read: one hit per node that holds
+    // the read, ascending by forward start.  A set too large for it is left to k_smem; the
+    // reads that end before their last base go on there.
+    auto emit = [&](uint32_t who, uint32_t j, bool ends, const NodeList& one, uint32_t n1, const NodeList& big, uint32_t nb) {
+      uint32_t later = 0, again = 0;
       for (; who; who &= who - 1) {
         const uint32_t r = __ffs(who) - 1;
+        if (r % TRIE_WARPS != warp) continue;
+        if (!ends) later |= 1u << r;
+        if (j < P.min_len) continue;
         uint32_t cnt = 0;
         for (int kind = 0; kind < 2; kind++) {
           const NodeList& l = kind ? big : one;
@@ -122,11 +153,11 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
             if (b + lane < m) v = l.get(b + lane);
             const bool has = (v.w >> r) & 1;
             const uint32_t bal = __ballot_sync(0xFFFFFFFFu, has), at = cnt + __popc(bal & lt);
-            if (has && at < TRIE_EMIT) S.set[at] = make_uint2(v.x, v.z);
+            if (has && at < TRIE_EMIT) set[at] = make_uint2(v.x, v.z);
             cnt += __popc(bal);
           }
         }
-        if (cnt > TRIE_EMIT) { too_large |= 1u << r; continue; }
+        if (cnt > TRIE_EMIT) { again |= 1u << r; continue; }
         __syncwarp();
         uint64_t off = 0;
         if (lane == r) off = thread_reserve(hitpool, cnt);
@@ -134,9 +165,9 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
         if (off != ~0ull) {
           uint4* dst = (uint4*)hitpool.base + off * 2;
           for (uint32_t e = lane; e < cnt; e += 32) {
-            const uint2 v = S.set[e];
+            const uint2 v = set[e];
             uint32_t rank = 0;
-            for (uint32_t t = 0; t < cnt; t++) rank += S.set[t].x < v.x ? 1u : 0u;
+            for (uint32_t t = 0; t < cnt; t++) rank += set[t].x < v.x ? 1u : 0u;
             dst[2 * rank] = make_uint4(0u, j, v.y, v.y > P.max_hits ? 1u : 0u);
             dst[2 * rank + 1] = make_uint4(v.x, P.resolve ? min(v.y, P.max_hits) : 0u, 0u, 0u);
           }
@@ -147,52 +178,43 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
         }
         __syncwarp();
       }
-      return too_large;
-    };
-    // Hands the reads in `who` to k_smem: after [0, j), or from the start.
-    auto leave = [&](uint32_t who, uint32_t j) {
-      if (!who) return;
-      uint32_t at = 0;
-      if (lane == 0) at = atomicAdd(W.n_left, (uint32_t)__popc(who));
-      at = __shfl_sync(0xFFFFFFFFu, at, 0);
-      if ((who >> lane) & 1) {
-        W.left[at + __popc(who & lt)] = read;
-        W.resume[read] = j;
-        if (j == RESUME_START) out.hit_count[slot] = 0;
-      }
+      leave(later & ~again, j);
+      leave(again, RESUME_START);
     };
 
     uint32_t t = 0, n1 = 0, nb = 0;
-    if (lane == 0) {
+    if (threadIdx.x == 0) {
       const uint4 full = make_uint4(0u, 0u, Fw.text_len, alive);
       if (Fw.text_len == 1) S.one[0][0] = full; else S.big[0][0] = full;
     }
     if (Fw.text_len == 1) n1 = 1; else nb = 1;
     uint32_t code = ((alive >> lane) & 1) ? p[0] : 16u;
-    __syncwarp();
-    for (uint32_t j = 0;; j++) {
+    __syncthreads();
+    for (uint32_t j = 0, c = 0;; j++) {
       const NodeList one{S.one[t], g + (size_t)t * TRIE_CAP, TRIE_S1}, big{S.big[t], g + (size_t)(2 + t) * TRIE_CAP, TRIE_SB};
       const NodeList one2{S.one[t ^ 1], g + (size_t)(t ^ 1) * TRIE_CAP, TRIE_S1},
           big2{S.big[t ^ 1], g + (size_t)(2 + (t ^ 1)) * TRIE_CAP, TRIE_SB};
       const uint32_t fin = alive & __ballot_sync(0xFFFFFFFFu, n == j);
       if (fin) {
-        leave(emit(fin, j, one, n1, big, nb), RESUME_START);
+        emit(fin, j, true, one, n1, big, nb);
         alive &= ~fin;
       }
       if (!alive) break;
-      const uint32_t match = ((alive >> lane) & 1) && code < 16 ? s_compat[code] : 0u;
+      const uint32_t cn = c == 2 ? 0 : c + 1;
+      if (threadIdx.x == 0) { S.n1[cn] = 0; S.nb[cn] = 0; S.still[cn] = 0; }
+      const uint32_t match = ((alive >> lane) & 1) && code < 16 ? S.compat[code] : 0u;
       // the next code is on its way while this position's nodes are split
       code = ((alive >> lane) & 1) && j + 1 < n ? p[j + 1] : 16u;
+      __syncwarp();
 #pragma unroll
       for (int s = 0; s < 16; s++) {
         const uint32_t b = __ballot_sync(0xFFFFFFFFu, (match >> s) & 1);
-        if (lane == s) S.reads[s] = b;
+        if (lane == s) reads[s] = b;
       }
       __syncwarp();
-      uint32_t m1 = 0, mb = 0, still = 0;
-      bool ovf = false;
+      uint32_t still = 0;
       // larger nodes: their one-row children go to the one-row list
-      for (uint32_t b = 0; b < nb && !ovf; b += 32) {
+      for (uint32_t b = warp * 32; b < nb; b += TRIE_WARPS * 32) {
         uint32_t r[16], d[16], kids = 0;
         uint4 v = make_uint4(0, 0, 0, 0);
         if (b + lane < nb) {
@@ -201,21 +223,27 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
           if (COUNT_TOUCH) touches += 2;
 #pragma unroll
           for (int s = 1; s < 16; s++)
-            if (d[s] && (v.w & S.reads[s])) kids += d[s] == 1 ? 1u : 0x10000u;
+            if (d[s] && (v.w & reads[s])) kids += d[s] == 1 ? 1u : 0x10000u;
         }
         uint32_t total;
-        uint32_t at = warp_excl_scan(kids, total);
-        uint32_t a1 = m1 + (at & 0xFFFFu), ab = mb + (at >> 16);
-        m1 += total & 0xFFFFu; mb += total >> 16;
-        if (m1 > TRIE_CAP || mb > TRIE_CAP) { ovf = true; break; }
+        const uint32_t at = warp_excl_scan(kids, total);
+        uint32_t a1 = 0, ab = 0;
+        if (lane == 0) {
+          if (total & 0xFFFFu) a1 = atomicAdd(&S.n1[c], total & 0xFFFFu);
+          if (total >> 16) ab = atomicAdd(&S.nb[c], total >> 16);
+        }
+        a1 = __shfl_sync(0xFFFFFFFFu, a1, 0);
+        ab = __shfl_sync(0xFFFFFFFFu, ab, 0);
+        if (a1 + (total & 0xFFFFu) > TRIE_CAP || ab + (total >> 16) > TRIE_CAP) break;   // the counts tell everyone
+        a1 += at & 0xFFFFu; ab += at >> 16;
         if (kids) {
           uint32_t run = d[0];
 #pragma unroll
           for (int s = 1; s < 16; s++) {
-            const uint32_t who = v.w & S.reads[s];
+            const uint32_t who = v.w & reads[s];
             if (d[s] && who) {
-              const uint4 c = make_uint4(v.x + run, s_C[s] + r[s], d[s], who);
-              if (d[s] == 1) one2.put(a1++, c); else big2.put(ab++, c);
+              const uint4 kid = make_uint4(v.x + run, S.C[s] + r[s], d[s], who);
+              if (d[s] == 1) one2.put(a1++, kid); else big2.put(ab++, kid);
               still |= who;
             }
             run += d[s];
@@ -223,35 +251,43 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
         }
       }
       // one-row nodes: one LF step each
-      for (uint32_t b = 0; b < n1 && !ovf; b += 32) {
-        uint4 c = make_uint4(0, 0, 0, 0);
+      for (uint32_t b = warp * 32; b < n1; b += TRIE_WARPS * 32) {
+        uint4 kid = make_uint4(0, 0, 0, 0);
         if (b + lane < n1) {
           const uint4 v = one.get(b + lane);
           uint32_t s, rk;
           row_code_rank<OCC_WIDE>(X, v.y, s, rk);
           if (COUNT_TOUCH) touches += 1;
-          const uint32_t who = v.w & S.reads[s];
-          c = make_uint4(v.x, s_C[s] + rk, 1u, who);
+          const uint32_t who = v.w & reads[s];
+          kid = make_uint4(v.x, S.C[s] + rk, 1u, who);
           still |= who;
         }
-        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, c.w != 0);
-        if (m1 + __popc(bal) > TRIE_CAP) { ovf = true; break; }
-        if (c.w) one2.put(m1 + __popc(bal & lt), c);
-        m1 += __popc(bal);
+        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, kid.w != 0);
+        if (!bal) continue;
+        uint32_t a1 = 0;
+        if (lane == 0) a1 = atomicAdd(&S.n1[c], (uint32_t)__popc(bal));
+        a1 = __shfl_sync(0xFFFFFFFFu, a1, 0);
+        if (a1 + __popc(bal) > TRIE_CAP) break;
+        if (kid.w) one2.put(a1 + __popc(bal & lt), kid);
       }
-      if (ovf) { leave(alive, RESUME_START); break; }
       still = __reduce_or_sync(0xFFFFFFFFu, still);
-      __syncwarp();
+      if (lane == 0 && still) atomicOr(&S.still[c], still);
+      __syncthreads();
+      const uint32_t m1 = S.n1[c], mb = S.nb[c];
+      if (m1 > TRIE_CAP || mb > TRIE_CAP) {
+        if (warp == 0) leave(alive, RESUME_START);
+        break;
+      }
+      still = S.still[c];
       const uint32_t dead = alive & ~still;
       if (dead) {
-        const uint32_t whole = j >= P.min_len ? emit(dead, j, one, n1, big, nb) : 0u;
-        leave(dead & ~whole, j);
-        leave(whole, RESUME_START);
+        emit(dead, j, false, one, n1, big, nb);
         alive = still;
+        __syncthreads();                    // the next position writes where these lists are
       }
-      n1 = m1; nb = mb; t ^= 1;
+      n1 = m1; nb = mb; t ^= 1; c = cn;
     }
-    __syncwarp();
+    __syncthreads();
   }
   if (COUNT_TOUCH && touches) atomicAdd(out.touches, (unsigned long long)touches);
 }
