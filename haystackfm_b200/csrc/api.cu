@@ -99,7 +99,7 @@ struct DevBuf {
 
 struct Counters {                    // device-side counters, one block per handle
   unsigned long long iv_used, hit_used, touches, steps, n_units;
-  uint32_t n_ovf, still_ovf, walk_err, queue, queue2, n_mid, n_wrp, queue3, n_long, trie_queue, n_left, _pad;
+  uint32_t n_ovf, still_ovf, walk_err, queue, queue2, n_mid, n_wrp, queue3, n_long, trie_queue, n_left, seg_len;
 };
 
 struct FmDev {
@@ -118,6 +118,8 @@ using namespace hfm;
 struct hfm_index {
   int device = 0, kind = 0;
   FmDev fwd, rev;
+  DevAux aux{};                   // ACGT texts, bidirectional: what the SMEM search keeps besides the records
+  DevBuf aux_kmer;                // (owned by the handle that loaded the index, like its records)
   cudaStream_t stream = nullptr;
   std::mutex mu;
   bool count_work = false;
@@ -273,6 +275,40 @@ static int build_device_fm(const HostFm& h, FmDev& f, cudaStream_t s) {
   f.text_len = n; f.num_seqs = h.num_sequences; f.lookup_depth = d.lut_depth; f.tag = h.tag;
   f.num_lanes = L; f.encoding = h.encoding; f.rate = h.sample_rate; f.seq_boundaries = h.seq_boundaries;
   f.fmt = fmt;
+  return HFM_OK;
+}
+
+// The k-mer table of an ACGT index (DevAux): k at most KMER_MAX, and the table (16 bytes an
+// entry) no larger than a byte per text position.  Without the memory for it the search does
+// without it.  (k 12 / 11 / 10 / none, SMEM search ms on 256 Mbp: 1M reads of 150 bp 9.0 /
+// 9.0 / 9.8 / 15.1, 60,000 mixed reads 6.0 / 6.0 / 6.6 / 11.2: one step less is worth no more
+// than the table's larger reach into memory from 11 on.)
+static constexpr uint32_t KMER_MAX = 11;
+static int build_aux(hfm_index* x) {
+  const FmDev& f = x->fwd;
+  if (x->kind != HFM_KIND_BIDIR || f.fmt != OCC_NARROW) return HFM_OK;
+  uint32_t k = 0;
+  while (k < KMER_MAX && (16ull << (2 * (k + 1))) <= f.text_len) k++;
+  if (k < 2) return HFM_OK;
+  DevBuf tmp;
+  if (x->aux_kmer.ensure(16ull << (2 * k)) != HFM_OK || tmp.ensure(16ull << (2 * (k - 1))) != HFM_OK) {
+    x->aux_kmer.release();
+    return HFM_OK;
+  }
+  // levels alternate between the two buffers so that level k ends in the table
+  const uint4* in = nullptr;
+  for (uint32_t l = 0; l < k; l++) {
+    uint4* out = ((k - l) & 1) ? x->aux_kmer.as<uint4>() : tmp.as<uint4>();
+    const uint64_t entries = 1ull << (2 * (l + 1));
+    k_kmer_table<<<(unsigned)((entries + 255) / 256), 256, 0, x->stream>>>(f.d, in, l, out);
+    in = out;
+  }
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(x->stream);
+  tmp.release();
+  CK(e);
+  x->aux.kmer = x->aux_kmer.as<uint4>();
+  x->aux.k = k;
   return HFM_OK;
 }
 
@@ -693,19 +729,23 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
   const uint32_t* fast_ids = order ? order + n_warp : nullptr;
   uint32_t n_fast = nq - n_warp, n_long = 0;
   uint64_t n_units = 0, n_slots = nq;
+  uint32_t seg_len = x->seg_len;
   const uint64_t* slot_base = nullptr;
   if (variant == 3 && n_fast > 0 && min_len > 0) {
     CK(cudaMemsetAsync(x->ctr.p, 0, sizeof(Counters), x->stream));
     RET(x->nslot.ensure((size_t)nq * 4 + 4));
     if (n_warp) CK(cudaMemsetAsync(x->nslot.p, 0, (size_t)nq * 4, x->stream));
     RET(x->lflag.ensure((size_t)n_fast * 4 + 4));
-    k_long_reads<<<(n_fast + 255) / 256, 256, 0, x->stream>>>(fast_ids, n_fast, d_qoff, x->seg_len, x->lflag.as<uint32_t>(),
-                                                              x->nslot.as<uint32_t>(), &dctr(x)->n_long, &dctr(x)->n_units);
+    k_long_reads<<<(n_fast + 255) / 256, 256, 0, x->stream>>>(fast_ids, n_fast, d_qoff, nq, x->seg_len,
+                                                              fmt == OCC_NARROW ? full_threads : 0, x->lflag.as<uint32_t>(),
+                                                              x->nslot.as<uint32_t>(), &dctr(x)->n_long, &dctr(x)->n_units,
+                                                              &dctr(x)->seg_len);
     other++;
     CK(cudaGetLastError());
     RET(read_ctr(x));
     n_long = x->h_ctr->n_long;
     n_units = x->h_ctr->n_units;
+    seg_len = x->h_ctr->seg_len;
     if (n_long) {
       RET(x->lpos.ensure(((size_t)n_fast + 1) * 8));
       RET(x->sids.ensure((size_t)n_fast * 4 + 4));
@@ -720,7 +760,7 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       k_split_ids<<<(n_fast + 255) / 256, 256, 0, x->stream>>>(fast_ids, n_fast, x->lflag.as<uint32_t>(),
                                                                x->lpos.as<uint64_t>(), x->sids.as<uint32_t>(),
                                                                x->lids.as<uint32_t>(), x->ucount.as<uint32_t>(), d_qoff,
-                                                               x->seg_len);
+                                                               seg_len);
       RET(scan(x, x->ucount.as<uint32_t>(), 1, n_long, x->ubase.as<uint64_t>(), other));
       k_unit_fill<<<(n_long + 255) / 256, 256, 0, x->stream>>>(x->lids.as<uint32_t>(), n_long, x->ubase.as<uint64_t>(),
                                                                x->uread.as<uint32_t>(), x->uk.as<uint32_t>());
@@ -810,7 +850,7 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       W.hits = variant == 3 ? x->cwork.as<uint4>() : nullptr; W.hit_cap = variant == 3 ? FAST_HIT_CAP : 0u;
       W.queue = &dctr(x)->queue; W.still_ovf = &dctr(x)->still_ovf; W.work_log = wlog; W.chunk = x->queue_chunk;
       SmemJobs J{};
-      J.unit_read = x->uread.as<uint32_t>(); J.unit_k = x->uk.as<uint32_t>(); J.seg_len = x->seg_len;
+      J.unit_read = x->uread.as<uint32_t>(); J.unit_k = x->uk.as<uint32_t>(); J.seg_len = seg_len;
       J.n_units = (uint32_t)n_units; J.ids = fast_ids; J.n_ids = n_fast; J.slot_base = slot_base;
       const unsigned grid = (unsigned)(threads / 128);
       if (x->memwork.cap < (size_t)grid * 128 * MEM_SET_BYTES) return set_error(HFM_E_ARG, "internal: work area too small");
@@ -831,7 +871,7 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       WITH_FMT(fmt, {
         auto go = [&](auto kern) {
           kern<<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(), Rv.compat.as<uint16_t>(), d_q, d_qoff, P,
-                                            hp, o, W, J);
+                                            hp, o, W, J, x->aux);
         };
         if (variant == 3) { if (counting) go(k_smem<true, 32, 0, 5, FM>); else go(k_smem<false, 32, 0, 8, FM>); }
         else { if (counting) go(k_smem<true, 32, MEM_KC, 5, FM>); else go(k_smem<false, 32, MEM_KC, 8, FM>); }
@@ -880,7 +920,7 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
         WITH_FMT(fmt, {
           auto go = [&](auto kern) {
             kern<<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(), Rv.compat.as<uint16_t>(), d_q, d_qoff,
-                                              P, hp, o2, W, J);
+                                              P, hp, o2, W, J, x->aux);
           };
           if (counting) go(k_smem<true, 32, 0, 5, FM>); else go(k_smem<false, 32, 0, 8, FM>);
         });
@@ -1132,8 +1172,9 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
   J.ids = ord; J.n_ids = nq; J.slot_base = slot_base;
   if (seg) {
     if (launch) {
-      k_long_reads<<<(nq + 255) / 256, 256, 0, x->stream>>>(ord, nq, c.d_qoff, x->seg_len, x->lflag.as<uint32_t>(),
-                                                            x->nslot.as<uint32_t>(), &dc->n_long, &dc->n_units);
+      k_long_reads<<<(nq + 255) / 256, 256, 0, x->stream>>>(ord, nq, c.d_qoff, nq, x->seg_len, 0, x->lflag.as<uint32_t>(),
+                                                            x->nslot.as<uint32_t>(), &dc->n_long, &dc->n_units,
+                                                            &dc->seg_len);
       CK(cudaGetLastError());
     }
     RET(SCAN(x->lflag.as<uint32_t>(), 1, nq, x->lpos.as<uint64_t>()));
@@ -1171,7 +1212,7 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
     }
     WITH_FMT(fmt, {
       k_smem<false, 32, 0, 8, FM><<<(unsigned)(threads / 128), 128, 0, x->stream>>>(Fw.d, Rv.d, cfw, crv, c.d_q, c.d_qoff,
-                                                                                    P, hp, o, W, J);
+                                                                                    P, hp, o, W, J, x->aux);
     });
     // reads that outgrew their sets or hit list: one warp per read, over the device list
     MemsWork Ww{};
@@ -1472,6 +1513,7 @@ static int make_shadow(hfm_index* x, hfm_index** out) {
   sh->queue_chunk = x->queue_chunk; sh->threads_per_read = x->threads_per_read; sh->read_order = x->read_order;
   sh->timeout_ms = x->timeout_ms;
   sh->shared_index = true;
+  sh->aux = x->aux;
   for (int k = 0; k < 2; k++) {
     const FmDev& src = k ? x->rev : x->fwd;
     FmDev& dst = k ? sh->rev : sh->fwd;
@@ -1536,6 +1578,7 @@ int hfm_index_load(const uint8_t* bytes, size_t len, int kind, const hfm_opts* o
   RET(x->ctr.ensure(sizeof(Counters)));
   RET(build_device_fm(hf, x->fwd, x->stream));
   if (kind == HFM_KIND_BIDIR) RET(build_device_fm(hr, x->rev, x->stream));
+  RET(build_aux(x.get()));
   *out = x.release();
   return HFM_OK;
 }
@@ -1693,6 +1736,7 @@ int hfm_index_load_layout(const uint8_t* bytes, uint64_t len, const hfm_opts* op
     f.seq_boundaries = D.bnd;
   }
   CK(cudaStreamSynchronize(x->stream));
+  RET(build_aux(x.get()));
   *out = x.release();
   return HFM_OK;
 }
@@ -1711,7 +1755,10 @@ int hfm_index_device_bytes(const hfm_index* x, uint64_t* index_bytes, uint64_t* 
       &x->lids, &x->ucount, &x->ubase, &x->uread, &x->uk, &x->nslot, &x->slot_base, &x->slot_hits, &x->npos,
       &x->iota, &x->loc_pairs, &x->okeys, &x->oids, &x->otemp, &x->trie_nodes, &x->trie_left, &x->trie_resume};
   uint64_t a = 0, b = 0;
-  if (!x->shared_index) for (const DevBuf* d : idx_bufs) a += d->cap;
+  if (!x->shared_index) {
+    for (const DevBuf* d : idx_bufs) a += d->cap;
+    a += x->aux_kmer.cap;
+  }
   for (const DevBuf* d : work_bufs) b += d->cap;
   if (index_bytes) *index_bytes = a;
   if (work_bytes) *work_bytes = b;
@@ -1736,7 +1783,7 @@ void hfm_index_free(hfm_index* x) {
                     &x->blockmap, &x->blockmap2, &x->ovf2, &x->ovf3, &x->lflag, &x->lpos, &x->sids, &x->lids,
                     &x->ucount, &x->ubase, &x->uread, &x->uk, &x->nslot, &x->slot_base, &x->slot_hits, &x->npos,
                     &x->iota, &x->loc_pairs, &x->okeys, &x->oids, &x->otemp, &x->trie_nodes, &x->trie_left,
-                    &x->trie_resume})
+                    &x->trie_resume, &x->aux_kmer})
     b->release();
   for (auto& e : x->ev) if (e) cudaEventDestroy(e);
   for (auto& e : x->evk) if (e) cudaEventDestroy(e);
@@ -1751,7 +1798,7 @@ int hfm_index_info_get(const hfm_index* x, hfm_index_info* o) {
   o->kind = x->kind; o->text_len = x->fwd.text_len; o->num_sequences = x->fwd.num_seqs;
   o->sample_rate = x->fwd.rate; o->lookup_depth = x->fwd.lookup_depth; o->alphabet_tag = x->fwd.tag;
   o->num_lanes = x->fwd.num_lanes; o->encoding = x->fwd.encoding;
-  o->device_bytes = x->fwd.bytes() + x->rev.bytes();
+  o->device_bytes = x->fwd.bytes() + x->rev.bytes() + x->aux_kmer.cap;
   return HFM_OK;
 }
 

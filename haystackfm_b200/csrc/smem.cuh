@@ -20,10 +20,10 @@
 //
 // A read costs about 2 min_len + its match lengths in steps; the sweep it replaces extended
 // every prefix of every pivot at which the coverage drops (some 15 per pivot) left again.
-// Measured on a B200, 256 Mbp ACGT repeat genome, kernel times of the sweep and of this
-// search: 1M reads of 150 bp 58.4 -> 11.6 ms; 60,000 mixed reads up to 10 kbp 71.2 -> 7.7 ms;
-// 250 of them 37.2 -> 5.2 ms; find_mems of 20,000 ragged reads 25.9 -> 1.9 ms.  Bound by the
-// latency of one dependent record load per step.
+// Measured on a B200, 256 Mbp ACGT repeat genome, kernel times of the sweep, of this search,
+// and with the k-mer table (DevAux) and short segments for small batches: 1M reads of 150 bp
+// 58.4 / 11.3 / 8.2 ms; 60,000 mixed reads up to 10 kbp 71.2 / 7.7 / 4.7 ms; 250 of them
+// 37.2 / 5.2 / 0.56 ms; find_mems of 20,000 ragged reads 25.9 / 1.9 / 0.9 ms.
 //
 // Segments.  A result belongs to the segment of a long read in which it starts.  A segment's
 // search begins at its first position a: if the window there does not match, everything
@@ -64,6 +64,17 @@ struct SmemJobs {
 
 constexpr uint32_t RESUME_START = 0xFFFFFFFFu;
 
+// What a bidirectional index of an ACGT text keeps besides its records, made on the device
+// when it is loaded (k_kmer_table):
+//   kmer  for every ACGT string of k codes (code 1 first, the first code in the top digit)
+//         its forward start, reverse start and rows: the window and next phases start k
+//         steps on, with one load.
+// It may be absent (no memory for it): the search then takes the steps.
+struct DevAux {
+  const uint4* kmer;
+  uint32_t k;
+};
+
 // One direction of the index as the step needs it.
 struct FmView { const uint4* occ; const uint32_t* sb; };
 
@@ -101,7 +112,7 @@ __device__ __forceinline__ bool acgt_step(const FmView& X, const uint32_t* C, ui
   const uint32_t last = lo + n - 1, bl = lo >> 6, bh = last >> 6;
   const uint4* pl = X.occ + (size_t)bl * OCC_NARROW_U4;
   const uint4 a = __ldg(pl), b = __ldg(pl + 1);
-  const uint32_t sbl = __ldg(X.sb + (size_t)(bl >> SB_BLOCK_SHIFT) * 16 + s);
+  uint32_t sbl = __ldg(X.sb + (size_t)(bl >> SB_BLOCK_SHIFT) * 16 + s);
   uint4 a2 = a, b2 = b;
   if (bh != bl) {
     const uint4* ph = X.occ + (size_t)bh * OCC_NARROW_U4;
@@ -215,7 +226,8 @@ template <bool COUNT_TOUCH, int STRIDE, int KC, int MINB, uint32_t FMT>
 __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const uint16_t* __restrict__ compat_fw,
                                                    const uint16_t* __restrict__ compat_rv,
                                                    const uint8_t* __restrict__ q, const uint64_t* __restrict__ qoff,
-                                                   MemsParams P, Pool hitpool, MemsOut out, MemsWork W, SmemJobs J) {
+                                                   MemsParams P, Pool hitpool, MemsOut out, MemsWork W, SmemJobs J,
+                                                   DevAux A) {
   __shared__ SmemFm Sf, Sr;
   smem_fm_init(Sf, Fw, compat_fw);
   smem_fm_init(Sr, Rv, compat_rv);
@@ -233,7 +245,7 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
     hits = W.hits + tid * W.hit_cap * 2;
     hit_cap = W.hit_cap;
   }
-  enum : uint32_t { FETCH, WINDOW, BACK, FORWARD, NEXT, LEFT_MAX, DONE };
+  enum : uint32_t { FETCH, WINDOW, BACK, FORWARD, NEXT_START, NEXT, LEFT_MAX, DONE };
   const uint32_t n_units = J.units(), n_jobs = n_units + J.whole(), chunk = W.step(), min_len = P.min_len;
   const uint32_t sym = Fw.sym_mask;
   QueueCursor qc;
@@ -266,20 +278,36 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
           for (uint32_t k = 0; k < 2 * have; k++) hits[k] = src[k];
           nh = have;
           if (end == 0) i = 1;
-          else { L.flo = 0; L.rlo = 0; L.sz = Fw.text_len; L.cnt = 1; pos = end; ph = NEXT; }
+          else ph = NEXT_START;
         }
       }
     }
-    if (ph == WINDOW) {
-      if (min_len == 0 || i >= stop || n - i < min_len) ph = DONE;
-      else {
-        L.flo = 0; L.rlo = 0; L.sz = Fw.text_len; L.cnt = 1;
-        pos = i + min_len - 1;
-        ph = BACK;
+    if (ph == WINDOW && (min_len == 0 || i >= stop || n - i < min_len)) ph = DONE;
+    if (ph == WINDOW || ph == NEXT_START) {
+      // start from the whole text, or from the last k codes at once (k <= min_len): where
+      // they do not occur, no result reaches past them from before the second of them
+      const bool window = ph == WINDOW;
+      L.flo = 0; L.rlo = 0; L.sz = Fw.text_len; L.cnt = 1;
+      pos = window ? i + min_len - 1 : end;
+      ph = window ? BACK : NEXT;
+      if (FMT == OCC_NARROW && A.kmer && A.k <= min_len) {
+        uint32_t x = 0, bad = 0;
+        const uint8_t* b = p + pos + 1 - A.k;
+        for (uint32_t k = 0; k < A.k; k++) { const uint32_t c = b[k] - 1u; bad |= c; x = x << 2 | (c & 3u); }
+        if (bad < 4) {
+          const uint4 v = __ldg(A.kmer + x);
+          if (COUNT_TOUCH) touches += 1;
+          const uint32_t at = pos + 1 - A.k;               // its first code
+          if (!v.z) { i = at + 1; first = false; ph = WINDOW; continue; }
+          L.flo = v.x; L.rlo = v.y; L.sz = v.z;
+          if (at > i) pos = at - 1;
+          else { pos = i + min_len; ph = FORWARD; }        // k == min_len: the window is matched
+        }
       }
     }
     bool matched = false;                 // q[i, end) is a longest match from i
-    if (ph != DONE) {
+    if (ph == FORWARD && pos == n) { end = n; matched = true; }
+    if (ph != DONE && !matched) {
       const bool left = ph != FORWARD;
       const FmView X{left ? Fw.occ : Rv.occ, left ? Fw.sb : Rv.sb};
       const uint8_t code = p[pos];
@@ -292,8 +320,8 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
         else if (pos > i) pos--;
         else {
           pos = i + min_len;
+          ph = FORWARD;
           if (pos == n) { end = n; matched = true; }
-          else ph = FORWARD;
         }
       } else if (ph == FORWARD) {
         if (ok) pos++;
@@ -304,7 +332,7 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
         else pos--;
       } else {                                                  // LEFT_MAX: the set is still that of q[i, end)
         first = false;
-        if (ok) { L.flo = 0; L.rlo = 0; L.sz = Fw.text_len; L.cnt = 1; pos = end; ph = end == n ? DONE : NEXT; }
+        if (ok) ph = end == n ? DONE : NEXT_START;
         else matched = true;
       }
     }
@@ -321,9 +349,7 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
           hits[2 * (nh + k) + 1] = make_uint4(fl, P.resolve ? min(sz, P.max_hits) : 0u, 0u, 0u);
         }
         nh += L.cnt;
-        L.flo = 0; L.rlo = 0; L.sz = Fw.text_len; L.cnt = 1;
-        pos = end;
-        ph = end == n ? DONE : NEXT;
+        ph = end == n ? DONE : NEXT_START;
       }
     }
     if (ph == DONE) {
@@ -355,6 +381,22 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
     }
   }
   if (COUNT_TOUCH && touches) atomicAdd(out.touches, (unsigned long long)touches);
+}
+
+// ---- DevAux, made when an index is loaded --------------------------------------------
+
+// One more code in front: out[c w] from in[w] for strings w of k codes (in: nullptr for k = 0).
+__global__ void k_kmer_table(DevFm Fw, const uint4* __restrict__ in, uint32_t k, uint4* __restrict__ out) {
+  const uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >> (2 * (k + 1))) return;
+  const uint32_t s = (uint32_t)(x >> (2 * k)) + 1u;
+  uint4 v = in ? in[x & ((1ull << (2 * k)) - 1ull)] : make_uint4(0u, 0u, Fw.text_len, 0u);
+  uint32_t C[5];
+  for (int c = 0; c < 5; c++) C[c] = Fw.C[c];
+  uint64_t touches = 0;
+  const FmView X{Fw.occ, Fw.sb};
+  if (v.z && !acgt_step<false>(X, C, s, v.x, v.y, v.z, touches)) v = make_uint4(0u, 0u, 0u, 0u);
+  out[x] = v;
 }
 
 }  // namespace hfm

@@ -386,21 +386,23 @@ int hfm_set_timeout(hfm_index* idx, uint32_t ms);
 /* Tunable parameters of the SMEM/MEM search and their autotuner (no counterpart in the
  * reference, whose shaders run a fixed workgroup_size(64), shaders/mem_find.wgsl:364-372).
  * Results never depend on them.
- *   mems_variant      persistent fast pass with 32-entry candidate lists in local memory (2)
- *                     or 1024-entry lists in global memory (3, default), 8 resident blocks
- *                     per SM; 4: the plain launch — one thread per read over a grid the size
+ *   mems_variant      persistent fast pass with 32-entry hit lists in local memory and whole
+ *                     reads (2), or 1024-entry lists in global memory and segments (3,
+ *                     default), 8 resident blocks per SM; 4: the plain launch — one thread per read over a grid the size
  *                     of the batch, sets and candidates in local memory, a count pass whose
  *                     totals are read back to size the outputs before the write pass (the
  *                     reference GPU search's structure, src/gpu/mem_find.rs:213-244), kept
  *                     as the baseline.
- *   seg_len           SMEM reads longer than 2*seg_len are swept in seg_len-position segments
- *                     (multiple of 32 in 64..4096, default 512).
+ *   seg_len           reads longer than 2*seg_len are searched in seg_len-position segments
+ *                     (multiple of 32 in 64..4096, default 512; on ACGT texts a batch that is
+ *                     too small to fill the GPU with them uses shorter ones, down to 64).
  *   queue_chunk       reads a per-thread kernel takes from its device work queue per atomic
  *                     (1..64, default 1).
  *   read_order        0 (default): the SMEM queue in the caller's read order (or the order of
  *                     hfm_mems_batch_device_sched); 1: reads queued in the order of their first
- *                     16 codes (a device radix sort; per-thread kernels only), so that reads
- *                     sharing a prefix — and the reference windows it selects — share a warp.
+ *                     16 codes (a device radix sort; per-thread kernels only).  On a text with
+ *                     ambiguity codes the reads of a block share their first sweep, and batches
+ *                     that fill the GPU with such groups are always queued by prefix.
  *   threads_per_read  1 (default): a thread per read; 4, 8 or 16: every read on a group of
  *                     that many lanes (sub-warp kernel, the fast pass's set capacities; a
  *                     read that outgrows them goes on to the warp tier); 32: every read on

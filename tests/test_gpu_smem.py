@@ -55,6 +55,8 @@ def test_read_lengths_and_group_sizes(oracle, kind):
     _check(oracle, b, h, ragged + noise + odd, 19, 0)
     _check(oracle, b, h, ragged[:60] + noise + odd, 1, 0, cap=4)
     _check(oracle, b, h, ragged[:40] + noise + odd, 12, 1)
+    for min_len in (6, 7, 8):                                           # around the k-mer table's k (7 here)
+        _check(oracle, b, h, ragged[:60] + noise + odd, min_len, 0, cap=4)
     _check(oracle, b, h, [r[:60] for r in rows[:24]], 61, 0)            # nothing is long enough
     _check(oracle, b, h, ragged[:24], 0, 0)                             # min_len 0: no results
     # a batch large enough for groups formed by prefix
