@@ -177,9 +177,9 @@ static int build_device_fm(const HostFm& h, FmDev& f, cudaStream_t s) {
   const uint64_t width = h.encoding == 0 ? h.num_planes : L;
   // Decode the reference records (compacted lanes, u32 superblock count + u16 delta per
   // lane) into whole per-symbol counts and 4 symbol-code bitplanes, then re-encode them as
-  // the device records: whole counts (wide; brought to row 32 on the device, k_wide_records)
-  // or counts from the start of the device superblock of 1024 records, which fit a u16
-  // (narrow).
+  // the device records: whole counts (wide) or counts from the start of the device
+  // superblock of 1024 records, which fit a u16 (narrow); k_device_records brings them to
+  // row 32.
   auto decode = [&](uint64_t b, uint32_t cnt[16], uint64_t planes[4]) {
     const uint8_t* r = h.block_data + b * h.block_stride;
     uint64_t words[16] = {0};
@@ -256,8 +256,8 @@ static int build_device_fm(const HostFm& h, FmDev& f, cudaStream_t s) {
     RET(upload(*bufs[k], srcs[k], sizes[k], s));
     f.nbytes[k] = sizes[k];
   }
-  if (fmt == OCC_WIDE) {
-    k_wide_records<<<(unsigned)((nblk + 255) / 256), 256, 0, s>>>(f.occ.as<uint4>(), (uint32_t)nblk);
+  if (nblk) {
+    k_device_records<<<(unsigned)((nblk + 255) / 256), 256, 0, s>>>(f.occ.as<uint4>(), (uint32_t)nblk, fmt);
     CK(cudaGetLastError());
   }
   CK(cudaStreamSynchronize(s));      // host vectors die at return
@@ -1593,21 +1593,44 @@ int hfm_index_load(const uint8_t* bytes, size_t len, int kind, const hfm_opts* o
 // ---------------------------------------------------------------------------
 static constexpr uint32_t LAYOUT_VERSION = 1;
 
-// Wide records as the blob holds them: counts before row 0 of the record and whole planes
-// (k_wide_records is the way back).
-static void blob_wide_records(uint8_t* rec, uint64_t n) {
-  auto work = [rec](uint64_t b0, uint64_t b1) {
-    for (uint64_t b = b0; b < b1; b++) {
-      uint32_t r[24], o[24];
-      std::memcpy(r, rec + b * 96, 96);
-      for (int c = 0; c < 16; c++) {
-        uint32_t m = ~0u;
-        for (int p = 0; p < 4; p++) m &= ((c >> p) & 1) ? r[16 + p] : ~r[16 + p];
-        o[c] = r[c] - (uint32_t)__builtin_popcount(m);
-      }
-      for (int p = 0; p < 4; p++) { o[16 + 2 * p] = r[16 + p]; o[17 + 2 * p] = r[20 + p]; }
-      std::memcpy(rec + b * 96, o, 96);
+// Records as the blob holds them: counts before row 0 of the record and whole planes of the
+// codes' bits (k_device_records is the way back).
+static void blob_records(uint8_t* rec, uint64_t n, uint32_t fmt) {
+  auto wide = [](uint8_t* at) {
+    uint32_t r[24], o[24];
+    std::memcpy(r, at, 96);
+    for (int c = 0; c < 16; c++) {
+      uint32_t m = ~0u;
+      for (int p = 0; p < 4; p++) m &= ((c >> p) & 1) ? r[16 + p] : ~r[16 + p];
+      o[c] = r[c] - (uint32_t)__builtin_popcount(m);
     }
+    for (int p = 0; p < 4; p++) { o[16 + 2 * p] = r[16 + p]; o[17 + 2 * p] = r[20 + p]; }
+    std::memcpy(at, o, 96);
+  };
+  auto narrow = [](uint8_t* at) {
+    uint32_t r[8], o[8];
+    std::memcpy(r, at, 32);
+    const uint32_t half[2][3] = {{r[2], r[3], r[4]}, {r[5], r[6], r[7]}};     // bits of code - 1, sentinels
+    uint32_t cnt[4];
+    for (int c = 0; c < 4; c++) {
+      const uint32_t m = ~half[0][2] & ((c & 1) ? half[0][0] : ~half[0][0]) & ((c & 2) ? half[0][1] : ~half[0][1]);
+      const uint32_t w = r[c >> 1];
+      cnt[c] = ((c & 1) ? w >> 16 : w & 0xFFFFu) - (uint32_t)__builtin_popcount(m);
+    }
+    o[0] = cnt[0] | cnt[1] << 16;
+    o[1] = cnt[2] | cnt[3] << 16;
+    for (int h = 0; h < 2; h++) {
+      const uint32_t b0 = half[h][0], b1 = half[h][1], z = half[h][2];
+      o[2 + h] = ~z & ~b0;                      // codes 1 and 3
+      o[4 + h] = ~z & (b0 ^ b1);                // codes 2 and 3
+      o[6 + h] = ~z & b0 & b1;                  // code 4
+    }
+    std::memcpy(at, o, 32);
+  };
+  auto work = [&](uint64_t b0, uint64_t b1) {
+    for (uint64_t b = b0; b < b1; b++)
+      if (fmt == OCC_WIDE) wide(rec + b * OCC_WIDE_U4 * 16);
+      else narrow(rec + b * OCC_NARROW_U4 * 16);
   };
   const unsigned nt = n < (1u << 16) ? 1 : std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
   std::vector<std::thread> th;
@@ -1649,7 +1672,7 @@ int hfm_index_export_layout(hfm_index* x, uint8_t** bytes_out, uint64_t* len_out
       if (f.nbytes[b]) {
         cudaError_t e = cudaMemcpy(w, bufs[b]->p, f.nbytes[b], cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) { std::free(out); cudaGetLastError(); return set_error(HFM_E_CUDA, "layout copy failed"); }
-        if (b == 0 && f.fmt == OCC_WIDE) blob_wide_records(w, f.nbytes[b] / (OCC_WIDE_U4 * 16));
+        if (b == 0) blob_records(w, f.d.num_blocks, f.fmt);
       }
       w += f.nbytes[b];
     }
@@ -1723,8 +1746,8 @@ int hfm_index_load_layout(const uint8_t* bytes, uint64_t len, const hfm_opts* op
       RET(upload(*bufs[b], bytes + D.at[b], D.nb[b], x->stream));
       f.nbytes[b] = D.nb[b];
     }
-    if (D.d.fmt == OCC_WIDE && D.d.num_blocks) {
-      k_wide_records<<<(D.d.num_blocks + 255) / 256, 256, 0, x->stream>>>(f.occ.as<uint4>(), D.d.num_blocks);
+    if (D.d.num_blocks) {
+      k_device_records<<<(D.d.num_blocks + 255) / 256, 256, 0, x->stream>>>(f.occ.as<uint4>(), D.d.num_blocks, D.d.fmt);
       CK(cudaGetLastError());
     }
     f.d = D.d;

@@ -12,9 +12,10 @@
 //                    popcounts (16 lanes a cycle) bound the search on IUPAC texts;
 //             narrow (32 B, texts of codes 0..4 only — ExactDna and ACGT-only IUPAC texts):
 //                    4 x u16 counts of codes 1..4 from the start of the record's superblock
-//                    (1,024 records = 65,536 rows) to the record, then 3 x u64 planes (one
-//                    sector); the count of code 0 is the rows before the border minus the
-//                    other four.
+//                    (1,024 records = 65,536 rows) to the record's row 32, then for rows
+//                    0..31 and for rows 32..63 three u32 planes: the two bits of code - 1,
+//                    and the sentinels (one sector); the count of code 0 is the rows before
+//                    the border minus the other four.
 //   sb    : (narrow) 16 x u32 per superblock: count of every code before the superblock
 //           (a few MB at 3.1 Gbp; it stays in L2).
 //   ssa   : one 16-byte record per 64 rows: u64 "row is sampled" bits + u32 count of
@@ -80,6 +81,14 @@ __device__ __forceinline__ uint32_t sel4(uint4 x, uint32_t i) {
 // (border 0: record 0 with no row selected; its counts and superblock entry are 0).
 template <uint32_t FMT> struct Border;
 
+// A border x rows (0..64) into a record: the rows between it and row 32, and whether they
+// are added to the counts there (1) or taken off (~0).
+__device__ __forceinline__ uint32_t half_rows(uint32_t x) {
+  const uint32_t k = x & 31;
+  return x >= 64 ? ~0u : x >= 32 ? (1u << k) - 1u : ~0u << k;
+}
+__device__ __forceinline__ uint32_t half_sign(uint32_t x) { return x >= 32 ? 1u : ~0u; }
+
 template <>
 struct Border<OCC_WIDE> {
   uint4 a, b, c, d;        // counts before row 32
@@ -87,11 +96,7 @@ struct Border<OCC_WIDE> {
   uint32_t m, sg;          // rows between row 32 and the border; 1 after row 32, ~0 before it
 
   // the rows of `w` counted for a border x rows (0..64) into the record
-  __device__ __forceinline__ void select(uint32_t x) {
-    const uint32_t k = x & 31;
-    m = x >= 64 ? ~0u : x >= 32 ? (1u << k) - 1u : ~0u << k;
-    sg = x >= 32 ? 1u : ~0u;
-  }
+  __device__ __forceinline__ void select(uint32_t x) { m = half_rows(x); sg = half_sign(x); }
   // rows of code s among the selected ones (s a compile-time constant after unrolling)
   __device__ __forceinline__ uint32_t eq(int s) const {
     return m & ((s & 1) ? w.x : ~w.x) & ((s & 2) ? w.y : ~w.y) & ((s & 4) ? w.z : ~w.z) & ((s & 8) ? w.w : ~w.w);
@@ -106,23 +111,26 @@ struct Border<OCC_WIDE> {
 
 template <>
 struct Border<OCC_NARROW> {
-  uint4 a, b;              // a = deltas + plane 0, b = planes 1, 2
-  uint64_t low;            // selected rows
+  uint32_t c12, c34;       // counts before row 32, from the superblock start
+  uint32_t b0, b1, z;      // the planes of the half that holds the border
+  uint32_t m, sg;          // rows between row 32 and the border; 1 after row 32, ~0 before it
   uint32_t sbi, i;         // superblock, the border itself
 
-  __device__ __forceinline__ uint64_t plane(int k) const {
-    return k == 0 ? u2to64(a.z, a.w) : k == 1 ? u2to64(b.x, b.y) : u2to64(b.z, b.w);
+  __device__ __forceinline__ void take(const uint4& u, const uint4& v, uint32_t x) {
+    c12 = u.x; c34 = u.y;
+    const bool up = x >= 32;
+    b0 = up ? v.y : u.z; b1 = up ? v.z : u.w; z = up ? v.w : v.x;
+    m = half_rows(x); sg = half_sign(x);
   }
-  __device__ __forceinline__ uint64_t eq(int s) const {
-    return low & ((s & 1) ? plane(0) : ~plane(0)) & ((s & 2) ? plane(1) : ~plane(1)) & ((s & 4) ? plane(2) : ~plane(2));
+  __device__ __forceinline__ uint32_t eq(int s) const {      // s in 1..4
+    return m & ~z & (((s - 1) & 1) ? b0 : ~b0) & (((s - 1) & 2) ? b1 : ~b1);
   }
-  // count of code s (1..4) from the superblock start to the record
   __device__ __forceinline__ uint32_t delta(int s) const {
-    const uint32_t w = s <= 2 ? a.x : a.y;
+    const uint32_t w = s <= 2 ? c12 : c34;
     return ((s - 1) & 1) ? (w >> 16) : (w & 0xFFFFu);
   }
   // rank of code s within the superblock
-  __device__ __forceinline__ uint32_t local(int s) const { return delta(s) + (uint32_t)__popcll(eq(s)); }
+  __device__ __forceinline__ uint32_t local(int s) const { return delta(s) + (uint32_t)__popc(eq(s)) * sg; }
 };
 
 template <uint32_t FMT, class FM>
@@ -136,11 +144,10 @@ __device__ __forceinline__ Border<FMT> load_border(const FM& F, uint32_t i) {
     r.w = __ldg(p + (x >= 32 ? 5 : 4));
     r.select(x);
   } else {
-    r.low = i ? (2ull << (pos & 63)) - 1ull : 0ull;        // rows 0..pos%64 (pos%64 = 63: all)
     r.sbi = blk >> SB_BLOCK_SHIFT;
     r.i = i;
     const uint4* p = F.occ + (size_t)blk * OCC_NARROW_U4;
-    r.a = __ldg(p); r.b = __ldg(p + 1);
+    r.take(__ldg(p), __ldg(p + 1), i ? (pos & 63) + 1u : 0u);
   }
   return r;
 }
@@ -233,19 +240,20 @@ __device__ __forceinline__ void row_code_rank(const FM& F, uint32_t row, uint32_
     code = c;
     rank = __ldg(reinterpret_cast<const uint32_t*>(p) + c) + (uint32_t)__popc(m) * B.sg;
   } else {
-    Border<FMT> B = load_border<FMT>(F, row + 1);     // the record of `row`, rows 0..row%64
-    const uint32_t c = (uint32_t)((B.plane(0) >> off) & 1) | ((uint32_t)((B.plane(1) >> off) & 1) << 1) |
-                       ((uint32_t)((B.plane(2) >> off) & 1) << 2);
-    B.low >>= 1;                                         // rows before `row` only
+    const uint4* p = F.occ + (size_t)(row >> 6) * OCC_NARROW_U4;
+    Border<FMT> B;
+    B.take(__ldg(p), __ldg(p + 1), off);               // rows before `row` only
+    B.sbi = row >> (6 + SB_BLOCK_SHIFT);
     B.i = row;
+    const uint32_t k = off & 31;
+    const uint32_t c = ((B.z >> k) & 1) ? 0u : 1u + (((B.b0 >> k) & 1) | ((B.b1 >> k) & 1) << 1);
     code = c;
     if (c == 0) {
       rank = border_rank(F, B, 0);
     } else {
-      const uint64_t m = B.low & ((c & 1) ? B.plane(0) : ~B.plane(0)) & ((c & 2) ? B.plane(1) : ~B.plane(1)) &
-                         ((c & 4) ? B.plane(2) : ~B.plane(2));
-      const uint32_t w = c <= 2 ? B.a.x : B.a.y;
-      rank = sb_count(F, B.sbi, c) + (((c - 1) & 1) ? (w >> 16) : (w & 0xFFFFu)) + (uint32_t)__popcll(m);
+      const uint32_t m = B.m & ~B.z & (((c - 1) & 1) ? B.b0 : ~B.b0) & (((c - 1) & 2) ? B.b1 : ~B.b1);
+      const uint32_t w = c <= 2 ? B.c12 : B.c34;
+      rank = sb_count(F, B.sbi, c) + (((c - 1) & 1) ? (w >> 16) : (w & 0xFFFFu)) + (uint32_t)__popc(m) * B.sg;
     }
   }
 }
@@ -303,23 +311,40 @@ __device__ __forceinline__ uint32_t upper_bound_u32(const uint32_t* b, uint32_t 
   return lo;
 }
 
-// The wide record between its form in the device-layout blob (counts before row 0, planes
-// as u64) and its form on the device.
-__global__ void k_wide_records(uint4* __restrict__ occ, uint32_t nblk) {
+// Records from their form in the device-layout blob (counts before row 0, planes of the
+// codes' bits as u64) to their form on the device.
+__global__ void k_device_records(uint4* __restrict__ occ, uint32_t nblk, uint32_t fmt) {
   const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nblk) return;
-  uint4* p = occ + (size_t)b * OCC_WIDE_U4;
-  Border<OCC_WIDE> B;
-  B.a = p[0]; B.b = p[1]; B.c = p[2]; B.d = p[3];
-  const uint4 e = p[4], f = p[5];
-  B.w = make_uint4(e.x, e.z, f.x, f.z);
-  B.m = ~0u; B.sg = 1u;
-  uint32_t r[16];
-  wide_ranks(B, r);
+  if (fmt == OCC_WIDE) {
+    uint4* p = occ + (size_t)b * OCC_WIDE_U4;
+    Border<OCC_WIDE> B;
+    B.a = p[0]; B.b = p[1]; B.c = p[2]; B.d = p[3];
+    const uint4 e = p[4], f = p[5];
+    B.w = make_uint4(e.x, e.z, f.x, f.z);
+    B.m = ~0u; B.sg = 1u;
+    uint32_t r[16];
+    wide_ranks(B, r);
 #pragma unroll
-  for (int k = 0; k < 4; k++) p[k] = make_uint4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
-  p[4] = B.w;
-  p[5] = make_uint4(e.y, e.w, f.y, f.w);
+    for (int k = 0; k < 4; k++) p[k] = make_uint4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
+    p[4] = B.w;
+    p[5] = make_uint4(e.y, e.w, f.y, f.w);
+  } else {
+    uint4* p = occ + (size_t)b * OCC_NARROW_U4;
+    const uint4 u = p[0], v = p[1];       // counts; planes 0, 1, 2 as u64
+    auto half = [](uint32_t p0, uint32_t p1, uint32_t p2, uint32_t& b0, uint32_t& b1, uint32_t& z) {
+      z = ~(p0 | p1 | p2);                // code 1..4 = 001 010 011 100 -> code - 1 = 00 01 10 11
+      b0 = (p1 & ~p0) | p2;
+      b1 = (p1 & p0) | p2;
+    };
+    uint4 x = u, y = v;
+    half(u.z, v.x, v.z, x.z, x.w, y.x);
+    half(u.w, v.y, v.w, y.y, y.z, y.w);
+    const uint32_t n1 = __popc(~x.z & ~x.w & ~y.x), n2 = __popc(x.z & ~x.w), n3 = __popc(~x.z & x.w), n4 = __popc(x.z & x.w);
+    x.x = u.x + (n1 | n2 << 16);
+    x.y = u.y + (n3 | n4 << 16);
+    p[0] = x; p[1] = y;
+  }
 }
 
 }  // namespace hfm

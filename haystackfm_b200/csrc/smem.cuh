@@ -23,7 +23,8 @@
 // Measured on a B200, 256 Mbp ACGT repeat genome, kernel times of the sweep, of this search,
 // and with the k-mer table (DevAux) and short segments for small batches: 1M reads of 150 bp
 // 58.4 / 11.3 / 8.2 ms; 60,000 mixed reads up to 10 kbp 71.2 / 7.7 / 4.7 ms; 250 of them
-// 37.2 / 5.2 / 0.56 ms; find_mems of 20,000 ragged reads 25.9 / 1.9 / 0.9 ms.
+// 37.2 / 5.2 / 0.56 ms; find_mems of 20,000 ragged reads 25.9 / 1.9 / 0.9 ms.  With records
+// that count from row 32 (32-bit masks, half the popcounts): 5.9, 3.5, 0.38 and 0.70 ms.
 //
 // Segments.  A result belongs to the segment of a long read in which it starts.  A segment's
 // search begins at its first position a: if the window there does not match, everything
@@ -78,59 +79,52 @@ struct DevAux {
 // One direction of the index as the step needs it.
 struct FmView { const uint4* occ; const uint32_t* sb; };
 
-// Rows of code s, and of codes s..4, among 64 rows of an ACGT record (codes 0..4; plane 2
-// is set for code 4 alone).
-__device__ __forceinline__ uint64_t acgt_eq(uint32_t s, uint64_t p0, uint64_t p1, uint64_t p2) {
-  const uint64_t x = s == 1 ? p0 & ~p1 : s == 2 ? p1 & ~p0 : p0 & p1;
-  return s == 4 ? p2 : x;
-}
-__device__ __forceinline__ uint64_t acgt_ge(uint32_t s, uint64_t p0, uint64_t p1, uint64_t p2) {
-  const uint64_t x = s == 1 ? p0 | p1 : s == 2 ? p1 : p0 & p1;
-  return s == 4 ? p2 : x | p2;
-}
-__device__ __forceinline__ uint32_t acgt_delta(const uint4& a, uint32_t s) {
-  const uint32_t w = s <= 2 ? a.x : a.y;
-  return (s & 1) ? (w & 0xFFFFu) : (w >> 16);
-}
-// Counts of codes s..4 in the record's deltas.
-__device__ __forceinline__ uint32_t acgt_delta_ge(uint32_t x, uint32_t y, uint32_t s) {
-  uint32_t t = y >> 16;
-  if (s <= 3) t += y & 0xFFFFu;
-  if (s <= 2) t += x >> 16;
-  if (s <= 1) t += x & 0xFFFFu;
-  return t;
-}
-
 // Extends one interval of an ACGT text by one code s (1..4): rows [lo, lo + n) of the
 // extended side become [lo', lo' + n'), `base` (the other side's start) moves past the rows
 // of smaller codes.  The border records are those of the first and the last row, so an
 // interval within 64 rows (every one-row interval) reads one sector.  Returns false, and
 // changes nothing, when no row has the code.
+//
+// Both borders count from row 32 of their records: 4 popcounts of 32 bits (rows of code s,
+// and of the codes from s on, at either border); the masks of s are two words made from its
+// bits, so that one form serves every code.
 template <bool COUNT_TOUCH>
 __device__ __forceinline__ bool acgt_step(const FmView& X, const uint32_t* C, uint32_t s, uint32_t& lo, uint32_t& base,
                                           uint32_t& n, uint64_t& touches) {
-  const uint32_t last = lo + n - 1, bl = lo >> 6, bh = last >> 6;
+  const uint32_t last = lo + n - 1, bl = lo >> 6, bh = last >> 6, sh = 16u * (s - 1u);
   const uint4* pl = X.occ + (size_t)bl * OCC_NARROW_U4;
-  const uint4 a = __ldg(pl), b = __ldg(pl + 1);
-  uint32_t sbl = __ldg(X.sb + (size_t)(bl >> SB_BLOCK_SHIFT) * 16 + s);
-  uint4 a2 = a, b2 = b;
+  const uint4 u = __ldg(pl), v = __ldg(pl + 1);
+  const uint32_t sbl = __ldg(X.sb + (size_t)(bl >> SB_BLOCK_SHIFT) * 16 + s);
+  uint4 u2 = u, v2 = v;
   if (bh != bl) {
     const uint4* ph = X.occ + (size_t)bh * OCC_NARROW_U4;
-    a2 = __ldg(ph); b2 = __ldg(ph + 1);
+    u2 = __ldg(ph); v2 = __ldg(ph + 1);
   }
   if (COUNT_TOUCH) touches += bh != bl ? 2 : 1;
-  const uint64_t ml = (1ull << (lo & 63)) - 1ull, mh = (2ull << (last & 63)) - 1ull;
-  const uint64_t p0 = u2to64(a.z, a.w), p1 = u2to64(b.x, b.y), p2 = u2to64(b.z, b.w);
-  const uint64_t h0 = u2to64(a2.z, a2.w), h1 = u2to64(b2.x, b2.y), h2 = u2to64(b2.z, b2.w);
-  const uint32_t rl = acgt_delta(a, s) + (uint32_t)__popcll(acgt_eq(s, p0, p1, p2) & ml);
-  uint32_t d = acgt_delta(a2, s) + (uint32_t)__popcll(acgt_eq(s, h0, h1, h2) & mh) - rl;
-  uint32_t g = acgt_delta_ge(a2.x, a2.y, s) - acgt_delta_ge(a.x, a.y, s) +
-               (uint32_t)__popcll(acgt_ge(s, h0, h1, h2) & mh) - (uint32_t)__popcll(acgt_ge(s, p0, p1, p2) & ml);
-  if ((bh >> SB_BLOCK_SHIFT) != (bl >> SB_BLOCK_SHIFT)) {
+  Border<OCC_NARROW> L, H;
+  L.take(u, v, lo & 63);
+  H.take(u2, v2, (last & 63) + 1u);
+  const uint32_t k0 = 0u - ((s - 1u) & 1u), k1 = 0u - ((s - 1u) >> 1);      // the bits of code s as masks
+  auto eq = [&](const Border<OCC_NARROW>& B) { return (uint32_t)__popc(B.m & ~B.z & ~((B.b0 ^ k0) | (B.b1 ^ k1))) * B.sg; };
+  auto ge = [&](const Border<OCC_NARROW>& B) {
+    return (uint32_t)__popc(B.m & ~B.z & ((B.b1 & ~k1) | (~(B.b1 ^ k1) & (B.b0 | ~k0)))) * B.sg;
+  };
+  auto count = [&](const Border<OCC_NARROW>& B) {
+    return (uint32_t)((((uint64_t)B.c34 << 32) | B.c12) >> sh) & 0xFFFFu;
+  };
+  const uint32_t rl = count(L) + eq(L);
+  uint32_t d = count(H) + eq(H) - rl;
+  // codes from s on: the records' counts differ by u16 fields that never borrow within a
+  // superblock
+  const uint64_t df = ((((uint64_t)H.c34 << 32) | H.c12) - (((uint64_t)L.c34 << 32) | L.c12)) >> sh;
+  uint32_t g = ge(H) - ge(L);
+  if ((bh >> SB_BLOCK_SHIFT) == (bl >> SB_BLOCK_SHIFT)) {
+    g += (uint32_t)(df & 0xFFFFu) + (uint32_t)(df >> 16 & 0xFFFFu) + (uint32_t)(df >> 32 & 0xFFFFu) + (uint32_t)(df >> 48);
+  } else {
     const uint32_t* q = X.sb + (size_t)(bl >> SB_BLOCK_SHIFT) * 16;
     const uint32_t* r = X.sb + (size_t)(bh >> SB_BLOCK_SHIFT) * 16;
     d += __ldg(r + s) - sbl;
-    for (uint32_t t = s; t <= 4; t++) g += __ldg(r + t) - __ldg(q + t);
+    for (uint32_t t = s; t <= 4; t++) g += __ldg(r + t) - __ldg(q + t) + H.delta((int)t) - L.delta((int)t);
   }
   if (!d) return false;
   base += n - g;

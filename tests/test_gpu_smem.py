@@ -114,18 +114,21 @@ def test_layout_blob_keeps_its_form(oracle, kind):
     again = _Handle.from_layout(blob)
     assert again.export_layout() == blob
     o = oracle.OracleIndex(b, KIND_BIDIR)
-    if kind != "acgt":
-        arr = np.frombuffer(blob, np.uint8)
-        n = o.text_len
-        nblk = (n + 63) // 64
-        # 16-byte head, DevFm, 8 scalars, bounds, 7 sizes, then the Occ records
-        nb = len(_header_fields(b, 4)[2])
-        at = blob.index(np.uint64(nblk * 96).tobytes(), 16)
-        rec = arr[at + 56:at + 56 + nblk * 96].reshape(nblk, 96)
-        counts = rec[:, :64].copy().view(np.uint32)
-        for blk in (0, 1, nblk // 2, nblk - 1):
+    arr = np.frombuffer(blob, np.uint8)
+    size = 32 if kind == "acgt" else 96
+    nblk = (o.text_len + 63) // 64
+    # the seven buffer sizes (the Occ records' first), then the records
+    at = blob.index(np.uint64(nblk * size).tobytes(), 16)
+    rec = arr[at + 56:at + 56 + nblk * size].reshape(nblk, size)
+    for blk in (0, 1, nblk // 2, nblk - 1):
+        if kind == "acgt":               # u16 counts of codes 1..4 from the superblock's start
+            counts = rec[blk, :8].copy().view(np.uint16)
+            first = blk // 1024 * 65536
+            for c in (1, 2, 3, 4):
+                assert counts[c - 1] == o.rank(c, blk * 64) - o.rank(c, first)
+        else:                            # u32 counts of every code
+            counts = rec[blk, :64].copy().view(np.uint32)
             for c in (0, 1, 4, 5, 9):
-                assert counts[blk, c] == o.rank(c, blk * 64)
-        assert nb >= 1
+                assert counts[c] == o.rank(c, blk * 64)
     reads = list(synth.sample_reads(ref, n_reads=50, read_len=100, seed=11))
     _check(oracle, b, again, reads, 19, 0)
