@@ -118,8 +118,10 @@ using namespace hfm;
 struct hfm_index {
   int device = 0, kind = 0;
   FmDev fwd, rev;
-  DevAux aux{};                   // ACGT texts, bidirectional: what the SMEM search keeps besides the records
-  DevBuf aux_kmer;                // (owned by the handle that loaded the index, like its records)
+  // made on the device when the index is loaded, owned by that handle like the records
+  DevAux aux{};                   // ACGT texts, bidirectional: the SMEM search's k-mer table
+  const uint32_t* sa = nullptr;   // position of every forward row (resolve.cuh)
+  DevBuf aux_kmer, aux_sa;
   cudaStream_t stream = nullptr;
   std::mutex mu;
   bool count_work = false;
@@ -284,7 +286,7 @@ static int build_device_fm(const HostFm& h, FmDev& f, cudaStream_t s) {
 // 9.0 / 9.8 / 15.1, 60,000 mixed reads 6.0 / 6.0 / 6.6 / 11.2: one step less is worth no more
 // than the table's larger reach into memory from 11 on.)
 static constexpr uint32_t KMER_MAX = 11;
-static int build_aux(hfm_index* x) {
+static int build_kmer(hfm_index* x) {
   const FmDev& f = x->fwd;
   if (x->kind != HFM_KIND_BIDIR || f.fmt != OCC_NARROW) return HFM_OK;
   uint32_t k = 0;
@@ -309,6 +311,20 @@ static int build_aux(hfm_index* x) {
   CK(e);
   x->aux.kmer = x->aux_kmer.as<uint4>();
   x->aux.k = k;
+  return HFM_OK;
+}
+
+// The position of every row of the forward index (k_sa_rows).
+static int build_sa(hfm_index* x) {
+  const FmDev& f = x->fwd;
+  if (f.rate < 1 || f.rate > SA_ROWS_RATE || f.d.num_seqs > f.text_len || !f.text_len) return HFM_OK;
+  if (x->aux_sa.ensure((size_t)f.text_len * 4) != HFM_OK) return HFM_OK;
+  CK(cudaMemsetAsync(x->aux_sa.p, 0xFF, (size_t)f.text_len * 4, x->stream));
+  const uint64_t items = (uint64_t)f.d.num_blocks + f.d.num_seqs;
+  WITH_FMT(f.fmt, { k_sa_rows<FM><<<(unsigned)((items + 127) / 128), 128, 0, x->stream>>>(f.d, x->aux_sa.as<uint32_t>()); });
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(x->stream));
+  x->sa = x->aux_sa.as<uint32_t>();
   return HFM_OK;
 }
 
@@ -469,7 +485,8 @@ static int resolve(hfm_index* x, const FmDev& F, const uint32_t* seg_row, uint32
                                                                      x->blockmap.as<uint32_t>());
   other++;
   ResolveArgs A{seg_row, stride, seg_off, (uint32_t)nseg, total, d_bounds, nb,
-                F.rate ? F.rate : F.text_len, out, &dctr(x)->walk_err, &dctr(x)->steps, x->blockmap.as<uint32_t>()};
+                F.rate ? F.rate : F.text_len, out, &dctr(x)->walk_err, &dctr(x)->steps, x->blockmap.as<uint32_t>(), nullptr,
+                x->sa};
   // grid.x limit 2^31-1 blocks covers 5e11 positions
   cudaEventRecord(x->evk[2], x->stream);
   if (x->count_work) k_resolve<true><<<(unsigned)blocks, RES_T, 0, x->stream>>>(F.d, A);
@@ -1269,7 +1286,7 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
                                                                           x->blockmap.as<uint32_t>(),
                                                                           (upcap + RES_T - 1) / RES_T);
       ResolveArgs A{x->urow.as<uint32_t>(), 1, x->uoff.as<uint64_t>(), (uint32_t)hcap, upcap, d_bounds, c.nb, guard,
-                    x->uout.as<uint32_t>(), &dc->walk_err, &dc->steps, x->blockmap.as<uint32_t>(), &c.d_tot->upos};
+                    x->uout.as<uint32_t>(), &dc->walk_err, &dc->steps, x->blockmap.as<uint32_t>(), &c.d_tot->upos, x->sa};
       k_resolve<false><<<(unsigned)((upcap + RES_T - 1) / RES_T), RES_T, 0, x->stream>>>(Fw.d, A);
       k_block_first<<<(unsigned)((hcap + 255) / 256), 256, 0, x->stream>>>(seg_off, (uint32_t)hcap, EXP_BLK,
                                                                           x->blockmap2.as<uint32_t>(), eblocks);
@@ -1284,7 +1301,7 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
     k_block_first<<<(unsigned)((hcap + 255) / 256), 256, 0, x->stream>>>(seg_off, (uint32_t)hcap, RES_T,
                                                                         x->blockmap.as<uint32_t>(), rblocks);
     ResolveArgs A{seg_row, 8, seg_off, (uint32_t)hcap, pcap, d_bounds, c.nb, guard, x->out_pairs.as<uint32_t>(),
-                  &dc->walk_err, &dc->steps, x->blockmap.as<uint32_t>(), &c.d_tot->npos};
+                  &dc->walk_err, &dc->steps, x->blockmap.as<uint32_t>(), &c.d_tot->npos, x->sa};
     k_resolve<false><<<(unsigned)((pcap + RES_T - 1) / RES_T), RES_T, 0, x->stream>>>(Fw.d, A);
     CK(cudaGetLastError());
   }
@@ -1410,7 +1427,7 @@ static int fixed_locate(hfm_index* x, FixedLocate& c, bool launch) {
                                                                           x->blockmap.as<uint32_t>(),
                                                                           (upcap + RES_T - 1) / RES_T);
       ResolveArgs A{x->urow.as<uint32_t>(), 1, x->uoff.as<uint64_t>(), (uint32_t)icap, upcap, d_bounds, nb, guard,
-                    x->uout.as<uint32_t>(), &dc->walk_err, &dc->steps, x->blockmap.as<uint32_t>(), &c.d_tot->upos};
+                    x->uout.as<uint32_t>(), &dc->walk_err, &dc->steps, x->blockmap.as<uint32_t>(), &c.d_tot->upos, x->sa};
       k_resolve<false><<<(unsigned)((upcap + RES_T - 1) / RES_T), RES_T, 0, x->stream>>>(F.d, A);
       k_block_first<<<(unsigned)((icap + 255) / 256), 256, 0, x->stream>>>(seg_off, (uint32_t)icap, EXP_BLK,
                                                                           x->blockmap2.as<uint32_t>(), eblocks);
@@ -1425,7 +1442,7 @@ static int fixed_locate(hfm_index* x, FixedLocate& c, bool launch) {
     k_block_first<<<(unsigned)((icap + 255) / 256), 256, 0, x->stream>>>(seg_off, (uint32_t)icap, RES_T,
                                                                         x->blockmap.as<uint32_t>(), rblocks);
     ResolveArgs A{seg_row, 1, seg_off, (uint32_t)icap, pcap, d_bounds, nb, guard, x->loc_pairs.as<uint32_t>(),
-                  &dc->walk_err, &dc->steps, x->blockmap.as<uint32_t>(), &c.d_tot->npos};
+                  &dc->walk_err, &dc->steps, x->blockmap.as<uint32_t>(), &c.d_tot->npos, x->sa};
     k_resolve<false><<<(unsigned)((pcap + RES_T - 1) / RES_T), RES_T, 0, x->stream>>>(F.d, A);
     CK(cudaGetLastError());
   }
@@ -1513,7 +1530,7 @@ static int make_shadow(hfm_index* x, hfm_index** out) {
   sh->queue_chunk = x->queue_chunk; sh->threads_per_read = x->threads_per_read; sh->read_order = x->read_order;
   sh->timeout_ms = x->timeout_ms;
   sh->shared_index = true;
-  sh->aux = x->aux;
+  sh->aux = x->aux; sh->sa = x->sa;
   for (int k = 0; k < 2; k++) {
     const FmDev& src = k ? x->rev : x->fwd;
     FmDev& dst = k ? sh->rev : sh->fwd;
@@ -1578,7 +1595,8 @@ int hfm_index_load(const uint8_t* bytes, size_t len, int kind, const hfm_opts* o
   RET(x->ctr.ensure(sizeof(Counters)));
   RET(build_device_fm(hf, x->fwd, x->stream));
   if (kind == HFM_KIND_BIDIR) RET(build_device_fm(hr, x->rev, x->stream));
-  RET(build_aux(x.get()));
+  RET(build_kmer(x.get()));
+  RET(build_sa(x.get()));
   *out = x.release();
   return HFM_OK;
 }
@@ -1759,7 +1777,8 @@ int hfm_index_load_layout(const uint8_t* bytes, uint64_t len, const hfm_opts* op
     f.seq_boundaries = D.bnd;
   }
   CK(cudaStreamSynchronize(x->stream));
-  RET(build_aux(x.get()));
+  RET(build_kmer(x.get()));
+  RET(build_sa(x.get()));
   *out = x.release();
   return HFM_OK;
 }
@@ -1780,7 +1799,7 @@ int hfm_index_device_bytes(const hfm_index* x, uint64_t* index_bytes, uint64_t* 
   uint64_t a = 0, b = 0;
   if (!x->shared_index) {
     for (const DevBuf* d : idx_bufs) a += d->cap;
-    a += x->aux_kmer.cap;
+    a += x->aux_kmer.cap + x->aux_sa.cap;
   }
   for (const DevBuf* d : work_bufs) b += d->cap;
   if (index_bytes) *index_bytes = a;
@@ -1806,7 +1825,7 @@ void hfm_index_free(hfm_index* x) {
                     &x->blockmap, &x->blockmap2, &x->ovf2, &x->ovf3, &x->lflag, &x->lpos, &x->sids, &x->lids,
                     &x->ucount, &x->ubase, &x->uread, &x->uk, &x->nslot, &x->slot_base, &x->slot_hits, &x->npos,
                     &x->iota, &x->loc_pairs, &x->okeys, &x->oids, &x->otemp, &x->trie_nodes, &x->trie_left,
-                    &x->trie_resume, &x->aux_kmer})
+                    &x->trie_resume, &x->aux_kmer, &x->aux_sa})
     b->release();
   for (auto& e : x->ev) if (e) cudaEventDestroy(e);
   for (auto& e : x->evk) if (e) cudaEventDestroy(e);
@@ -1821,7 +1840,7 @@ int hfm_index_info_get(const hfm_index* x, hfm_index_info* o) {
   o->kind = x->kind; o->text_len = x->fwd.text_len; o->num_sequences = x->fwd.num_seqs;
   o->sample_rate = x->fwd.rate; o->lookup_depth = x->fwd.lookup_depth; o->alphabet_tag = x->fwd.tag;
   o->num_lanes = x->fwd.num_lanes; o->encoding = x->fwd.encoding;
-  o->device_bytes = x->fwd.bytes() + x->rev.bytes() + x->aux_kmer.cap;
+  o->device_bytes = x->fwd.bytes() + x->rev.bytes() + x->aux_kmer.cap + x->aux_sa.cap;
   return HFM_OK;
 }
 
