@@ -29,6 +29,7 @@
 #include "search.cuh"
 #include "smem.cuh"
 #include "trie.cuh"
+#include "acgt.cuh"
 
 namespace hfm {
 
@@ -98,8 +99,8 @@ struct DevBuf {
 };
 
 struct Counters {                    // device-side counters, one block per handle
-  unsigned long long iv_used, hit_used, touches, steps, n_units;
-  uint32_t n_ovf, still_ovf, walk_err, queue, queue2, n_mid, n_wrp, queue3, n_long, trie_queue, n_left, seg_len;
+  unsigned long long iv_used, hit_used, touches, steps, n_units, bases;
+  uint32_t n_ovf, still_ovf, walk_err, queue, queue2, n_mid, n_wrp, queue3, n_long, trie_queue, n_left, seg_len, queue4, _pad;
 };
 
 struct FmDev {
@@ -119,9 +120,9 @@ struct hfm_index {
   int device = 0, kind = 0;
   FmDev fwd, rev;
   // made on the device when the index is loaded, owned by that handle like the records
-  DevAux aux{};                   // ACGT texts, bidirectional: the SMEM search's k-mer table
+  DevAux aux{};                   // ACGT texts, bidirectional: for the SMEM search
   const uint32_t* sa = nullptr;   // position of every forward row (resolve.cuh)
-  DevBuf aux_kmer, aux_sa;
+  DevBuf aux_kmer, aux_sa, aux_text, aux_seen;
   cudaStream_t stream = nullptr;
   std::mutex mu;
   bool count_work = false;
@@ -130,7 +131,7 @@ struct hfm_index {
       scan_tmp, out_pairs, ref_bounds, hit_start, hit_count, hit_base, hits, npos_scan, work, cwork, ctr,
       mivpool, bswork, memwork, hkeys, hslot, hflags, huid, urow, ulen, uoff, uout, blockmap, blockmap2, ovf2, ovf3,
       lflag, lpos, sids, lids, ucount, ubase, uread, uk, nslot, slot_base, slot_hits, npos, loc_pairs, okeys, oids,
-      otemp, trie_nodes, trie_left, trie_resume;
+      otemp, trie_nodes, trie_left, trie_resume, left_jobs, pack_words, pack_anchors;
   uint32_t flags = 0;
   uint32_t seg_len = 512;  // SMEM reads longer than 2 * seg_len take the segmented sweep
   uint32_t queue_chunk = 1;       // reads a per-thread kernel takes from its queue per atomic
@@ -281,16 +282,15 @@ static int build_device_fm(const HostFm& h, FmDev& f, cudaStream_t s) {
 }
 
 // The k-mer table of an ACGT index (DevAux): k at most KMER_MAX, and the table (16 bytes an
-// entry) no larger than a byte per text position.  Without the memory for it the search does
-// without it.  (k 12 / 11 / 10 / none, SMEM search ms on 256 Mbp: 1M reads of 150 bp 9.0 /
-// 9.0 / 9.8 / 15.1, 60,000 mixed reads 6.0 / 6.0 / 6.6 / 11.2: one step less is worth no more
-// than the table's larger reach into memory from 11 on.)
-static constexpr uint32_t KMER_MAX = 11;
+// entry) at most two bytes per text position.  Without the memory for it the search does
+// without it.  (k 13 / 12 / 11, search of 1M reads of 150 bp on 256 Mbp: 4.2 / 4.2 / 4.35 ms,
+// of 60,000 mixed reads 1.93 / 1.96 / 2.00; none at all: 1.7 times as long.)
+static constexpr uint32_t KMER_MAX = 13;
 static int build_kmer(hfm_index* x) {
   const FmDev& f = x->fwd;
   if (x->kind != HFM_KIND_BIDIR || f.fmt != OCC_NARROW) return HFM_OK;
   uint32_t k = 0;
-  while (k < KMER_MAX && (16ull << (2 * (k + 1))) <= f.text_len) k++;
+  while (k < KMER_MAX && (16ull << (2 * (k + 1))) <= 2ull * f.text_len) k++;
   if (k < 2) return HFM_OK;
   DevBuf tmp;
   if (x->aux_kmer.ensure(16ull << (2 * k)) != HFM_OK || tmp.ensure(16ull << (2 * (k - 1))) != HFM_OK) {
@@ -302,7 +302,7 @@ static int build_kmer(hfm_index* x) {
   for (uint32_t l = 0; l < k; l++) {
     uint4* out = ((k - l) & 1) ? x->aux_kmer.as<uint4>() : tmp.as<uint4>();
     const uint64_t entries = 1ull << (2 * (l + 1));
-    k_kmer_table<<<(unsigned)((entries + 255) / 256), 256, 0, x->stream>>>(f.d, in, l, out);
+    k_kmer_table<<<(unsigned)((entries + 255) / 256), 256, 0, x->stream>>>(f.d, in, l, l + 1 == k, out);
     in = out;
   }
   cudaError_t e = cudaGetLastError();
@@ -314,18 +314,56 @@ static int build_kmer(hfm_index* x) {
   return HFM_OK;
 }
 
-// The position of every row of the forward index (k_sa_rows).
+// The position of every row of the forward index (k_sa_rows), and what the SMEM search of an
+// ACGT text keeps with it.
+static constexpr uint32_t SEEN_K_MAX = 18;      // 8 GB of bits, for texts near 2^32
 static int build_sa(hfm_index* x) {
   const FmDev& f = x->fwd;
   if (f.rate < 1 || f.rate > SA_ROWS_RATE || f.d.num_seqs > f.text_len || !f.text_len) return HFM_OK;
-  if (x->aux_sa.ensure((size_t)f.text_len * 4) != HFM_OK) return HFM_OK;
+  if (x->aux_sa.ensure((size_t)f.text_len * 4 + 16) != HFM_OK) return HFM_OK;    // read 16 bytes at a time
   CK(cudaMemsetAsync(x->aux_sa.p, 0xFF, (size_t)f.text_len * 4, x->stream));
   const uint64_t items = (uint64_t)f.d.num_blocks + f.d.num_seqs;
   WITH_FMT(f.fmt, { k_sa_rows<FM><<<(unsigned)((items + 127) / 128), 128, 0, x->stream>>>(f.d, x->aux_sa.as<uint32_t>()); });
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(x->stream));
   x->sa = x->aux_sa.as<uint32_t>();
-  return HFM_OK;
+  if (x->kind != HFM_KIND_BIDIR || f.fmt != OCC_NARROW) return HFM_OK;
+  // the text, for the SMEM search of ACGT texts; not kept when a row has no position (an
+  // inconsistent index)
+  const uint64_t n = f.text_len, words = n / 32 + 2;
+  DevBuf bytes;
+  if (bytes.ensure(n) != HFM_OK) return HFM_OK;
+  if (x->aux_text.ensure(words * 16) != HFM_OK) { bytes.release(); return HFM_OK; }
+  auto run = [&]() -> int {
+    uint32_t* unknown = &x->ctr.as<Counters>()->walk_err;
+    CK(cudaMemsetAsync(unknown, 0, 4, x->stream));
+    CK(cudaMemsetAsync(bytes.p, 0, n, x->stream));
+    const unsigned grid = (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)x->num_sms * 32);
+    k_text_bytes<<<grid, 256, 0, x->stream>>>(f.d, x->sa, bytes.as<uint8_t>(), unknown);
+    k_text_planes<<<grid, 256, 0, x->stream>>>(bytes.as<uint8_t>(), n, words, x->aux_text.as<uint4>());
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(&x->h_ctr->walk_err, unknown, 4, cudaMemcpyDeviceToHost, x->stream));
+    CK(cudaStreamSynchronize(x->stream));
+    if (x->h_ctr->walk_err) { x->aux_text.release(); return HFM_OK; }
+    x->aux.sa = x->sa;
+    x->aux.text = x->aux_text.as<uint4>();
+    // one bit per string of seen_k codes, 4 to 16 bits per text position
+    uint32_t k = 3;
+    while ((1ull << (2 * k)) < 4ull * n) k++;
+    const uint64_t seen_bytes = (1ull << (2 * k)) / 8;
+    if (k > SEEN_K_MAX || x->aux_seen.ensure(seen_bytes) != HFM_OK) return HFM_OK;
+    CK(cudaMemsetAsync(x->aux_seen.p, 0, seen_bytes, x->stream));
+    k_seen_bits<<<(unsigned)((n + 8191) / 8192), 256, 0, x->stream>>>(bytes.as<uint8_t>(), (uint32_t)n, k,
+                                                                     x->aux_seen.as<uint32_t>());
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(x->stream));
+    x->aux.seen = x->aux_seen.as<uint32_t>();
+    x->aux.seen_k = k;
+    return HFM_OK;
+  };
+  const int rc = run();
+  bytes.release();
+  return rc;
 }
 
 // ---------------------------------------------------------------------------
@@ -391,6 +429,7 @@ static constexpr uint32_t MID_HIT_CAP = 1024;  // hit list of the per-thread rer
 static constexpr uint32_t MID_THREADS_PER_SM = 256;
 static constexpr uint32_t FAST_HIT_CAP = 1024;   // hit list of fast-pass variant 3 (global memory)
 static constexpr uint64_t MEM_SET_BYTES = 2ull * MEM_SET_CAP * 12;   // the two interval sets of a thread
+static constexpr int ACGT_BLOCKS = 8;            // resident blocks per SM that k_acgt is compiled for
 static constexpr int MEMS_PLAIN = 4;             // mems_variant of the plain one-thread-per-read launch
 
 // Backward search for a batch.  with_ivs = false: counts only.
@@ -675,6 +714,33 @@ static int trie_plan(hfm_index* x, uint32_t nq, uint32_t& blocks, uint32_t& grou
   RET(x->trie_resume.ensure((size_t)nq * 4 + 4));
   return HFM_OK;
 }
+// Packs the reads of a batch for k_acgt (k_acgt_pack): `bases` codes in nq reads.  launch =
+// false makes the allocations only (a graph capture's sizing pass).
+static int pack_reads(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff, uint32_t nq, uint64_t bases, uint32_t min_len,
+                      const SmemJobs& J, uint64_t max_jobs, bool counting, PackedReads& R, bool launch = true) {
+  const DevAux& A = x->aux;
+  R = PackedReads{};
+  RET(x->pack_words.ensure((bases / 32 + nq + 1) * 16));
+  R.words = x->pack_words.as<uint4>();
+  if (A.seen && A.seen_k <= min_len) {
+    R.seen_k = A.seen_k;
+    R.stride = min_len - A.seen_k + 1;
+    const uint64_t bytes = (bases / (32ull * R.stride) + nq + 1) * 4;
+    RET(x->pack_anchors.ensure(bytes));
+    R.anchors = x->pack_anchors.as<uint32_t>();
+    if (launch) CK(cudaMemsetAsync(R.anchors, 0, bytes, x->stream));
+  }
+  if (!launch || !max_jobs) return HFM_OK;
+  const unsigned grid = (unsigned)std::min<uint64_t>((max_jobs + 7) / 8, (uint64_t)x->num_sms * 8 * 4);
+  auto go = [&](auto kern) {
+    kern<<<grid, 256, 0, x->stream>>>(x->fwd.compat.as<uint16_t>(), x->fwd.d.sym_mask, d_q, d_qoff, J, A, R,
+                                      &dctr(x)->touches);
+  };
+  if (counting) go(k_acgt_pack<true>); else go(k_acgt_pack<false>);
+  CK(cudaGetLastError());
+  return HFM_OK;
+}
+
 static constexpr uint32_t TRIE_SORT_GROUP = 4;   // groups of this many reads or more are formed by prefix
 
 static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff, uint32_t nq, uint32_t min_len,
@@ -736,16 +802,14 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
   int variant = x->mems_variant;
   int bpsm = 0;
   const uint32_t fmt = Fw.fmt;
-  WITH_FMT(fmt, {
-    if (variant == 2) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_smem<false, 32, MEM_KC, 8, FM>, 128, 0));
-    else CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_smem<false, 32, 0, 8, FM>, 128, 0));
-  });
+  if (fmt == OCC_NARROW) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_acgt<false, 0, ACGT_BLOCKS>, 128, 0));
+  else CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_smem<false, 32, 0, 8, OCC_WIDE>, 128, 0));
   const uint64_t full_threads = (uint64_t)std::max(1, bpsm) * x->num_sms * 128;
   // Reads longer than 2 * seg_len (variant 3) are searched as segments; the fast pass gets
   // the other reads whole, in the same relative order.
   const uint32_t* fast_ids = order ? order + n_warp : nullptr;
   uint32_t n_fast = nq - n_warp, n_long = 0;
-  uint64_t n_units = 0, n_slots = nq;
+  uint64_t n_units = 0, n_slots = nq, bases = 0;
   uint32_t seg_len = x->seg_len;
   const uint64_t* slot_base = nullptr;
   if (variant == 3 && n_fast > 0 && min_len > 0) {
@@ -756,13 +820,14 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
     k_long_reads<<<(n_fast + 255) / 256, 256, 0, x->stream>>>(fast_ids, n_fast, d_qoff, nq, x->seg_len,
                                                               fmt == OCC_NARROW ? full_threads : 0, x->lflag.as<uint32_t>(),
                                                               x->nslot.as<uint32_t>(), &dctr(x)->n_long, &dctr(x)->n_units,
-                                                              &dctr(x)->seg_len);
+                                                              &dctr(x)->seg_len, &dctr(x)->bases);
     other++;
     CK(cudaGetLastError());
     RET(read_ctr(x));
     n_long = x->h_ctr->n_long;
     n_units = x->h_ctr->n_units;
     seg_len = x->h_ctr->seg_len;
+    bases = x->h_ctr->bases;
     if (n_long) {
       RET(x->lpos.ensure(((size_t)n_fast + 1) * 8));
       RET(x->sids.ensure((size_t)n_fast * 4 + 4));
@@ -791,12 +856,26 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       if (n_slots >= 0xFFFFFFFFull) return set_error(HFM_E_ARG, "too many read segments in one call");
     }
   }
-  const uint64_t threads = std::min<uint64_t>(full_threads, (n_units + n_fast + 127) / 128 * 128);
+  if (!bases && fmt == OCC_NARROW && variant != MEMS_PLAIN && n_fast) {      // not counted above
+    uint64_t from = 0;
+    RET(read_u64(x, d_qoff, from));
+    RET(read_u64(x, d_qoff + nq, bases));
+    bases -= from;
+  }
+  // A small batch is spread over all resident warps, with a job on a few lanes of each
+  // (k_acgt): a warp runs the code of every phase that one of its lanes is in.
+  uint32_t lanes = 32;
+  uint64_t threads = std::min<uint64_t>(full_threads, (n_units + n_fast + 127) / 128 * 128);
+  if (fmt == OCC_NARROW) {
+    lanes = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, ((n_units + n_fast) * 32 + full_threads - 1) / full_threads));
+    threads = std::min<uint64_t>(full_threads, ((n_units + n_fast + lanes - 1) / lanes + 3) / 4 * 128);
+  }
   RET(x->hit_start.ensure(n_slots * 8 + 8)); RET(x->hit_count.ensure(n_slots * 4 + 4));
   const bool plain = variant == MEMS_PLAIN;
   if (plain && (order || n_warp)) return set_error(HFM_E_ARG, "the plain launch takes no schedule");
   if (!plain) {
-    RET(x->memwork.ensure(std::max<uint64_t>(threads, 128) * MEM_SET_BYTES));
+    if (fmt == OCC_WIDE) RET(x->memwork.ensure(std::max<uint64_t>(threads, 128) * MEM_SET_BYTES));
+    else RET(x->left_jobs.ensure((n_units + n_fast) * 4 + 4));
     if (variant == 3) RET(x->cwork.ensure((size_t)std::max<uint64_t>(threads, 128) * FAST_HIT_CAP * 32));
   } else if (nq) {
     // plain launch, count pass: every read's MemHits and positions counted by a full
@@ -870,7 +949,6 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       J.unit_read = x->uread.as<uint32_t>(); J.unit_k = x->uk.as<uint32_t>(); J.seg_len = seg_len;
       J.n_units = (uint32_t)n_units; J.ids = fast_ids; J.n_ids = n_fast; J.slot_base = slot_base;
       const unsigned grid = (unsigned)(threads / 128);
-      if (x->memwork.cap < (size_t)grid * 128 * MEM_SET_BYTES) return set_error(HFM_E_ARG, "internal: work area too small");
       if (variant == 3 && x->cwork.cap < (size_t)grid * 128 * FAST_HIT_CAP * 32)
         return set_error(HFM_E_ARG, "internal: hit list area too small");
       if (trie && n_fast > 0) {
@@ -885,16 +963,47 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
         CK(cudaGetLastError());
         J.ids = T.left; J.n_ids_dev = T.n_left; J.resume = T.resume;
       }
-      WITH_FMT(fmt, {
+      if (fmt == OCC_NARROW) {
+        PackedReads R;
+        RET(pack_reads(x, d_q, d_qoff, nq, bases, min_len, J, n_units + n_fast, counting, R));
+        launches++;
+        auto go = [&](auto kern) {
+          kern<<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, d_qoff, P, hp, o, W, J, x->aux, R, lanes,
+                                            x->left_jobs.as<uint32_t>(), &dctr(x)->n_left);
+        };
+        if (variant == 3) { if (counting) go(k_acgt<true, 0, 5>); else go(k_acgt<false, 0, ACGT_BLOCKS>); }
+        else { if (counting) go(k_acgt<true, MEM_KC, 5>); else go(k_acgt<false, MEM_KC, ACGT_BLOCKS>); }
+        launches++;
+        CK(cudaGetLastError());
+        if (Fw.tag != 1) {                    // IUPAC queries: jobs with codes of several symbols
+          RET(read_ctr(x));
+          if (x->h_ctr->n_left) {
+            const unsigned g2 = (unsigned)std::min<uint64_t>(grid, ((uint64_t)x->h_ctr->n_left + 127) / 128);
+            RET(x->memwork.ensure((size_t)g2 * 128 * MEM_SET_BYTES));
+            W.sets = x->memwork.as<BIv>();
+            W.queue = &dctr(x)->queue3;
+            J.jobs = x->left_jobs.as<uint32_t>(); J.n_jobs = x->h_ctr->n_left;
+            auto rest = [&](auto kern) {
+              kern<<<g2, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(), Rv.compat.as<uint16_t>(), d_q, d_qoff, P,
+                                              hp, o, W, J, x->aux);
+            };
+            if (variant == 3) { if (counting) rest(k_smem<true, 32, 0, 5, OCC_NARROW>); else rest(k_smem<false, 32, 0, 8, OCC_NARROW>); }
+            else { if (counting) rest(k_smem<true, 32, MEM_KC, 5, OCC_NARROW>); else rest(k_smem<false, 32, MEM_KC, 8, OCC_NARROW>); }
+            launches++;
+            CK(cudaGetLastError());
+          }
+        }
+      } else {
+        if (x->memwork.cap < (size_t)grid * 128 * MEM_SET_BYTES) return set_error(HFM_E_ARG, "internal: work area too small");
         auto go = [&](auto kern) {
           kern<<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, Fw.compat.as<uint16_t>(), Rv.compat.as<uint16_t>(), d_q, d_qoff, P,
                                             hp, o, W, J, x->aux);
         };
-        if (variant == 3) { if (counting) go(k_smem<true, 32, 0, 5, FM>); else go(k_smem<false, 32, 0, 8, FM>); }
-        else { if (counting) go(k_smem<true, 32, MEM_KC, 5, FM>); else go(k_smem<false, 32, MEM_KC, 8, FM>); }
-      });
-      launches++;
-      CK(cudaGetLastError());
+        if (variant == 3) { if (counting) go(k_smem<true, 32, 0, 5, OCC_WIDE>); else go(k_smem<false, 32, 0, 8, OCC_WIDE>); }
+        else { if (counting) go(k_smem<true, 32, MEM_KC, 5, OCC_WIDE>); else go(k_smem<false, 32, MEM_KC, 8, OCC_WIDE>); }
+        launches++;
+        CK(cudaGetLastError());
+      }
     }
     if (!plain && (n_fast > 0 || n_long > 0)) {
       cudaEventRecord(x->evk[1], x->stream);
@@ -923,11 +1032,11 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
                                           threads / 128 * 128});
         tm = std::max<uint64_t>(tm, 128);
         unsigned grid = (unsigned)(tm / 128);
-        if (x->memwork.cap < (size_t)grid * 128 * MEM_SET_BYTES) return set_error(HFM_E_ARG, "internal: work area too small");
+        RET(x->memwork.ensure((size_t)grid * 128 * MEM_SET_BYTES));
         RET(x->cwork.ensure((size_t)grid * 128 * MID_HIT_CAP * 32));
         MemsWork W{};
         W.sets = x->memwork.as<BIv>(); W.set_cap = MEM_SET_CAP; W.hits = x->cwork.as<uint4>(); W.hit_cap = MID_HIT_CAP;
-        W.queue = &dctr(x)->queue3; W.still_ovf = &dctr(x)->still_ovf; W.work_log = wlog;
+        W.queue = &dctr(x)->queue4; W.still_ovf = &dctr(x)->still_ovf; W.work_log = wlog;
         SmemJobs J{};
         J.ids = x->ovf3.as<uint32_t>(); J.n_ids = n_mid; J.slot_base = slot_base;
         CK(cudaMemsetAsync(x->status.p, 0, (size_t)nq * 4, x->stream));
@@ -1135,13 +1244,18 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
   RET(x->mivpool.ensure(x->miv_cap * 16)); RET(x->hitpool.ensure(hcap * 32));
   if (!launch) {                     // occupancy queried outside the capture
     int bpsm = 0;
-    WITH_FMT(fmt, { CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_smem<false, 32, 0, 8, FM>, 128, 0)); });
+    if (fmt == OCC_NARROW) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_acgt<false, 0, ACGT_BLOCKS>, 128, 0));
+    else CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_smem<false, 32, 0, 8, OCC_WIDE>, 128, 0));
     c.threads = (uint64_t)std::max(1, bpsm) * x->num_sms * 128;
     c.trie = fmt == OCC_WIDE && x->mems_variant == 3 && x->threads_per_read == 1 && seg;
     if (c.trie) RET(trie_plan(x, nq, c.tblocks, c.tgroup));
   }
   const uint64_t threads = c.threads;
-  RET(x->memwork.ensure(threads * MEM_SET_BYTES));
+  if (fmt == OCC_WIDE || Fw.tag != 1) RET(x->memwork.ensure(threads * MEM_SET_BYTES));
+  RET(x->left_jobs.ensure(scap * 4 + 4));
+  PackedReads R;
+  if (fmt == OCC_NARROW)
+    RET(pack_reads(x, c.d_q, c.d_qoff, nq, c.max_bases, c.P.min_len, SmemJobs{}, 0, false, R, false));
   if (seg) {
     RET(x->lflag.ensure((size_t)nq * 4 + 4)); RET(x->lpos.ensure(((size_t)nq + 1) * 8));
     RET(x->sids.ensure((size_t)nq * 4 + 4)); RET(x->lids.ensure((size_t)nq * 4 + 4));
@@ -1191,7 +1305,7 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
     if (launch) {
       k_long_reads<<<(nq + 255) / 256, 256, 0, x->stream>>>(ord, nq, c.d_qoff, nq, x->seg_len, 0, x->lflag.as<uint32_t>(),
                                                             x->nslot.as<uint32_t>(), &dc->n_long, &dc->n_units,
-                                                            &dc->seg_len);
+                                                            &dc->seg_len, &dc->bases);
       CK(cudaGetLastError());
     }
     RET(SCAN(x->lflag.as<uint32_t>(), 1, nq, x->lpos.as<uint64_t>()));
@@ -1227,10 +1341,21 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
       CK(cudaGetLastError());
       J.ids = T.left; J.n_ids_dev = T.n_left; J.resume = T.resume;
     }
-    WITH_FMT(fmt, {
-      k_smem<false, 32, 0, 8, FM><<<(unsigned)(threads / 128), 128, 0, x->stream>>>(Fw.d, Rv.d, cfw, crv, c.d_q, c.d_qoff,
-                                                                                    P, hp, o, W, J, x->aux);
-    });
+    const unsigned grid = (unsigned)(threads / 128);
+    if (fmt == OCC_NARROW) {
+      RET(pack_reads(x, c.d_q, c.d_qoff, nq, c.max_bases, P.min_len, J, scap, false, R));
+      k_acgt<false, 0, ACGT_BLOCKS><<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, c.d_qoff, P, hp, o, W, J, x->aux, R, 32u,
+                                                                 x->left_jobs.as<uint32_t>(), &dc->n_left);
+      if (Fw.tag != 1) {
+        W.queue = &dc->queue3;
+        J.jobs = x->left_jobs.as<uint32_t>(); J.n_jobs_dev = &dc->n_left;
+        k_smem<false, 32, 0, 8, OCC_NARROW><<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, cfw, crv, c.d_q, c.d_qoff, P, hp, o, W, J,
+                                                                         x->aux);
+      }
+    } else {
+      k_smem<false, 32, 0, 8, OCC_WIDE><<<grid, 128, 0, x->stream>>>(Fw.d, Rv.d, cfw, crv, c.d_q, c.d_qoff, P, hp, o, W, J,
+                                                                     x->aux);
+    }
     // reads that outgrew their sets or hit list: one warp per read, over the device list
     MemsWork Ww{};
     Ww.sets = x->work.as<BIv>(); Ww.set_cap = c.warp_cap; Ww.cands = x->cwork.as<Cand>(); Ww.cand_cap = c.warp_cands;
@@ -1795,11 +1920,12 @@ int hfm_index_device_bytes(const hfm_index* x, uint64_t* index_bytes, uint64_t* 
       &x->mivpool, &x->bswork, &x->memwork, &x->hkeys, &x->hslot, &x->hflags, &x->huid, &x->urow, &x->ulen,
       &x->uoff, &x->uout, &x->blockmap, &x->blockmap2, &x->ovf2, &x->ovf3, &x->lflag, &x->lpos, &x->sids,
       &x->lids, &x->ucount, &x->ubase, &x->uread, &x->uk, &x->nslot, &x->slot_base, &x->slot_hits, &x->npos,
-      &x->iota, &x->loc_pairs, &x->okeys, &x->oids, &x->otemp, &x->trie_nodes, &x->trie_left, &x->trie_resume};
+      &x->iota, &x->loc_pairs, &x->okeys, &x->oids, &x->otemp, &x->trie_nodes, &x->trie_left, &x->trie_resume,
+      &x->left_jobs, &x->pack_words, &x->pack_anchors};
   uint64_t a = 0, b = 0;
   if (!x->shared_index) {
     for (const DevBuf* d : idx_bufs) a += d->cap;
-    a += x->aux_kmer.cap + x->aux_sa.cap;
+    a += x->aux_kmer.cap + x->aux_sa.cap + x->aux_text.cap + x->aux_seen.cap;
   }
   for (const DevBuf* d : work_bufs) b += d->cap;
   if (index_bytes) *index_bytes = a;
@@ -1825,7 +1951,8 @@ void hfm_index_free(hfm_index* x) {
                     &x->blockmap, &x->blockmap2, &x->ovf2, &x->ovf3, &x->lflag, &x->lpos, &x->sids, &x->lids,
                     &x->ucount, &x->ubase, &x->uread, &x->uk, &x->nslot, &x->slot_base, &x->slot_hits, &x->npos,
                     &x->iota, &x->loc_pairs, &x->okeys, &x->oids, &x->otemp, &x->trie_nodes, &x->trie_left,
-                    &x->trie_resume, &x->aux_kmer, &x->aux_sa})
+                    &x->trie_resume, &x->left_jobs, &x->pack_words, &x->pack_anchors, &x->aux_kmer, &x->aux_sa,
+                    &x->aux_text, &x->aux_seen})
     b->release();
   for (auto& e : x->ev) if (e) cudaEventDestroy(e);
   for (auto& e : x->evk) if (e) cudaEventDestroy(e);
@@ -1840,7 +1967,7 @@ int hfm_index_info_get(const hfm_index* x, hfm_index_info* o) {
   o->kind = x->kind; o->text_len = x->fwd.text_len; o->num_sequences = x->fwd.num_seqs;
   o->sample_rate = x->fwd.rate; o->lookup_depth = x->fwd.lookup_depth; o->alphabet_tag = x->fwd.tag;
   o->num_lanes = x->fwd.num_lanes; o->encoding = x->fwd.encoding;
-  o->device_bytes = x->fwd.bytes() + x->rev.bytes() + x->aux_kmer.cap + x->aux_sa.cap;
+  o->device_bytes = x->fwd.bytes() + x->rev.bytes() + x->aux_kmer.cap + x->aux_sa.cap + x->aux_text.cap + x->aux_seen.cap;
   return HFM_OK;
 }
 

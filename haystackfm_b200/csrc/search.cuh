@@ -718,13 +718,16 @@ __global__ void __launch_bounds__(128) k_mems_plain(DevFm Fw, DevFm Rv, const ui
 constexpr uint32_t SEG_MAX = 4096;   // longest segment
 
 // The segment length of a batch: the tuned one, or for an ACGT text (threads > 0) a smaller
-// one, down to 64, while the batch's codes do not fill the resident threads with segments of
-// it: a small batch is bound by its longest chain of steps, and a segment's chain is its
-// length plus a match.  (250 mixed reads up to 10 kbp, 256 Mbp ACGT: 4.4 ms at 512.)
+// one, down to 64, while the batch's codes do not give every resident thread SEGS_PER_THREAD
+// segments of it: a small batch is bound by its longest chain of steps, which is a segment's
+// length plus a match, and a larger one by the last segments while most lanes are idle.
+// (Search of 60,000 mixed reads up to 10 kbp, 49 M codes for 151,552 threads: 3.2 ms at 512,
+// 2.2 at 256, 2.0 at 128, 2.3 at 64, where the windows that segments share cost more.)
+constexpr uint64_t SEGS_PER_THREAD = 4;
 __device__ __forceinline__ uint32_t batch_seg_len(uint64_t bases, uint32_t seg_len, uint64_t threads) {
   if (!threads) return seg_len;
   uint32_t s = 64;
-  while (s < seg_len && bases / s > threads) s *= 2;
+  while (s < seg_len && bases / s > SEGS_PER_THREAD * threads) s *= 2;
   return min(s, seg_len);
 }
 
@@ -733,11 +736,12 @@ __device__ __forceinline__ uint32_t batch_seg_len(uint64_t bases, uint32_t seg_l
 __global__ void k_long_reads(const uint32_t* __restrict__ ids, uint32_t n, const uint64_t* __restrict__ qoff,
                              uint32_t nq, uint32_t tuned_len, uint64_t threads, uint32_t* __restrict__ flags,
                              uint32_t* __restrict__ nslot, uint32_t* __restrict__ n_long,
-                             unsigned long long* __restrict__ n_units, uint32_t* __restrict__ used_len) {
+                             unsigned long long* __restrict__ n_units, uint32_t* __restrict__ used_len,
+                             unsigned long long* __restrict__ bases) {
   uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const uint32_t seg_len = batch_seg_len(qoff[nq] - qoff[0], tuned_len, threads);
-  if (k == 0) *used_len = seg_len;
+  if (k == 0) { *used_len = seg_len; *bases = qoff[nq] - qoff[0]; }
   const uint32_t i = ids ? ids[k] : k;
   const uint64_t len = qoff[i + 1] - qoff[i];
   const bool is_long = len > 2 * (uint64_t)seg_len;

@@ -52,6 +52,9 @@ struct SmemJobs {
   uint32_t n_ids;
   const uint64_t* n_long_dev;     // when set, n_ids counts the long reads too
   const uint32_t* n_ids_dev;      // when set, the number of whole reads
+  const uint32_t* jobs;           // when set, only these n_jobs jobs (of the ones above)
+  uint32_t n_jobs;
+  const uint32_t* n_jobs_dev;     // when set, their number
   const uint32_t* resume;         // per whole read: position after a result [0, e) that is already in its slot
                                   // (k_trie), or RESUME_START; nullptr: every read from its start
   // Results are written per slot: a read's segments in order (one slot for a read in one
@@ -67,13 +70,20 @@ constexpr uint32_t RESUME_START = 0xFFFFFFFFu;
 
 // What a bidirectional index of an ACGT text keeps besides its records, made on the device
 // when it is loaded (k_kmer_table):
-//   kmer  for every ACGT string of k codes (code 1 first, the first code in the top digit)
-//         its forward start, reverse start and rows: the window and next phases start k
-//         steps on, with one load.
-// It may be absent (no memory for it): the search then takes the steps.
+//   kmer  for every ACGT string of k codes its forward start, reverse start and rows: the
+//         window and next phases start k steps on, with one load;
+//   sa    the position of every forward row, and
+//   text  the text as bit planes: the rest of a one-row match is read off them;
+//   seen  a bit for every string of seen_k codes, set when it occurs in the text.
+// A string's place in kmer and seen: the second bits of its symbols - 1, then their first
+// bits, the string's first code in the lowest bit of either (plane_key, acgt.cuh).
+// Any may be absent (no memory for it): the search then takes the steps.
 struct DevAux {
   const uint4* kmer;
-  uint32_t k;
+  const uint32_t* sa;
+  const uint4* text;              // 32 codes a word (k_text_planes); only with sa
+  const uint32_t* seen;           // only with text
+  uint32_t k, seen_k;
 };
 
 // One direction of the index as the step needs it.
@@ -87,20 +97,20 @@ struct FmView { const uint4* occ; const uint32_t* sb; };
 //
 // Both borders count from row 32 of their records: 4 popcounts of 32 bits (rows of code s,
 // and of the codes from s on, at either border); the masks of s are two words made from its
-// bits, so that one form serves every code.
+// bits, so that one form serves every code.  acgt_use takes the first half of the lower
+// border's record (at pl) from its caller.
 template <bool COUNT_TOUCH>
-__device__ __forceinline__ bool acgt_step(const FmView& X, const uint32_t* C, uint32_t s, uint32_t& lo, uint32_t& base,
-                                          uint32_t& n, uint64_t& touches) {
+__device__ __forceinline__ bool acgt_use(const FmView& X, const uint32_t* C, uint32_t s, const uint4& u, const uint4* pl,
+                                         uint32_t& lo, uint32_t& base, uint32_t& n, uint64_t& touches) {
   const uint32_t last = lo + n - 1, bl = lo >> 6, bh = last >> 6, sh = 16u * (s - 1u);
-  const uint4* pl = X.occ + (size_t)bl * OCC_NARROW_U4;
-  const uint4 u = __ldg(pl), v = __ldg(pl + 1);
+  const uint4 v = __ldg(pl + 1);
   const uint32_t sbl = __ldg(X.sb + (size_t)(bl >> SB_BLOCK_SHIFT) * 16 + s);
   uint4 u2 = u, v2 = v;
   if (bh != bl) {
     const uint4* ph = X.occ + (size_t)bh * OCC_NARROW_U4;
     u2 = __ldg(ph); v2 = __ldg(ph + 1);
+    if (COUNT_TOUCH) touches += 1;
   }
-  if (COUNT_TOUCH) touches += bh != bl ? 2 : 1;
   Border<OCC_NARROW> L, H;
   L.take(u, v, lo & 63);
   H.take(u2, v2, (last & 63) + 1u);
@@ -131,6 +141,15 @@ __device__ __forceinline__ bool acgt_step(const FmView& X, const uint32_t* C, ui
   lo = C[s] + sbl + rl;
   n = d;
   return true;
+}
+
+template <bool COUNT_TOUCH>
+__device__ __forceinline__ bool acgt_step(const FmView& X, const uint32_t* C, uint32_t s, uint32_t& lo, uint32_t& base,
+                                          uint32_t& n, uint64_t& touches) {
+  const uint4* pl = X.occ + (size_t)(lo >> 6) * OCC_NARROW_U4;
+  const uint4 u = __ldg(pl);
+  if (COUNT_TOUCH) touches += 1;
+  return acgt_use<COUNT_TOUCH>(X, C, s, u, pl, lo, base, n, touches);
 }
 
 // A lane's interval set: one interval in registers, or cnt > 1 of them in `cur` (in any
@@ -240,7 +259,8 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
     hit_cap = W.hit_cap;
   }
   enum : uint32_t { FETCH, WINDOW, BACK, FORWARD, NEXT_START, NEXT, LEFT_MAX, DONE };
-  const uint32_t n_units = J.units(), n_jobs = n_units + J.whole(), chunk = W.step(), min_len = P.min_len;
+  const uint32_t n_units = J.units(), chunk = W.step(), min_len = P.min_len;
+  const uint32_t n_jobs = !J.jobs ? n_units + J.whole() : J.n_jobs_dev ? *J.n_jobs_dev : J.n_jobs;
   const uint32_t sym = Fw.sym_mask;
   QueueCursor qc;
   uint64_t touches = 0, t0 = 0;
@@ -250,7 +270,7 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
   const uint8_t* p = q;
   for (;;) {
     if (ph == FETCH) {
-      if (!next_read_chunked(W.queue, n_jobs, nullptr, chunk, qc, u)) break;
+      if (!next_read_chunked(W.queue, n_jobs, J.jobs, chunk, qc, u)) break;
       const bool unit = u < n_units;
       read = unit ? J.unit_read[u] : J.ids ? J.ids[u - n_units] : u - n_units;
       const uint64_t o = qoff[read];
@@ -285,11 +305,11 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
       pos = window ? i + min_len - 1 : end;
       ph = window ? BACK : NEXT;
       if (FMT == OCC_NARROW && A.kmer && A.k <= min_len) {
-        uint32_t x = 0, bad = 0;
+        uint32_t b0 = 0, b1 = 0, bad = 0;
         const uint8_t* b = p + pos + 1 - A.k;
-        for (uint32_t k = 0; k < A.k; k++) { const uint32_t c = b[k] - 1u; bad |= c; x = x << 2 | (c & 3u); }
+        for (uint32_t k = 0; k < A.k; k++) { const uint32_t c = b[k] - 1u; bad |= c; b0 |= (c & 1u) << k; b1 |= (c >> 1 & 1u) << k; }
         if (bad < 4) {
-          const uint4 v = __ldg(A.kmer + x);
+          const uint4 v = __ldg(A.kmer + (b1 << A.k | b0));
           if (COUNT_TOUCH) touches += 1;
           const uint32_t at = pos + 1 - A.k;               // its first code
           if (!v.z) { i = at + 1; first = false; ph = WINDOW; continue; }
@@ -379,8 +399,10 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
 
 // ---- DevAux, made when an index is loaded --------------------------------------------
 
-// One more code in front: out[c w] from in[w] for strings w of k codes (in: nullptr for k = 0).
-__global__ void k_kmer_table(DevFm Fw, const uint4* __restrict__ in, uint32_t k, uint4* __restrict__ out) {
+// One more code in front: out[c w] from in[w] for strings w of k codes (in: nullptr for k = 0);
+// strings are numbered with their first code in the top digit, in the last level as DevAux has
+// them.
+__global__ void k_kmer_table(DevFm Fw, const uint4* __restrict__ in, uint32_t k, bool last, uint4* __restrict__ out) {
   const uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (x >> (2 * (k + 1))) return;
   const uint32_t s = (uint32_t)(x >> (2 * k)) + 1u;
@@ -390,7 +412,16 @@ __global__ void k_kmer_table(DevFm Fw, const uint4* __restrict__ in, uint32_t k,
   uint64_t touches = 0;
   const FmView X{Fw.occ, Fw.sb};
   if (v.z && !acgt_step<false>(X, C, s, v.x, v.y, v.z, touches)) v = make_uint4(0u, 0u, 0u, 0u);
-  out[x] = v;
+  uint64_t at = x;
+  if (last) {
+    uint32_t b0 = 0, b1 = 0;
+    for (uint32_t t = 0; t <= k; t++) {
+      const uint32_t d = (uint32_t)(x >> (2 * (k - t))) & 3u;
+      b0 |= (d & 1u) << t; b1 |= (d >> 1) << t;
+    }
+    at = (uint64_t)b1 << (k + 1) | b0;
+  }
+  out[at] = v;
 }
 
 }  // namespace hfm

@@ -89,6 +89,27 @@ def test_segment_edges(oracle, kind):
         _check(oracle, b, h, reads[:20], 25, 1)
 
 
+def test_iupac_codes_of_one_symbol(oracle):
+    """A text of two bases: query codes such as R match one symbol of it, others two or none,
+    inside long one-row matches and next to sequence ends."""
+    rng = np.random.default_rng(12)
+    seqs = [rng.integers(1, 3, size=n).astype(np.uint8) for n in (40_000, 90, 3000)]
+    b = _build([al.DnaSequence(c) for c in seqs], FmIndexConfig(sa_sample_rate=8), 0, KIND_BIDIR)
+    h = _Handle(b, KIND_BIDIR)
+    reads = []
+    for k in range(160):
+        s = seqs[k % 3]
+        n = int(rng.integers(30, 90))
+        a = int(rng.integers(0, len(s) - n + 1)) if k % 5 else len(s) - n
+        r = np.concatenate([s[a:a + n], rng.integers(1, 3, size=k % 4).astype(np.uint8)])
+        for at in rng.integers(0, len(r), size=k % 6):
+            r[at] = rng.integers(1, 16)
+        reads.append(r)
+    for min_len in (1, 12, 25):
+        _check(oracle, b, h, reads, min_len, 0)
+    _check(oracle, b, h, reads, 20, 1)
+
+
 def test_set_overflow_tiers(oracle):
     """N stretches in the reads grow interval sets past the shared node lists and the
     per-thread sets; the reads around them keep their results."""
