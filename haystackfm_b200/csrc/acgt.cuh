@@ -54,23 +54,14 @@ struct PackedReads {
   uint32_t seen_k, stride;                  // 0: no anchors (every window is searched)
 };
 
-__device__ __forceinline__ uint64_t plane_key(uint32_t b0, uint32_t b1, uint32_t k) {
-  const uint32_t m = (1u << k) - 1u;        // k < 32
-  return (uint64_t)(b1 & m) << k | (b0 & m);
-}
-
 // A warp per job (segment or whole read): its words, and the bits of the anchors that start
 // in it (anchors is zeroed by the caller).
 template <bool COUNT_TOUCH>
 __global__ void __launch_bounds__(256) k_acgt_pack(const uint16_t* __restrict__ compat, uint32_t sym_mask,
                                                   const uint8_t* __restrict__ q, const uint64_t* __restrict__ qoff,
                                                   SmemJobs J, DevAux A, PackedReads R, unsigned long long* touches) {
-  __shared__ uint8_t s_sym[256];            // query code -> its one symbol, 0 (none) or MANY
-  constexpr uint32_t MANY = 15;
-  {
-    const uint32_t c = threadIdx.x, m = c < 16 ? (uint32_t)(compat[c] & sym_mask) & 0x1Eu : 0u;
-    s_sym[c] = (uint8_t)(!m ? 0u : m & (m - 1) ? MANY : 31u - (uint32_t)__clz(m));
-  }
+  __shared__ uint8_t s_sym[256];
+  sym_table_init(s_sym, compat, sym_mask);
   __syncthreads();
   const uint32_t lane = threadIdx.x & 31, n_units = J.units(), n_jobs = n_units + J.whole();
   const uint64_t first_off = qoff[0];
@@ -99,7 +90,7 @@ __global__ void __launch_bounds__(256) k_acgt_pack(const uint16_t* __restrict__ 
         for (int k = 0; k < 4; k++) {
           const uint32_t c = sym[k] - 1u;
           const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, sym[k] && (c & 1)), b1 = __ballot_sync(0xFFFFFFFFu, sym[k] && (c & 2)),
-                         none = __ballot_sync(0xFFFFFFFFu, sym[k] == 0), many = __ballot_sync(0xFFFFFFFFu, sym[k] == MANY);
+                         none = __ballot_sync(0xFFFFFFFFu, sym[k] == 0), many = __ballot_sync(0xFFFFFFFFu, sym[k] == SYM_MANY);
           if (lane == w + k) mine = make_uint4(b0, b1, none, many);
         }
       }

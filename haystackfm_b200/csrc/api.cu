@@ -281,6 +281,13 @@ static int build_device_fm(const HostFm& h, FmDev& f, cudaStream_t s) {
   return HFM_OK;
 }
 
+// What a handle keeps besides the records may take a quarter of the memory that is free when
+// it is loaded, each part: an index that leaves no room for it is searched without it.
+static bool aux_room(uint64_t bytes) {
+  size_t free_bytes = 0, total = 0;
+  return cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && bytes <= free_bytes / 4;
+}
+
 // The k-mer table of an ACGT index (DevAux): k at most KMER_MAX, and the table (16 bytes an
 // entry) at most two bytes per text position.  Without the memory for it the search does
 // without it.  (k 13 / 12 / 11, search of 1M reads of 150 bp on 256 Mbp: 4.2 / 4.2 / 4.35 ms,
@@ -288,10 +295,10 @@ static int build_device_fm(const HostFm& h, FmDev& f, cudaStream_t s) {
 static constexpr uint32_t KMER_MAX = 13;
 static int build_kmer(hfm_index* x) {
   const FmDev& f = x->fwd;
-  if (x->kind != HFM_KIND_BIDIR || f.fmt != OCC_NARROW) return HFM_OK;
+  if (f.fmt != OCC_NARROW) return HFM_OK;
   uint32_t k = 0;
   while (k < KMER_MAX && (16ull << (2 * (k + 1))) <= 2ull * f.text_len) k++;
-  if (k < 2) return HFM_OK;
+  if (k < 2 || !aux_room(20ull << (2 * k))) return HFM_OK;
   DevBuf tmp;
   if (x->aux_kmer.ensure(16ull << (2 * k)) != HFM_OK || tmp.ensure(16ull << (2 * (k - 1))) != HFM_OK) {
     x->aux_kmer.release();
@@ -320,16 +327,15 @@ static constexpr uint32_t SEEN_K_MAX = 18;      // 8 GB of bits, for texts near 
 static int build_sa(hfm_index* x) {
   const FmDev& f = x->fwd;
   if (f.rate < 1 || f.rate > SA_ROWS_RATE || f.d.num_seqs > f.text_len || !f.text_len) return HFM_OK;
-  if (x->aux_sa.ensure((size_t)f.text_len * 4 + 16) != HFM_OK) return HFM_OK;    // read 16 bytes at a time
+  if (!aux_room((uint64_t)f.text_len * 4) || x->aux_sa.ensure((size_t)f.text_len * 4 + 16) != HFM_OK) return HFM_OK;    // read 16 bytes at a time
   CK(cudaMemsetAsync(x->aux_sa.p, 0xFF, (size_t)f.text_len * 4, x->stream));
   const uint64_t items = (uint64_t)f.d.num_blocks + f.d.num_seqs;
   WITH_FMT(f.fmt, { k_sa_rows<FM><<<(unsigned)((items + 127) / 128), 128, 0, x->stream>>>(f.d, x->aux_sa.as<uint32_t>()); });
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(x->stream));
   x->sa = x->aux_sa.as<uint32_t>();
-  if (x->kind != HFM_KIND_BIDIR || f.fmt != OCC_NARROW) return HFM_OK;
-  // the text, for the SMEM search of ACGT texts; not kept when a row has no position (an
-  // inconsistent index)
+  if (f.fmt != OCC_NARROW || !aux_room((uint64_t)f.text_len * 2)) return HFM_OK;
+  // the text of ACGT texts; not kept when a row has no position (an inconsistent index)
   const uint64_t n = f.text_len, words = n / 32 + 2;
   DevBuf bytes;
   if (bytes.ensure(n) != HFM_OK) return HFM_OK;
@@ -351,7 +357,7 @@ static int build_sa(hfm_index* x) {
     uint32_t k = 3;
     while ((1ull << (2 * k)) < 4ull * n) k++;
     const uint64_t seen_bytes = (1ull << (2 * k)) / 8;
-    if (k > SEEN_K_MAX || x->aux_seen.ensure(seen_bytes) != HFM_OK) return HFM_OK;
+    if (x->kind != HFM_KIND_BIDIR || k > SEEN_K_MAX || !aux_room(seen_bytes) || x->aux_seen.ensure(seen_bytes) != HFM_OK) return HFM_OK;
     CK(cudaMemsetAsync(x->aux_seen.p, 0, seen_bytes, x->stream));
     k_seen_bits<<<(unsigned)((n + 8191) / 8192), 256, 0, x->stream>>>(bytes.as<uint8_t>(), (uint32_t)n, k,
                                                                      x->aux_seen.as<uint32_t>());
@@ -446,7 +452,7 @@ static int run_bsearch(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
   }
   // persistent fast pass: one wave of resident threads, BS_SET_CAP intervals per set
   int bpsm = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_bsearch<false, 32>, 256, 0));
+  WITH_FMT(F.fmt, { CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_bsearch<false, 32, FM>, 256, 0)); });
   uint64_t threads = (uint64_t)std::max(1, bpsm) * x->num_sms * 256;
   threads = std::min<uint64_t>(threads, ((uint64_t)nq + 255) / 256 * 256);
   RET(x->bswork.ensure(std::max<uint64_t>(threads, 32) * 2 * BS_SET_CAP * 8));
@@ -459,14 +465,11 @@ static int run_bsearch(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       unsigned grid = (unsigned)(threads / 256);
       if (x->bswork.cap < (size_t)grid * 256 * 2 * BS_SET_CAP * 8) return set_error(HFM_E_ARG, "internal: work area too small");
       cudaEventRecord(x->evk[0], x->stream);
-      if (x->count_work)
-        k_bsearch<true, 32><<<grid, 256, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, nullptr, nq, cap,
-                                                        x->bswork.as<uint2>(), BS_SET_CAP, &dctr(x)->queue, pool, o,
-                                                        &dctr(x)->still_ovf);
-      else
-        k_bsearch<false, 32><<<grid, 256, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, nullptr, nq, cap,
-                                                         x->bswork.as<uint2>(), BS_SET_CAP, &dctr(x)->queue, pool, o,
-                                                         &dctr(x)->still_ovf);
+      auto go = [&](auto kern) {
+        kern<<<grid, 256, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, nq, cap, x->bswork.as<uint2>(), BS_SET_CAP,
+                                          &dctr(x)->queue, pool, o, x->aux);
+      };
+      WITH_FMT(F.fmt, { if (x->count_work) go(k_bsearch<true, 32, FM>); else go(k_bsearch<false, 32, FM>); });
       cudaEventRecord(x->evk[1], x->stream);
       x->k_search_rec = true;
       launches++;
@@ -486,14 +489,12 @@ static int run_bsearch(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
         RET(x->work.ensure((size_t)grid * 4 * per_warp));
         CK(cudaMemsetAsync(&dctr(x)->still_ovf, 0, 4, x->stream));
         CK(cudaMemsetAsync(&dctr(x)->queue2, 0, 4, x->stream));
-        if (x->count_work)
-          k_bsearch_warp<true><<<grid, 128, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, x->ovf.as<uint32_t>(),
-                                                           n_ovf, cap, x->work.as<uint2>(), set_cap, &dctr(x)->queue2, pool,
-                                                           o, &dctr(x)->still_ovf);
-        else
-          k_bsearch_warp<false><<<grid, 128, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, x->ovf.as<uint32_t>(),
-                                                            n_ovf, cap, x->work.as<uint2>(), set_cap, &dctr(x)->queue2, pool,
-                                                            o, &dctr(x)->still_ovf);
+        auto go = [&](auto kern) {
+          kern<<<grid, 128, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, x->ovf.as<uint32_t>(), n_ovf, cap,
+                                            x->work.as<uint2>(), set_cap, &dctr(x)->queue2, pool, o, &dctr(x)->still_ovf, x->aux,
+                                            (const uint32_t*)nullptr);
+        };
+        WITH_FMT(F.fmt, { if (x->count_work) go(k_bsearch_warp<true, FM>); else go(k_bsearch_warp<false, FM>); });
         launches++;
         CK(cudaGetLastError());
         RET(read_ctr(x));
@@ -1471,7 +1472,7 @@ static int fixed_locate(hfm_index* x, FixedLocate& c, bool launch) {
   RET(x->ivpool.ensure(icap * 8));
   if (!launch) {
     int bpsm = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_bsearch<false, 32>, 256, 0));
+    WITH_FMT(F.fmt, { CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_bsearch<false, 32, FM>, 256, 0)); });
     c.threads = std::min<uint64_t>((uint64_t)std::max(1, bpsm) * x->num_sms * 256, ((uint64_t)nq + 255) / 256 * 256);
   }
   RET(x->bswork.ensure(std::max<uint64_t>(c.threads, 32) * 2 * BS_SET_CAP * 8));
@@ -1500,12 +1501,13 @@ static int fixed_locate(hfm_index* x, FixedLocate& c, bool launch) {
   const uint16_t* cm = F.compat.as<uint16_t>();
   if (launch) {
     CK(cudaMemsetAsync(dc, 0, sizeof(Counters), x->stream));
-    k_bsearch<false, 32><<<(unsigned)(c.threads / 256), 256, 0, x->stream>>>(F.d, cm, c.d_q, c.d_qoff, nullptr, nq,
-                                                                            c.max_hits, x->bswork.as<uint2>(), BS_SET_CAP,
-                                                                            &dc->queue, pool, o, &dc->still_ovf);
-    k_bsearch_warp<false><<<wgrid, 128, 0, x->stream>>>(F.d, cm, c.d_q, c.d_qoff, x->ovf.as<uint32_t>(), 0u, c.max_hits,
-                                                       x->work.as<uint2>(), c.warp_cap, &dc->queue2, pool, o,
-                                                       &dc->still_ovf, &dc->n_ovf);
+    WITH_FMT(F.fmt, {
+      k_bsearch<false, 32, FM><<<(unsigned)(c.threads / 256), 256, 0, x->stream>>>(
+          F.d, cm, c.d_q, c.d_qoff, nq, c.max_hits, x->bswork.as<uint2>(), BS_SET_CAP, &dc->queue, pool, o, x->aux);
+      k_bsearch_warp<false, FM><<<wgrid, 128, 0, x->stream>>>(F.d, cm, c.d_q, c.d_qoff, x->ovf.as<uint32_t>(), 0u, c.max_hits,
+                                                              x->work.as<uint2>(), c.warp_cap, &dc->queue2, pool, o,
+                                                              &dc->still_ovf, x->aux, &dc->n_ovf);
+    });
     k_zero_failed<<<(nq + 255) / 256, 256, 0, x->stream>>>(x->status.as<uint32_t>(), nq, x->niv.as<uint32_t>(),
                                                            x->nhits.as<uint64_t>());
     CK(cudaGetLastError());
@@ -2474,17 +2476,20 @@ extern "C" int hfm_count_batch_noalloc(hfm_index* x, const uint8_t* d_q, const u
   CK(cudaMemsetAsync(ctr, 0, sizeof(NoallocCtr), x->stream));
   Pool pool{nullptr, &ctr->used, 0};
   BsOut o{d_counts, nullptr, nullptr, nullptr, status, ovf, &ctr->n_ovf, &ctr->touches};
-  k_bsearch<false, 32><<<NOALLOC_THREADS / 256, 256, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, nullptr,
-                                                                     nq, 0, fast, NOALLOC_SET_CAP, &ctr->queue, pool,
-                                                                     o, &ctr->still_ovf);
+  WITH_FMT(F.fmt, {
+    k_bsearch<false, 32, FM><<<NOALLOC_THREADS / 256, 256, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, nq, 0, fast,
+                                                                          NOALLOC_SET_CAP, &ctr->queue, pool, o, x->aux);
+  });
   CK(cudaGetLastError());
   uint32_t n_ovf = 0;
   CK(cudaMemcpyAsync(&n_ovf, &ctr->n_ovf, sizeof(uint32_t), cudaMemcpyDeviceToHost, x->stream));
   CK(cudaStreamSynchronize(x->stream));
   if (n_ovf) {
-    k_bsearch_warp<false><<<NOALLOC_WARPS / 4, 128, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, ovf, n_ovf,
-                                                                   0, tail, NOALLOC_WARP_SET_CAP, &ctr->queue2, pool,
-                                                                   o, &ctr->still_ovf);
+    WITH_FMT(F.fmt, {
+      k_bsearch_warp<false, FM><<<NOALLOC_WARPS / 4, 128, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, ovf, n_ovf, 0,
+                                                                         tail, NOALLOC_WARP_SET_CAP, &ctr->queue2, pool, o,
+                                                                         &ctr->still_ovf, x->aux);
+    });
     CK(cudaGetLastError());
     uint32_t still = 0;
     CK(cudaMemcpyAsync(&still, &ctr->still_ovf, sizeof(uint32_t), cudaMemcpyDeviceToHost, x->stream));

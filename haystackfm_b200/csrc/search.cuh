@@ -126,28 +126,6 @@ __device__ __forceinline__ bool next_read_chunked(unsigned int* ctr, uint32_t n,
 // Backward search (FmIndex::backward_search, src/fm_index/query.rs:219-277)
 // =====================================================================================
 
-// Insert a non-empty interval into a sorted, coalesced set (the effect of
-// merge_intervals_inplace, src/fm_index/query.rs:390-407, applied incrementally).
-template <class SR>
-__device__ __forceinline__ bool iv_insert(const SR& a, uint32_t& n, uint32_t cap, uint32_t lo, uint32_t hi) {
-  uint32_t j = n;
-  while (j > 0 && a[j - 1].x > lo) j--;
-  if (j > 0 && a[j - 1].y >= lo) { j--; lo = a[j].x; hi = max(hi, a[j].y); }
-  uint32_t e = j;
-  while (e < n && a[e].x <= hi) { hi = max(hi, a[e].y); e++; }
-  uint32_t removed = e - j;
-  if (removed == 0) {
-    if (n >= cap) return false;
-    for (uint32_t k = n; k > j; k--) a[k] = a[k - 1];
-    n++;
-  } else if (removed > 1) {
-    for (uint32_t k = e; k < n; k++) a[k - removed + 1] = a[k];
-    n -= removed - 1;
-  }
-  a[j] = make_uint2(lo, hi);
-  return true;
-}
-
 struct BsOut {
   uint32_t* counts;      // exact count per query
   uint64_t* nhits;       // sum of min(size, cap) per query (nullptr: count only)
@@ -159,135 +137,309 @@ struct BsOut {
   unsigned long long* touches;  // Occ record touches (counted only with COUNT_TOUCH)
 };
 
-// Returns the final number of intervals in cur (0 = no match), or ~0u on set overflow.
-template <bool COUNT_TOUCH, class SR>
-__device__ __forceinline__ uint32_t backward_search_one(const DevFm& F, const SmemFm& S, const uint8_t* p,
-                                                        uint32_t m, SR& cur, SR& nxt, uint32_t cap,
-                                                        uint64_t& touches) {
-  cur[0] = make_uint2(0, F.text_len);
-  if (m == 0) return 1;
-  uint32_t n = 1, start = m;
-  if (F.lut && m >= F.lut_depth) {
-    // LookupTable::get (src/fm_index/lookup.rs:101-111): rightmost code is the most
-    // significant digit of the base-radix index.
-    uint64_t idx = 0; bool ok = true;
-    for (int k = (int)F.lut_depth - 1; k >= 0; --k) {
-      uint8_t c = p[m - F.lut_depth + k];
-      uint32_t d = c < 16 ? S.dig[c] : 0xFF;
-      if (d == 0xFF) { ok = false; break; }
-      idx = idx * F.lut_radix + d;
-    }
-    if (ok) {
-      uint2 iv = __ldg(F.lut + idx);
+// What a handle keeps for queries besides the records, made on the device when an index is
+// loaded: sa is the position of every forward row (resolve.cuh); the others exist for ACGT
+// texts only:
+//   kmer  for every ACGT string of k codes its forward start, reverse start and rows: a search
+//         starts k steps on, with one load;
+//   text  the text as bit planes (with sa): the rest of a one-row match is read off them;
+//   seen  a bit for every string of seen_k codes, set when it occurs in the text.
+// A string's place in kmer and seen: the second bits of its symbols - 1, then their first
+// bits, the string's first code in the lowest bit of either (plane_key).
+// Any may be absent (no memory for it): the searches then take the steps.
+struct DevAux {
+  const uint4* kmer;
+  const uint32_t* sa;
+  const uint4* text;              // 32 codes a word (k_text_planes); only with sa
+  const uint32_t* seen;           // only with text
+  uint32_t k, seen_k;
+};
+
+__device__ __forceinline__ uint64_t plane_key(uint32_t b0, uint32_t b1, uint32_t k) {
+  const uint32_t m = (1u << k) - 1u;        // k < 32
+  return (uint64_t)(b1 & m) << k | (b0 & m);
+}
+
+// Query code -> the one symbol of the text that it matches, 0 for none, SYM_MANY for several
+// (256 entries, every code a byte can hold).
+constexpr uint32_t SYM_MANY = 0xFF;
+__device__ __forceinline__ void sym_table_init(uint8_t* t, const uint16_t* compat, uint32_t sym_mask) {
+  for (uint32_t c = threadIdx.x; c < 256; c += blockDim.x) {
+    const uint32_t m = c < 16 ? (uint32_t)compat[c] & sym_mask : 0u;
+    t[c] = (uint8_t)(!m ? 0u : m & (m - 1) ? SYM_MANY : 31u - (uint32_t)__clz(m));
+  }
+}
+
+// Rows [lo, lo + n) narrowed to those preceded by code s (1..4) of an ACGT text; false, and
+// nothing changed, when there are none.
+template <bool COUNT_TOUCH>
+__device__ __forceinline__ bool acgt_rows(const DevFm& F, const uint32_t* C, uint32_t s, uint32_t& lo, uint32_t& n,
+                                          uint64_t& touches) {
+  const uint32_t last = lo + n - 1, bl = lo >> 6, bh = last >> 6, sh = 16u * (s - 1u);
+  const uint4* pl = F.occ + (size_t)bl * OCC_NARROW_U4;
+  const uint4 u = __ldg(pl), v = __ldg(pl + 1);
+  const uint32_t sbl = __ldg(F.sb + (size_t)(bl >> SB_BLOCK_SHIFT) * 16 + s);
+  uint4 u2 = u, v2 = v;
+  uint32_t sbh = sbl;
+  if (bh != bl) {
+    const uint4* ph = F.occ + (size_t)bh * OCC_NARROW_U4;
+    u2 = __ldg(ph); v2 = __ldg(ph + 1);
+    sbh = __ldg(F.sb + (size_t)(bh >> SB_BLOCK_SHIFT) * 16 + s);
+  }
+  if (COUNT_TOUCH) touches += bh != bl ? 2 : 1;
+  Border<OCC_NARROW> L, H;
+  L.take(u, v, lo & 63);
+  H.take(u2, v2, (last & 63) + 1u);
+  const uint32_t k0 = 0u - ((s - 1u) & 1u), k1 = 0u - ((s - 1u) >> 1);
+  auto rank = [&](const Border<OCC_NARROW>& B) {
+    return ((uint32_t)((((uint64_t)B.c34 << 32) | B.c12) >> sh) & 0xFFFFu) +
+           (uint32_t)__popc(B.m & ~B.z & ~((B.b0 ^ k0) | (B.b1 ^ k1))) * B.sg;
+  };
+  const uint32_t rl = sbl + rank(L), d = sbh + rank(H) - rl;
+  if (!d) return false;
+  lo = C[s] + rl;
+  n = d;
+  return true;
+}
+
+// 16 counts at the borders of rows [lo, lo + n), n >= 1, of a wide index: r[s] = rank of s at
+// lo, d[s] = rows of code s.  The records are those of the first and the last row, one when
+// they are the same.
+__device__ __forceinline__ void wide_split(const uint4* __restrict__ occ, uint32_t lo, uint32_t n, uint32_t r[16],
+                                           uint32_t d[16]) {
+  const uint32_t last = lo + n - 1, bl = lo >> 6, bh = last >> 6, xl = lo & 63, xh = (last & 63) + 1;
+  const uint4* pl = occ + (size_t)bl * OCC_WIDE_U4;
+  const uint4* ph = occ + (size_t)bh * OCC_WIDE_U4;
+  Border<OCC_WIDE> L, H;
+  L.a = __ldg(pl); L.b = __ldg(pl + 1); L.c = __ldg(pl + 2); L.d = __ldg(pl + 3);
+  L.w = __ldg(pl + (xl >= 32 ? 5 : 4));
+  H.w = __ldg(ph + (xh >= 32 ? 5 : 4));
+  H.a = L.a; H.b = L.b; H.c = L.c; H.d = L.d;
+  if (bh != bl) { H.a = __ldg(ph); H.b = __ldg(ph + 1); H.c = __ldg(ph + 2); H.d = __ldg(ph + 3); }
+  L.select(xl); H.select(xh);
+  wide_ranks(L, r);
+  wide_ranks(H, d);
+#pragma unroll
+  for (int s = 0; s < 16; s++) d[s] -= r[s];
+}
+
+// Ranks at lo and rows of every code in [lo, hi), hi > lo, for either record format.
+template <uint32_t FMT>
+__device__ __forceinline__ void rows_by_code(const DevFm& F, uint32_t lo, uint32_t hi, uint32_t r[16], uint32_t d[16]) {
+  if constexpr (FMT == OCC_WIDE) {
+    wide_split(F.occ, lo, hi - lo, r, d);
+  } else {
+    sym_ranks_t<FMT>(F, lo, r);
+    sym_ranks_t<FMT>(F, hi, d);
+#pragma unroll
+    for (int s = 0; s < 16; s++) d[s] -= r[s];
+  }
+}
+
+// The last codes of a pattern at once: the index's own lookup table (LookupTable::get,
+// src/fm_index/lookup.rs:101-111: only when all of them are ACGT, and whatever it holds is
+// the answer, which on IUPAC texts leaves out strings with other codes), or the k-mer table
+// of an ACGT text when that reaches further.  Sets [lo, lo + n) and the codes still to search;
+// n = 0 when there is no match, start = m when nothing was looked up.
+template <bool COUNT_TOUCH>
+__device__ __forceinline__ void seed_pattern(const DevFm& F, const DevAux& A, const uint8_t* dig, const uint8_t* p, uint32_t m,
+                                             uint32_t& lo, uint32_t& n, uint32_t& start, uint64_t& touches) {
+  lo = 0; n = F.text_len; start = m;
+  if (A.kmer && m >= A.k && A.k >= F.lut_depth) {
+    uint32_t b0 = 0, b1 = 0, bad = 0;
+    const uint8_t* b = p + (m - A.k);
+    for (uint32_t k = 0; k < A.k; k++) { const uint32_t c = b[k] - 1u; bad |= c; b0 |= (c & 1u) << k; b1 |= (c >> 1 & 1u) << k; }
+    if (bad < 4) {
+      const uint4 v = __ldg(A.kmer + plane_key(b0, b1, A.k));
       if (COUNT_TOUCH) touches++;
-      if (iv.x >= iv.y) return 0;
-      cur[0] = iv; start = m - F.lut_depth;
+      lo = v.x; n = v.z; start = m - A.k;
+      return;
     }
   }
-  for (uint32_t k = start; k-- > 0;) {
-    uint8_t c = p[k];
-    uint32_t mask = c < 16 ? S.compat_mask[c] : 0;
-    mask &= F.sym_mask;                   // symbol_count(r) == 0 -> skipped
+  if (F.lut && m >= F.lut_depth) {
+    uint64_t idx = 0;
+    for (int k = (int)F.lut_depth - 1; k >= 0; --k) {
+      const uint8_t c = p[m - F.lut_depth + k];
+      const uint32_t d = c < 16 ? dig[c] : 0xFF;
+      if (d == 0xFF) return;
+      idx = idx * F.lut_radix + d;
+    }
+    const uint2 iv = __ldg(F.lut + idx);
+    if (COUNT_TOUCH) touches++;
+    lo = iv.x; n = iv.y > iv.x ? iv.y - iv.x : 0u; start = m - F.lut_depth;
+  }
+}
+
+// Codes left from which on a counted one-row match of an ACGT text is compared with the text.
+constexpr uint32_t COUNT_TEXT_LEFT = 4;
+
+// Do the codes p[0..k) stand before the suffix of row `row`?  1 yes, 0 no, -1 one of the codes
+// matches several symbols.
+template <bool COUNT_TOUCH>
+__device__ __forceinline__ int text_before(const DevAux& A, const uint8_t* sym, const uint8_t* p, uint32_t k, uint32_t row,
+                                           uint64_t& touches) {
+  const uint32_t at = __ldg(A.sa + row);
+  if (COUNT_TOUCH) touches += 1;
+  for (uint32_t e = k; e > 0;) {                       // up to 32 codes at a time, the last ones first
+    const uint32_t len = min(e, 32u), from = at - (k - e) - len;       // text place of the first of them
+    uint32_t b0 = 0, b1 = 0, odd = 0;
+    for (uint32_t t = 0; t < len; t++) {
+      const uint32_t s = sym[p[e - len + t]];
+      if (s == SYM_MANY) return -1;
+      odd |= s == 0;
+      b0 |= ((s - 1u) & 1u) << t; b1 |= ((s - 1u) >> 1 & 1u) << t;
+    }
+    if (odd || at < k - e + len) return 0;
+    const uint4 x = __ldg(A.text + (from >> 5)), y = __ldg(A.text + (from >> 5) + 1);
+    if (COUNT_TOUCH) touches += 1;
+    const uint32_t sh = from & 31, part = len == 32 ? ~0u : (1u << len) - 1u;
+    const uint32_t diff = (__funnelshift_r(x.x, y.x, sh) ^ b0) | (__funnelshift_r(x.y, y.y, sh) ^ b1) | __funnelshift_r(x.z, y.z, sh);
+    if (diff & part) return 0;
+    e -= len;
+  }
+  return 1;
+}
+
+// Backward search of one pattern (FmIndex::backward_search, src/fm_index/query.rs:219-277).
+// One interval stays in registers (lo, rows); more are in cur, sorted and coalesced.  Returns
+// their number (0 = no match), or ~0u on set overflow.
+template <bool COUNT_TOUCH, uint32_t FMT, class SR>
+__device__ __forceinline__ uint32_t backward_search_one(const DevFm& F, const SmemFm& S, const DevAux& A, const uint8_t* sym,
+                                                        bool count_only, const uint8_t* p, uint32_t m, SR& cur, SR& nxt,
+                                                        uint32_t cap, uint32_t& lo, uint32_t& rows, uint64_t& touches) {
+  uint32_t n = 1, k;
+  seed_pattern<COUNT_TOUCH>(F, A, S.dig, p, m, lo, rows, k, touches);
+  if (!rows) return 0;
+  while (k > 0) {
+    if (FMT == OCC_NARROW && n == 1) {
+      if (count_only && A.text && rows == 1 && k >= COUNT_TEXT_LEFT) {
+        const int r = text_before<COUNT_TOUCH>(A, sym, p, k, lo, touches);
+        if (r >= 0) return (uint32_t)r;
+      }
+      const uint32_t s = sym[p[k - 1]];
+      if (!s) return 0;
+      if (s != SYM_MANY) {
+        if (!acgt_rows<COUNT_TOUCH>(F, S.C, s, lo, rows, touches)) return 0;
+        k--;
+        continue;
+      }
+    }
+    const uint8_t c = p[--k];
+    const uint32_t mask = (c < 16 ? S.compat_mask[c] : 0u) & F.sym_mask;   // symbol_count(r) == 0 -> skipped
     if (!mask) return 0;
-    uint32_t nn = 0;
+    if (FMT == OCC_WIDE && n == 1 && rows == 1) {
+      uint32_t s, rk;
+      row_code_rank<FMT>(F, lo, s, rk);
+      if (COUNT_TOUCH) touches += 1;
+      if (!((mask >> s) & 1)) return 0;
+      lo = S.C[s] + rk;
+      continue;
+    }
+    uint32_t nn = 0, f0 = 0, f1 = 0;                   // the last interval is held back: it may still grow
+    bool ovf = false;
+    auto add = [&](uint32_t a, uint32_t e) {           // ascending; touching neighbours are one
+      if (nn && a <= f1) { f1 = max(f1, e); return; }
+      if (nn) { if (nn >= cap) { ovf = true; return; } nxt[nn - 1] = make_uint2(f0, f1); }
+      f0 = a; f1 = e; nn++;
+    };
     if (n == 1) {
       // one source interval: symbol order is already ascending row order
-      uint2 iv = cur[0];
-      uint32_t rl[16], rh[16];
-      sym_ranks(F, S, iv.x, rl);
-      sym_ranks(F, S, iv.y, rh);
-      if (COUNT_TOUCH) touches += (iv.x != 0) + (iv.y != 0);
+      uint32_t r[16], d[16];
+      rows_by_code<FMT>(F, lo, lo + rows, r, d);
+      if (COUNT_TOUCH) touches += 2;
 #pragma unroll
-      for (int r = 0; r < 16; r++) {
-        if (!((mask >> r) & 1)) continue;
-        uint32_t nl = S.C[r] + rl[r], nh = S.C[r] + rh[r];
-        if (nl < nh && !iv_insert(nxt, nn, cap, nl, nh)) return ~0u;
-      }
+      for (int s = 0; s < 16; s++)
+        if (((mask >> s) & 1) && d[s]) add(S.C[s] + r[s], S.C[s] + r[s] + d[s]);
     } else {
-      // Outputs for symbol r lie in [C[r], C[r+1]) in source order, so a stable counting
-      // sort by symbol yields ascending rows: count per symbol, then place.
+      // Outputs for symbol s lie in [C[s], C[s+1]) in source order: a pass per symbol that
+      // occurs would read the records over, so a stable counting sort by symbol places them.
       uint32_t cnt[16];
 #pragma unroll
-      for (int r = 0; r < 16; r++) cnt[r] = 0;
+      for (int s = 0; s < 16; s++) cnt[s] = 0;
       for (uint32_t i = 0; i < n; i++) {
-        uint2 iv = cur[i];
-        uint32_t rl[16], rh[16];
-        sym_ranks(F, S, iv.x, rl);
-        sym_ranks(F, S, iv.y, rh);
-        if (COUNT_TOUCH) touches += (iv.x != 0) + (iv.y != 0);
+        const uint2 iv = cur[i];
+        uint32_t r[16], d[16];
+        rows_by_code<FMT>(F, iv.x, iv.y, r, d);
+        if (COUNT_TOUCH) touches += 2;
 #pragma unroll
-        for (int r = 0; r < 16; r++) cnt[r] += (((mask >> r) & 1) && rh[r] > rl[r]) ? 1u : 0u;
+        for (int s = 0; s < 16; s++) cnt[s] += (((mask >> s) & 1) && d[s]) ? 1u : 0u;
       }
       uint32_t total = 0;
 #pragma unroll
-      for (int r = 0; r < 16; r++) { uint32_t t = cnt[r]; cnt[r] = total; total += t; }
+      for (int s = 0; s < 16; s++) { const uint32_t t = cnt[s]; cnt[s] = total; total += t; }
       if (total > cap) return ~0u;
       for (uint32_t i = 0; i < n; i++) {
-        uint2 iv = cur[i];
-        uint32_t rl[16], rh[16];
-        sym_ranks(F, S, iv.x, rl);
-        sym_ranks(F, S, iv.y, rh);
+        const uint2 iv = cur[i];
+        uint32_t r[16], d[16];
+        rows_by_code<FMT>(F, iv.x, iv.y, r, d);
 #pragma unroll
-        for (int r = 0; r < 16; r++)
-          if (((mask >> r) & 1) && rh[r] > rl[r]) nxt[cnt[r]++] = make_uint2(S.C[r] + rl[r], S.C[r] + rh[r]);
+        for (int s = 0; s < 16; s++)
+          if (((mask >> s) & 1) && d[s]) nxt[cnt[s]++] = make_uint2(S.C[s] + r[s], S.C[s] + r[s] + d[s]);
       }
       // coalesce touching neighbours (merge_intervals_inplace, query.rs:390-407)
-      for (uint32_t e = 0; e < total; e++) {
-        uint2 v = nxt[e];
-        if (nn > 0) {
-          uint2 last = nxt[nn - 1];
-          if (v.x <= last.y) { nxt[nn - 1] = make_uint2(last.x, max(last.y, v.y)); continue; }
-        }
-        nxt[nn++] = v;
-      }
+      for (uint32_t e = 0; e < total; e++) { const uint2 v = nxt[e]; add(v.x, v.y); }
     }
+    if (ovf) return ~0u;
     if (nn == 0) return 0;
-    SR t = cur; cur = nxt; nxt = t; n = nn;
+    if (nn == 1) { lo = f0; rows = f1 - f0; }
+    else {
+      if (nn > cap) return ~0u;
+      nxt[nn - 1] = make_uint2(f0, f1);
+      const SR t = cur; cur = nxt; nxt = t;
+    }
+    n = nn;
   }
   return n;
 }
 
-// Persistent backward search.  ids == nullptr: every query 0..n-1; otherwise the listed
-// queries (fallback pass; reads that overflow there bump *still_ovf).
-template <bool COUNT_TOUCH, int STRIDE>
+// Persistent backward search of queries 0..n-1.  Queries whose sets outgrow set_cap are listed
+// for k_bsearch_warp.
+template <bool COUNT_TOUCH, int STRIDE, uint32_t FMT>
 __global__ void __launch_bounds__(256) k_bsearch(DevFm F, const uint16_t* __restrict__ compat_masks,
                                                 const uint8_t* __restrict__ q, const uint64_t* __restrict__ qoff,
-                                                const uint32_t* __restrict__ ids, uint32_t n, uint32_t hit_cap,
-                                                uint2* work, uint32_t set_cap, unsigned int* queue, Pool pool,
-                                                BsOut out, uint32_t* still_ovf) {
+                                                uint32_t n, uint32_t hit_cap, uint2* work, uint32_t set_cap,
+                                                unsigned int* queue, Pool pool, BsOut out, DevAux A) {
   __shared__ SmemFm S;
+  __shared__ uint8_t s_sym[256];
   smem_fm_init(S, F, compat_masks);
+  if (FMT == OCC_NARROW) sym_table_init(s_sym, compat_masks, F.sym_mask);
   __syncthreads();
-  SetRef<uint2, STRIDE> A = thread_set<uint2, STRIDE>(work, set_cap, 2, 0);
-  SetRef<uint2, STRIDE> B = thread_set<uint2, STRIDE>(work, set_cap, 2, 1);
+  SetRef<uint2, STRIDE> A0 = thread_set<uint2, STRIDE>(work, set_cap, 2, 0);
+  SetRef<uint2, STRIDE> B0 = thread_set<uint2, STRIDE>(work, set_cap, 2, 1);
   uint64_t touches = 0;
   uint32_t i;
-  while (next_read(queue, n, ids, i)) {
-    SetRef<uint2, STRIDE> cur = A, nxt = B;
-    uint64_t o = qoff[i];
-    uint32_t niv = backward_search_one<COUNT_TOUCH>(F, S, q + o, (uint32_t)(qoff[i + 1] - o), cur, nxt, set_cap,
-                                                    touches);
+  while (next_read(queue, n, nullptr, i)) {
+    SetRef<uint2, STRIDE> cur = A0, nxt = B0;
+    const uint64_t o = qoff[i];
+    uint32_t lo, rows;
+    uint32_t niv = backward_search_one<COUNT_TOUCH, FMT>(F, S, A, s_sym, out.nhits == nullptr, q + o,
+                                                         (uint32_t)(qoff[i + 1] - o), cur, nxt, set_cap, lo, rows, touches);
     uint32_t st = ST_OK;
     if (niv == ~0u) { st = ST_SET_OVF; niv = 0; }
     uint32_t cnt = 0; uint64_t hits = 0;
-    for (uint32_t k = 0; k < niv; k++) {
-      uint2 v = cur[k];
-      uint32_t sz = v.y - v.x;
-      cnt += sz; hits += (hit_cap && sz > hit_cap) ? hit_cap : sz;
+    if (niv == 1) {
+      cnt = rows; hits = (hit_cap && rows > hit_cap) ? hit_cap : rows;
+    } else {
+      for (uint32_t k = 0; k < niv; k++) {
+        const uint2 v = cur[k];
+        const uint32_t sz = v.y - v.x;
+        cnt += sz; hits += (hit_cap && sz > hit_cap) ? hit_cap : sz;
+      }
     }
     uint64_t off = 0;
     if (out.nhits && niv) {
       off = thread_reserve(pool, niv);
       if (off == ~0ull) st |= ST_POOL_OVF;
-      else { uint2* dst = (uint2*)pool.base + off; for (uint32_t k = 0; k < niv; k++) dst[k] = cur[k]; }
+      else {
+        uint2* dst = (uint2*)pool.base + off;
+        if (niv == 1) dst[0] = make_uint2(lo, lo + rows);
+        else for (uint32_t k = 0; k < niv; k++) dst[k] = cur[k];
+      }
     }
     out.counts[i] = cnt;
     if (out.nhits) { out.nhits[i] = hits; out.niv[i] = niv; out.ivoff[i] = off; }
     out.status[i] = st;
-    if (st & ST_SET_OVF) {
-      if (ids) atomicAdd(still_ovf, 1u);
-      else out.ovf_list[atomicAdd(out.n_ovf, 1u)] = i;
-    }
+    if (st & ST_SET_OVF) out.ovf_list[atomicAdd(out.n_ovf, 1u)] = i;
   }
   if (COUNT_TOUCH && touches) atomicAdd(out.touches, (unsigned long long)touches);
 }
@@ -845,90 +997,89 @@ __device__ __forceinline__ uint32_t grp_excl_scan(uint32_t v, uint32_t& total) {
   return x - v;
 }
 
-// Backward-search step set (sorted, coalesced) with the warp: counting sort by symbol
-// (pass 1 counts with ballots, pass 2 places), then lane 0 coalesces touching neighbours.
-template <bool COUNT_TOUCH>
-__device__ uint32_t warp_backward_search(const DevFm& F, const SmemFm& S, const uint8_t* p, uint32_t m,
+// Backward search of one pattern by a warp: a counting sort by symbol (pass 1 counts with
+// ballots, pass 2 places), then touching neighbours coalesced: an interval is the first of its
+// run when it does not touch the one before it, so a run's place is the number of firsts up
+// to it and every lane writes the ends that it knows.  (Coalesced by lane 0 alone, 5,000
+// patterns with an N among the seeded codes took WARP_BEFORE ms of 500,000; now WARP_AFTER.)
+template <bool COUNT_TOUCH, uint32_t FMT>
+__device__ uint32_t warp_backward_search(const DevFm& F, const SmemFm& S, const DevAux& A, const uint8_t* p, uint32_t m,
                                          uint2*& cur, uint2*& nxt, uint32_t cap, uint64_t& touches) {
   const int lane = threadIdx.x & 31;
-  cur[0] = make_uint2(0, F.text_len);
-  if (m == 0) return 1;
-  uint32_t n = 1, start = m;
-  if (F.lut && m >= F.lut_depth) {
-    uint64_t idx = 0; bool ok = true;
-    for (int k = (int)F.lut_depth - 1; k >= 0; --k) {
-      uint8_t c = p[m - F.lut_depth + k];
-      uint32_t d = c < 16 ? S.dig[c] : 0xFF;
-      if (d == 0xFF) { ok = false; break; }
-      idx = idx * F.lut_radix + d;
-    }
-    if (ok) {
-      uint2 iv = __ldg(F.lut + idx);
-      if (COUNT_TOUCH && lane == 0) touches++;
-      if (iv.x >= iv.y) return 0;
-      if (lane == 0) cur[0] = iv;
-      start = m - F.lut_depth;
-    }
-  }
+  const uint32_t lt = lane_lt_mask();
+  uint32_t lo, rows, start;
+  uint64_t seeds = 0;
+  seed_pattern<COUNT_TOUCH>(F, A, S.dig, p, m, lo, rows, start, seeds);
+  if (lane == 0) touches += seeds;
+  if (!rows) return 0;
+  if (lane == 0) cur[0] = make_uint2(lo, lo + rows);
+  uint32_t n = 1;
   __syncwarp();
   for (uint32_t k = start; k-- > 0;) {
-    uint8_t c = p[k];
-    uint32_t mask = (c < 16 ? S.compat_mask[c] : 0) & F.sym_mask;
+    const uint8_t c = p[k];
+    const uint32_t mask = (c < 16 ? S.compat_mask[c] : 0) & F.sym_mask;
     if (!mask) return 0;
     uint32_t cnt[16];
 #pragma unroll
-    for (int r = 0; r < 16; r++) cnt[r] = 0;
+    for (int s = 0; s < 16; s++) cnt[s] = 0;
     for (uint32_t b = 0; b < n; b += 32) {
-      uint32_t i = b + lane;
-      uint32_t rl[16], rh[16];
-      uint2 iv = i < n ? cur[i] : make_uint2(0, 0);
-      sym_ranks(F, S, iv.x, rl);
-      sym_ranks(F, S, iv.y, rh);
-      if (COUNT_TOUCH && i < n) touches += (iv.x != 0) + (iv.y != 0);
+      const uint32_t i = b + lane;
+      uint32_t r[16], d[16];
+      const uint2 iv = i < n ? cur[i] : make_uint2(0, 1);
+      rows_by_code<FMT>(F, iv.x, iv.y, r, d);
+      if (COUNT_TOUCH && i < n) touches += 2;
 #pragma unroll
-      for (int r = 0; r < 16; r++) cnt[r] += __popc(__ballot_sync(0xFFFFFFFFu, i < n && ((mask >> r) & 1) && rh[r] > rl[r]));
+      for (int s = 0; s < 16; s++) cnt[s] += __popc(__ballot_sync(0xFFFFFFFFu, i < n && ((mask >> s) & 1) && d[s]));
     }
     uint32_t total = 0;
 #pragma unroll
-    for (int r = 0; r < 16; r++) { uint32_t t = cnt[r]; cnt[r] = total; total += t; }
+    for (int s = 0; s < 16; s++) { const uint32_t t = cnt[s]; cnt[s] = total; total += t; }
     if (total > cap) return ~0u;
     if (total == 0) return 0;
     for (uint32_t b = 0; b < n; b += 32) {
-      uint32_t i = b + lane;
-      uint32_t rl[16], rh[16];
-      uint2 iv = i < n ? cur[i] : make_uint2(0, 0);
-      sym_ranks(F, S, iv.x, rl);
-      sym_ranks(F, S, iv.y, rh);
+      const uint32_t i = b + lane;
+      uint32_t r[16], d[16];
+      const uint2 iv = i < n ? cur[i] : make_uint2(0, 1);
+      rows_by_code<FMT>(F, iv.x, iv.y, r, d);
 #pragma unroll
-      for (int r = 0; r < 16; r++) {
-        bool e = i < n && ((mask >> r) & 1) && rh[r] > rl[r];
-        uint32_t bal = __ballot_sync(0xFFFFFFFFu, e);
-        if (e) nxt[cnt[r] + __popc(bal & lane_lt_mask())] = make_uint2(S.C[r] + rl[r], S.C[r] + rh[r]);
-        cnt[r] += __popc(bal);
+      for (int s = 0; s < 16; s++) {
+        const bool e = i < n && ((mask >> s) & 1) && d[s];
+        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, e);
+        if (e) nxt[cnt[s] + __popc(bal & lt)] = make_uint2(S.C[s] + r[s], S.C[s] + r[s] + d[s]);
+        cnt[s] += __popc(bal);
       }
     }
     __syncwarp();
-    uint32_t nn = 0;
-    if (lane == 0) {   // coalesce touching neighbours (merge_intervals_inplace, query.rs:390-407)
-      for (uint32_t e = 0; e < total; e++) {
-        uint2 v = nxt[e];
-        if (nn > 0) { uint2 last = nxt[nn - 1]; if (v.x <= last.y) { nxt[nn - 1] = make_uint2(last.x, max(last.y, v.y)); continue; } }
-        nxt[nn++] = v;
+    // coalesce touching neighbours into cur (merge_intervals_inplace, query.rs:390-407)
+    uint32_t nn = 0, before = 0;                        // runs so far; end of the interval before this chunk
+    for (uint32_t b = 0; b < total; b += 32) {
+      const uint32_t i = b + lane;
+      const uint2 v = i < total ? nxt[i] : make_uint2(0, 0);
+      uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, v.y, 1);
+      if (lane == 0) prev = before;
+      const bool first = i < total && (i == 0 || v.x > prev);
+      const uint32_t bal = __ballot_sync(0xFFFFFFFFu, first);
+      const uint32_t run = nn + __popc(bal & (lt | 1u << lane));          // runs up to and with this interval
+      if (first) {
+        cur[run - 1].x = v.x;
+        if (i) cur[run - 2].y = prev;
       }
+      nn += __popc(bal);
+      before = __shfl_sync(0xFFFFFFFFu, v.y, 31);
+      if (i == total - 1) cur[run - 1].y = v.y;
     }
-    nn = __shfl_sync(0xFFFFFFFFu, nn, 0);
     __syncwarp();
-    uint2* t = cur; cur = nxt; nxt = t; n = nn;
+    n = nn;
   }
   return n;
 }
 
-template <bool COUNT_TOUCH>
+template <bool COUNT_TOUCH, uint32_t FMT>
 __global__ void __launch_bounds__(128) k_bsearch_warp(DevFm F, const uint16_t* __restrict__ compat_masks,
                                                      const uint8_t* __restrict__ q, const uint64_t* __restrict__ qoff,
                                                      const uint32_t* __restrict__ ids, uint32_t n, uint32_t hit_cap,
                                                      uint2* work, uint32_t set_cap, unsigned int* queue, Pool pool,
-                                                     BsOut out, uint32_t* still_ovf,
+                                                     BsOut out, uint32_t* still_ovf, DevAux X,
                                                      const uint32_t* __restrict__ n_dev = nullptr) {
   __shared__ SmemFm S;
   smem_fm_init(S, F, compat_masks);
@@ -947,7 +1098,7 @@ __global__ void __launch_bounds__(128) k_bsearch_warp(DevFm F, const uint16_t* _
     uint32_t i = ids[k];
     uint2* cur = A; uint2* nxt = B;
     uint64_t o = qoff[i];
-    uint32_t niv = warp_backward_search<COUNT_TOUCH>(F, S, q + o, (uint32_t)(qoff[i + 1] - o), cur, nxt, set_cap, touches);
+    uint32_t niv = warp_backward_search<COUNT_TOUCH, FMT>(F, S, X, q + o, (uint32_t)(qoff[i + 1] - o), cur, nxt, set_cap, touches);
     if (niv == ~0u) {
       if (lane == 0) { atomicAdd(still_ovf, 1u); out.status[i] = ST_SET_OVF; }
       continue;

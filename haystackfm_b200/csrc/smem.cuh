@@ -68,24 +68,6 @@ struct SmemJobs {
 
 constexpr uint32_t RESUME_START = 0xFFFFFFFFu;
 
-// What a bidirectional index of an ACGT text keeps besides its records, made on the device
-// when it is loaded (k_kmer_table):
-//   kmer  for every ACGT string of k codes its forward start, reverse start and rows: the
-//         window and next phases start k steps on, with one load;
-//   sa    the position of every forward row, and
-//   text  the text as bit planes: the rest of a one-row match is read off them;
-//   seen  a bit for every string of seen_k codes, set when it occurs in the text.
-// A string's place in kmer and seen: the second bits of its symbols - 1, then their first
-// bits, the string's first code in the lowest bit of either (plane_key, acgt.cuh).
-// Any may be absent (no memory for it): the search then takes the steps.
-struct DevAux {
-  const uint4* kmer;
-  const uint32_t* sa;
-  const uint4* text;              // 32 codes a word (k_text_planes); only with sa
-  const uint32_t* seen;           // only with text
-  uint32_t k, seen_k;
-};
-
 // One direction of the index as the step needs it.
 struct FmView { const uint4* occ; const uint32_t* sb; };
 

@@ -69,26 +69,6 @@ struct NodeList {
   __device__ __forceinline__ void put(uint32_t k, const uint4& v) const { if (k < sc) s[k] = v; else g[k] = v; }
 };
 
-// 16 counts at the borders of rows [lo, lo + n), n > 1: r[s] = rank of s at lo, d[s] = rows
-// of code s.  The records are those of the first and the last row, one when they are the same.
-__device__ __forceinline__ void wide_split(const uint4* __restrict__ occ, uint32_t lo, uint32_t n, uint32_t r[16],
-                                           uint32_t d[16]) {
-  const uint32_t last = lo + n - 1, bl = lo >> 6, bh = last >> 6, xl = lo & 63, xh = (last & 63) + 1;
-  const uint4* pl = occ + (size_t)bl * OCC_WIDE_U4;
-  const uint4* ph = occ + (size_t)bh * OCC_WIDE_U4;
-  Border<OCC_WIDE> L, H;
-  L.a = __ldg(pl); L.b = __ldg(pl + 1); L.c = __ldg(pl + 2); L.d = __ldg(pl + 3);
-  L.w = __ldg(pl + (xl >= 32 ? 5 : 4));
-  H.w = __ldg(ph + (xh >= 32 ? 5 : 4));
-  H.a = L.a; H.b = L.b; H.c = L.c; H.d = L.d;
-  if (bh != bl) { H.a = __ldg(ph); H.b = __ldg(ph + 1); H.c = __ldg(ph + 2); H.d = __ldg(ph + 3); }
-  L.select(xl); H.select(xh);
-  wide_ranks(L, r);
-  wide_ranks(H, d);
-#pragma unroll
-  for (int s = 0; s < 16; s++) d[s] -= r[s];
-}
-
 template <bool COUNT_TOUCH>
 __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv, const uint16_t* __restrict__ compat,
                                                              const uint8_t* __restrict__ q,
