@@ -176,17 +176,22 @@ __global__ void __launch_bounds__(128, MINB) k_acgt(DevFm Fw, DevFm Rv, const ui
       if (ph == DONE) {
         const bool unit = u < n_units;
         const uint64_t slot = (J.slot_base ? J.slot_base[read] : (uint64_t)read) + (unit ? J.unit_k[u] : 0u);
-        uint64_t hs = 0;
+        uint64_t hs = 0, hp = 0;
         if (st) nh = 0;
         if (nh) {
           hs = thread_reserve(hitpool, nh);
           if (hs == ~0ull) { st |= ST_POOL_OVF; hs = 0; nh = 0; }
           else {
             uint4* dst = (uint4*)hitpool.base + hs * 2;
-            for (uint32_t k = 0; k < 2 * nh; k++) dst[k] = hits[k];
+#pragma unroll 1
+            for (uint32_t k = 0; k < nh; k++) {
+              const uint4 v = hits[2 * k + 1];
+              dst[2 * k] = hits[2 * k]; dst[2 * k + 1] = v;
+              hp += v.y;
+            }
           }
         }
-        out.hit_start[slot] = hs; out.hit_count[slot] = nh;
+        out.hit_start[slot] = hs; out.hit_count[slot] = nh; out.pos_count[slot] = hp;
         if (st == ST_LEAVE) {
           left_jobs[atomicAdd(n_left, 1u)] = u;
         } else {

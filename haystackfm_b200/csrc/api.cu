@@ -100,6 +100,7 @@ struct DevBuf {
 
 struct Counters {                    // device-side counters, one block per handle
   unsigned long long iv_used, hit_used, touches, steps, n_units, bases;
+  ScanPair totals;                   // of the last scan of a pair: intervals or hits, positions
   uint32_t n_ovf, still_ovf, walk_err, queue, queue2, n_mid, n_wrp, queue3, n_long, trie_queue, n_left, seg_len, queue4, _pad;
 };
 
@@ -128,7 +129,7 @@ struct hfm_index {
   bool count_work = false;
   // per-call work buffers (grow-only)
   DevBuf q, qoff, counts, nhits, niv, ivoff, status, ovf, ivpool, hitpool, seg_row, seg_off, pos_base, seg_base,
-      scan_tmp, out_pairs, ref_bounds, hit_start, hit_count, hit_base, hits, npos_scan, work, cwork, ctr,
+      scan_tmp, out_pairs, ref_bounds, hit_start, hit_count, pos_count, slot_pos, hit_base, hits, npos_scan, work, cwork, ctr,
       mivpool, bswork, memwork, hkeys, hslot, hflags, huid, urow, ulen, uoff, uout, blockmap, blockmap2, ovf2, ovf3,
       lflag, lpos, sids, lids, ucount, ubase, uread, uk, nslot, slot_base, slot_hits, npos, loc_pairs, okeys, oids,
       otemp, trie_nodes, trie_left, trie_resume, left_jobs, pack_words, pack_anchors;
@@ -389,6 +390,22 @@ static int scan(hfm_index* x, const T* in, uint32_t stride, uint64_t n, uint64_t
   return HFM_OK;
 }
 
+// out_a[0..n], out_b[0..n] = exclusive scans of in_a and in_b, their totals in out_a[n],
+// out_b[n] and in the counters.
+static int scan_pair(hfm_index* x, const uint32_t* in_a, const uint64_t* in_b, uint64_t n, uint64_t* out_a, uint64_t* out_b,
+                     ScanPair* totals, uint32_t& launches, bool launch = true) {
+  const uint64_t tiles = std::max<uint64_t>(1, (n + SCAN_TILE - 1) / SCAN_TILE);
+  if (tiles > 0x7FFFFFFFull) return set_error(HFM_E_ARG, "too many entries in one call");
+  RET(x->scan_tmp.ensure(tiles * sizeof(ScanPair)));
+  if (!launch) return HFM_OK;
+  ScanPair* sums = x->scan_tmp.as<ScanPair>();
+  k_scan_pair_tiles<<<(unsigned)tiles, SCAN_T, 0, x->stream>>>(in_a, in_b, n, out_a, out_b, sums, totals);
+  if (tiles > 1) k_scan_pair_add<<<(unsigned)tiles, SCAN_T, 0, x->stream>>>(n, out_a, out_b, sums, totals);
+  launches += tiles > 1 ? 2 : 1;
+  CK(cudaGetLastError());
+  return HFM_OK;
+}
+
 // Waits until `ev` has completed.  Without a deadline this is cudaEventSynchronize; with
 // one (hfm_set_timeout) the host polls the event and gives up with HFM_E_TIMEOUT once the
 // deadline has passed.  The abandoned work stays queued on the handle's stream: the next
@@ -440,7 +457,7 @@ static constexpr int MEMS_PLAIN = 4;             // mems_variant of the plain on
 
 // Backward search for a batch.  with_ivs = false: counts only.
 static int run_bsearch(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff, uint32_t nq, uint32_t cap,
-                       bool with_ivs, uint32_t* d_counts, uint32_t& launches) {
+                       bool with_ivs, uint32_t* d_counts, uint32_t& launches, uint32_t& other) {
   const FmDev& F = x->fwd;
   RET(x->nhits.ensure((size_t)nq * 8 + 8)); RET(x->niv.ensure((size_t)nq * 4 + 4));
   RET(x->ivoff.ensure((size_t)nq * 8 + 8)); RET(x->status.ensure((size_t)nq * 4 + 4));
@@ -475,6 +492,11 @@ static int run_bsearch(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       launches++;
       CK(cudaGetLastError());
     }
+    auto scan_counts = [&]() -> int {
+      return with_ivs ? scan_pair(x, x->niv.as<uint32_t>(), x->nhits.as<uint64_t>(), nq, x->seg_base.as<uint64_t>(),
+                                  x->pos_base.as<uint64_t>(), &dctr(x)->totals, other) : HFM_OK;
+    };
+    RET(scan_counts());
     RET(read_ctr(x));
     uint32_t n_ovf = x->h_ctr->n_ovf;
     if (n_ovf) {
@@ -497,6 +519,7 @@ static int run_bsearch(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
         WITH_FMT(F.fmt, { if (x->count_work) go(k_bsearch_warp<true, FM>); else go(k_bsearch_warp<false, FM>); });
         launches++;
         CK(cudaGetLastError());
+        RET(scan_counts());
         RET(read_ctr(x));
         if (x->h_ctr->still_ovf == 0) break;
         if (set_cap >= (1u << 24)) return set_error(HFM_E_OVERFLOW, "interval set exceeds 2^24 intervals");
@@ -590,8 +613,9 @@ static void begin_stats(hfm_index* x) {
   x->k_search_rec = x->k_resolve_rec = false;
   cudaEventRecord(x->ev[0], x->stream);
 }
-static int end_stats(hfm_index* x) {
+static int end_stats(hfm_index* x, bool counters = false) {
   cudaEventRecord(x->ev[2], x->stream);
+  if (counters) RET(read_ctr(x));        // the same wait serves both
   RET(wait_event(x, x->ev[2]));
   float a = 0, b = 0;
   cudaEventElapsedTime(&a, x->ev[0], x->ev[1]);
@@ -610,7 +634,8 @@ static int end_stats(hfm_index* x) {
 static int count_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff, uint32_t nq, uint32_t* d_counts) {
   begin_stats(x);
   uint32_t launches = 0;
-  RET(run_bsearch(x, d_q, d_qoff, nq, 0, false, d_counts, launches));
+  uint32_t other = 0;
+  RET(run_bsearch(x, d_q, d_qoff, nq, 0, false, d_counts, launches, other));
   cudaEventRecord(x->ev[1], x->stream);
   RET(end_stats(x));
   x->stats.search_launches = launches;
@@ -622,14 +647,11 @@ static int locate_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qof
   begin_stats(x);
   uint32_t launches = 0, other = 0;
   RET(x->counts.ensure((size_t)nq * 4 + 4));
-  RET(run_bsearch(x, d_q, d_qoff, nq, cap, true, x->counts.as<uint32_t>(), launches));
   RET(x->seg_base.ensure(((size_t)nq + 1) * 8));
   RET(x->pos_base.ensure(((size_t)nq + 1) * 8));
-  RET(scan(x, x->niv.as<uint32_t>(), 1, nq, x->seg_base.as<uint64_t>(), other));
-  RET(scan(x, x->nhits.as<uint64_t>(), 1, nq, x->pos_base.as<uint64_t>(), other));
-  uint64_t nseg = 0, total = 0;
-  RET(read_u64(x, x->seg_base.as<uint64_t>() + nq, nseg));
-  RET(read_u64(x, x->pos_base.as<uint64_t>() + nq, total));
+  // the search scans its interval and hit counts itself, before it reads its counters
+  RET(run_bsearch(x, d_q, d_qoff, nq, cap, true, x->counts.as<uint32_t>(), launches, other));
+  const uint64_t nseg = x->h_ctr->totals.a, total = x->h_ctr->totals.b;
   RET(x->seg_row.ensure(nseg * 4 + 4));
   RET(x->seg_off.ensure((nseg + 1) * 8));
   RET(x->out_pairs.ensure(total * 8 + 8));
@@ -641,13 +663,12 @@ static int locate_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qof
     other++;
     CK(cudaGetLastError());
   }
-  CK(cudaMemcpyAsync(x->seg_off.as<uint64_t>() + nseg, &total, 8, cudaMemcpyHostToDevice, x->stream));
+  CK(cudaMemcpyAsync(x->seg_off.as<uint64_t>() + nseg, x->pos_base.as<uint64_t>() + nq, 8, cudaMemcpyDeviceToDevice, x->stream));
   cudaEventRecord(x->ev[1], x->stream);
   uint32_t rl = 0;
   RET(resolve_segments(x, x->fwd, x->seg_row.as<uint32_t>(), 1, x->seg_off.as<uint64_t>(), nseg, total,
               x->fwd.bounds.as<uint32_t>(), (uint32_t)x->fwd.seq_boundaries.size(), x->out_pairs.as<uint32_t>(), rl, other));
-  RET(read_ctr(x));
-  RET(end_stats(x));
+  RET(end_stats(x, true));
   x->stats.search_launches = launches; x->stats.resolve_launches = rl; x->stats.other_launches = other;
   x->stats.rows_resolved = total; x->stats.lf_calls = x->h_ctr->steps;
   if (x->h_ctr->walk_err) return set_error(HFM_E_WALK, "LF walk exceeded sample_rate steps: index inconsistent");
@@ -872,6 +893,15 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
     threads = std::min<uint64_t>(full_threads, ((n_units + n_fast + lanes - 1) / lanes + 3) / 4 * 128);
   }
   RET(x->hit_start.ensure(n_slots * 8 + 8)); RET(x->hit_count.ensure(n_slots * 4 + 4));
+  RET(x->pos_count.ensure(n_slots * 8 + 8)); RET(x->slot_pos.ensure((n_slots + 1) * 8));
+  RET(x->hit_base.ensure(((size_t)nq + 1) * 8));
+  if (slot_base) RET(x->slot_hits.ensure((n_slots + 1) * 8));
+  uint64_t* slot_hits = slot_base ? x->slot_hits.as<uint64_t>() : x->hit_base.as<uint64_t>();
+  // the totals come with the counters of the last search pass
+  auto scan_hits = [&]() -> int {
+    return scan_pair(x, x->hit_count.as<uint32_t>(), x->pos_count.as<uint64_t>(), n_slots, slot_hits,
+                     x->slot_pos.as<uint64_t>(), &dctr(x)->totals, other);
+  };
   const bool plain = variant == MEMS_PLAIN;
   if (plain && (order || n_warp)) return set_error(HFM_E_ARG, "the plain launch takes no schedule");
   if (!plain) {
@@ -883,7 +913,7 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
     // search, read back and prefix-summed to size the outputs before the write pass
     RET(x->npos.ensure((size_t)nq * 4 + 4));
     CK(cudaMemsetAsync(x->ctr.p, 0, sizeof(Counters), x->stream));
-    MemsOut oc{x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), x->status.as<uint32_t>(),
+    MemsOut oc{x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), x->pos_count.as<uint64_t>(), x->status.as<uint32_t>(),
                x->ovf.as<uint32_t>(), &dctr(x)->n_ovf, &dctr(x)->touches};
     Pool none{nullptr, &dctr(x)->iv_used, 0};
     cudaEventRecord(x->evk[0], x->stream);
@@ -917,7 +947,7 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
     if (wlog && nq) CK(cudaMemsetAsync(wlog, 0, (size_t)nq * 16, x->stream));
     if (!plain && nq) CK(cudaMemsetAsync(x->status.p, 0, (size_t)nq * 4, x->stream));
     Pool ivp{x->mivpool.p, &dctr(x)->iv_used, x->miv_cap}, hp{x->hitpool.p, &dctr(x)->hit_used, x->hit_cap};
-    MemsOut o{x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), x->status.as<uint32_t>(),
+    MemsOut o{x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), x->pos_count.as<uint64_t>(), x->status.as<uint32_t>(),
               x->ovf.as<uint32_t>(), &dctr(x)->n_ovf, &dctr(x)->touches};
     if (n_warp) {   // reads the schedule sends straight to the warp-per-read kernel head the long-tail list
       CK(cudaMemcpyAsync(x->ovf.p, order, (size_t)n_warp * 4, cudaMemcpyDeviceToDevice, x->stream));
@@ -1010,8 +1040,10 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       cudaEventRecord(x->evk[1], x->stream);
       x->k_search_rec = true;
     }
+    RET(scan_hits());
     RET(read_ctr(x));
     uint32_t n_ovf = x->h_ctr->n_ovf;
+    const bool later_pass = n_ovf != 0;
     const uint32_t* wlist = x->ovf.as<uint32_t>();
     if (n_ovf) {
       x->stats.fallback_reads += n_ovf;
@@ -1122,6 +1154,7 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
         set_cap *= 4; cand_cap *= 4;
       }
     }
+    if (later_pass) { RET(scan_hits()); RET(read_ctr(x)); }
     if (x->h_ctr->iv_used <= x->miv_cap && x->h_ctr->hit_used <= x->hit_cap) { done = true; break; }
     x->miv_cap = std::max(x->miv_cap, (uint64_t)(x->h_ctr->iv_used * 3 / 2 + 4096));
     x->hit_cap = std::max(x->hit_cap, (uint64_t)(x->h_ctr->hit_used * 3 / 2 + 4096));
@@ -1129,33 +1162,22 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
   if (!done) return set_error(HFM_E_OVERFLOW, "MEM pools did not converge");
   x->stats.occ_touches += x->h_ctr->touches;
   // CSR of hits (over the slots, then per read), then positions
-  RET(x->hit_base.ensure(((size_t)nq + 1) * 8));
-  if (slot_base) RET(x->slot_hits.ensure((n_slots + 1) * 8));
-  uint64_t* slot_hits = slot_base ? x->slot_hits.as<uint64_t>() : x->hit_base.as<uint64_t>();
-  RET(scan(x, x->hit_count.as<uint32_t>(), 1, n_slots, slot_hits, other));
-  uint64_t nh = 0;
-  RET(read_u64(x, slot_hits + n_slots, nh));
+  const uint64_t nh = x->h_ctr->totals.a, npos = x->h_ctr->totals.b;
   RET(x->hits.ensure(nh * 32 + 32));
+  RET(x->npos_scan.ensure((nh + 1) * 8));
   if (nq) {
     if (slot_base) {
       k_slot_to_read<<<(nq + 256) / 256, 256, 0, x->stream>>>(slot_hits, slot_base, nq, x->hit_base.as<uint64_t>());
       other++;
     }
     k_gather_hits<<<(unsigned)((n_slots + 255) / 256), 256, 0, x->stream>>>(
-        x->hitpool.as<uint4>(), x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), slot_hits, (uint32_t)n_slots,
-        x->hits.as<uint4>());
+        x->hitpool.as<uint4>(), x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), slot_hits, x->slot_pos.as<uint64_t>(),
+        n_slots, x->hits.as<uint4>(), x->npos_scan.as<uint64_t>());
     other++;
     CK(cudaGetLastError());
   }
-  RET(x->npos_scan.ensure((nh + 1) * 8));
-  RET(scan(x, x->hits.as<uint32_t>() + 5, 8, nh, x->npos_scan.as<uint64_t>(), other));
-  uint64_t npos = 0;
-  RET(read_u64(x, x->npos_scan.as<uint64_t>() + nh, npos));
-  if (nh) {
-    k_set_pos_off<<<(unsigned)((nh + 255) / 256), 256, 0, x->stream>>>(x->hits.as<uint32_t>(), x->npos_scan.as<uint64_t>(), nh);
-    other++;
-    CK(cudaGetLastError());
-  }
+  CK(cudaMemcpyAsync(x->npos_scan.as<uint64_t>() + nh, x->slot_pos.as<uint64_t>() + n_slots, 8, cudaMemcpyDeviceToDevice,
+                     x->stream));
   if (wlog && nq) {
     k_work_log<<<(nq + 255) / 256, 256, 0, x->stream>>>(x->hit_base.as<uint64_t>(), x->npos_scan.as<uint64_t>(), nq, wlog);
     other++;
@@ -1166,8 +1188,7 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
   uint32_t rl = 0;
   RET(resolve_segments(x, Fw, x->hits.as<uint32_t>() + 4, 8, x->npos_scan.as<uint64_t>(), nh, npos,
               x->ref_bounds.as<uint32_t>(), nb, x->out_pairs.as<uint32_t>(), rl, other));
-  RET(read_ctr(x));
-  RET(end_stats(x));
+  RET(end_stats(x, true));
   x->stats.search_launches = launches; x->stats.resolve_launches = rl; x->stats.other_launches = other;
   x->stats.rows_resolved = npos; x->stats.lf_calls = x->h_ctr->steps; x->stats.hits_out = nh;
   if (x->h_ctr->walk_err) return set_error(HFM_E_WALK, "LF walk exceeded sample_rate steps: index inconsistent");
@@ -1241,6 +1262,7 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
   if (scap >= 0xFFFFFFFFull) return set_error(HFM_E_ARG, "read segment capacity above 2^32");
   // work buffers
   RET(x->hit_start.ensure(scap * 8 + 8)); RET(x->hit_count.ensure(scap * 4 + 4));
+  RET(x->pos_count.ensure(scap * 8 + 8)); RET(x->slot_pos.ensure((scap + 1) * 8));
   RET(x->status.ensure((size_t)nq * 4 + 4)); RET(x->ovf.ensure((size_t)nq * 4 + 4));
   RET(x->mivpool.ensure(x->miv_cap * 16)); RET(x->hitpool.ensure(hcap * 32));
   if (!launch) {                     // occupancy queried outside the capture
@@ -1289,7 +1311,7 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
   const MemsParams& P = c.P;
   Counters* dc = dctr(x);
   Pool ivp{x->mivpool.p, &dc->iv_used, x->miv_cap}, hp{x->hitpool.p, &dc->hit_used, hcap};
-  MemsOut o{x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), x->status.as<uint32_t>(),
+  MemsOut o{x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), x->pos_count.as<uint64_t>(), x->status.as<uint32_t>(),
             x->ovf.as<uint32_t>(), &dc->n_ovf, &dc->touches};
   const uint16_t* cfw = Fw.compat.as<uint16_t>();
   const uint16_t* crv = Rv.compat.as<uint16_t>();
@@ -1332,6 +1354,7 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
   if (launch) {
     CK(cudaMemsetAsync(x->status.p, 0, (size_t)nq * 4, x->stream));
     CK(cudaMemsetAsync(x->hit_count.p, 0, scap * 4, x->stream));        // slots past the count stay empty
+    CK(cudaMemsetAsync(x->pos_count.p, 0, scap * 8, x->stream));
     MemsWork W{};
     W.sets = x->memwork.as<BIv>(); W.set_cap = MEM_SET_CAP; W.hits = x->cwork.as<uint4>(); W.hit_cap = FAST_HIT_CAP;
     W.queue = &dc->queue; W.still_ovf = &dc->still_ovf; W.chunk = x->queue_chunk;
@@ -1365,21 +1388,17 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
     k_mems_warp<false><<<wgrid, 128, 0, x->stream>>>(Fw.d, Rv.d, cfw, crv, c.d_q, c.d_qoff, P, ivp, hp, o, Ww);
     CK(cudaGetLastError());
   }
-  // CSR of MemHits (hits past the count stay zero, so their position counts add nothing)
+  // CSR of MemHits; segments past the count are empty
   uint64_t* slot_hits = seg ? x->slot_hits.as<uint64_t>() : x->hit_base.as<uint64_t>();
-  RET(SCAN(x->hit_count.as<uint32_t>(), 1, scap, slot_hits));
+  RET(scan_pair(x, x->hit_count.as<uint32_t>(), x->pos_count.as<uint64_t>(), scap, slot_hits, x->slot_pos.as<uint64_t>(),
+                &dc->totals, dummy, launch));
   if (launch) {
     if (seg) k_slot_to_read<<<(nq + 256) / 256, 256, 0, x->stream>>>(slot_hits, slot_base, nq, x->hit_base.as<uint64_t>());
-    CK(cudaMemsetAsync(x->hits.p, 0, (hcap + 1) * 32, x->stream));
     k_gather_hits<<<(unsigned)((scap + 255) / 256), 256, 0, x->stream>>>(
-        x->hitpool.as<uint4>(), x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), slot_hits, (uint32_t)scap,
-        x->hits.as<uint4>());
-    CK(cudaGetLastError());
-  }
-  RET(SCAN(x->hits.as<uint32_t>() + 5, 8, hcap, x->npos_scan.as<uint64_t>()));
-  if (launch) {
-    k_set_pos_off<<<(unsigned)((hcap + 255) / 256), 256, 0, x->stream>>>(x->hits.as<uint32_t>(), x->npos_scan.as<uint64_t>(),
-                                                                        hcap);
+        x->hitpool.as<uint4>(), x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), slot_hits, x->slot_pos.as<uint64_t>(),
+        scap, x->hits.as<uint4>(), x->npos_scan.as<uint64_t>(), hcap);
+    k_seal_segments<<<(unsigned)std::min<uint64_t>((hcap + 256) / 256, 65535), 256, 0, x->stream>>>(
+        x->npos_scan.as<uint64_t>(), slot_hits + scap, x->slot_pos.as<uint64_t>() + scap, hcap);
     CK(cudaGetLastError());
   }
   const uint32_t* seg_row = x->hits.as<uint32_t>() + 4;
@@ -1512,8 +1531,9 @@ static int fixed_locate(hfm_index* x, FixedLocate& c, bool launch) {
                                                            x->nhits.as<uint64_t>());
     CK(cudaGetLastError());
   }
-  RET(SCAN(x->niv.as<uint32_t>(), 1, nq, x->seg_base.as<uint64_t>()));      // seg_base[nq] = intervals
-  RET(SCAN(x->nhits.as<uint64_t>(), 1, nq, x->pos_base.as<uint64_t>()));    // pos_base[nq] = positions
+  // seg_base[nq] = intervals, pos_base[nq] = positions
+  RET(scan_pair(x, x->niv.as<uint32_t>(), x->nhits.as<uint64_t>(), nq, x->seg_base.as<uint64_t>(), x->pos_base.as<uint64_t>(),
+                &dc->totals, dummy, launch));
   const uint64_t* seg_off = x->seg_off.as<uint64_t>();
   const uint32_t* seg_row = x->seg_row.as<uint32_t>();
   const uint32_t guard = F.rate ? F.rate : F.text_len;
@@ -1918,7 +1938,7 @@ int hfm_index_device_bytes(const hfm_index* x, uint64_t* index_bytes, uint64_t* 
   const DevBuf* work_bufs[] = {
       &x->q, &x->qoff, &x->counts, &x->nhits, &x->niv, &x->ivoff, &x->status, &x->ovf, &x->ivpool, &x->hitpool,
       &x->seg_row, &x->seg_off, &x->pos_base, &x->seg_base, &x->scan_tmp, &x->out_pairs, &x->ref_bounds,
-      &x->hit_start, &x->hit_count, &x->hit_base, &x->hits, &x->npos_scan, &x->work, &x->cwork, &x->ctr,
+      &x->hit_start, &x->hit_count, &x->pos_count, &x->slot_pos, &x->hit_base, &x->hits, &x->npos_scan, &x->work, &x->cwork, &x->ctr,
       &x->mivpool, &x->bswork, &x->memwork, &x->hkeys, &x->hslot, &x->hflags, &x->huid, &x->urow, &x->ulen,
       &x->uoff, &x->uout, &x->blockmap, &x->blockmap2, &x->ovf2, &x->ovf3, &x->lflag, &x->lpos, &x->sids,
       &x->lids, &x->ucount, &x->ubase, &x->uread, &x->uk, &x->nslot, &x->slot_base, &x->slot_hits, &x->npos,
@@ -1947,7 +1967,7 @@ void hfm_index_free(hfm_index* x) {
                     &x->fwd.compat, &x->rev.occ, &x->rev.ssa, &x->rev.sa_vals, &x->rev.lut,
                     &x->rev.bounds, &x->rev.compat, &x->q, &x->qoff, &x->counts, &x->nhits, &x->niv, &x->ivoff,
                     &x->status, &x->ovf, &x->ivpool, &x->hitpool, &x->seg_row, &x->seg_off, &x->pos_base,
-                    &x->seg_base, &x->scan_tmp, &x->out_pairs, &x->ref_bounds, &x->hit_start, &x->hit_count,
+                    &x->seg_base, &x->scan_tmp, &x->out_pairs, &x->ref_bounds, &x->hit_start, &x->hit_count, &x->pos_count, &x->slot_pos,
                     &x->hit_base, &x->hits, &x->npos_scan, &x->work, &x->cwork, &x->ctr, &x->mivpool, &x->bswork, &x->memwork,
                     &x->hkeys, &x->hslot, &x->hflags, &x->huid, &x->urow, &x->ulen, &x->uoff, &x->uout,
                     &x->blockmap, &x->blockmap2, &x->ovf2, &x->ovf3, &x->lflag, &x->lpos, &x->sids, &x->lids,
@@ -2056,6 +2076,7 @@ int hfm_mems_reserve(hfm_index* x, uint32_t nq, uint64_t intervals, uint64_t hit
   RET(x->npos_scan.ensure((hits + 1) * 8));
   RET(x->out_pairs.ensure(positions * 8 + 8));
   RET(x->hit_start.ensure((size_t)nq * 8 + 8)); RET(x->hit_count.ensure((size_t)nq * 4 + 4));
+  RET(x->pos_count.ensure((size_t)nq * 8 + 8)); RET(x->slot_pos.ensure(((size_t)nq + 1) * 8));
   RET(x->hit_base.ensure(((size_t)nq + 1) * 8));
   RET(x->status.ensure((size_t)nq * 4 + 4)); RET(x->ovf.ensure((size_t)nq * 4 + 4));
   return HFM_OK;

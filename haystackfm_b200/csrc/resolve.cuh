@@ -335,6 +335,75 @@ __global__ void k_scan_add(uint64_t* out, uint64_t n, const uint64_t* __restrict
   if (i == 0) out[n] = sums[ntiles];
 }
 
+// ---- exclusive scans of two arrays at once (u32 and u64), out[n] = totals ------------
+// The tiles' own sums first; then every block adds the sums of the tiles before its own, which
+// it sums itself (a launch and a round through one block less than a scan of the sums: the
+// scan of a batch of up to SCAN_TILE is one launch).
+struct ScanPair { unsigned long long a, b; };
+
+__device__ __forceinline__ ScanPair block_scan_pair(ScanPair v, ScanPair* s_warp, ScanPair& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  ScanPair x = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned long long ya = __shfl_up_sync(0xFFFFFFFFu, x.a, d), yb = __shfl_up_sync(0xFFFFFFFFu, x.b, d);
+    if (lane >= d) { x.a += ya; x.b += yb; }
+  }
+  if (lane == 31) s_warp[warp] = x;
+  __syncthreads();
+  ScanPair before{0, 0};
+  total = ScanPair{0, 0};
+#pragma unroll
+  for (int w = 0; w < SCAN_T / 32; w++) {
+    const ScanPair t = s_warp[w];
+    if (w < warp) { before.a += t.a; before.b += t.b; }
+    total.a += t.a; total.b += t.b;
+  }
+  __syncthreads();
+  return ScanPair{x.a - v.a + before.a, x.b - v.b + before.b};
+}
+
+__global__ void __launch_bounds__(SCAN_T) k_scan_pair_tiles(const uint32_t* __restrict__ in_a, const uint64_t* __restrict__ in_b,
+                                                           uint64_t n, uint64_t* __restrict__ out_a, uint64_t* __restrict__ out_b,
+                                                           ScanPair* __restrict__ sums, ScanPair* __restrict__ totals) {
+  __shared__ ScanPair s_warp[SCAN_T / 32];
+  const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE + (uint64_t)threadIdx.x * SCAN_ITEMS;
+  unsigned long long va[SCAN_ITEMS], vb[SCAN_ITEMS];
+  ScanPair sum{0, 0}, total;
+#pragma unroll
+  for (int k = 0; k < SCAN_ITEMS; k++) {
+    const uint64_t i = base + k;
+    va[k] = i < n ? in_a[i] : 0; vb[k] = i < n ? in_b[i] : 0;
+    sum.a += va[k]; sum.b += vb[k];
+  }
+  ScanPair run = block_scan_pair(sum, s_warp, total);
+#pragma unroll
+  for (int k = 0; k < SCAN_ITEMS; k++) {
+    const uint64_t i = base + k;
+    if (i < n) { out_a[i] = run.a; out_b[i] = run.b; }
+    run.a += va[k]; run.b += vb[k];
+  }
+  if (threadIdx.x == 0) {
+    sums[blockIdx.x] = total;
+    if (gridDim.x == 1) { out_a[n] = total.a; out_b[n] = total.b; *totals = total; }
+  }
+}
+
+__global__ void __launch_bounds__(SCAN_T) k_scan_pair_add(uint64_t n, uint64_t* __restrict__ out_a, uint64_t* __restrict__ out_b,
+                                                         const ScanPair* __restrict__ sums, ScanPair* __restrict__ totals) {
+  __shared__ ScanPair s_warp[SCAN_T / 32];
+  ScanPair mine{0, 0}, before;
+  for (uint32_t t = threadIdx.x; t < blockIdx.x; t += SCAN_T) { mine.a += sums[t].a; mine.b += sums[t].b; }
+  block_scan_pair(mine, s_warp, before);
+  const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
+  for (uint64_t i = base + threadIdx.x; i < min(n, base + SCAN_TILE); i += SCAN_T) { out_a[i] += before.a; out_b[i] += before.b; }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    const ScanPair last = sums[blockIdx.x], total{before.a + last.a, before.b + last.b};
+    out_a[n] = total.a; out_b[n] = total.b;
+    *totals = total;
+  }
+}
+
 // ---- gathers ------------------------------------------------------------------
 // Locate: query intervals (pool) -> resolve segments in query order.
 __global__ void k_gather_locate(const uint2* __restrict__ ivpool, const uint64_t* __restrict__ ivoff,
@@ -353,22 +422,26 @@ __global__ void k_gather_locate(const uint2* __restrict__ ivpool, const uint64_t
   }
 }
 
-// Mems: per-read hits (pool) -> CSR hit array.
+// Mems: hits of every slot (pool) -> CSR hit array, with the offsets of their positions, also
+// as the resolve's segment offsets.
 __global__ void k_gather_hits(const uint4* __restrict__ hitpool, const uint64_t* __restrict__ hit_start,
                               const uint32_t* __restrict__ hit_count, const uint64_t* __restrict__ hit_base,
-                              uint32_t nq, uint4* __restrict__ hits) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nq) return;
+                              const uint64_t* __restrict__ pos_base, uint64_t n_slots, uint4* __restrict__ hits,
+                              uint64_t* __restrict__ seg_off, uint64_t hit_cap = ~0ull) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_slots) return;
+  const uint32_t n = hit_count[i];
   const uint4* src = hitpool + hit_start[i] * 2;
-  uint4* dst = hits + hit_base[i] * 2;
-  for (uint32_t k = 0; k < hit_count[i] * 2; k++) dst[k] = src[k];
-}
-
-__global__ void k_set_pos_off(uint32_t* __restrict__ hits, const uint64_t* __restrict__ pos_off, uint64_t nh) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nh) return;
-  uint64_t o = pos_off[i];
-  hits[i * 8 + 6] = (uint32_t)o; hits[i * 8 + 7] = (uint32_t)(o >> 32);
+  const uint64_t base = hit_base[i];
+  uint64_t run = pos_base[i];
+  for (uint32_t k = 0; k < n && base + k < hit_cap; k++) {
+    uint4 b = src[2 * k + 1];
+    b.z = (uint32_t)run; b.w = (uint32_t)(run >> 32);
+    hits[2 * (base + k)] = src[2 * k];
+    hits[2 * (base + k) + 1] = b;
+    seg_off[base + k] = run;
+    run += b.y;
+  }
 }
 
 // Per-read work record, words 1 and 2: MemHits and positions reported for read i.

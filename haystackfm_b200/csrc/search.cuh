@@ -539,8 +539,9 @@ __device__ __forceinline__ bool any_extend(const DevFm& X, const SmemFm& S, uint
 struct Cand { uint32_t qs, qe, count, nivs; uint64_t ivoff; uint32_t pivot, _pad; };
 
 struct MemsOut {
-  uint64_t* hit_start;      // per read: offset of its hits in the hit pool
-  uint32_t* hit_count;      // per read: number of hits
+  uint64_t* hit_start;      // per slot (read or segment): offset of its hits in the hit pool
+  uint32_t* hit_count;      // per slot: number of hits
+  uint64_t* pos_count;      // per slot: positions of its hits
   uint32_t* status;
   uint32_t* ovf_list;
   uint32_t* n_ovf;
@@ -718,8 +719,9 @@ __device__ __forceinline__ uint32_t finalize_smems(Cand* c, uint32_t n) {
 // Writes the hits of one read (one per SA interval of each surviving MEM) into the hit
 // pool; returns false on pool exhaustion.
 __device__ __forceinline__ bool write_hits(Cand* c, uint32_t n, const MemsParams& P, Pool& ivpool,
-                                           Pool& hitpool, uint64_t& start, uint32_t& count) {
+                                           Pool& hitpool, uint64_t& start, uint32_t& count, uint64_t& positions) {
   uint32_t total = 0;
+  positions = 0;
   for (uint32_t k = 0; k < n; k++) total += c[k].nivs;
   count = total;
   if (total == 0) { start = 0; return true; }
@@ -733,6 +735,7 @@ __device__ __forceinline__ bool write_hits(Cand* c, uint32_t n, const MemsParams
     for (uint32_t t = 0; t < c[k].nivs; t++) {
       uint32_t sz = ivs[t].fhi - ivs[t].flo;
       uint32_t eff = P.resolve ? min(sz, P.max_hits) : 0u;
+      positions += eff;
       uint4 a = make_uint4(c[k].qs, c[k].qe, sz, sz > P.max_hits ? 1u : 0u);
       uint4 b = make_uint4(ivs[t].flo, eff, 0u, 0u);
       reinterpret_cast<uint4*>(h)[0] = a; reinterpret_cast<uint4*>(h)[1] = b;
@@ -845,19 +848,19 @@ __global__ void __launch_bounds__(128) k_mems_plain(DevFm Fw, DevFm Rv, const ui
     // reads the count pass found too large for local memory keep their flags; a pool
     // overflow of an earlier attempt is cleared (the host regrew the pools)
     uint32_t st = out.status[i] & (ST_SET_OVF | ST_CAND_OVF);
-    uint64_t hs = 0; uint32_t hc = 0;
+    uint64_t hs = 0, hp = 0; uint32_t hc = 0;
     if (st == ST_OK) {
       CandSink<SR> sink{cands, 0, (uint32_t)PLAIN_KC, &ivpool, &st, PLAIN_SET_CAP};
       uint32_t nc = mems_sweep<COUNT_TOUCH, FMT>(Fw, Rv, Sf, Sr, q + o, len, P, s0, s1, s2, s3, PLAIN_SET_CAP, sink,
                                                  st, touches);
       if (nc != ~0u) {
         if (P.mode == 0) nc = finalize_smems(cands, nc);
-        if (!write_hits(cands, nc, P, ivpool, hitpool, hs, hc)) st |= ST_POOL_OVF;
+        if (!write_hits(cands, nc, P, ivpool, hitpool, hs, hc, hp)) st |= ST_POOL_OVF;
       }
-      if (st) { hs = 0; hc = 0; }
+      if (st) { hs = 0; hc = 0; hp = 0; }
     }
     out.status[i] = st;
-    out.hit_start[i] = hs; out.hit_count[i] = hc;
+    out.hit_start[i] = hs; out.hit_count[i] = hc; out.pos_count[i] = hp;
     if (st & (ST_SET_OVF | ST_CAND_OVF)) out.ovf_list[atomicAdd(out.n_ovf, 1u)] = i;
   }
   if (COUNT_TOUCH && touches) atomicAdd(out.touches, (unsigned long long)touches);
@@ -1001,7 +1004,7 @@ __device__ __forceinline__ uint32_t grp_excl_scan(uint32_t v, uint32_t& total) {
 // ballots, pass 2 places), then touching neighbours coalesced: an interval is the first of its
 // run when it does not touch the one before it, so a run's place is the number of firsts up
 // to it and every lane writes the ends that it knows.  (Coalesced by lane 0 alone, 5,000
-// patterns with an N among the seeded codes took WARP_BEFORE ms of 500,000; now WARP_AFTER.)
+// patterns with an N among the seeded codes took 2.4 ms of 500,000; now 1.1.)
 template <bool COUNT_TOUCH, uint32_t FMT>
 __device__ uint32_t warp_backward_search(const DevFm& F, const SmemFm& S, const DevAux& A, const uint8_t* p, uint32_t m,
                                          uint2*& cur, uint2*& nxt, uint32_t cap, uint64_t& touches) {
@@ -1267,15 +1270,15 @@ __global__ void __launch_bounds__(128) k_mems_warp(DevFm Fw, DevFm Rv, const uin
       if (lane == 0) { W.work_log[4 * (size_t)i] += d; W.work_log[4 * (size_t)i + 3] |= 3u; }
     }
     if (lane == 0) {
-      uint64_t hs = 0; uint32_t hc = 0;
+      uint64_t hs = 0, hp = 0; uint32_t hc = 0;
       if (nc != ~0u) {
-        if (!write_hits(cands, nc, P, ivpool, hitpool, hs, hc)) st |= ST_POOL_OVF;
+        if (!write_hits(cands, nc, P, ivpool, hitpool, hs, hc, hp)) st |= ST_POOL_OVF;
       }
-      if (st) { hs = 0; hc = 0; }
+      if (st) { hs = 0; hc = 0; hp = 0; }
       const uint64_t slot = W.slot_base ? W.slot_base[i] : (uint64_t)i;
-      out.hit_start[slot] = hs; out.hit_count[slot] = hc; out.status[i] = st;
+      out.hit_start[slot] = hs; out.hit_count[slot] = hc; out.pos_count[slot] = hp; out.status[i] = st;
       if (W.slot_base)
-        for (uint64_t x = slot + 1; x < W.slot_base[i + 1]; x++) out.hit_count[x] = 0;
+        for (uint64_t x = slot + 1; x < W.slot_base[i + 1]; x++) { out.hit_count[x] = 0; out.pos_count[x] = 0; }
       if (st & (ST_SET_OVF | ST_CAND_OVF)) {
         if (W.rerun) atomicAdd(W.still_ovf, 1u);
         else out.ovf_list[atomicAdd(out.n_ovf, 1u)] = i;      // on to the warp tier

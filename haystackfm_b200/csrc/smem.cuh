@@ -349,21 +349,21 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
       }
     }
     if (ph == DONE) {
-      uint64_t hs = 0;
+      uint64_t hs = 0, hp = 0;
       if (st) nh = 0;
       if (nh) {
         hs = thread_reserve(hitpool, nh);
         if (hs == ~0ull) { st |= ST_POOL_OVF; hs = 0; nh = 0; }
         else {
           uint4* dst = (uint4*)hitpool.base + hs * 2;
-          for (uint32_t k = 0; k < 2 * nh; k++) dst[k] = hits[k];
+          for (uint32_t k = 0; k < 2 * nh; k++) { const uint4 v = hits[k]; dst[k] = v; if (k & 1) hp += v.y; }
         }
       }
       const bool unit = u < n_units;
       const uint64_t slot = (J.slot_base ? J.slot_base[read] : (uint64_t)read) + (unit ? J.unit_k[u] : 0u);
-      out.hit_start[slot] = hs; out.hit_count[slot] = nh;
+      out.hit_start[slot] = hs; out.hit_count[slot] = nh; out.pos_count[slot] = hp;
       if (!unit && J.slot_base)
-        for (uint64_t k = slot + 1; k < J.slot_base[read + 1]; k++) out.hit_count[k] = 0;
+        for (uint64_t k = slot + 1; k < J.slot_base[read + 1]; k++) { out.hit_count[k] = 0; out.pos_count[k] = 0; }
       if (COUNT_TOUCH && W.work_log) {
         atomicAdd(W.work_log + 4 * (size_t)read, (uint32_t)(touches - t0));
         if (st & (ST_SET_OVF | ST_CAND_OVF)) atomicOr(W.work_log + 4 * (size_t)read + 3, 1u);

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
     const uint32_t n = mine ? (uint32_t)(qoff[read + 1] - o) : 0u;
     const uint8_t* p = q + o;
     const uint64_t slot = mine ? (J.slot_base ? J.slot_base[read] : (uint64_t)read) : 0;
-    if (mine && warp == 0) { out.hit_start[slot] = 0; out.hit_count[slot] = 0; }
+    if (mine && warp == 0) { out.hit_start[slot] = 0; out.hit_count[slot] = 0; out.pos_count[slot] = 0; }
     uint32_t alive = __ballot_sync(0xFFFFFFFFu, mine && n >= P.min_len);      // min_len >= 1 here
 
     // Hands the reads in `who` to k_smem: after [0, j), or from the start.
@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
         uint64_t off = 0;
         if (lane == r) off = thread_reserve(hitpool, cnt);
         off = __shfl_sync(0xFFFFFFFFu, off, r);
+        uint64_t hp = 0;
         if (off != ~0ull) {
           uint4* dst = (uint4*)hitpool.base + off * 2;
           for (uint32_t e = lane; e < cnt; e += 32) {
@@ -149,12 +150,16 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
             uint32_t rank = 0;
             for (uint32_t t = 0; t < cnt; t++) rank += set[t].x < v.x ? 1u : 0u;
             dst[2 * rank] = make_uint4(0u, j, v.y, v.y > P.max_hits ? 1u : 0u);
-            dst[2 * rank + 1] = make_uint4(v.x, P.resolve ? min(v.y, P.max_hits) : 0u, 0u, 0u);
+            const uint32_t positions = P.resolve ? min(v.y, P.max_hits) : 0u;
+            dst[2 * rank + 1] = make_uint4(v.x, positions, 0u, 0u);
+            hp += positions;
           }
         }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) hp += __shfl_xor_sync(0xFFFFFFFFu, hp, d);
         if (lane == r) {
           if (off == ~0ull) atomicOr(out.status + read, (uint32_t)ST_POOL_OVF);
-          else { out.hit_start[slot] = off; out.hit_count[slot] = cnt; }
+          else { out.hit_start[slot] = off; out.hit_count[slot] = cnt; out.pos_count[slot] = hp; }
         }
         __syncwarp();
       }
