@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import struct
+import weakref
 from dataclasses import dataclass, field
 from typing import List, Sequence, Tuple
 
@@ -82,6 +83,47 @@ def _take_bytes(ptr, n: int) -> bytes:
     """Copy n bytes from a library-allocated block (ctypes.string_at takes a C int size,
     too small for genome-scale indices)."""
     return np.ctypeslib.as_array(ptr, shape=(n,)).tobytes() if n else b""
+
+
+# A result block of the library (pinned host memory that the device copied into) is handed out
+# as numpy views and released when the last of them is gone: copying 98 MB of positions into
+# fresh pages took 20 ms of a 24 ms call.  Small results are copied; so is everything while the
+# views in use hold RESULT_VIEW_MAX bytes, so that a program that keeps its results does not pin
+# memory without bound.
+RESULT_VIEW_MIN = 1 << 20
+RESULT_VIEW_MAX = 4 << 30
+_viewed: dict = {}                 # address -> bytes of the blocks that views hold
+
+
+def _release_block(addr: int) -> None:
+    _viewed.pop(addr, None)
+    L.lib().hfm_free(C.c_void_p(addr))
+
+
+class _Result:
+    """The block at `addr`: arrays from it, then close()."""
+
+    def __init__(self, addr: int, nbytes: int):
+        self.addr = addr
+        self.buf = None
+        if nbytes >= RESULT_VIEW_MIN and sum(list(_viewed.values())) + nbytes <= RESULT_VIEW_MAX:
+            self.buf = (C.c_uint8 * nbytes).from_address(addr)
+            _viewed[addr] = nbytes
+            weakref.finalize(self.buf, _release_block, addr).atexit = False
+
+    def array(self, p, dtype, n: int) -> np.ndarray:
+        if not n:
+            return np.zeros(0, dtype=dtype)
+        at = C.cast(p, C.c_void_p).value
+        if self.buf is not None:
+            return np.frombuffer(self.buf, dtype=dtype, count=n, offset=at - self.addr)
+        size = n * np.dtype(dtype).itemsize
+        return np.frombuffer((C.c_uint8 * size).from_address(at), dtype=dtype).copy()
+
+    def close(self) -> None:
+        if self.buf is None:
+            L.lib().hfm_free(C.c_void_p(self.addr))
+        self.buf = None
 
 
 def _build(sequences: Sequence[DnaSequence], config: FmIndexConfig, tag: int, kind: int) -> bytes:
@@ -204,14 +246,14 @@ class _Handle:
         nq = len(off) - 1
         res = C.POINTER(L.HfmHits)()
         L.check(L.lib().hfm_locate_batch(self.h, L.ptr(flat, L.u8p), L.ptr(off, L.u64p), nq, max_hits, C.byref(res)))
+        r = res.contents
+        block = _Result(C.addressof(r), C.sizeof(L.HfmHits) + 8 * (nq + 1) + 4 * nq + 4 + 8 * r.total)
         try:
-            r = res.contents
-            offsets = np.ctypeslib.as_array(r.offsets, shape=(nq + 1,)).copy()
-            counts = np.ctypeslib.as_array(r.counts, shape=(nq,)).copy() if nq else np.zeros(0, np.uint32)
-            pairs = (np.ctypeslib.as_array(r.pairs, shape=(2 * r.total,)).reshape(-1, 2).copy()
-                     if r.total else np.zeros((0, 2), np.uint32))
+            offsets = block.array(r.offsets, np.uint64, nq + 1)
+            counts = block.array(r.counts, np.uint32, nq)
+            pairs = block.array(r.pairs, np.uint32, 2 * r.total).reshape(-1, 2)
         finally:
-            L.lib().hfm_free(res)
+            block.close()
         return counts, offsets, pairs
 
     def mems_packed(self, flat: np.ndarray, off: np.ndarray, min_len: int, mode: int, ref_bounds, max_hits: int):
@@ -224,15 +266,14 @@ class _Handle:
         res = C.POINTER(L.HfmMemOut)()
         L.check(L.lib().hfm_mems_batch(self.h, L.ptr(flat, L.u8p), L.ptr(off, L.u64p), nq, min_len, mode, rbp,
                                        len(rb), max_hits, C.byref(res)))
+        r = res.contents
+        block = _Result(C.addressof(r), C.sizeof(L.HfmMemOut) + 8 * (nq + 1) + 32 * r.n_hits + 8 * r.n_positions + 8)
         try:
-            r = res.contents
-            hit_off = np.ctypeslib.as_array(r.hit_offsets, shape=(nq + 1,)).copy()
-            hits = (np.ctypeslib.as_array(C.cast(r.hits, L.u32p), shape=(8 * r.n_hits,)).reshape(-1, 8).copy()
-                    if r.n_hits else np.zeros((0, 8), np.uint32))
-            pos = (np.ctypeslib.as_array(r.positions, shape=(2 * r.n_positions,)).reshape(-1, 2).copy()
-                   if r.n_positions else np.zeros((0, 2), np.uint32))
+            hit_off = block.array(r.hit_offsets, np.uint64, nq + 1)
+            hits = block.array(r.hits, np.uint32, 8 * r.n_hits).reshape(-1, 8)
+            pos = block.array(r.positions, np.uint32, 2 * r.n_positions).reshape(-1, 2)
         finally:
-            L.lib().hfm_free(res)
+            block.close()
         return hit_off, hits, pos
 
 
