@@ -23,12 +23,13 @@
 // forward phases there (smem.cuh): the SA intervals of the text strings that match.
 //
 // Measured on a B200, 150 bp reads on the 100 Mbp IUPAC text, kernel times of a thread per
-// read, of this sweep with a warp per group, and as it is: 200,000 reads by prefix 39.5 /
-// 12.6 / 12.7 ms, 60,000 reads - / 7.7 / 5.0, 4,099 reads 16.2 / 1.30 / 0.88, 64 reads (one
-// a block: its nodes share the threads) 10.7 / 0.67 / 0.65.  Bound by issue: some 400
-// instructions for 32 larger nodes (the 16 masks and popcounts of two borders, then their
-// children); 30 reads carry about 130 of those and as many one-row nodes a position, where
-// one read alone carries some 35.
+// read, of this sweep with a warp per group, with a block, and as it is (one warp prepares a
+// position, symbols without children skipped, both kinds of nodes at a time, five blocks an SM
+// where four had 124 registers): 200,000 reads by prefix 39.5 / 12.6 / 12.7 / 10.4 ms, 4,099
+// reads 16.2 / 1.30 / 0.88 / 0.82 ms, 64 reads (one a block: its nodes share the threads) 10.7
+// / 0.67 / 0.65 / 0.46 ms.  Bound by issue: some 400 instructions for 32 larger nodes (the 16
+// masks and popcounts of two borders, then their children); 30 reads carry about 130 of those
+// and as many one-row nodes a position, where one read alone carries some 35.
 #pragma once
 #include "smem.cuh"
 
@@ -45,7 +46,7 @@ struct TrieShared {
   uint4 one[2][TRIE_S1];
   uint4 big[2][TRIE_SB];
   uint2 set[TRIE_WARPS][TRIE_EMIT];
-  uint32_t reads[TRIE_WARPS][16];           // reads whose code matches symbol s (a copy per warp)
+  uint32_t reads[2][16];                    // reads whose code at this (the next) position matches symbol s
   // of the next list: nodes, reads that hold one.  Position j counts in [j % 3] and clears
   // the one after it, which every thread has read two barriers ago.
   uint32_t n1[3], nb[3], still[3];
@@ -70,7 +71,7 @@ struct NodeList {
 };
 
 template <bool COUNT_TOUCH>
-__global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv, const uint16_t* __restrict__ compat,
+__global__ void __launch_bounds__(TRIE_WARPS * 32, 5) k_trie(DevFm Fw, DevFm Rv, const uint16_t* __restrict__ compat,
                                                              const uint8_t* __restrict__ q,
                                                              const uint64_t* __restrict__ qoff, MemsParams P,
                                                              Pool hitpool, MemsOut out, TrieWork W, SmemJobs J) {
@@ -78,7 +79,6 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
   TrieShared& S = *reinterpret_cast<TrieShared*>(trie_smem);
   if (threadIdx.x < 16) { S.C[threadIdx.x] = Rv.C[threadIdx.x]; S.compat[threadIdx.x] = compat[threadIdx.x] & Fw.sym_mask; }
   const uint32_t lane = threadIdx.x & 31, lt = lane_lt_mask(), warp = threadIdx.x >> 5;
-  uint32_t* reads = S.reads[warp];
   uint2* set = S.set[warp];
   uint4* g = W.nodes + (size_t)blockIdx.x * 4 * TRIE_CAP;
   const uint32_t n_reads = J.whole(), n_groups = (n_reads + W.group - 1) / W.group;
@@ -173,7 +173,17 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
       if (Fw.text_len == 1) S.one[0][0] = full; else S.big[0][0] = full;
     }
     if (Fw.text_len == 1) n1 = 1; else nb = 1;
-    uint32_t code = ((alive >> lane) & 1) ? p[0] : 16u;
+    // the reads whose code c matches each symbol; a read that has ended or whose set is empty
+    // may keep its bits: no node has it any more, and one that ends here is taken out
+    auto match_reads = [&](uint32_t code, uint32_t* to) {
+      const uint32_t match = code < 16 ? S.compat[code] : 0u;
+#pragma unroll
+      for (int s = 0; s < 16; s++) {
+        const uint32_t b = __ballot_sync(0xFFFFFFFFu, (match >> s) & 1);
+        if (lane == s) to[s] = b;
+      }
+    };
+    if (warp == 0) match_reads(((alive >> lane) & 1) ? p[0] : 16u, S.reads[0]);
     __syncthreads();
     for (uint32_t j = 0, c = 0;; j++) {
       const NodeList one{S.one[t], g + (size_t)t * TRIE_CAP, TRIE_S1}, big{S.big[t], g + (size_t)(2 + t) * TRIE_CAP, TRIE_SB};
@@ -187,20 +197,13 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
       if (!alive) break;
       const uint32_t cn = c == 2 ? 0 : c + 1;
       if (threadIdx.x == 0) { S.n1[cn] = 0; S.nb[cn] = 0; S.still[cn] = 0; }
-      const uint32_t match = ((alive >> lane) & 1) && code < 16 ? S.compat[code] : 0u;
-      // the next code is on its way while this position's nodes are split
-      code = ((alive >> lane) & 1) && j + 1 < n ? p[j + 1] : 16u;
-      __syncwarp();
-#pragma unroll
-      for (int s = 0; s < 16; s++) {
-        const uint32_t b = __ballot_sync(0xFFFFFFFFu, (match >> s) & 1);
-        if (lane == s) reads[s] = b;
-      }
-      __syncwarp();
+      const uint32_t* reads = S.reads[j & 1];
+      // one warp, another each time, prepares the next position
+      if ((j & (TRIE_WARPS - 1)) == warp) match_reads(((alive >> lane) & 1) && j + 1 < n ? p[j + 1] : 16u, S.reads[(j + 1) & 1]);
       uint32_t still = 0;
       // larger nodes: their one-row children go to the one-row list
       for (uint32_t b = warp * 32; b < nb; b += TRIE_WARPS * 32) {
-        uint32_t r[16], d[16], kids = 0;
+        uint32_t r[16], d[16], kids = 0, syms = 0;
         uint4 v = make_uint4(0, 0, 0, 0);
         if (b + lane < nb) {
           v = big.get(b + lane);
@@ -208,7 +211,7 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
           if (COUNT_TOUCH) touches += 2;
 #pragma unroll
           for (int s = 1; s < 16; s++)
-            if (d[s] && (v.w & reads[s])) kids += d[s] == 1 ? 1u : 0x10000u;
+            if (d[s] && (v.w & reads[s])) { kids += d[s] == 1 ? 1u : 0x10000u; syms |= 1u << s; }
         }
         uint32_t total;
         const uint32_t at = warp_excl_scan(kids, total);
@@ -221,22 +224,24 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 4) k_trie(DevFm Fw, DevFm Rv,
         ab = __shfl_sync(0xFFFFFFFFu, ab, 0);
         if (a1 + (total & 0xFFFFu) > TRIE_CAP || ab + (total >> 16) > TRIE_CAP) break;   // the counts tell everyone
         a1 += at & 0xFFFFu; ab += at >> 16;
-        if (kids) {
-          uint32_t run = d[0];
+        const uint32_t any = __reduce_or_sync(0xFFFFFFFFu, syms);       // half of the symbols, on average
+        uint32_t run = d[0];
 #pragma unroll
-          for (int s = 1; s < 16; s++) {
-            const uint32_t who = v.w & reads[s];
-            if (d[s] && who) {
+        for (int s = 1; s < 16; s++) {
+          if ((any >> s) & 1) {
+            if ((syms >> s) & 1) {
+              const uint32_t who = v.w & reads[s];
               const uint4 kid = make_uint4(v.x + run, S.C[s] + r[s], d[s], who);
               if (d[s] == 1) one2.put(a1++, kid); else big2.put(ab++, kid);
               still |= who;
             }
-            run += d[s];
           }
+          run += d[s];
         }
       }
-      // one-row nodes: one LF step each
-      for (uint32_t b = warp * 32; b < n1; b += TRIE_WARPS * 32) {
+      // one-row nodes: one LF step each; from the last warp on, so that short lists of both
+      // kinds are worked off at the same time
+      for (uint32_t b = (TRIE_WARPS - 1 - warp) * 32; b < n1; b += TRIE_WARPS * 32) {
         uint4 kid = make_uint4(0, 0, 0, 0);
         if (b + lane < n1) {
           const uint4 v = one.get(b + lane);
