@@ -1170,7 +1170,7 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       k_slot_to_read<<<(nq + 256) / 256, 256, 0, x->stream>>>(slot_hits, slot_base, nq, x->hit_base.as<uint64_t>());
       other++;
     }
-    k_gather_hits<<<(unsigned)((n_slots + 255) / 256), 256, 0, x->stream>>>(
+    k_gather_hits<<<(unsigned)((n_slots * GATHER_LANES + 255) / 256), 256, 0, x->stream>>>(
         x->hitpool.as<uint4>(), x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), slot_hits, x->slot_pos.as<uint64_t>(),
         n_slots, x->hits.as<uint4>(), x->npos_scan.as<uint64_t>());
     other++;
@@ -1394,7 +1394,7 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
                 &dc->totals, dummy, launch));
   if (launch) {
     if (seg) k_slot_to_read<<<(nq + 256) / 256, 256, 0, x->stream>>>(slot_hits, slot_base, nq, x->hit_base.as<uint64_t>());
-    k_gather_hits<<<(unsigned)((scap + 255) / 256), 256, 0, x->stream>>>(
+    k_gather_hits<<<(unsigned)((scap * GATHER_LANES + 255) / 256), 256, 0, x->stream>>>(
         x->hitpool.as<uint4>(), x->hit_start.as<uint64_t>(), x->hit_count.as<uint32_t>(), slot_hits, x->slot_pos.as<uint64_t>(),
         scap, x->hits.as<uint4>(), x->npos_scan.as<uint64_t>(), hcap);
     k_seal_segments<<<(unsigned)std::min<uint64_t>((hcap + 256) / 256, 65535), 256, 0, x->stream>>>(
