@@ -202,21 +202,26 @@ __device__ __forceinline__ bool acgt_rows(const DevFm& F, const uint32_t* C, uin
   return true;
 }
 
-// 16 counts at the borders of rows [lo, lo + n), n >= 1, of a wide index: r[s] = rank of s at
-// lo, d[s] = rows of code s.  The records are those of the first and the last row, one when
-// they are the same.
-__device__ __forceinline__ void wide_split(const uint4* __restrict__ occ, uint32_t lo, uint32_t n, uint32_t r[16],
-                                           uint32_t d[16]) {
+// The borders of rows [lo, lo + n), n >= 1, of a wide index.  The records are those of the first
+// and the last row, one when they are the same.
+__device__ __forceinline__ void wide_borders(const uint4* __restrict__ occ, uint32_t lo, uint32_t n, Border<OCC_WIDE>& L,
+                                             Border<OCC_WIDE>& H) {
   const uint32_t last = lo + n - 1, bl = lo >> 6, bh = last >> 6, xl = lo & 63, xh = (last & 63) + 1;
   const uint4* pl = occ + (size_t)bl * OCC_WIDE_U4;
   const uint4* ph = occ + (size_t)bh * OCC_WIDE_U4;
-  Border<OCC_WIDE> L, H;
   L.a = __ldg(pl); L.b = __ldg(pl + 1); L.c = __ldg(pl + 2); L.d = __ldg(pl + 3);
   L.w = __ldg(pl + (xl >= 32 ? 5 : 4));
   H.w = __ldg(ph + (xh >= 32 ? 5 : 4));
   H.a = L.a; H.b = L.b; H.c = L.c; H.d = L.d;
   if (bh != bl) { H.a = __ldg(ph); H.b = __ldg(ph + 1); H.c = __ldg(ph + 2); H.d = __ldg(ph + 3); }
   L.select(xl); H.select(xh);
+}
+
+// 16 counts at those borders: r[s] = rank of s at lo, d[s] = rows of code s.
+__device__ __forceinline__ void wide_split(const uint4* __restrict__ occ, uint32_t lo, uint32_t n, uint32_t r[16],
+                                           uint32_t d[16]) {
+  Border<OCC_WIDE> L, H;
+  wide_borders(occ, lo, n, L, H);
   wide_ranks(L, r);
   wide_ranks(H, d);
 #pragma unroll
@@ -233,6 +238,28 @@ __device__ __forceinline__ void rows_by_code(const DevFm& F, uint32_t lo, uint32
     sym_ranks_t<FMT>(F, hi, d);
 #pragma unroll
     for (int s = 0; s < 16; s++) d[s] -= r[s];
+  }
+}
+
+// Calls f(code, rank at lo, rows) for each code of `mask` (the same in all lanes that call it)
+// in ascending order; rows may be 0.
+template <uint32_t FMT, class FN>
+__device__ __forceinline__ void each_code(const DevFm& F, uint32_t lo, uint32_t hi, uint32_t mask, FN f) {
+  if constexpr (FMT == OCC_WIDE) {
+    Border<OCC_WIDE> L, H;
+    wide_borders(F.occ, lo, hi - lo, L, H);
+#pragma unroll
+    for (int s = 0; s < 16; s++) {
+      if (!(mask >> s & 1)) continue;
+      const uint32_t r = L.local(s);
+      f(s, r, H.local(s) - r);
+    }
+  } else {
+    uint32_t r[16], d[16];
+    rows_by_code<FMT>(F, lo, hi, r, d);
+#pragma unroll
+    for (int s = 1; s < 5; s++)
+      if (mask >> s & 1) f(s, r[s], d[s]);
   }
 }
 
@@ -351,33 +378,44 @@ __device__ __forceinline__ uint32_t backward_search_one(const DevFm& F, const Sm
       for (int s = 0; s < 16; s++)
         if (((mask >> s) & 1) && d[s]) add(S.C[s] + r[s], S.C[s] + r[s] + d[s]);
     } else {
-      // Outputs for symbol s lie in [C[s], C[s+1]) in source order: a pass per symbol that
-      // occurs would read the records over, so a stable counting sort by symbol places them.
-      uint32_t cnt[16];
+      // Children of symbol s lie in [C[s], C[s+1]) in source order: they are written to nxt
+      // source by source, then placed into cur by symbol (a stable counting sort).  (Extending
+      // the sources again to place the children: 0.64 ms against 0.49 for 500,000 patterns of
+      // 32 codes on an IUPAC assembly.)
+      constexpr int S0 = FMT == OCC_NARROW ? 1 : 0, S1 = FMT == OCC_NARROW ? 5 : 16;
+      uint32_t cnt[16], total = 0;
 #pragma unroll
-      for (int s = 0; s < 16; s++) cnt[s] = 0;
+      for (int s = S0; s < S1; s++) cnt[s] = 0;
       for (uint32_t i = 0; i < n; i++) {
         const uint2 iv = cur[i];
         uint32_t r[16], d[16];
         rows_by_code<FMT>(F, iv.x, iv.y, r, d);
         if (COUNT_TOUCH) touches += 2;
 #pragma unroll
-        for (int s = 0; s < 16; s++) cnt[s] += (((mask >> s) & 1) && d[s]) ? 1u : 0u;
+        for (int s = S0; s < S1; s++) {
+          if (!((mask >> s) & 1) || !d[s]) continue;
+          cnt[s]++;
+          if (total < cap) nxt[total] = make_uint2(S.C[s] + r[s], S.C[s] + r[s] + d[s]);
+          total++;
+        }
+        if (total > cap) return ~0u;
       }
-      uint32_t total = 0;
+      uint32_t below = 0;
 #pragma unroll
-      for (int s = 0; s < 16; s++) { const uint32_t t = cnt[s]; cnt[s] = total; total += t; }
-      if (total > cap) return ~0u;
-      for (uint32_t i = 0; i < n; i++) {
-        const uint2 iv = cur[i];
-        uint32_t r[16], d[16];
-        rows_by_code<FMT>(F, iv.x, iv.y, r, d);
+      for (int s = S0; s < S1; s++) { const uint32_t t = cnt[s]; cnt[s] = below; below += t; }
+      for (uint32_t e = 0; e < total; e++) {
+        const uint2 v = nxt[e];
+        uint32_t at = 0;
 #pragma unroll
-        for (int s = 0; s < 16; s++)
-          if (((mask >> s) & 1) && d[s]) nxt[cnt[s]++] = make_uint2(S.C[s] + r[s], S.C[s] + r[s] + d[s]);
+        for (int s = S0; s < S1; s++) {
+          const bool is = v.x >= S.C[s] && (s == S1 - 1 || v.x < S.C[s + 1]);
+          at = is ? cnt[s] : at;
+          cnt[s] += is ? 1u : 0u;
+        }
+        cur[at] = v;
       }
       // coalesce touching neighbours (merge_intervals_inplace, query.rs:390-407)
-      for (uint32_t e = 0; e < total; e++) { const uint2 v = nxt[e]; add(v.x, v.y); }
+      for (uint32_t e = 0; e < total; e++) { const uint2 v = cur[e]; add(v.x, v.y); }
     }
     if (ovf) return ~0u;
     if (nn == 0) return 0;
@@ -1000,11 +1038,14 @@ __device__ __forceinline__ uint32_t grp_excl_scan(uint32_t v, uint32_t& total) {
   return x - v;
 }
 
-// Backward search of one pattern by a warp: a counting sort by symbol (pass 1 counts with
-// ballots, pass 2 places), then touching neighbours coalesced: an interval is the first of its
-// run when it does not touch the one before it, so a run's place is the number of firsts up
-// to it and every lane writes the ends that it knows.  (Coalesced by lane 0 alone, 5,000
-// patterns with an N among the seeded codes took 2.4 ms of 500,000; now 1.1.)
+// Backward search of one pattern by a warp.  The sources are extended once, 32 at a time and
+// only by the symbols of the code; the children are placed by symbol (a stable counting sort);
+// then touching neighbours are coalesced: an interval is the first of its run when it does not
+// touch the one before it, so a run's place is the number of firsts up to it and every lane
+// writes the ends that it knows.  Bound by the chain of dependent loads of a pattern, some 90
+// groups of 32 intervals on an IUPAC assembly.  5,000 patterns with an N among the seeded codes,
+// of 500,000: 2.4 ms when lane 0 coalesced alone, 1.1 when the sources were extended a second
+// time to place the children, 0.8 now.
 template <bool COUNT_TOUCH, uint32_t FMT>
 __device__ uint32_t warp_backward_search(const DevFm& F, const SmemFm& S, const DevAux& A, const uint8_t* p, uint32_t m,
                                          uint2*& cur, uint2*& nxt, uint32_t cap, uint64_t& touches) {
@@ -1022,42 +1063,50 @@ __device__ uint32_t warp_backward_search(const DevFm& F, const SmemFm& S, const 
     const uint8_t c = p[k];
     const uint32_t mask = (c < 16 ? S.compat_mask[c] : 0) & F.sym_mask;
     if (!mask) return 0;
-    uint32_t cnt[16];
-#pragma unroll
-    for (int s = 0; s < 16; s++) cnt[s] = 0;
+    // extend: 32 sources at a time, symbol by symbol; lane s < 16 counts the children of s
+    uint32_t total = 0, mine = 0;
     for (uint32_t b = 0; b < n; b += 32) {
       const uint32_t i = b + lane;
-      uint32_t r[16], d[16];
       const uint2 iv = i < n ? cur[i] : make_uint2(0, 1);
-      rows_by_code<FMT>(F, iv.x, iv.y, r, d);
       if (COUNT_TOUCH && i < n) touches += 2;
-#pragma unroll
-      for (int s = 0; s < 16; s++) cnt[s] += __popc(__ballot_sync(0xFFFFFFFFu, i < n && ((mask >> s) & 1) && d[s]));
+      each_code<FMT>(F, iv.x, iv.y, mask, [&](int s, uint32_t r, uint32_t d) {
+        const bool e = i < n && d;
+        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, e), at = total + __popc(bal & lt), k = __popc(bal);
+        if (e && at < cap) nxt[at] = make_uint2(S.C[s] + r, S.C[s] + r + d);
+        mine += lane == s ? k : 0u;
+        total += k;
+      });
+      if (total > cap) return ~0u;
     }
-    uint32_t total = 0;
-#pragma unroll
-    for (int s = 0; s < 16; s++) { const uint32_t t = cnt[s]; cnt[s] = total; total += t; }
-    if (total > cap) return ~0u;
     if (total == 0) return 0;
-    for (uint32_t b = 0; b < n; b += 32) {
-      const uint32_t i = b + lane;
-      uint32_t r[16], d[16];
-      const uint2 iv = i < n ? cur[i] : make_uint2(0, 1);
-      rows_by_code<FMT>(F, iv.x, iv.y, r, d);
-#pragma unroll
-      for (int s = 0; s < 16; s++) {
-        const bool e = i < n && ((mask >> s) & 1) && d[s];
-        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, e);
-        if (e) nxt[cnt[s] + __popc(bal & lt)] = make_uint2(S.C[s] + r[s], S.C[s] + r[s] + d[s]);
-        cnt[s] += __popc(bal);
-      }
-    }
     __syncwarp();
-    // coalesce touching neighbours into cur (merge_intervals_inplace, query.rs:390-407)
-    uint32_t nn = 0, before = 0;                        // runs so far; end of the interval before this chunk
+    // place: a child's symbol is that of the C range that holds it; its place, the symbol's
+    // first, the earlier ones of the symbol and those of lower lanes
+    uint32_t all;
+    uint32_t place = grp_excl_scan<32>(mine, all);                 // lane s: the next place of symbol s
     for (uint32_t b = 0; b < total; b += 32) {
       const uint32_t i = b + lane;
       const uint2 v = i < total ? nxt[i] : make_uint2(0, 0);
+      uint32_t s = 0;
+#pragma unroll
+      for (int t = 1; t < 16; t++) s += v.x >= S.C[t] ? 1u : 0u;
+      uint32_t same = __ballot_sync(0xFFFFFFFFu, i < total), own = same;   // of this child's symbol; of symbol `lane`
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const uint32_t bit = __ballot_sync(0xFFFFFFFFu, s >> t & 1);
+        same &= s >> t & 1 ? bit : ~bit;
+        own &= lane >> t & 1 ? bit : ~bit;
+      }
+      const uint32_t at = __shfl_sync(0xFFFFFFFFu, place, s) + __popc(same & lt);
+      if (i < total) cur[at] = v;
+      place += __popc(own);
+    }
+    __syncwarp();
+    // coalesce touching neighbours in place (merge_intervals_inplace, query.rs:390-407)
+    uint32_t nn = 0, before = 0;                        // runs so far; end of the interval before this chunk
+    for (uint32_t b = 0; b < total; b += 32) {
+      const uint32_t i = b + lane;
+      const uint2 v = i < total ? cur[i] : make_uint2(0, 0);
       uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, v.y, 1);
       if (lane == 0) prev = before;
       const bool first = i < total && (i == 0 || v.x > prev);
