@@ -1628,7 +1628,7 @@ struct PinnedCache {
 static PinnedCache& pinned_cache() { static PinnedCache* c = new PinnedCache(); return *c; }
 static constexpr size_t PINNED_CACHE_MAX = 48ull << 30;
 
-static void* host_result_alloc(size_t bytes) {
+void* host_result_alloc(size_t bytes) {
   PinnedCache& P = pinned_cache();
   std::lock_guard<std::mutex> lk(P.mu);
   auto it = P.free_blocks.lower_bound(bytes);
@@ -1648,7 +1648,7 @@ static void* host_result_alloc(size_t bytes) {
   return p;
 }
 
-static void host_result_free(void* p) {
+void host_result_free(void* p) {
   PinnedCache& P = pinned_cache();
   std::lock_guard<std::mutex> lk(P.mu);
   auto it = P.owned.find(p);

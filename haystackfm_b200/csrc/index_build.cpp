@@ -98,41 +98,21 @@ void suffix_array(const uint8_t* text, uint32_t n, uint32_t* sa) {
   sais<uint8_t>(t.data(), sa, n, 17);
 }
 
-// ---------------------------------------------------------------------------
-// bincode-1 writer (fixint, little endian; src/fm_index/serialize.rs:55-67)
-// ---------------------------------------------------------------------------
 struct BinWriter {
+  const BuiltFm& f;
   std::vector<uint8_t>& b;
   void put(const void* p, size_t k) { const uint8_t* s = (const uint8_t*)p; b.insert(b.end(), s, s + k); }
-  void u8(uint8_t v) { b.push_back(v); }
-  void u32(uint32_t v) { put(&v, 4); }
-  void u64(uint64_t v) { put(&v, 8); }
+  void section(FmSection id, uint64_t bytes) {
+    const void* p[5] = {f.sb.data(), f.block_data.data(), f.ssa_words.data(), f.sa_vals.data(), f.lut.data()};
+    put(p[id], bytes);
+  }
 };
 
-void write_fm(const BuiltFm& f, std::vector<uint8_t>& out) {
-  BinWriter w{out};
-  for (int c = 0; c < 16; c++) w.u32(f.C[c]);
-  // OccTable field order (src/occ/mod.rs:45-78)
-  w.u8(f.num_lanes); w.u8(f.num_planes); w.put(f.s2l, 16); w.put(f.l2s, 16);
-  w.u64(f.sb.size()); w.put(f.sb.data(), f.sb.size() * 4);
-  w.u64(f.block_data.size()); w.put(f.block_data.data(), f.block_data.size());
-  w.u64(f.block_stride); w.u32(f.encoding); w.u32(f.text_len);
-  // SampledSuffixArray (src/suffix_array/mod.rs:54-63)
-  w.u64(f.ssa_words.size()); w.put(f.ssa_words.data(), f.ssa_words.size());
-  w.u64(f.sa_vals.size()); w.put(f.sa_vals.data(), f.sa_vals.size() * 4);
-  w.u32(f.rate); w.u32(f.text_len);
-  w.u32(f.text_len); w.u32(f.num_sequences);
-  w.u64(f.bounds.size()); w.put(f.bounds.data(), f.bounds.size() * 4);
-  w.u64(f.headers.size());
-  for (auto& h : f.headers) { w.u64(h.size()); w.put(h.data(), h.size()); }
-  if (f.lookup_depth > 0) {   // Option<LookupTable> (src/fm_index/lookup.rs:19-27)
-    w.u8(1); w.u32(f.lookup_depth);
-    static const uint8_t core[4] = {1, 2, 3, 4};
-    w.u64(4); w.put(core, 4);
-    w.u64(f.lut.size());
-    for (auto& iv : f.lut) { w.u32(iv.first); w.u32(iv.second); }
-  } else w.u8(0);
-  w.u8(f.tag);
+static void write_built(BuiltFm& f, std::vector<uint8_t>& out) {
+  f.n_sb = f.sb.size(); f.n_block = f.block_data.size(); f.n_ssa = f.ssa_words.size();
+  f.n_vals = f.sa_vals.size(); f.n_lut = f.lut.size();
+  BinWriter w{f, out};
+  write_fm(f, w);
 }
 
 // Rank over the Occ records just built (same arithmetic as OccTable::rank, src/occ/mod.rs:330-363).
@@ -257,43 +237,56 @@ static void build_fm(const uint8_t* text, uint32_t n, const std::vector<uint32_t
 }
 
 
-// concatenate_sequences (src/alphabet.rs:375-393): codes 1..15 per sequence, a 0 sentinel
-// after each; bounds = exclusive ends; headers default to "seq_{i}".
-int concat_text(const uint8_t* codes, const uint64_t* seq_off, uint32_t nseq, const char* const* headers,
-                std::vector<uint8_t>& text, std::vector<uint32_t>& bounds, std::vector<std::string>& hs) {
+int sequence_bounds(const uint8_t* codes, const uint64_t* seq_off, uint32_t nseq, const char* const* headers,
+                    std::vector<uint32_t>& bounds, std::vector<std::string>& hs) {
   uint64_t total = 0;
   for (uint32_t s = 0; s < nseq; s++) total += seq_off[s + 1] - seq_off[s] + 1;
   if (total > 0xFFFFFFFFull) return set_error(HFM_E_ARG, "text too large: exceeds u32::MAX");
-  const uint32_t n = (uint32_t)total;
   try {
-    text.assign(n, 0); bounds.assign(nseq, 0); hs.assign(nseq, std::string());
+    bounds.assign(nseq, 0); hs.assign(nseq, std::string());
+    uint64_t pos = 0;
+    for (uint32_t s = 0; s < nseq; s++) {
+      const uint8_t* c = codes + seq_off[s];
+      const uint64_t len = seq_off[s + 1] - seq_off[s];
+      uint8_t bad = 0;                                      // no early exit: the loop is vectorised
+      for (uint64_t k = 0; k < len; k++) bad |= (uint8_t)(c[k] - 1) > 14 ? 1 : 0;
+      if (bad) return set_error(HFM_E_ARG, "invalid code in sequence");
+      pos += len + 1;
+      bounds[s] = (uint32_t)pos;
+      std::string h = headers && headers[s] ? headers[s] : "";
+      hs[s] = h.empty() ? "seq_" + std::to_string(s) : h;
+    }
   } catch (const std::bad_alloc&) {
     return set_error(HFM_E_OOM, "host allocation failed");
   }
-  uint64_t pos = 0;
+  return HFM_OK;
+}
+
+// The sequences joined, a 0 sentinel after each.
+static int concat_text(const uint8_t* codes, const uint64_t* seq_off, uint32_t nseq, const char* const* headers,
+                       std::vector<uint8_t>& text, std::vector<uint32_t>& bounds, std::vector<std::string>& hs) {
+  RET_STATUS(sequence_bounds(codes, seq_off, nseq, headers, bounds, hs));
+  try {
+    text.assign(bounds.back(), 0);
+  } catch (const std::bad_alloc&) {
+    return set_error(HFM_E_OOM, "host allocation failed");
+  }
   for (uint32_t s = 0; s < nseq; s++) {
-    uint64_t len = seq_off[s + 1] - seq_off[s];
-    for (uint64_t k = 0; k < len; k++) {
-      uint8_t c = codes[seq_off[s] + k];
-      if (c == 0 || c > 15) return set_error(HFM_E_ARG, "invalid code in sequence");
-      text[pos + k] = c;
-    }
-    pos += len; text[pos++] = 0; bounds[s] = (uint32_t)pos;
-    std::string h = headers && headers[s] ? headers[s] : "";
-    hs[s] = h.empty() ? "seq_" + std::to_string(s) : h;
+    const uint64_t len = seq_off[s + 1] - seq_off[s];
+    if (len) std::memcpy(text.data() + bounds[s] - 1 - len, codes + seq_off[s], len);
   }
   return HFM_OK;
 }
 
 // FmIndex bytes (kind 0) or BidirFmIndex bytes, [u32 fwd_len][fwd][rev] (kind 1,
 // src/fm_index/bidir_index.rs:183-192), in one malloc block.
-int emit_bytes(const BuiltFm& fwd, const BuiltFm& rev, int kind, uint8_t** bytes_out, size_t* len_out) {
+static int emit_bytes(BuiltFm& fwd, BuiltFm& rev, int kind, uint8_t** bytes_out, size_t* len_out) {
   std::vector<uint8_t> out;
   try {
-    if (kind == HFM_KIND_FM) write_fm(fwd, out);
+    if (kind == HFM_KIND_FM) write_built(fwd, out);
     else {
       std::vector<uint8_t> fb, rb;
-      write_fm(fwd, fb); write_fm(rev, rb);
+      write_built(fwd, fb); write_built(rev, rb);
       uint32_t fl = (uint32_t)fb.size();
       out.resize(4); std::memcpy(out.data(), &fl, 4);
       out.insert(out.end(), fb.begin(), fb.end());
