@@ -542,14 +542,16 @@ static int run_bsearch(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
 
 static int resolve(hfm_index* x, const FmDev& F, const uint32_t* seg_row, uint32_t stride, const uint64_t* seg_off,
                    uint64_t nseg, uint64_t total, const uint32_t* d_bounds, uint32_t nb, uint32_t* out,
-                   uint32_t& launches, uint32_t& other) {
+                   uint32_t& launches, uint32_t& other, bool have_map = false) {
   if (total == 0) return HFM_OK;
   if (nseg >= 0xFFFFFFFFull) return set_error(HFM_E_ARG, "too many intervals in one call");
   uint64_t blocks = (total + RES_T - 1) / RES_T;
-  RET(x->blockmap.ensure(blocks * 4 + 4));
-  k_block_first<<<(unsigned)((nseg + 255) / 256), 256, 0, x->stream>>>(seg_off, (uint32_t)nseg, RES_T,
-                                                                     x->blockmap.as<uint32_t>());
-  other++;
+  if (!have_map) {
+    RET(x->blockmap.ensure(blocks * 4 + 4));
+    k_block_first<<<(unsigned)((nseg + 255) / 256), 256, 0, x->stream>>>(seg_off, (uint32_t)nseg, RES_T,
+                                                                       x->blockmap.as<uint32_t>());
+    other++;
+  }
   ResolveArgs A{seg_row, stride, seg_off, (uint32_t)nseg, total, d_bounds, nb,
                 F.rate ? F.rate : F.text_len, out, &dctr(x)->walk_err, &dctr(x)->steps, x->blockmap.as<uint32_t>(), nullptr,
                 x->sa};
@@ -564,14 +566,19 @@ static int resolve(hfm_index* x, const FmDev& F, const uint32_t* seg_row, uint32
   return HFM_OK;
 }
 
+static bool dedups(const hfm_index* x, uint64_t nseg, uint64_t total) {
+  return nseg >= 2 && ((x->flags & HFM_FLAG_DEDUP_ALWAYS) || (!(x->flags & HFM_FLAG_DEDUP_NEVER) && total >= 4 * nseg));
+}
+
 // Resolve with deduplication of identical segments (see k_dedup_*): each distinct
-// (first row, length) is walked once and copied to every hit that has it.
+// (first row, length) is walked once and copied to every hit that has it.  have_map: blockmap
+// holds k_block_first's map of these segments (for a resolve without deduplication).
 static int resolve_segments(hfm_index* x, const FmDev& F, const uint32_t* seg_row, uint32_t stride,
                             const uint64_t* seg_off, uint64_t nseg, uint64_t total, const uint32_t* d_bounds,
-                            uint32_t nb, uint32_t* out, uint32_t& launches, uint32_t& other) {
+                            uint32_t nb, uint32_t* out, uint32_t& launches, uint32_t& other, bool have_map = false) {
   if (total == 0) return HFM_OK;
-  bool dedup = (x->flags & HFM_FLAG_DEDUP_ALWAYS) || (!(x->flags & HFM_FLAG_DEDUP_NEVER) && total >= 4 * nseg);
-  if (!dedup || nseg < 2) return resolve(x, F, seg_row, stride, seg_off, nseg, total, d_bounds, nb, out, launches, other);
+  if (!dedups(x, nseg, total))
+    return resolve(x, F, seg_row, stride, seg_off, nseg, total, d_bounds, nb, out, launches, other, have_map);
   uint64_t size = 1024;
   while (size < 2 * nseg) size <<= 1;
   RET(x->hkeys.ensure(size * 8)); RET(x->hslot.ensure(nseg * 4 + 4));
@@ -616,8 +623,11 @@ static void begin_stats(hfm_index* x) {
   x->k_search_rec = x->k_resolve_rec = false;
   cudaEventRecord(x->ev[0], x->stream);
 }
-static int end_stats(hfm_index* x, bool counters = false) {
+// `queue` puts what the caller wants behind the work (copies of the result) before the wait.
+template <class Q>
+static int end_stats(hfm_index* x, bool counters, Q&& queue) {
   cudaEventRecord(x->ev[2], x->stream);
+  RET(queue());
   if (counters) RET(read_ctr(x));        // the same wait serves both
   RET(wait_event(x, x->ev[2]));
   float a = 0, b = 0;
@@ -629,6 +639,9 @@ static int end_stats(hfm_index* x, bool counters = false) {
   if (x->k_resolve_rec) cudaEventElapsedTime(&kr, x->evk[2], x->evk[3]);
   x->stats.ms_search_kernel = ks; x->stats.ms_resolve_kernel = kr;
   return HFM_OK;
+}
+static int end_stats(hfm_index* x, bool counters = false) {
+  return end_stats(x, counters, [] { return HFM_OK; });
 }
 
 // ---------------------------------------------------------------------------
@@ -645,8 +658,10 @@ static int count_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff
   return HFM_OK;
 }
 
+// `copies` is called once the result is queued: its copies share the last wait.
+template <class Q>
 static int locate_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff, uint32_t nq, uint32_t cap,
-                         hfm_dev_hits* out) {
+                         hfm_dev_hits* out, Q&& copies) {
   begin_stats(x);
   uint32_t launches = 0, other = 0;
   RET(x->counts.ensure((size_t)nq * 4 + 4));
@@ -658,27 +673,35 @@ static int locate_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qof
   RET(x->seg_row.ensure(nseg * 4 + 4));
   RET(x->seg_off.ensure((nseg + 1) * 8));
   RET(x->out_pairs.ensure(total * 8 + 8));
+  // the map of the resolve's blocks comes with the gather where no deduplication is in between
+  const bool map = total > 0 && !dedups(x, nseg, total);
+  if (map) RET(x->blockmap.ensure((total + RES_T - 1) / RES_T * 4 + 4));
   if (nq) {
     k_gather_locate<<<(nq + 255) / 256, 256, 0, x->stream>>>(x->ivpool.as<uint2>(), x->ivoff.as<uint64_t>(),
                                                             x->niv.as<uint32_t>(), x->seg_base.as<uint64_t>(),
                                                             x->pos_base.as<uint64_t>(), nq, cap,
-                                                            x->seg_row.as<uint32_t>(), x->seg_off.as<uint64_t>());
+                                                            x->seg_row.as<uint32_t>(), x->seg_off.as<uint64_t>(),
+                                                            map ? RES_T : 0u, x->blockmap.as<uint32_t>());
     other++;
     CK(cudaGetLastError());
   }
-  CK(cudaMemcpyAsync(x->seg_off.as<uint64_t>() + nseg, x->pos_base.as<uint64_t>() + nq, 8, cudaMemcpyDeviceToDevice, x->stream));
+  if (!map)
+    CK(cudaMemcpyAsync(x->seg_off.as<uint64_t>() + nseg, x->pos_base.as<uint64_t>() + nq, 8, cudaMemcpyDeviceToDevice, x->stream));
   cudaEventRecord(x->ev[1], x->stream);
   uint32_t rl = 0;
   RET(resolve_segments(x, x->fwd, x->seg_row.as<uint32_t>(), 1, x->seg_off.as<uint64_t>(), nseg, total,
-              x->fwd.bounds.as<uint32_t>(), (uint32_t)x->fwd.seq_boundaries.size(), x->out_pairs.as<uint32_t>(), rl, other));
-  RET(end_stats(x, true));
+              x->fwd.bounds.as<uint32_t>(), (uint32_t)x->fwd.seq_boundaries.size(), x->out_pairs.as<uint32_t>(), rl, other, map));
+  const hfm_dev_hits done{nq, 0, total, x->pos_base.as<uint64_t>(), x->counts.as<uint32_t>(), x->out_pairs.as<uint32_t>()};
+  RET(end_stats(x, true, [&] { return copies(done); }));
   x->stats.search_launches = launches; x->stats.resolve_launches = rl; x->stats.other_launches = other;
   x->stats.rows_resolved = total; x->stats.lf_calls = x->h_ctr->steps;
   if (x->h_ctr->walk_err) return set_error(HFM_E_WALK, "LF walk exceeded sample_rate steps: index inconsistent");
-  out->nq = nq; out->total = total;
-  out->d_offsets = x->pos_base.as<uint64_t>(); out->d_counts = x->counts.as<uint32_t>();
-  out->d_pairs = x->out_pairs.as<uint32_t>();
+  *out = done;
   return HFM_OK;
+}
+static int locate_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff, uint32_t nq, uint32_t cap,
+                         hfm_dev_hits* out) {
+  return locate_device(x, d_q, d_qoff, nq, cap, out, [](const hfm_dev_hits&) { return HFM_OK; });
 }
 
 // Sort key of a read for the prefix queue order: its first 16 codes, 4 bits each, the first
@@ -2142,23 +2165,25 @@ int hfm_locate_batch(hfm_index* x, const uint8_t* q, const uint64_t* q_off, uint
   Guard g(x);
   RET(stage_queries(x, q, q_off, nq));
   hfm_dev_hits d{};
-  RET(locate_device(x, x->q.as<uint8_t>(), x->qoff.as<uint64_t>(), nq, cap, &d));
-  // one malloc block: struct | offsets | counts | pairs
-  size_t bytes = sizeof(hfm_hits) + ((size_t)nq + 1) * 8 + (size_t)nq * 4 + 4 + (size_t)d.total * 8;
-  uint8_t* blk = (uint8_t*)host_result_alloc(bytes);
-  if (!blk) return set_error(HFM_E_OOM, "host allocation failed");
-  hfm_hits* h = (hfm_hits*)blk;
-  h->nq = nq; h->_pad = 0; h->total = d.total;
-  h->offsets = (uint64_t*)(blk + sizeof(hfm_hits));
-  h->pairs = (uint32_t*)(h->offsets + nq + 1);
-  h->counts = h->pairs + d.total * 2;
-  CK(cudaMemcpyAsync(h->offsets, d.d_offsets, ((size_t)nq + 1) * 8, cudaMemcpyDeviceToHost, x->stream));
-  if (d.total) CK(cudaMemcpyAsync(h->pairs, d.d_pairs, (size_t)d.total * 8, cudaMemcpyDeviceToHost, x->stream));
-  if (nq) CK(cudaMemcpyAsync(h->counts, d.d_counts, (size_t)nq * 4, cudaMemcpyDeviceToHost, x->stream));
-  int rc = wait_stream(x);
+  hfm_hits* h = nullptr;
+  const int rc = locate_device(x, x->q.as<uint8_t>(), x->qoff.as<uint64_t>(), nq, cap, &d, [&](const hfm_dev_hits& r) -> int {
+    // one block: struct | offsets | pairs | counts
+    size_t bytes = sizeof(hfm_hits) + ((size_t)nq + 1) * 8 + (size_t)nq * 4 + 4 + (size_t)r.total * 8;
+    uint8_t* blk = (uint8_t*)host_result_alloc(bytes);
+    if (!blk) return set_error(HFM_E_OOM, "host allocation failed");
+    h = (hfm_hits*)blk;
+    h->nq = nq; h->_pad = 0; h->total = r.total;
+    h->offsets = (uint64_t*)(blk + sizeof(hfm_hits));
+    h->pairs = (uint32_t*)(h->offsets + nq + 1);
+    h->counts = h->pairs + r.total * 2;
+    CK(cudaMemcpyAsync(h->offsets, r.d_offsets, ((size_t)nq + 1) * 8, cudaMemcpyDeviceToHost, x->stream));
+    if (r.total) CK(cudaMemcpyAsync(h->pairs, r.d_pairs, (size_t)r.total * 8, cudaMemcpyDeviceToHost, x->stream));
+    if (nq) CK(cudaMemcpyAsync(h->counts, r.d_counts, (size_t)nq * 4, cudaMemcpyDeviceToHost, x->stream));
+    return HFM_OK;
+  });
   if (rc != HFM_OK) {
-    if (rc == HFM_E_TIMEOUT) x->orphans.push_back(blk);   // copies may still land in blk
-    else host_result_free(blk);
+    if (rc == HFM_E_TIMEOUT && h) x->orphans.push_back(h);   // copies may still land in it
+    else if (h) host_result_free(h);
     return rc;
   }
   *out = h;
