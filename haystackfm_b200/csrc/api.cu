@@ -815,8 +815,8 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
   uint32_t launches = 0, other = 0;
   // IUPAC texts: the first sweep of the reads in one piece is shared by the reads of a warp
   // (k_trie).  A per-read work log needs every read's own work.
-  const bool trie = x->fwd.fmt == OCC_WIDE && x->mems_variant == 3 && x->threads_per_read == 1 && !wlog && min_len > 0 &&
-                    nq > n_warp;
+  const bool trie = x->fwd.fmt == OCC_WIDE && x->mems_variant != MEMS_PLAIN && x->threads_per_read == 1 && !wlog &&
+                    min_len > 0 && nq > n_warp;
   uint32_t tblocks = 0, tgroup = 0;
   if (trie) RET(trie_plan(x, nq - n_warp, tblocks, tgroup));
   if (!order && x->threads_per_read == 1 && x->mems_variant != MEMS_PLAIN && nq > 1 &&
@@ -1073,13 +1073,13 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
     const uint32_t* wlist = x->ovf.as<uint32_t>();
     if (n_ovf) {
       x->stats.fallback_reads += n_ovf;
-      // Reads that outgrew only a 32-entry hit list (variant 2) rerun on the per-thread kernel
-      // with MID_HIT_CAP entries in global memory; set overflows, reads the schedule routed,
+      // Reads that outgrew only a 32-entry hit list (variant 2 and the plain launch) rerun on the
+      // per-thread kernel with MID_HIT_CAP entries in global memory; set overflows, reads the schedule routed,
       // and what still overflows go to the warp-per-read kernel.
       RET(x->ovf2.ensure((size_t)nq * 4 + 4));
       RET(x->ovf3.ensure((size_t)nq * 4 + 4));
       CK(cudaMemsetAsync(&dctr(x)->n_mid, 0, 12, x->stream));
-      k_split_ovf<<<(n_ovf + 255) / 256, 256, 0, x->stream>>>(x->ovf.as<uint32_t>(), n_ovf, variant == 2 ? n_warp : n_ovf,
+      k_split_ovf<<<(n_ovf + 255) / 256, 256, 0, x->stream>>>(x->ovf.as<uint32_t>(), n_ovf, variant == 3 ? n_ovf : n_warp,
                                                               x->status.as<uint32_t>(), x->ovf3.as<uint32_t>(),
                                                               &dctr(x)->n_mid, x->ovf2.as<uint32_t>(), &dctr(x)->n_wrp);
       other++;
