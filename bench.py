@@ -327,7 +327,7 @@ def profile_smem(args):
     s = h.stats()
     h.set_counters(True)
     L.check(lib.hfm_mems_batch_device(h.h, rd.data_ptr(), off.data_ptr(), n, 19, 0, None, 0, 1024, C.byref(dm)))
-    print(json.dumps({"profile": "smem_search", "reads": n, "k_mems_ms": s.ms_search_kernel,
+    print(json.dumps({"profile": "smem_search", "reads": n, "search_kernels_ms": s.ms_search_kernel,
                       "fallback_reads": s.fallback_reads, "mem_hits": dm.n_hits,
                       "occ_touches": h.stats().occ_touches}), flush=True)
 
@@ -1000,7 +1000,7 @@ def main():
     b_res_mem = 32 * (2 * c_mem.lf_calls + rows_walked(c_mem)) + 8 * rows_walked(c_mem)
     b_bs = 32 * c_loc.occ_touches + 32 * n
     b_res_loc = 32 * (2 * c_loc.lf_calls + rows_walked(c_loc)) + 8 * rows_walked(c_loc)
-    kern = {"k_mems": (k_mems_ms, b_mems, c_mem.occ_touches, "Occ touches"),
+    kern = {"smem_search": (k_mems_ms, b_mems, c_mem.occ_touches, "Occ touches"),
             "k_resolve(smem)": (k_res_mem_ms, b_res_mem, c_mem.lf_calls, "LF steps"),
             "k_bsearch": (k_bs_ms, b_bs, c_loc.occ_touches, "Occ touches"),
             "k_resolve(locate)": (k_res_loc_ms, b_res_loc, c_loc.lf_calls, "LF steps")}
