@@ -55,8 +55,8 @@ struct SmemJobs {
   const uint32_t* jobs;           // when set, only these n_jobs jobs (of the ones above)
   uint32_t n_jobs;
   const uint32_t* n_jobs_dev;     // when set, their number
-  const uint32_t* resume;         // per whole read: position after a result [0, e) that is already in its slot
-                                  // (k_trie), or RESUME_START; nullptr: every read from its start
+  const uint32_t* resume;         // per entry of ids: position after a result [0, e) that is already in its read's
+                                  // slot (k_trie), or RESUME_START; nullptr: every read from its start
   // Results are written per slot: a read's segments in order (one slot for a read in one
   // piece).  slot_base[i] = first slot of read i; nullptr: slot i.
   const uint64_t* slot_base;
@@ -263,9 +263,9 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
       first = i > 0;
       nh = 0; st = ST_OK; t0 = touches;
       ph = WINDOW;
-      if (!unit && J.resume && J.resume[read] != RESUME_START) {
+      if (!unit && J.resume && J.resume[u - n_units] != RESUME_START) {
         // behind a first result that is already known: its hits lead this read's list
-        end = J.resume[read];
+        end = J.resume[u - n_units];
         const uint64_t slot = J.slot_base ? J.slot_base[read] : (uint64_t)read;
         const uint4* src = (const uint4*)hitpool.base + out.hit_start[slot] * 2;
         const uint32_t have = out.hit_count[slot];

@@ -60,7 +60,7 @@ struct TrieWork {
   unsigned int* queue;
   uint32_t group;                           // reads per block, 1..32
   uint32_t* left; uint32_t* n_left;         // reads that k_smem goes on with
-  uint32_t* resume;                         // per read: where, or RESUME_START
+  uint32_t* resume;                         // for each of them: where, or RESUME_START
 };
 
 // A node list: the first SC nodes in shared memory, the others in the warp's global area.
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 5) k_trie(DevFm Fw, DevFm Rv,
       at = __shfl_sync(0xFFFFFFFFu, at, 0);
       if ((who >> lane) & 1) {
         W.left[at + __popc(who & lt)] = read;
-        W.resume[read] = j;
+        W.resume[at + __popc(who & lt)] = j;
       }
     };
     // The result [0, j) of the reads in `who`, a warp per read: one hit per node that holds
