@@ -269,7 +269,9 @@ __global__ void __launch_bounds__(128, MINB) k_acgt(DevFm Fw, DevFm Rv, const ui
     } else if (ph == PLACE) {
       a = reinterpret_cast<const uint4*>(A.sa) + (flo >> 2);
     } else if (ph == TEXT) {
-      a = A.text + ((rlo + pos) >> 5);                         // rlo: text position of code 0 (may wrap below 0)
+      // rlo: text position of code 0 (may wrap below 0).  Directions of an index that disagree
+      // give rows whose text ends before the match does: nothing matches there.
+      a = A.text + (min(rlo + pos, Fw.text_len) >> 5);
     }
     const uint4 va = __ldg(a);
     if (COUNT_TOUCH) touches += 1;
@@ -322,7 +324,7 @@ __global__ void __launch_bounds__(128, MINB) k_acgt(DevFm Fw, DevFm Rv, const ui
     } else {
       // the codes of this word against the text
       const uint4 vb = __ldg(a + 1);
-      const uint32_t b = pos & 31, sh = (rlo + pos) & 31;
+      const uint32_t b = pos & 31, sh = min(rlo + pos, Fw.text_len) & 31;
       const uint32_t x0 = __funnelshift_r(va.x, vb.x, sh) ^ (r.x >> b), x1 = __funnelshift_r(va.y, vb.y, sh) ^ (r.y >> b);
       const uint32_t diff = (x0 | x1 | __funnelshift_r(va.z, vb.z, sh) | (r.z | r.w) >> b) & (~0u >> b);
       const uint32_t same = diff ? (uint32_t)__ffs(diff) - 1u : 32u - b;

@@ -1,0 +1,53 @@
+"""Index bytes that pass the format checks without being an index of any text: the parts
+disagree with one another.  Whatever such a handle answers, no search leaves its buffers: the
+calls return, and a proper index is still searched correctly afterwards."""
+from __future__ import annotations
+
+import struct
+
+import numpy as np
+import pytest
+
+from haystackfm_b200 import alphabet as al
+from haystackfm_b200._lib import pack_queries
+from haystackfm_b200.fm_index import FmIndexConfig, KIND_BIDIR, KIND_FM, _Handle, _build
+
+pytestmark = pytest.mark.gpu
+
+
+def _two_texts(seed, p=(0.25, 0.25, 0.25, 0.25)):
+    """A forward index of one text and a reverse index of another of the same length."""
+    rng = np.random.default_rng(seed)
+    a = rng.integers(1, 5, size=60_000).astype(np.uint8)
+    c = rng.permutation(a) if p is None else rng.choice(np.arange(1, 5, dtype=np.uint8), size=len(a), p=p)
+    cfg = FmIndexConfig(sa_sample_rate=16, lookup_depth=4)
+    fwd = _build([al.DnaSequence(a)], cfg, 1, KIND_FM)
+    rev = _build([al.DnaSequence(c[::-1].copy())], FmIndexConfig(sa_sample_rate=16), 1, KIND_FM)
+    return a, c, struct.pack("<I", len(fwd)) + fwd + rev
+
+
+def _search(h, reads):
+    flat, off = pack_queries(reads)
+    for variant, mode in ((3, 0), (2, 0), (3, 1)):
+        h.set_tuning(variant, 64)
+        hit_off, hits, pos = h.mems_packed(flat, off, 19, mode, None, 64)
+        assert hit_off[-1] == len(hits)
+
+
+def _proper(oracle, a, reads):
+    b = _build([al.DnaSequence(a)], FmIndexConfig(sa_sample_rate=16, lookup_depth=4), 1, KIND_BIDIR)
+    flat, off = pack_queries(reads)
+    want = oracle.OracleIndex(b, KIND_BIDIR).mems_packed(flat, off, 19, 0, None, 64)
+    for g, w in zip(_Handle(b, KIND_BIDIR).mems_packed(flat, off, 19, 0, None, 64), want):
+        assert np.array_equal(g, w)
+
+
+def test_directions_of_different_texts(oracle):
+    """Same codes in another order: a match's forward row is that of some other string, and the
+    text behind it may end long before the read does."""
+    a, c, b = _two_texts(1, None)
+    h = _Handle(b, KIND_BIDIR)
+    reads = [a[k:k + 4000].copy() for k in range(0, 56_000, 3500)] + [c[k:k + 4000].copy() for k in range(0, 56_000, 3500)]
+    reads += [a[-3000:].copy(), c[-3000:].copy(), a[-40:].copy(), c[-40:].copy()]
+    _search(h, reads)
+    _proper(oracle, a, reads)
