@@ -129,8 +129,8 @@ __global__ void __launch_bounds__(128, MINB) k_acgt(DevFm Fw, DevFm Rv, const ui
                                                    Pool hitpool, MemsOut out, MemsWork W, SmemJobs J, DevAux A,
                                                    PackedReads R, uint32_t lanes, uint32_t* __restrict__ left_jobs,
                                                    uint32_t* __restrict__ n_left) {
-  __shared__ uint32_t s_C[5];
-  if (threadIdx.x < 5) s_C[threadIdx.x] = Fw.C[threadIdx.x];
+  __shared__ uint32_t s_C[2][8];            // of the reverse and of the forward index: the same in an index of one text
+  if (threadIdx.x < 5) { s_C[0][threadIdx.x] = Rv.C[threadIdx.x]; s_C[1][threadIdx.x] = Fw.C[threadIdx.x]; }
   __syncthreads();
   uint4 local_h[KC > 0 ? 2 * KC : 1];
   uint4* hits = local_h;
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(128, MINB) k_acgt(DevFm Fw, DevFm Rv, const ui
       bool ok = false;
       if ((r.w >> b) & 1) { st = ST_LEAVE; ph = DONE; continue; }
       if (!((r.z >> b) & 1)) {
-        ok = acgt_use<COUNT_TOUCH>(X, s_C, 1u + ((r.x >> b) & 1) + 2u * ((r.y >> b) & 1), va, a, lo, base, sz, touches);
+        ok = acgt_use<COUNT_TOUCH>(X, s_C[left], 1u + ((r.x >> b) & 1) + 2u * ((r.y >> b) & 1), va, a, lo, base, sz, touches);
         if (ok) { flo = left ? lo : base; rlo = left ? base : lo; }
       }
       if (ph == BACK) {

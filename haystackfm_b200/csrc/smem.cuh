@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
       const uint8_t code = p[pos];
       const uint32_t mask = code < 16 ? (uint32_t)Sf.compat_mask[code] & sym : 0u;
       bool ovf = false;
-      const bool ok = lane_step<COUNT_TOUCH, FMT>(X, Sf.C, left, mask, L, SCAP, ovf, touches);
+      const bool ok = lane_step<COUNT_TOUCH, FMT>(X, left ? Sf.C : Sr.C, left, mask, L, SCAP, ovf, touches);
       if (ovf) { st |= ST_SET_OVF; ph = DONE; }
       else if (ph == BACK) {
         if (!ok) { i = pos + 1; first = false; ph = WINDOW; }

@@ -51,3 +51,30 @@ def test_directions_of_different_texts(oracle):
     reads += [a[-3000:].copy(), c[-3000:].copy(), a[-40:].copy(), c[-40:].copy()]
     _search(h, reads)
     _proper(oracle, a, reads)
+
+
+@pytest.mark.parametrize("p", [(0.05, 0.05, 0.05, 0.85), (0.85, 0.05, 0.05, 0.05)])
+def test_directions_of_different_code_counts(oracle, p):
+    """A step of either direction counts from that direction's own rows of smaller codes."""
+    a, c, b = _two_texts(2, p)
+    h = _Handle(b, KIND_BIDIR)
+    reads = [a[k:k + 300].copy() for k in range(0, 56_000, 3500)] + [c[k:k + 300].copy() for k in range(0, 56_000, 3500)]
+    for codes in (1, 4):
+        reads += [np.full(200, codes, np.uint8), np.concatenate([a[:100], np.full(100, codes, np.uint8)])]
+    _search(h, reads)
+    _proper(oracle, a, reads)
+
+
+def test_directions_of_different_code_counts_wide(oracle):
+    rng = np.random.default_rng(3)
+    a = rng.integers(1, 16, size=20_000).astype(np.uint8)
+    c = np.where(rng.random(len(a)) < 0.9, 15, a).astype(np.uint8)
+    fwd = _build([al.DnaSequence(a)], FmIndexConfig(sa_sample_rate=16), 0, KIND_FM)
+    rev = _build([al.DnaSequence(c[::-1].copy())], FmIndexConfig(sa_sample_rate=16), 0, KIND_FM)
+    h = _Handle(struct.pack("<I", len(fwd)) + fwd + rev, KIND_BIDIR)
+    reads = [a[k:k + 60].copy() for k in range(0, 18_000, 900)] + [c[k:k + 60].copy() for k in range(0, 18_000, 900)]
+    flat, off = pack_queries(reads)
+    for variant in (3, 2):
+        h.set_tuning(variant, 64)
+        hit_off, hits, pos = h.mems_packed(flat, off, 25, 0, None, 64)
+        assert hit_off[-1] == len(hits)
