@@ -307,16 +307,20 @@ static int build_kmer(hfm_index* x) {
   }
   // levels alternate between the two buffers so that level k ends in the table
   const uint4* in = nullptr;
+  uint32_t* bad = &x->ctr.as<Counters>()->walk_err;
+  cudaError_t e = cudaMemsetAsync(bad, 0, 4, x->stream);
   for (uint32_t l = 0; l < k; l++) {
     uint4* out = ((k - l) & 1) ? x->aux_kmer.as<uint4>() : tmp.as<uint4>();
     const uint64_t entries = 1ull << (2 * (l + 1));
-    k_kmer_table<<<(unsigned)((entries + 255) / 256), 256, 0, x->stream>>>(f.d, in, l, l + 1 == k, out);
+    k_kmer_table<<<(unsigned)((entries + 255) / 256), 256, 0, x->stream>>>(f.d, in, l, l + 1 == k, out, bad);
     in = out;
   }
-  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&x->h_ctr->walk_err, bad, 4, cudaMemcpyDeviceToHost, x->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(x->stream);
   tmp.release();
   CK(e);
+  if (x->h_ctr->walk_err) { x->aux_kmer.release(); return HFM_OK; }
   x->aux.kmer = x->aux_kmer.as<uint4>();
   x->aux.k = k;
   return HFM_OK;
@@ -327,11 +331,11 @@ static int build_kmer(hfm_index* x) {
 static constexpr uint32_t SEEN_K_MAX = 18;      // 8 GB of bits, for texts near 2^32
 static int build_sa(hfm_index* x) {
   const FmDev& f = x->fwd;
-  if (f.rate < 1 || f.rate > SA_ROWS_RATE || f.d.num_seqs > f.text_len || !f.text_len) return HFM_OK;
+  if (f.rate < 1 || f.rate > SA_ROWS_RATE || f.d.sample_rate != f.rate || f.d.num_seqs > f.text_len || !f.text_len) return HFM_OK;
   if (!aux_room((uint64_t)f.text_len * 4) || x->aux_sa.ensure((size_t)f.text_len * 4 + 16) != HFM_OK) return HFM_OK;    // read 16 bytes at a time
   CK(cudaMemsetAsync(x->aux_sa.p, 0xFF, (size_t)f.text_len * 4, x->stream));
   const uint64_t items = (uint64_t)f.d.num_blocks + f.d.num_seqs;
-  WITH_FMT(f.fmt, { k_sa_rows<FM><<<(unsigned)((items + 127) / 128), 128, 0, x->stream>>>(f.d, x->aux_sa.as<uint32_t>()); });
+  WITH_FMT(f.fmt, { k_sa_rows<FM><<<(unsigned)((items + 127) / 128), 128, 0, x->stream>>>(f.d, f.nbytes[3] / 4, x->aux_sa.as<uint32_t>()); });
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(x->stream));
   x->sa = x->aux_sa.as<uint32_t>();

@@ -43,9 +43,10 @@ constexpr uint32_t SA_ROWS_RATE = 1024;     // longest walks that k_sa_rows is r
 // from it by LF steps are those of the positions before it, down to the next sampled one.
 // The rows of the sentinels (the first num_seqs rows) cover the ends of the sequences; their
 // positions come from a walk first.  sa is filled with SA_UNKNOWN by the caller; rows that an
-// inconsistent index does not reach stay so.
+// inconsistent index does not reach stay so.  A layout blob is not checked beyond its sizes: marks
+// past the text and places outside the n_vals sampled values count for nothing.
 template <uint32_t FMT>
-__global__ void __launch_bounds__(128) k_sa_rows(DevFm F, uint32_t* __restrict__ sa) {
+__global__ void __launch_bounds__(128) k_sa_rows(DevFm F, uint64_t n_vals, uint32_t* __restrict__ sa) {
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   auto step = [&](uint32_t& row) -> bool {
     uint32_t c, rk;
@@ -58,7 +59,9 @@ __global__ void __launch_bounds__(128) k_sa_rows(DevFm F, uint32_t* __restrict__
     const uint4 w = __ldg(F.ssa + (row >> 6));
     const uint64_t word = u2to64(w.x, w.y);
     if (!((word >> (row & 63)) & 1)) return false;
-    val = __ldg(F.sa_vals + w.z + (uint32_t)__popcll(word & ((1ull << (row & 63)) - 1ull)));
+    const uint64_t at = (uint64_t)w.z + (uint32_t)__popcll(word & ((1ull << (row & 63)) - 1ull));
+    if (at >= n_vals) return false;
+    val = __ldg(F.sa_vals + at);
     return true;
   };
   auto fill = [&](uint32_t row, uint32_t v) {
@@ -68,9 +71,11 @@ __global__ void __launch_bounds__(128) k_sa_rows(DevFm F, uint32_t* __restrict__
   };
   if (t < F.num_blocks) {
     const uint4 w = __ldg(F.ssa + t);
-    uint32_t k = 0;
-    for (uint64_t m = u2to64(w.x, w.y); m; m &= m - 1, k++)
-      fill((uint32_t)(t * 64) + (uint32_t)__ffsll((long long)m) - 1u, __ldg(F.sa_vals + w.z + k));
+    uint64_t at = w.z;
+    for (uint64_t m = u2to64(w.x, w.y); m; m &= m - 1, at++) {
+      const uint64_t row = t * 64 + (uint32_t)__ffsll((long long)m) - 1u;
+      if (row < F.text_len && at < n_vals) fill((uint32_t)row, __ldg(F.sa_vals + at));
+    }
   } else if (t - F.num_blocks < F.num_seqs) {
     const uint32_t first = (uint32_t)(t - F.num_blocks);
     uint32_t row = first, steps = 0, v = 0;

@@ -383,8 +383,10 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
 
 // One more code in front: out[c w] from in[w] for strings w of k codes (in: nullptr for k = 0);
 // strings are numbered with their first code in the top digit, in the last level as DevAux has
-// them.
-__global__ void k_kmer_table(DevFm Fw, const uint4* __restrict__ in, uint32_t k, bool last, uint4* __restrict__ out) {
+// them.  *bad counts intervals past the last row, which records that no text gives (a layout
+// blob's are not checked) may lead to: they are not gone on with.
+__global__ void k_kmer_table(DevFm Fw, const uint4* __restrict__ in, uint32_t k, bool last, uint4* __restrict__ out,
+                             uint32_t* __restrict__ bad) {
   const uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (x >> (2 * (k + 1))) return;
   const uint32_t s = (uint32_t)(x >> (2 * k)) + 1u;
@@ -394,6 +396,10 @@ __global__ void k_kmer_table(DevFm Fw, const uint4* __restrict__ in, uint32_t k,
   uint64_t touches = 0;
   const FmView X{Fw.occ, Fw.sb};
   if (v.z && !acgt_step<false>(X, C, s, v.x, v.y, v.z, touches)) v = make_uint4(0u, 0u, 0u, 0u);
+  if ((uint64_t)v.x + v.z > Fw.text_len || (uint64_t)v.y + v.z > Fw.text_len) {
+    atomicAdd(bad, 1u);
+    v = make_uint4(0u, 0u, 0u, 0u);
+  }
   uint64_t at = x;
   if (last) {
     uint32_t b0 = 0, b1 = 0;
