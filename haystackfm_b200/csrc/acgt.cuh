@@ -343,7 +343,9 @@ __global__ void __launch_bounds__(128, MINB) k_acgt(DevFm Fw, DevFm Rv, const ui
 // ---- what the search keeps besides the records (DevAux), made when an index is loaded ----
 
 // The text, one code a byte, from the BWT and the whole suffix array; *unknown counts rows
-// without a position.
+// without a position.  Every byte is TEXT_NONE before: one that stays so (two rows claim
+// another position) shows samples that belong to no text.
+constexpr uint8_t TEXT_NONE = 0xFF;
 __global__ void k_text_bytes(DevFm F, const uint32_t* __restrict__ sa, uint8_t* __restrict__ text,
                              uint32_t* __restrict__ unknown) {
   for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < F.text_len; r += (uint64_t)gridDim.x * blockDim.x) {
@@ -351,17 +353,20 @@ __global__ void k_text_bytes(DevFm F, const uint32_t* __restrict__ sa, uint8_t* 
     if (v == 0xFFFFFFFFu || v >= F.text_len) { atomicAdd(unknown, 1u); continue; }
     uint32_t c, rk;
     row_code_rank<OCC_NARROW>(F, (uint32_t)r, c, rk);
-    if (v > 0) text[v - 1] = (uint8_t)c;
+    if (v == 0 && c) atomicAdd(unknown, 1u);
+    text[v > 0 ? v - 1 : F.text_len - 1] = (uint8_t)c;
   }
 }
 
 // Bit planes of 32 codes a word: the bits of symbol - 1, then the sentinels (and the places
-// from n on).
-__global__ void k_text_planes(const uint8_t* __restrict__ text, uint64_t n, uint64_t words, uint4* __restrict__ out) {
+// from n on).  *unknown counts bytes that are TEXT_NONE.
+__global__ void k_text_planes(const uint8_t* __restrict__ text, uint64_t n, uint64_t words, uint4* __restrict__ out,
+                              uint32_t* __restrict__ unknown) {
   const uint32_t lane = threadIdx.x & 31;
   for (uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; w < words; w += ((uint64_t)gridDim.x * blockDim.x) >> 5) {
     const uint64_t t = w * 32 + lane;
     const uint32_t c = t < n ? text[t] : 0u;
+    if (c == TEXT_NONE) atomicAdd(unknown, 1u);
     const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, c && ((c - 1) & 1)), b1 = __ballot_sync(0xFFFFFFFFu, c && ((c - 1) & 2)),
                    z = __ballot_sync(0xFFFFFFFFu, c == 0);
     if (lane == 0) out[w] = make_uint4(b0, b1, z, 0u);

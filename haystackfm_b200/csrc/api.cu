@@ -340,7 +340,8 @@ static int build_sa(hfm_index* x) {
   CK(cudaStreamSynchronize(x->stream));
   x->sa = x->aux_sa.as<uint32_t>();
   if (f.fmt != OCC_NARROW || !aux_room((uint64_t)f.text_len * 2)) return HFM_OK;
-  // the text of ACGT texts; not kept when a row has no position (an inconsistent index)
+  // the text of ACGT texts; not kept when a row has no position or a position no row (an
+  // inconsistent index)
   const uint64_t n = f.text_len, words = n / 32 + 2;
   DevBuf bytes;
   if (bytes.ensure(n) != HFM_OK) return HFM_OK;
@@ -348,10 +349,10 @@ static int build_sa(hfm_index* x) {
   auto run = [&]() -> int {
     uint32_t* unknown = &x->ctr.as<Counters>()->walk_err;
     CK(cudaMemsetAsync(unknown, 0, 4, x->stream));
-    CK(cudaMemsetAsync(bytes.p, 0, n, x->stream));
+    CK(cudaMemsetAsync(bytes.p, TEXT_NONE, n, x->stream));
     const unsigned grid = (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)x->num_sms * 32);
     k_text_bytes<<<grid, 256, 0, x->stream>>>(f.d, x->sa, bytes.as<uint8_t>(), unknown);
-    k_text_planes<<<grid, 256, 0, x->stream>>>(bytes.as<uint8_t>(), n, words, x->aux_text.as<uint4>());
+    k_text_planes<<<grid, 256, 0, x->stream>>>(bytes.as<uint8_t>(), n, words, x->aux_text.as<uint4>(), unknown);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(&x->h_ctr->walk_err, unknown, 4, cudaMemcpyDeviceToHost, x->stream));
     CK(cudaStreamSynchronize(x->stream));

@@ -42,9 +42,11 @@ constexpr uint32_t SA_ROWS_RATE = 1024;     // longest walks that k_sa_rows is r
 // The suffix array from its samples: every sampled row knows its position, the rows reached
 // from it by LF steps are those of the positions before it, down to the next sampled one.
 // The rows of the sentinels (the first num_seqs rows) cover the ends of the sequences; their
-// positions come from a walk first.  sa is filled with SA_UNKNOWN by the caller; rows that an
-// inconsistent index does not reach stay so.  A layout blob is not checked beyond its sizes: marks
-// past the text and places outside the n_vals sampled values count for nothing.
+// positions come from a walk first.  sa is filled with SA_UNKNOWN by the caller.  A chain counts
+// only when the sampled row at its end has the position that it leads to: every entry is what a
+// walk from that row gives, and rows whose samples disagree (or that no chain reaches) stay
+// unknown and are walked, with the walk's answer or error.  A layout blob is not checked beyond
+// its sizes: marks past the text and places outside the n_vals sampled values count for nothing.
 template <uint32_t FMT>
 __global__ void __launch_bounds__(128) k_sa_rows(DevFm F, uint64_t n_vals, uint32_t* __restrict__ sa) {
   const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -64,10 +66,17 @@ __global__ void __launch_bounds__(128) k_sa_rows(DevFm F, uint64_t n_vals, uint3
     val = __ldg(F.sa_vals + at);
     return true;
   };
-  auto fill = [&](uint32_t row, uint32_t v) {
-    sa[row] = v;
-    uint32_t x;
-    for (uint32_t k = 0; k < F.sample_rate && v > 0 && step(row) && !sampled(row, x); k++) sa[row] = --v;
+  auto fill = [&](uint32_t first, uint32_t v) {
+    sa[first] = v;
+    uint32_t row = first, k = 0, x;
+    bool met = false;
+    for (; k < F.sample_rate && v > 0 && step(row); k++) {
+      v--;
+      if (sampled(row, x)) { met = x == v; break; }
+      sa[row] = v;
+    }
+    if (met || !k) return;
+    for (row = first; k && step(row); k--) sa[row] = SA_UNKNOWN;
   };
   if (t < F.num_blocks) {
     const uint4 w = __ldg(F.ssa + t);

@@ -78,3 +78,49 @@ def test_directions_of_different_code_counts_wide(oracle):
         h.set_tuning(variant, 64)
         hit_off, hits, pos = h.mems_packed(flat, off, 25, 0, None, 64)
         assert hit_off[-1] == len(hits)
+
+
+def _fm_parts(b, at):
+    """Offsets of the sampled values and of the marker words of the FmIndex at `at`."""
+    o = at + 64 + 2 + 32
+    o += 8 + 4 * struct.unpack_from("<Q", b, o)[0]
+    o += 8 + struct.unpack_from("<Q", b, o)[0]
+    o += 8 + 4 + 4
+    n_ssa = struct.unpack_from("<Q", b, o)[0]
+    ssa = o + 8
+    n_vals = struct.unpack_from("<Q", b, ssa + n_ssa)[0]
+    return ssa + n_ssa + 8, n_vals
+
+
+@pytest.mark.parametrize("change", ["one_value", "swapped", "short_sequence_moved"])
+def test_samples_that_disagree(oracle, change):
+    """Sampled positions changed within the text: positions are those that walks to the samples
+    give (the oracle's), searches do not depend on them."""
+    rng = np.random.default_rng(5)
+    seqs = [rng.integers(1, 5, size=n).astype(np.uint8) for n in (9000, 11, 13, 7000, 200)]
+    b = bytearray(_build([al.DnaSequence(s) for s in seqs], FmIndexConfig(sa_sample_rate=32, lookup_depth=4), 1, KIND_BIDIR))
+    at, n_vals = _fm_parts(b, 4)
+    vals = np.frombuffer(b, "<u4", n_vals, at).copy()
+    if change == "one_value":
+        vals[vals == 3200] = 4800
+    elif change == "swapped":
+        i, k = np.flatnonzero(vals == 320)[0], np.flatnonzero(vals == 12_000 // 32 * 32)[0]
+        vals[i], vals[k] = vals[k], vals[i]
+    else:                                                # every sample of the second sequence
+        start = len(seqs[0]) + 1
+        inside = (vals >= start) & (vals < start + len(seqs[1]) + 1)
+        assert inside.sum() >= 1
+        vals[inside] += 3000
+    b[at:at + 4 * n_vals] = vals.astype("<u4").tobytes()
+    b = bytes(b)
+    o = oracle.OracleIndex(b, KIND_BIDIR)
+    h = _Handle(b, KIND_BIDIR)
+    reads = [s[k:k + 120].copy() for s in seqs for k in range(0, max(1, len(s) - 120), 64)] + [s.copy() for s in seqs]
+    flat, off = pack_queries(reads)
+    bounds = np.cumsum([len(s) + 1 for s in seqs]).astype(np.uint32)
+    for g, w in zip(h.mems_packed(flat, off, 11, 0, bounds, 64), o.mems_packed(flat, off, 11, 0, bounds, 64)):
+        assert np.array_equal(g, w)
+    assert np.array_equal(h.count_packed(flat, off), o.count_packed(flat, off))
+    cut, cut_off = pack_queries([r[k:k + 9] for r in reads for k in range(0, len(r) - 8, 5)])
+    for g, w in zip(h.locate_packed(cut, cut_off, 64), o.locate_packed(cut, cut_off, 64)):
+        assert np.array_equal(g, w)
