@@ -240,7 +240,10 @@ static void build_fm(const uint8_t* text, uint32_t n, const std::vector<uint32_t
 int sequence_bounds(const uint8_t* codes, const uint64_t* seq_off, uint32_t nseq, const char* const* headers,
                     std::vector<uint32_t>& bounds, std::vector<std::string>& hs) {
   uint64_t total = 0;
-  for (uint32_t s = 0; s < nseq; s++) total += seq_off[s + 1] - seq_off[s] + 1;
+  for (uint32_t s = 0; s < nseq; s++) {
+    if (seq_off[s + 1] < seq_off[s]) return set_error(HFM_E_ARG, "seq_off not ascending");
+    total += seq_off[s + 1] - seq_off[s] + 1;
+  }
   if (total > 0xFFFFFFFFull) return set_error(HFM_E_ARG, "text too large: exceeds u32::MAX");
   try {
     bounds.assign(nseq, 0); hs.assign(nseq, std::string());
