@@ -1225,6 +1225,28 @@ __device__ uint32_t warp_extend_set(const DevFm& X, const SmemFm& S, uint32_t ma
   return nout;
 }
 
+// Codes of several symbols that a window may hold and still be searched from its end, and the
+// run of ACGT that a search is started from without looking for a longer one.
+constexpr uint32_t SEED_AMBIGUOUS = 3, SEED_RUN = 12;
+
+// Where the search of the window q[i, e) starts: its codes before the returned place are taken
+// to the left first, those from it on to the right after them.  A code that matches nothing
+// ends the window at once.
+__device__ __forceinline__ uint32_t seed_end(const uint16_t* compat, const uint8_t* q, uint32_t i, uint32_t e) {
+  uint32_t run = 0, best = 0, at = e, others = 0;
+  for (uint32_t k = e; k > i && best < SEED_RUN; k--) {
+    const uint32_t c = q[k - 1];
+    if (c > 15 || !compat[c]) return k;
+    if (c <= 4) {
+      if (++run > best) { best = run; at = k - 1 + run; }
+    } else {
+      run = 0;
+      others++;
+    }
+  }
+  return others > SEED_AMBIGUOUS ? at : e;
+}
+
 // The search of one read (window, forward, next: smem.cuh) by a group of G lanes; control
 // flow is group-uniform.
 template <bool COUNT_TOUCH, int G = 32>
@@ -1260,13 +1282,13 @@ __device__ uint32_t warp_mems_one(const DevFm& Fw, const DevFm& Rv, const SmemFm
   uint32_t i = 0;
   while (n - i >= P.min_len) {
     reset();
-    uint32_t k = i + P.min_len;
+    uint32_t e = seed_end(Sf.compat_mask, q, i, i + P.min_len), k = e;
     while (k > i && left(k - 1)) k--;
     if (ovf) { st |= ST_SET_OVF; return ~0u; }
     if (k > i) { i = k; continue; }
-    uint32_t e = i + P.min_len;
     while (e < n && right(e)) e++;
     if (ovf) { st |= ST_SET_OVF; return ~0u; }
+    if (e < i + P.min_len) { i++; continue; }          // the window at i does not match
     if (nc >= cand_cap) { st |= ST_CAND_OVF; return ~0u; }
     uint64_t off = 0;
     if (lane == 0) off = thread_reserve(ivpool, ncur);

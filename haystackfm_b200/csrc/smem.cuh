@@ -26,6 +26,16 @@
 // 37.2 / 5.2 / 0.56 ms; find_mems of 20,000 ragged reads 25.9 / 1.9 / 0.9 ms.  With records
 // that count from row 32 (32-bit masks, half the popcounts): 5.9, 3.5, 0.38 and 0.70 ms.
 //
+// Where a window starts.  Codes of several symbols multiply a set, an N fourfold and more, until
+// the codes around it have narrowed it down; a window that ended in a run of N was extended from
+// that run and had 4^run intervals.  A window with more than SEED_AMBIGUOUS of them starts at the
+// end of its longest run of ACGT instead (seed_end), goes left to i and then right: where the
+// left part empties, the same holds as above; where the right one does within the window, no
+// match of min_len starts at i.  B200, 1,000 reads of 150 bp on 64 Mbp ACGT, the sweep / from the
+// window's end / so, with ACGT sets of more than ACGT_SET_CAP intervals left to the warp kernel:
+// 8 N at a random place 140 / 188 / 90 ms, N from 60 to 69 4.2 / 13.2 / 5.3 s, N from 13 to 18 18.2 /
+// 12.9 / 8.5 ms, 4 N at a random place 142 / 38 / 4.7 ms.
+//
 // Segments.  A result belongs to the segment of a long read in which it starts.  A segment's
 // search begins at its first position a: if the window there does not match, everything
 // after it is left-maximal by construction; if it does, its match is a result only when it
@@ -214,6 +224,12 @@ __device__ __forceinline__ void sort_set(const SR& a, uint32_t n) {
     }
 }
 
+// Sets that a thread extends on ACGT texts: they have several intervals only behind codes of
+// several symbols, in few reads of a batch, and a thread takes them one at a time where the warp
+// kernel takes 32.  (64 reads of 150 bp with 4 N, 256 intervals: a thread each 30 ms, a warp 3.0.)
+constexpr uint32_t ACGT_SET_CAP = 96;
+static_assert(ACGT_SET_CAP <= FAST_SET_CAP, "the sets' areas");
+
 // Persistent search.  KC > 0: hit lists of KC entries in local memory; KC = 0: W.hit_cap
 // entries per thread in global memory.  A job that outgrows its sets or its list is queued
 // for a later tier (out.ovf_list, once per read).
@@ -227,7 +243,7 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
   smem_fm_init(Sf, Fw, compat_fw);
   smem_fm_init(Sr, Rv, compat_rv);
   __syncthreads();
-  const uint32_t SCAP = STRIDE == 32 ? FAST_SET_CAP : W.set_cap;
+  const uint32_t SCAP = FMT == OCC_NARROW ? ACGT_SET_CAP : STRIDE == 32 ? FAST_SET_CAP : W.set_cap;
   using SR = SetRef<BIv, STRIDE>;
   LaneSet<SR> L;
   L.cur = thread_set<BIv, STRIDE>(W.sets, SCAP, 2, 0);
@@ -284,8 +300,10 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
       // they do not occur, no result reaches past them from before the second of them
       const bool window = ph == WINDOW;
       L.flo = 0; L.rlo = 0; L.sz = Fw.text_len; L.cnt = 1;
-      pos = window ? i + min_len - 1 : end;
+      if (window) end = i + min_len;
+      pos = window ? end - 1 : end;
       ph = window ? BACK : NEXT;
+      bool seeded = false;
       if (FMT == OCC_NARROW && A.kmer && A.k <= min_len) {
         uint32_t b0 = 0, b1 = 0, bad = 0;
         const uint8_t* b = p + pos + 1 - A.k;
@@ -297,9 +315,11 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
           if (!v.z) { i = at + 1; first = false; ph = WINDOW; continue; }
           L.flo = v.x; L.rlo = v.y; L.sz = v.z;
           if (at > i) pos = at - 1;
-          else { pos = i + min_len; ph = FORWARD; }        // k == min_len: the window is matched
+          else { pos = end; ph = FORWARD; }                // all of q[i, end) is matched
+          seeded = true;
         }
       }
+      if (window && !seeded) { end = seed_end(Sf.compat_mask, p, i, end); pos = end - 1; }
     }
     bool matched = false;                 // q[i, end) is a longest match from i
     if (ph == FORWARD && pos == n) { end = n; matched = true; }
@@ -315,13 +335,14 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
         if (!ok) { i = pos + 1; first = false; ph = WINDOW; }
         else if (pos > i) pos--;
         else {
-          pos = i + min_len;
+          pos = end;                      // of q[i, end) so far: the window, or up to its seed_end
           ph = FORWARD;
-          if (pos == n) { end = n; matched = true; }
+          if (pos == n) matched = true;
         }
       } else if (ph == FORWARD) {
         if (ok) pos++;
-        if (!ok || pos == n) { end = pos; matched = true; }
+        if (!ok && pos < i + min_len) { i = i + 1; first = false; ph = WINDOW; }   // the window at i does not match
+        else if (!ok || pos == n) { end = pos; matched = true; }
       } else if (ph == NEXT) {
         if (!ok) { i = pos + 1; ph = WINDOW; }
         else if (pos <= i + 1) { i = i + 1; ph = WINDOW; }      // q[i, end] is known not to match
