@@ -136,8 +136,9 @@ __global__ void __launch_bounds__(128, MINB) k_acgt(DevFm Fw, DevFm Rv, const ui
   uint4* hits = local_h;
   uint32_t hit_cap = KC;
   if (KC == 0) {
-    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    hits = W.hits + tid * W.hit_cap * 2;
+    // a list for each lane that takes jobs
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    hits = W.hits + (warp * lanes + min(threadIdx.x & 31, lanes - 1)) * W.hit_cap * 2;
     hit_cap = W.hit_cap;
   }
   // BACK .. LEFT_MAX take a step; SEEN, KMER, PLACE and TEXT make another load; the others wait

@@ -923,6 +923,10 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
     lanes = (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, ((n_units + n_fast) * 32 + full_threads - 1) / full_threads));
     threads = std::min<uint64_t>(full_threads, ((n_units + n_fast + lanes - 1) / lanes + 3) / 4 * 128);
   }
+  // Hit lists of variant 3.  k_acgt finds one hit at a position at most, and has one list for each
+  // lane that takes jobs: lists for every thread of a batch of 250 reads took 3.1 GB.
+  const uint64_t lists = fmt == OCC_NARROW ? threads / 32 * lanes : std::max<uint64_t>(threads, 128);
+  const uint32_t list_cap = fmt == OCC_NARROW ? std::min(FAST_HIT_CAP, 2 * seg_len) : FAST_HIT_CAP;
   RET(x->hit_start.ensure(n_slots * 8 + 8)); RET(x->hit_count.ensure(n_slots * 4 + 4));
   RET(x->pos_count.ensure(n_slots * 8 + 8)); RET(x->slot_pos.ensure((n_slots + 1) * 8));
   RET(x->hit_base.ensure(((size_t)nq + 1) * 8));
@@ -938,7 +942,7 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
   if (!plain) {
     if (fmt == OCC_WIDE) RET(x->memwork.ensure(std::max<uint64_t>(threads, 128) * MEM_SET_BYTES));
     else RET(x->left_jobs.ensure((n_units + n_fast) * 4 + 4));
-    if (variant == 3) RET(x->cwork.ensure((size_t)std::max<uint64_t>(threads, 128) * FAST_HIT_CAP * 32));
+    if (variant == 3) RET(x->cwork.ensure((size_t)lists * list_cap * 32));
   } else if (nq) {
     // plain launch, count pass: every read's MemHits and positions counted by a full
     // search, read back and prefix-summed to size the outputs before the write pass
@@ -1005,13 +1009,13 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
     if (!plain && (n_fast > 0 || n_long > 0)) {
       MemsWork W{};
       W.sets = x->memwork.as<BIv>(); W.set_cap = MEM_SET_CAP;
-      W.hits = variant == 3 ? x->cwork.as<uint4>() : nullptr; W.hit_cap = variant == 3 ? FAST_HIT_CAP : 0u;
+      W.hits = variant == 3 ? x->cwork.as<uint4>() : nullptr; W.hit_cap = variant == 3 ? list_cap : 0u;
       W.queue = &dctr(x)->queue; W.still_ovf = &dctr(x)->still_ovf; W.work_log = wlog; W.chunk = x->queue_chunk;
       SmemJobs J{};
       J.unit_read = x->uread.as<uint32_t>(); J.unit_k = x->uk.as<uint32_t>(); J.seg_len = seg_len;
       J.n_units = (uint32_t)n_units; J.ids = fast_ids; J.n_ids = n_fast; J.slot_base = slot_base;
       const unsigned grid = (unsigned)(threads / 128);
-      if (variant == 3 && x->cwork.cap < (size_t)grid * 128 * FAST_HIT_CAP * 32)
+      if (variant == 3 && x->cwork.cap < (size_t)lists * list_cap * 32)
         return set_error(HFM_E_ARG, "internal: hit list area too small");
       if (trie && n_fast > 0) {
         TrieWork T{x->trie_nodes.as<uint4>(), &dctr(x)->trie_queue, tgroup, x->trie_left.as<uint32_t>(), &dctr(x)->n_left,
@@ -1043,6 +1047,10 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
             const unsigned g2 = (unsigned)std::min<uint64_t>(grid, ((uint64_t)x->h_ctr->n_left + 127) / 128);
             RET(x->memwork.ensure((size_t)g2 * 128 * MEM_SET_BYTES));
             W.sets = x->memwork.as<BIv>();
+            if (variant == 3) {
+              RET(x->cwork.ensure((size_t)g2 * 128 * FAST_HIT_CAP * 32));
+              W.hits = x->cwork.as<uint4>(); W.hit_cap = FAST_HIT_CAP;
+            }
             W.queue = &dctr(x)->queue3;
             J.jobs = x->left_jobs.as<uint32_t>(); J.n_jobs = x->h_ctr->n_left;
             auto rest = [&](auto kern) {
