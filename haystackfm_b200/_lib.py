@@ -18,6 +18,7 @@ LIB_PATH = os.path.join(_HERE, "libhfm.so")
 
 HFM_FLAG_DEDUP_ALWAYS = 1
 HFM_FLAG_DEDUP_NEVER = 2
+HFM_FLAG_RECORDS_ONLY = 4
 
 u8p = C.POINTER(C.c_uint8)
 u32p = C.POINTER(C.c_uint32)

@@ -378,6 +378,13 @@ static int build_sa(hfm_index* x) {
   return rc;
 }
 
+// All of it, unless the caller declines it.
+static int build_aux(hfm_index* x) {
+  if (x->flags & HFM_FLAG_RECORDS_ONLY) return HFM_OK;
+  RET(build_kmer(x));
+  return build_sa(x);
+}
+
 // ---------------------------------------------------------------------------
 // Scan helper: out[0..n] = exclusive scan of in (stride in elements), out[n] = total.
 // ---------------------------------------------------------------------------
@@ -1781,8 +1788,7 @@ int hfm_index_load(const uint8_t* bytes, size_t len, int kind, const hfm_opts* o
   RET(x->ctr.ensure(sizeof(Counters)));
   RET(build_device_fm(hf, x->fwd, x->stream));
   if (kind == HFM_KIND_BIDIR) RET(build_device_fm(hr, x->rev, x->stream));
-  RET(build_kmer(x.get()));
-  RET(build_sa(x.get()));
+  RET(build_aux(x.get()));
   *out = x.release();
   return HFM_OK;
 }
@@ -1963,8 +1969,7 @@ int hfm_index_load_layout(const uint8_t* bytes, uint64_t len, const hfm_opts* op
     f.seq_boundaries = D.bnd;
   }
   CK(cudaStreamSynchronize(x->stream));
-  RET(build_kmer(x.get()));
-  RET(build_sa(x.get()));
+  RET(build_aux(x.get()));
   *out = x.release();
   return HFM_OK;
 }

@@ -44,6 +44,7 @@ typedef struct hfm_index hfm_index;   /* device-resident index, opaque */
 
 #define HFM_FLAG_DEDUP_ALWAYS 1u  /* resolve repeated SA intervals once per call, always      */
 #define HFM_FLAG_DEDUP_NEVER 2u   /* never deduplicate (default: when hits average >= 4 rows) */
+#define HFM_FLAG_RECORDS_ONLY 4u  /* load the index's own records and nothing beside them     */
 
 typedef struct hfm_opts {
   int32_t device;          /* CUDA device ordinal (one index per GPU; replicate for multi-GPU) */
@@ -134,6 +135,14 @@ int hfm_build_index_gpu(const uint8_t* codes, const uint64_t* seq_off, uint32_t 
  *      src/fm_index/serialize.rs:32-52, src/fm_index/bidir_index.rs:195-210, and the
  *      per-call uploads of src/gpu/locate.rs:69-111, src/gpu/mem_find.rs:56-102,
  *      src/gpu/mem_resolve.rs:44-85) ---------------------------------------- */
+/* Both loads also make, on the device, what the searches are faster with: the position of
+ * every row (4 bytes a row, for sample rates up to 1,024) and on texts of ACGT alone the text
+ * (half a byte a position), a table of all k-mers (at most 2 bytes a position and 1.1 GB) and,
+ * for a bidirectional index, the bits of the strings that occur (half a byte to 2 bytes a
+ * position, 2.1 GB at most).  Each is made only when it takes at most a quarter of the memory
+ * that is free then.  HFM_FLAG_RECORDS_ONLY declines them all: for a load as short as the
+ * upload, or where the memory is wanted otherwise (3.1 Gbp: 5.4 GB and 17 GB beside it, 0.55 s
+ * more).  Results do not depend on it; searches then take steps and walks in their place. */
 int hfm_index_load(const uint8_t* bincode, size_t len, int kind, const hfm_opts* opts, hfm_index** out);
 /* Device-layout blob (no counterpart in the reference): hfm_index_export_layout writes the
  * handle's device records — after the transform from the bincode records that
