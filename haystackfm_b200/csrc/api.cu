@@ -79,11 +79,12 @@ static void compat_masks(uint32_t tag, uint16_t out[16]) {
 struct DevBuf {
   void* p = nullptr;
   size_t cap = 0;
-  int ensure(size_t bytes) {
+  // grows: false for a buffer that is made once, as large as it is asked for
+  int ensure(size_t bytes, bool grows = true) {
     if (bytes <= cap) return HFM_OK;
     if (p) cudaFree(p);
     p = nullptr; cap = 0;
-    size_t want = std::max<size_t>(bytes + std::min<size_t>(bytes / 4, 256ull << 20), 256);   // growth slack
+    size_t want = std::max<size_t>(bytes + (grows ? std::min<size_t>(bytes / 4, 256ull << 20) : 0), 256);   // growth slack
     cudaError_t e = cudaMalloc(&p, want);
     if (e != cudaSuccess) {
       cudaGetLastError();
@@ -301,7 +302,7 @@ static int build_kmer(hfm_index* x) {
   while (k < KMER_MAX && (16ull << (2 * (k + 1))) <= 2ull * f.text_len) k++;
   if (k < 2 || !aux_room(20ull << (2 * k))) return HFM_OK;
   DevBuf tmp;
-  if (x->aux_kmer.ensure(16ull << (2 * k)) != HFM_OK || tmp.ensure(16ull << (2 * (k - 1))) != HFM_OK) {
+  if (x->aux_kmer.ensure(16ull << (2 * k), false) != HFM_OK || tmp.ensure(16ull << (2 * (k - 1)), false) != HFM_OK) {
     x->aux_kmer.release();
     return HFM_OK;
   }
@@ -332,7 +333,7 @@ static constexpr uint32_t SEEN_K_MAX = 18;      // 8 GB of bits, for texts near 
 static int build_sa(hfm_index* x) {
   const FmDev& f = x->fwd;
   if (f.rate < 1 || f.rate > SA_ROWS_RATE || f.d.sample_rate != f.rate || f.d.num_seqs > f.text_len || !f.text_len) return HFM_OK;
-  if (!aux_room((uint64_t)f.text_len * 4) || x->aux_sa.ensure((size_t)f.text_len * 4 + 16) != HFM_OK) return HFM_OK;    // read 16 bytes at a time
+  if (!aux_room((uint64_t)f.text_len * 4) || x->aux_sa.ensure((size_t)f.text_len * 4 + 16, false) != HFM_OK) return HFM_OK;    // read 16 bytes at a time
   CK(cudaMemsetAsync(x->aux_sa.p, 0xFF, (size_t)f.text_len * 4, x->stream));
   const uint64_t items = (uint64_t)f.d.num_blocks + f.d.num_seqs;
   WITH_FMT(f.fmt, { k_sa_rows<FM><<<(unsigned)((items + 127) / 128), 128, 0, x->stream>>>(f.d, f.nbytes[3] / 4, x->aux_sa.as<uint32_t>()); });
@@ -344,8 +345,8 @@ static int build_sa(hfm_index* x) {
   // inconsistent index)
   const uint64_t n = f.text_len, words = n / 32 + 2;
   DevBuf bytes;
-  if (bytes.ensure(n) != HFM_OK) return HFM_OK;
-  if (x->aux_text.ensure(words * 16) != HFM_OK) { bytes.release(); return HFM_OK; }
+  if (bytes.ensure(n, false) != HFM_OK) return HFM_OK;
+  if (x->aux_text.ensure(words * 16, false) != HFM_OK) { bytes.release(); return HFM_OK; }
   auto run = [&]() -> int {
     uint32_t* unknown = &x->ctr.as<Counters>()->walk_err;
     CK(cudaMemsetAsync(unknown, 0, 4, x->stream));
@@ -363,7 +364,7 @@ static int build_sa(hfm_index* x) {
     uint32_t k = 3;
     while ((1ull << (2 * k)) < 4ull * n) k++;
     const uint64_t seen_bytes = (1ull << (2 * k)) / 8;
-    if (x->kind != HFM_KIND_BIDIR || k > SEEN_K_MAX || !aux_room(seen_bytes) || x->aux_seen.ensure(seen_bytes) != HFM_OK) return HFM_OK;
+    if (x->kind != HFM_KIND_BIDIR || k > SEEN_K_MAX || !aux_room(seen_bytes) || x->aux_seen.ensure(seen_bytes, false) != HFM_OK) return HFM_OK;
     CK(cudaMemsetAsync(x->aux_seen.p, 0, seen_bytes, x->stream));
     k_seen_bits<<<(unsigned)((n + 8191) / 8192), 256, 0, x->stream>>>(bytes.as<uint8_t>(), (uint32_t)n, k,
                                                                      x->aux_seen.as<uint32_t>());

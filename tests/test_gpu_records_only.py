@@ -58,3 +58,15 @@ def test_records_only_forward_index(oracle):
     for g, w in zip(h.locate_packed(flat, off, 0), o.locate_packed(flat, off, 0)):
         assert np.array_equal(g, w)
     assert np.array_equal(h.count_packed(flat, off), o.count_packed(flat, off))
+
+
+def test_arrays_beside_the_records_have_no_slack():
+    """They never grow: 4 bytes a row, and on an ACGT text what its length says."""
+    ref = synth.repeat_reference(total=3_000_000, n_contigs=2, seed=6)
+    b = _build([al.DnaSequence(c) for c in ref.contigs], FmIndexConfig(sa_sample_rate=32), 1, KIND_BIDIR)
+    full, bare = _Handle(b, KIND_BIDIR), _Handle(b, KIND_BIDIR, 0, HFM_FLAG_RECORDS_ONLY)
+    n = 3_000_002
+    k = max(k for k in range(2, 14) if 16 << 2 * k <= 2 * n)
+    seen = min(4 ** k for k in range(3, 18) if 4 ** k >= 4 * n) // 8
+    beside = (4 * n + 16) + (n // 32 + 2) * 16 + (16 << 2 * k) + seen
+    assert full.device_bytes()["index"] - bare.device_bytes()["index"] == beside
