@@ -329,7 +329,6 @@ static int build_kmer(hfm_index* x) {
 
 // The position of every row of the forward index (k_sa_rows), and what the SMEM search of an
 // ACGT text keeps with it.
-static constexpr uint32_t SEEN_K_MAX = 18;      // 8 GB of bits, for texts near 2^32
 static int build_sa(hfm_index* x) {
   const FmDev& f = x->fwd;
   if (f.rate < 1 || f.rate > SA_ROWS_RATE || f.d.sample_rate != f.rate || f.d.num_seqs > f.text_len || !f.text_len) return HFM_OK;
@@ -360,11 +359,11 @@ static int build_sa(hfm_index* x) {
     if (x->h_ctr->walk_err) { x->aux_text.release(); return HFM_OK; }
     x->aux.sa = x->sa;
     x->aux.text = x->aux_text.as<uint4>();
-    // one bit per string of seen_k codes, 4 to 16 bits per text position
+    // one bit per string of seen_k codes, 4 to 16 bits per text position: at most 17 codes, 2 GB
     uint32_t k = 3;
     while ((1ull << (2 * k)) < 4ull * n) k++;
     const uint64_t seen_bytes = (1ull << (2 * k)) / 8;
-    if (x->kind != HFM_KIND_BIDIR || k > SEEN_K_MAX || !aux_room(seen_bytes) || x->aux_seen.ensure(seen_bytes, false) != HFM_OK) return HFM_OK;
+    if (x->kind != HFM_KIND_BIDIR || !aux_room(seen_bytes) || x->aux_seen.ensure(seen_bytes, false) != HFM_OK) return HFM_OK;
     CK(cudaMemsetAsync(x->aux_seen.p, 0, seen_bytes, x->stream));
     k_seen_bits<<<(unsigned)((n + 8191) / 8192), 256, 0, x->stream>>>(bytes.as<uint8_t>(), (uint32_t)n, k,
                                                                      x->aux_seen.as<uint32_t>());
