@@ -534,6 +534,8 @@ extern "C" int hfm_build_index_gpu(const uint8_t* codes, const uint64_t* seq_off
   GCK(cudaGetDeviceCount(&ndev));
   if (device < 0 || device >= ndev) return set_error(HFM_E_ARG, "device ordinal out of range");
   GCK(cudaSetDevice(device));
+  int sms = 0;
+  GCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   const uint64_t n = fwd.bounds.back(), raw = n - nseq;
   const bool both = kind == HFM_KIND_BIDIR;
   fwd.text_len = rev.text_len = (uint32_t)n;
@@ -589,7 +591,7 @@ extern "C" int hfm_build_index_gpu(const uint8_t* codes, const uint64_t* seq_off
   if (raw) GCK(cudaMemcpyAsync(staged, codes + seq_off[0], raw, cudaMemcpyHostToDevice, R.s));
   GCK(cudaMemcpyAsync(d_bounds, fwd.bounds.data(), (size_t)nseq * 4, cudaMemcpyHostToDevice, R.s));
   GCK(cudaMemsetAsync(d_freq, 0, 64, R.s));
-  k_join<<<std::min<unsigned>(grid_for((n + 15) / 16), 148 * 4), 256, 0, R.s>>>(staged, d_bounds, nseq, n, text, d_freq);
+  k_join<<<std::min<unsigned>(grid_for((n + 15) / 16), (unsigned)sms * 4), 256, 0, R.s>>>(staged, d_bounds, nseq, n, text, d_freq);
   GCK(cudaGetLastError());
   GCK(cudaMemcpyAsync(freq, d_freq, 64, cudaMemcpyDeviceToHost, R.s));
   GCK(cudaStreamSynchronize(R.s));
