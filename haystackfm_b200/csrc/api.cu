@@ -825,10 +825,10 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
   if (n_warp && !order) return set_error(HFM_E_ARG, "sched.n_warp needs sched.d_order");
   begin_stats(x);
   uint32_t launches = 0, other = 0;
-  // IUPAC texts: the first sweep of the reads in one piece is shared by the reads of a warp
-  // (k_trie).  A per-read work log needs every read's own work.
-  const bool trie = x->fwd.fmt == OCC_WIDE && x->mems_variant != MEMS_PLAIN && x->threads_per_read == 1 && !wlog &&
-                    min_len > 0 && nq > n_warp;
+  // IUPAC texts: the first sweep of the reads in one piece is shared by the reads of a block
+  // (k_trie).
+  const bool trie = x->fwd.fmt == OCC_WIDE && x->mems_variant != MEMS_PLAIN && x->threads_per_read == 1 && min_len > 0 &&
+                    nq > n_warp;
   uint32_t tblocks = 0, tgroup = 0;
   if (trie) RET(trie_plan(x, nq - n_warp, tblocks, tgroup));
   if (!order && x->threads_per_read == 1 && x->mems_variant != MEMS_PLAIN && nq > 1 &&
@@ -1026,7 +1026,7 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
         return set_error(HFM_E_ARG, "internal: hit list area too small");
       if (trie && n_fast > 0) {
         TrieWork T{x->trie_nodes.as<uint4>(), &dctr(x)->trie_queue, tgroup, x->trie_left.as<uint32_t>(), &dctr(x)->n_left,
-                   x->trie_resume.as<uint32_t>()};
+                   x->trie_resume.as<uint32_t>(), wlog};
         auto run = [&](auto kern) {
           kern<<<tblocks, TRIE_WARPS * 32, TRIE_SMEM, x->stream>>>(Fw.d, Rv.d, Rv.compat.as<uint16_t>(), d_q, d_qoff, P, hp, o,
                                                                   T, J);
@@ -1406,7 +1406,7 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
     W.queue = &dc->queue; W.still_ovf = &dc->still_ovf; W.chunk = x->queue_chunk;
     if (c.trie) {
       TrieWork T{x->trie_nodes.as<uint4>(), &dc->trie_queue, c.tgroup, x->trie_left.as<uint32_t>(), &dc->n_left,
-                 x->trie_resume.as<uint32_t>()};
+                 x->trie_resume.as<uint32_t>(), nullptr};
       k_trie<false><<<c.tblocks, TRIE_WARPS * 32, TRIE_SMEM, x->stream>>>(Fw.d, Rv.d, crv, c.d_q, c.d_qoff, P, hp, o, T, J);
       CK(cudaGetLastError());
       J.ids = T.left; J.n_ids_dev = T.n_left; J.resume = T.resume;

@@ -22,6 +22,10 @@
 // in k_smem, which starts behind it (SmemJobs::resume).  The set is that of the window and
 // forward phases there (smem.cuh): the SA intervals of the text strings that match.
 //
+// With a work log every read is charged with the nodes that hold it, as if its set were extended
+// for it alone: what it costs does not depend on the reads around it, unless a list outgrows its
+// area (the log says so).
+//
 // Measured on a B200, 150 bp reads on the 100 Mbp IUPAC text, kernel times of a thread per
 // read, of this sweep with a warp per group, with a block, and as it is (one warp prepares a
 // position, symbols without children skipped, both kinds of nodes at a time, five blocks an SM
@@ -61,6 +65,7 @@ struct TrieWork {
   uint32_t group;                           // reads per block, 1..32
   uint32_t* left; uint32_t* n_left;         // reads that k_smem goes on with
   uint32_t* resume;                         // for each of them: where, or RESUME_START
+  uint32_t* work_log;                       // COUNT_TOUCH only, 4 u32 per read (MemsWork), or nullptr
 };
 
 // A node list: the first SC nodes in shared memory, the others in the warp's global area.
@@ -102,6 +107,14 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 5) k_trie(DevFm Fw, DevFm Rv,
     const uint64_t slot = mine ? (J.slot_base ? J.slot_base[read] : (uint64_t)read) : 0;
     if (mine && warp == 0) { out.hit_start[slot] = 0; out.hit_count[slot] = 0; out.pos_count[slot] = 0; }
     uint32_t alive = __ballot_sync(0xFFFFFFFFu, mine && n >= P.min_len);      // min_len >= 1 here
+    uint32_t work = 0;                      // COUNT_TOUCH: this warp's touches for read `lane`
+    auto charge = [&](uint32_t holds, uint32_t touch) {
+      if (!W.work_log) return;
+      for (uint32_t m = __reduce_or_sync(0xFFFFFFFFu, holds); m; m &= m - 1) {
+        const uint32_t r = __ffs(m) - 1, b = __ballot_sync(0xFFFFFFFFu, (holds >> r) & 1);
+        if (lane == r) work += touch * (uint32_t)__popc(b);
+      }
+    };
 
     // Hands the reads in `who` to k_smem: after [0, j), or from the start.
     auto leave = [&](uint32_t who, uint32_t j) {
@@ -112,6 +125,7 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 5) k_trie(DevFm Fw, DevFm Rv,
       if ((who >> lane) & 1) {
         W.left[at + __popc(who & lt)] = read;
         W.resume[at + __popc(who & lt)] = j;
+        if (COUNT_TOUCH && W.work_log && j == RESUME_START) atomicOr(W.work_log + 4 * (size_t)read + 3, 1u);
       }
     };
     // The result [0, j) of the reads in `who`, a warp per read: one hit per node that holds
@@ -213,6 +227,7 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 5) k_trie(DevFm Fw, DevFm Rv,
           for (int s = 1; s < 16; s++)
             if (d[s] && (v.w & reads[s])) { kids += d[s] == 1 ? 1u : 0x10000u; syms |= 1u << s; }
         }
+        if (COUNT_TOUCH) charge(v.w & alive, 2);
         uint32_t total;
         const uint32_t at = warp_excl_scan(kids, total);
         uint32_t a1 = 0, ab = 0;
@@ -242,9 +257,9 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 5) k_trie(DevFm Fw, DevFm Rv,
       // one-row nodes: one LF step each; from the last warp on, so that short lists of both
       // kinds are worked off at the same time
       for (uint32_t b = (TRIE_WARPS - 1 - warp) * 32; b < n1; b += TRIE_WARPS * 32) {
-        uint4 kid = make_uint4(0, 0, 0, 0);
+        uint4 kid = make_uint4(0, 0, 0, 0), v = kid;
         if (b + lane < n1) {
-          const uint4 v = one.get(b + lane);
+          v = one.get(b + lane);
           uint32_t s, rk;
           row_code_rank<OCC_WIDE>(X, v.y, s, rk);
           if (COUNT_TOUCH) touches += 1;
@@ -252,6 +267,7 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 5) k_trie(DevFm Fw, DevFm Rv,
           kid = make_uint4(v.x, S.C[s] + rk, 1u, who);
           still |= who;
         }
+        if (COUNT_TOUCH) charge(v.w & alive, 1);
         const uint32_t bal = __ballot_sync(0xFFFFFFFFu, kid.w != 0);
         if (!bal) continue;
         uint32_t a1 = 0;
@@ -277,6 +293,7 @@ __global__ void __launch_bounds__(TRIE_WARPS * 32, 5) k_trie(DevFm Fw, DevFm Rv,
       }
       n1 = m1; nb = mb; t ^= 1; c = cn;
     }
+    if (COUNT_TOUCH && W.work_log && mine && work) atomicAdd(W.work_log + 4 * (size_t)read, work);
     __syncthreads();
   }
   if (COUNT_TOUCH && touches) atomicAdd(out.touches, (unsigned long long)touches);
