@@ -1282,13 +1282,29 @@ __device__ uint32_t warp_mems_one(const DevFm& Fw, const DevFm& Rv, const SmemFm
   uint32_t i = 0;
   while (n - i >= P.min_len) {
     reset();
-    uint32_t e = seed_end(Sf.compat_mask, q, i, i + P.min_len), k = e;
-    while (k > i && left(k - 1)) k--;
+    // from the window's end, and from its seed_end where that gives a large set (looking for it
+    // in every window costs a load's wait: 4% with a warp a read).  Smaller groups leave reads
+    // with such sets to the warp.
+    uint32_t k = i + P.min_len, from = k;
+    if constexpr (G < 32) {
+      while (k > i && left(k - 1)) k--;
+    } else {
+      bool looked = false;
+      while (k > i && left(k - 1)) {
+        k--;
+        if (ncur > (Fw.fmt == OCC_NARROW ? 64u : 256u) && !looked && k > i) {
+          looked = true;
+          const uint32_t at = seed_end(Sf.compat_mask, q, i, from);
+          if (at < from) { from = k = at; reset(); }
+        }
+      }
+    }
     if (ovf) { st |= ST_SET_OVF; return ~0u; }
     if (k > i) { i = k; continue; }
+    uint32_t e = G < 32 ? i + P.min_len : from;
     while (e < n && right(e)) e++;
     if (ovf) { st |= ST_SET_OVF; return ~0u; }
-    if (e < i + P.min_len) { i++; continue; }          // the window at i does not match
+    if (G == 32 && e < i + P.min_len) { i++; continue; }          // the window at i does not match
     if (nc >= cand_cap) { st |= ST_CAND_OVF; return ~0u; }
     uint64_t off = 0;
     if (lane == 0) off = thread_reserve(ivpool, ncur);

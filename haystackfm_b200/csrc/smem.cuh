@@ -28,13 +28,14 @@
 //
 // Where a window starts.  Codes of several symbols multiply a set, an N fourfold and more, until
 // the codes around it have narrowed it down; a window that ended in a run of N was extended from
-// that run and had 4^run intervals.  A window with more than SEED_AMBIGUOUS of them starts at the
-// end of its longest run of ACGT instead (seed_end), goes left to i and then right: where the
-// left part empties, the same holds as above; where the right one does within the window, no
-// match of min_len starts at i.  B200, 1,000 reads of 150 bp on 64 Mbp ACGT, the sweep / from the
-// window's end / so, with ACGT sets of more than ACGT_SET_CAP intervals left to the warp kernel:
-// 8 N at a random place 140 / 188 / 90 ms, N from 60 to 69 4.2 / 13.2 / 5.3 s, N from 13 to 18 18.2 /
-// 12.9 / 8.5 ms, 4 N at a random place 142 / 38 / 4.7 ms.
+// that run and had 4^run intervals.  A window whose set grows like that and that holds more than
+// SEED_AMBIGUOUS of them starts anew, at the end of its longest run of ACGT (seed_end), goes left
+// to i and then right: where the left part empties, the same holds as above; where the right one
+// does within the window, no match of min_len starts at i.  B200, 1,000 reads of 150 bp on 64 Mbp
+// ACGT, the sweep / from the window's end / so, with ACGT sets of more than ACGT_SET_CAP intervals
+// left to the warp kernel: 8 N at a random place 140 / 188 / 90 ms, N from 60 to 69 4.2 / 13.2 / 5.2
+// s, N from 13 to 18 18.2 / 12.9 / 9.1 ms, 4 N at a random place 142 / 38 / 7.6 ms.  (Looked for in
+// every window before its first step: 3 to 6% for reads with a single N, 4.7 ms for the last.)
 //
 // Segments.  A result belongs to the segment of a long read in which it starts.  A segment's
 // search begins at its first position a: if the window there does not match, everything
@@ -243,6 +244,9 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
   smem_fm_init(Sf, Fw, compat_fw);
   smem_fm_init(Sr, Rv, compat_rv);
   __syncthreads();
+  // a window's set from which on its seed_end is looked for: three codes of several symbols and
+  // more, on texts with such codes more than the usual set
+  constexpr uint32_t SEED_SET = FMT == OCC_NARROW ? 16 : 128;
   const uint32_t SCAP = FMT == OCC_NARROW ? ACGT_SET_CAP : STRIDE == 32 ? FAST_SET_CAP : W.set_cap;
   using SR = SetRef<BIv, STRIDE>;
   LaneSet<SR> L;
@@ -265,6 +269,7 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
   uint32_t ph = FETCH, u = 0, read = 0, st = ST_OK;
   uint32_t n = 0, i = 0, stop = 0, pos = 0, end = 0, nh = 0;
   bool first = false;                     // the left-maximality of i is not known yet
+  bool looked = false;                    // BACK: seed_end of this window has been looked for
   const uint8_t* p = q;
   for (;;) {
     if (ph == FETCH) {
@@ -300,10 +305,9 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
       // they do not occur, no result reaches past them from before the second of them
       const bool window = ph == WINDOW;
       L.flo = 0; L.rlo = 0; L.sz = Fw.text_len; L.cnt = 1;
-      if (window) end = i + min_len;
+      if (window) { end = i + min_len; looked = false; }
       pos = window ? end - 1 : end;
       ph = window ? BACK : NEXT;
-      bool seeded = false;
       if (FMT == OCC_NARROW && A.kmer && A.k <= min_len) {
         uint32_t b0 = 0, b1 = 0, bad = 0;
         const uint8_t* b = p + pos + 1 - A.k;
@@ -315,11 +319,9 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
           if (!v.z) { i = at + 1; first = false; ph = WINDOW; continue; }
           L.flo = v.x; L.rlo = v.y; L.sz = v.z;
           if (at > i) pos = at - 1;
-          else { pos = end; ph = FORWARD; }                // all of q[i, end) is matched
-          seeded = true;
+          else { pos = end; ph = FORWARD; }                // k == min_len: the window is matched
         }
       }
-      if (window && !seeded) { end = seed_end(Sf.compat_mask, p, i, end); pos = end - 1; }
     }
     bool matched = false;                 // q[i, end) is a longest match from i
     if (ph == FORWARD && pos == n) { end = n; matched = true; }
@@ -333,8 +335,14 @@ __global__ void __launch_bounds__(128, MINB) k_smem(DevFm Fw, DevFm Rv, const ui
       if (ovf) { st |= ST_SET_OVF; ph = DONE; }
       else if (ph == BACK) {
         if (!ok) { i = pos + 1; first = false; ph = WINDOW; }
-        else if (pos > i) pos--;
-        else {
+        else if (pos > i) {
+          pos--;
+          if (L.cnt > SEED_SET && !looked) {
+            looked = true;
+            const uint32_t at = seed_end(Sf.compat_mask, p, i, end);
+            if (at < end) { end = at; pos = at - 1; L.flo = 0; L.rlo = 0; L.sz = Fw.text_len; L.cnt = 1; }
+          }
+        } else {
           pos = end;                      // of q[i, end) so far: the window, or up to its seed_end
           ph = FORWARD;
           if (pos == n) matched = true;
