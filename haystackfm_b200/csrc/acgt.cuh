@@ -270,9 +270,7 @@ __global__ void __launch_bounds__(128, MINB) k_acgt(DevFm Fw, DevFm Rv, const ui
     } else if (ph == PLACE) {
       a = reinterpret_cast<const uint4*>(A.sa) + (flo >> 2);
     } else if (ph == TEXT) {
-      // rlo: text position of code 0 (may wrap below 0).  Directions of an index that disagree
-      // give rows whose text ends before the match does: nothing matches there.
-      a = A.text + (min(rlo + pos, Fw.text_len) >> 5);
+      a = A.text + ((rlo + pos) >> 5);                         // rlo: text position of code 0 (may wrap below 0)
     }
     const uint4 va = __ldg(a);
     if (COUNT_TOUCH) touches += 1;
@@ -320,12 +318,15 @@ __global__ void __launch_bounds__(128, MINB) k_acgt(DevFm Fw, DevFm Rv, const ui
         }
       }
     } else if (ph == PLACE) {
-      rlo = sel4(va, flo & 3u) - i;
+      // Directions of an index that disagree give rows whose text ends before the match does:
+      // nothing matches at the end.  Further words are compared only when this one is the same,
+      // so its codes are in front of the end.
+      rlo = min(sel4(va, flo & 3u) - i + pos, Fw.text_len) - pos;
       ph = TEXT;
     } else {
       // the codes of this word against the text
       const uint4 vb = __ldg(a + 1);
-      const uint32_t b = pos & 31, sh = min(rlo + pos, Fw.text_len) & 31;
+      const uint32_t b = pos & 31, sh = (rlo + pos) & 31;
       const uint32_t x0 = __funnelshift_r(va.x, vb.x, sh) ^ (r.x >> b), x1 = __funnelshift_r(va.y, vb.y, sh) ^ (r.y >> b);
       const uint32_t diff = (x0 | x1 | __funnelshift_r(va.z, vb.z, sh) | (r.z | r.w) >> b) & (~0u >> b);
       const uint32_t same = diff ? (uint32_t)__ffs(diff) - 1u : 32u - b;
