@@ -122,7 +122,8 @@ struct hfm_index {
   int device = 0, kind = 0;
   FmDev fwd, rev;
   // made on the device when the index is loaded, owned by that handle like the records
-  DevAux aux{};                   // ACGT texts, bidirectional: for the SMEM search
+  DevAux aux{};                   // ACGT texts: for the SMEM search
+  DevAux aux_bs{};                // the same for the backward search
   const uint32_t* sa = nullptr;   // position of every forward row (resolve.cuh)
   DevBuf aux_kmer, aux_sa, aux_text, aux_seen;
   cudaStream_t stream = nullptr;
@@ -378,11 +379,37 @@ static int build_sa(hfm_index* x) {
   return rc;
 }
 
+// Does the index's own lookup table hold the rows of every string, so that the k-mer table may
+// answer for it?  Any table of the right size is accepted when an index is loaded, and what it
+// holds is the answer.  (4^depth searches of `depth` steps.)
+static int lookup_agrees(hfm_index* x, bool& agrees) {
+  const FmDev& f = x->fwd;
+  agrees = f.d.lut_radix == 4 && f.nbytes[4] == 8ull << (2 * f.d.lut_depth);
+  for (int c = 0; c < 16; c++) agrees = agrees && f.d.lut_digit[c] == (c >= 1 && c <= 4 ? c - 1 : 0xFF);
+  if (!agrees) return HFM_OK;
+  uint32_t* differ = &x->ctr.as<Counters>()->walk_err;
+  CK(cudaMemsetAsync(differ, 0, 4, x->stream));
+  const uint64_t entries = 1ull << (2 * f.d.lut_depth);
+  k_lookup_differs<<<(unsigned)((entries + 255) / 256), 256, 0, x->stream>>>(f.d, differ);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(&x->h_ctr->walk_err, differ, 4, cudaMemcpyDeviceToHost, x->stream));
+  CK(cudaStreamSynchronize(x->stream));
+  agrees = x->h_ctr->walk_err == 0;
+  return HFM_OK;
+}
+
 // All of it, unless the caller declines it.
 static int build_aux(hfm_index* x) {
   if (x->flags & HFM_FLAG_RECORDS_ONLY) return HFM_OK;
   RET(build_kmer(x));
-  return build_sa(x);
+  RET(build_sa(x));
+  x->aux_bs = x->aux;
+  if (x->aux.kmer && x->fwd.d.lut && x->aux.k >= x->fwd.d.lut_depth) {     // the k-mer table would be used
+    bool agrees = false;
+    RET(lookup_agrees(x, agrees));
+    if (!agrees) x->aux_bs.kmer = nullptr;
+  }
+  return HFM_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -499,7 +526,7 @@ static int run_bsearch(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
       cudaEventRecord(x->evk[0], x->stream);
       auto go = [&](auto kern) {
         kern<<<grid, 256, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, nq, cap, x->bswork.as<uint2>(), BS_SET_CAP,
-                                          &dctr(x)->queue, pool, o, x->aux);
+                                          &dctr(x)->queue, pool, o, x->aux_bs);
       };
       WITH_FMT(F.fmt, { if (x->count_work) go(k_bsearch<true, 32, FM>); else go(k_bsearch<false, 32, FM>); });
       cudaEventRecord(x->evk[1], x->stream);
@@ -528,7 +555,7 @@ static int run_bsearch(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
         CK(cudaMemsetAsync(&dctr(x)->queue2, 0, 4, x->stream));
         auto go = [&](auto kern) {
           kern<<<grid, 128, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, x->ovf.as<uint32_t>(), n_ovf, cap,
-                                            x->work.as<uint2>(), set_cap, &dctr(x)->queue2, pool, o, &dctr(x)->still_ovf, x->aux,
+                                            x->work.as<uint2>(), set_cap, &dctr(x)->queue2, pool, o, &dctr(x)->still_ovf, x->aux_bs,
                                             (const uint32_t*)nullptr);
         };
         WITH_FMT(F.fmt, { if (x->count_work) go(k_bsearch_warp<true, FM>); else go(k_bsearch_warp<false, FM>); });
@@ -1568,10 +1595,10 @@ static int fixed_locate(hfm_index* x, FixedLocate& c, bool launch) {
     CK(cudaMemsetAsync(dc, 0, sizeof(Counters), x->stream));
     WITH_FMT(F.fmt, {
       k_bsearch<false, 32, FM><<<(unsigned)(c.threads / 256), 256, 0, x->stream>>>(
-          F.d, cm, c.d_q, c.d_qoff, nq, c.max_hits, x->bswork.as<uint2>(), BS_SET_CAP, &dc->queue, pool, o, x->aux);
+          F.d, cm, c.d_q, c.d_qoff, nq, c.max_hits, x->bswork.as<uint2>(), BS_SET_CAP, &dc->queue, pool, o, x->aux_bs);
       k_bsearch_warp<false, FM><<<wgrid, 128, 0, x->stream>>>(F.d, cm, c.d_q, c.d_qoff, x->ovf.as<uint32_t>(), 0u, c.max_hits,
                                                               x->work.as<uint2>(), c.warp_cap, &dc->queue2, pool, o,
-                                                              &dc->still_ovf, x->aux, &dc->n_ovf);
+                                                              &dc->still_ovf, x->aux_bs, &dc->n_ovf);
     });
     k_zero_failed<<<(nq + 255) / 256, 256, 0, x->stream>>>(x->status.as<uint32_t>(), nq, x->niv.as<uint32_t>(),
                                                            x->nhits.as<uint64_t>());
@@ -1723,7 +1750,7 @@ static int make_shadow(hfm_index* x, hfm_index** out) {
   sh->queue_chunk = x->queue_chunk; sh->threads_per_read = x->threads_per_read; sh->read_order = x->read_order;
   sh->timeout_ms = x->timeout_ms;
   sh->shared_index = true;
-  sh->aux = x->aux; sh->sa = x->sa;
+  sh->aux = x->aux; sh->aux_bs = x->aux_bs; sh->sa = x->sa;
   for (int k = 0; k < 2; k++) {
     const FmDev& src = k ? x->rev : x->fwd;
     FmDev& dst = k ? sh->rev : sh->fwd;
@@ -2545,7 +2572,7 @@ extern "C" int hfm_count_batch_noalloc(hfm_index* x, const uint8_t* d_q, const u
   BsOut o{d_counts, nullptr, nullptr, nullptr, status, ovf, &ctr->n_ovf, &ctr->touches};
   WITH_FMT(F.fmt, {
     k_bsearch<false, 32, FM><<<NOALLOC_THREADS / 256, 256, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, nq, 0, fast,
-                                                                          NOALLOC_SET_CAP, &ctr->queue, pool, o, x->aux);
+                                                                          NOALLOC_SET_CAP, &ctr->queue, pool, o, x->aux_bs);
   });
   CK(cudaGetLastError());
   uint32_t n_ovf = 0;
@@ -2555,7 +2582,7 @@ extern "C" int hfm_count_batch_noalloc(hfm_index* x, const uint8_t* d_q, const u
     WITH_FMT(F.fmt, {
       k_bsearch_warp<false, FM><<<NOALLOC_WARPS / 4, 128, 0, x->stream>>>(F.d, F.compat.as<uint16_t>(), d_q, d_qoff, ovf, n_ovf, 0,
                                                                          tail, NOALLOC_WARP_SET_CAP, &ctr->queue2, pool, o,
-                                                                         &ctr->still_ovf, x->aux);
+                                                                         &ctr->still_ovf, x->aux_bs);
     });
     CK(cudaGetLastError());
     uint32_t still = 0;

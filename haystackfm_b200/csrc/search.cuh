@@ -263,6 +263,22 @@ __device__ __forceinline__ void each_code(const DevFm& F, uint32_t lo, uint32_t 
   }
 }
 
+// Entries of a lookup table over ACGT (last code in the top digit) that are not the rows of their
+// string, empty for none: the k-mer table stands in for one that has no such entry.
+__global__ void k_lookup_differs(DevFm F, uint32_t* __restrict__ differ) {
+  const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >> (2 * F.lut_depth)) return;
+  uint32_t C[5], lo = 0, n = F.text_len;
+  for (int c = 0; c < 5; c++) C[c] = F.C[c];
+  uint64_t touches = 0;
+  for (int k = (int)F.lut_depth - 1; k >= 0 && n; k--) {
+    if (!acgt_rows<false>(F, C, 1u + ((uint32_t)(idx >> (2 * k)) & 3u), lo, n, touches) || (uint64_t)lo + n > F.text_len) n = 0;
+  }
+  const uint2 iv = F.lut[idx];
+  const uint32_t rows = iv.y > iv.x ? iv.y - iv.x : 0u;
+  if (rows != n || (n && iv.x != lo)) atomicAdd(differ, 1u);
+}
+
 // The last codes of a pattern at once: the index's own lookup table (LookupTable::get,
 // src/fm_index/lookup.rs:101-111: only when all of them are ACGT, and whatever it holds is
 // the answer, which on IUPAC texts leaves out strings with other codes), or the k-mer table

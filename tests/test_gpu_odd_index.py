@@ -124,3 +124,28 @@ def test_samples_that_disagree(oracle, change):
     cut, cut_off = pack_queries([r[k:k + 9] for r in reads for k in range(0, len(r) - 8, 5)])
     for g, w in zip(h.locate_packed(cut, cut_off, 64), o.locate_packed(cut, cut_off, 64)):
         assert np.array_equal(g, w)
+
+
+@pytest.mark.parametrize("change", ["emptied", "exchanged"])
+def test_lookup_table_is_the_answer(oracle, change):
+    """What the index's lookup table holds for a pattern's last codes is the answer, also where the
+    records say otherwise."""
+    rng = np.random.default_rng(7)
+    a = rng.integers(1, 5, size=60_000).astype(np.uint8)
+    depth = 4
+    b = bytearray(_build([al.DnaSequence(a)], FmIndexConfig(sa_sample_rate=16, lookup_depth=depth), 1, KIND_FM))
+    lut = np.frombuffer(b, "<u4", 2 * 4 ** depth, len(b) - 1 - 8 * 4 ** depth).copy().reshape(-1, 2)
+    assert (lut[:, 1] >= lut[:, 0]).all() and int((lut[:, 1] - lut[:, 0]).sum()) > 50_000
+    if change == "emptied":
+        lut[::3] = 0
+    else:
+        lut[[5, 77]] = lut[[77, 5]]
+    b[len(b) - 1 - 8 * 4 ** depth:len(b) - 1] = lut.astype("<u4").tobytes()
+    b = bytes(b)
+    o = oracle.OracleIndex(b, KIND_FM)
+    h = _Handle(b, KIND_FM)
+    flat, off = pack_queries([a[k:k + n].copy() for n in (4, 6, 12, 40) for k in range(0, 50_000, 331)])
+    assert np.array_equal(h.count_packed(flat, off), o.count_packed(flat, off))
+    for g, w in zip(h.locate_packed(flat, off, 64), o.locate_packed(flat, off, 64)):
+        assert np.array_equal(g, w)
+    assert np.array_equal(h.share().count_packed(flat, off), o.count_packed(flat, off))
