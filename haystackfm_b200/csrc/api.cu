@@ -1343,7 +1343,8 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
     if (fmt == OCC_NARROW) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_acgt<false, 0, ACGT_BLOCKS>, 128, 0));
     else CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, k_smem<false, 32, 0, 8, OCC_WIDE>, 128, 0));
     c.threads = (uint64_t)std::max(1, bpsm) * x->num_sms * 128;
-    c.trie = fmt == OCC_WIDE && x->mems_variant == 3 && x->threads_per_read == 1 && seg;
+    // the chain runs the per-thread kernels whatever the handle's tuning is
+    c.trie = fmt == OCC_WIDE && seg;
     if (c.trie) RET(trie_plan(x, nq, c.tblocks, c.tgroup));
   }
   const uint64_t threads = c.threads;
@@ -1391,7 +1392,7 @@ static int fixed_chain(hfm_index* x, FixedChain& c, bool launch) {
   if (launch) CK(cudaMemsetAsync(x->ctr.p, 0, sizeof(Counters), x->stream));
   // the prefix queue order (read_order 1), inside the captured work like the rest
   const uint32_t* ord = nullptr;
-  if (x->threads_per_read == 1 && nq > 1 && (x->read_order == 1 || (c.trie && c.tgroup >= TRIE_SORT_GROUP)))
+  if (nq > 1 && ((x->threads_per_read == 1 && x->read_order == 1) || (c.trie && c.tgroup >= TRIE_SORT_GROUP)))
     RET(prefix_order(x, c.d_q, c.d_qoff, nq, ord, dummy, launch));
   // search: long reads cut into segments, the others whole, in one launch
   const uint64_t* slot_base = seg ? x->slot_base.as<uint64_t>() : nullptr;
