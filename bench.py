@@ -75,7 +75,7 @@ def parse():
     ap.add_argument("--serving-batches", type=int, default=1000)
     ap.add_argument("--serving-workers", type=int, default=3)
     ap.add_argument("--read-order", type=int, default=1,
-                    help="read_order of the profile modes (1: the autotuner's choice on the IUPAC workload)")
+                    help="read_order of the profile modes")
     ap.add_argument("--profile-step", action="store_true",
                     help="only the W + K headline steps (the launch-list command)")
     ap.add_argument("--profile-smem", action="store_true",
@@ -991,19 +991,23 @@ def main():
     k_bs_ms = statistics.mean(s1.ms_search_kernel for s1, *_ in per)
     k_res_loc_ms = statistics.mean(s1.ms_resolve_kernel for s1, *_ in per)
     # algorithmic bytes (32 B per random Occ / SA-marker / sa_vals / lookup touch, read bytes,
-    # 8 B per output position, 16 B per MEM hit header).  The resolve kernel walks each
-    # distinct SA row once (rows_unique after deduplication); copying the positions to every
-    # hit is a separate streaming kernel.
-    def rows_walked(c):
+    # 8 B per output position, 16 B per MEM hit header).  The resolve kernel reads each distinct
+    # row's 4-byte entry of the suffix array once (rows_unique after deduplication; without the
+    # array it walks: two sectors a step and the sample); copying the positions to every hit is
+    # a separate streaming kernel.
+    def rows_read(c):
         return c.rows_unique if c.rows_unique else c.rows_resolved
+
+    def resolve_bytes(c):
+        return 64 * c.lf_calls + (32 if c.lf_calls else 4) * rows_read(c) + 8 * rows_read(c)
     b_mems = 32 * c_mem.occ_touches + 150 * n + 16 * c_mem.hits_out
-    b_res_mem = 32 * (2 * c_mem.lf_calls + rows_walked(c_mem)) + 8 * rows_walked(c_mem)
+    b_res_mem = resolve_bytes(c_mem)
     b_bs = 32 * c_loc.occ_touches + 32 * n
-    b_res_loc = 32 * (2 * c_loc.lf_calls + rows_walked(c_loc)) + 8 * rows_walked(c_loc)
+    b_res_loc = resolve_bytes(c_loc)
     kern = {"smem_search": (k_mems_ms, b_mems, c_mem.occ_touches, "Occ touches"),
-            "k_resolve(smem)": (k_res_mem_ms, b_res_mem, c_mem.lf_calls, "LF steps"),
+            "k_resolve(smem)": (k_res_mem_ms, b_res_mem, rows_read(c_mem), "rows"),
             "k_bsearch": (k_bs_ms, b_bs, c_loc.occ_touches, "Occ touches"),
-            "k_resolve(locate)": (k_res_loc_ms, b_res_loc, c_loc.lf_calls, "LF steps")}
+            "k_resolve(locate)": (k_res_loc_ms, b_res_loc, rows_read(c_loc), "rows")}
     for k, v in kern.items():
         print(f"[bench] {k}: {v[0]:.3f} ms/launch, alg {v[1] / 1e9:.3f} GB, {v[2]} {v[3]}", file=sys.stderr)
     s1, s2 = per[-1][0], per[-1][1]
@@ -1179,7 +1183,7 @@ def main():
                     "index_build_s": round(build_s, 1), "index_cached": not built,
                     "index_sha256": hashlib.sha256(data).hexdigest(),
                     "locate_positions": int(loc_total), "mem_hits": int(n_hits), "mem_positions": int(n_pos),
-                    "distinct_rows_walked": int(rows_walked(c_mem) + rows_walked(c_loc)),
+                    "distinct_rows_walked": int(rows_read(c_mem) + rows_read(c_loc)),
                     "autotuned": tuning_main},
             "parity": parity,
             "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": int(launches), "memory": memory,
