@@ -141,7 +141,7 @@ int hfm_build_index_gpu(const uint8_t* codes, const uint64_t* seq_off, uint32_t 
  * for a bidirectional index, the bits of the strings that occur (half a byte to 2 bytes a
  * position, 2.1 GB at most).  Each is made only when it takes at most a quarter of the memory
  * that is free then.  HFM_FLAG_RECORDS_ONLY declines them all: for a load as short as the
- * upload, or where the memory is wanted otherwise (3.1 Gbp: 5.4 GB and 17 GB beside it, 0.55 s
+ * upload, or where the memory is wanted otherwise (3.1 Gbp: 6.6 GB and 17 GB beside it, 0.6 s
  * more).  Results do not depend on it; searches then take steps and walks in their place. */
 int hfm_index_load(const uint8_t* bincode, size_t len, int kind, const hfm_opts* opts, hfm_index** out);
 /* Device-layout blob (no counterpart in the reference): hfm_index_export_layout writes the

@@ -38,7 +38,7 @@ def test_every_tuning_takes_the_sweep(oracle):
                                               L.ptr(bounds, L.u32p), len(bounds), 8, 8_000_000, C.byref(g)))
         try:
             best = 1e9
-            for _ in range(6):
+            for _ in range(25):
                 d, replayed = L.HfmDevMems(), C.c_uint32()
                 t = time.perf_counter()
                 L.check(L.lib().hfm_mems_graph_launch(g, C.byref(d), C.byref(replayed)))
