@@ -834,6 +834,7 @@ static int mems_device(hfm_index* x, const uint8_t* d_q, const uint64_t* d_qoff,
                        uint32_t mode, const uint32_t* h_bounds, uint32_t nb, uint32_t cap, hfm_dev_mems* out,
                        const hfm_sched* sc = nullptr) {
   if (x->kind != HFM_KIND_BIDIR) return set_error(HFM_E_ARG, "MEM/SMEM search needs a bidirectional index");
+  if (x->fwd.fmt != x->rev.fmt) return set_error(HFM_E_FORMAT, "the directions are of different texts: one holds ambiguity codes");
   if (mode > 1) return set_error(HFM_E_ARG, "mode must be 0 (SMEM) or 1 (MEM)");
   const uint32_t* order = sc ? sc->d_order : nullptr;
   uint32_t n_warp = sc ? sc->n_warp : 0;
@@ -2327,6 +2328,7 @@ extern "C" int hfm_mems_graph_create(hfm_index* x, const uint8_t* d_q, const uin
                                      uint32_t nb, uint32_t max_hits, uint64_t max_positions, hfm_graph** out) {
   if (!x || !out || !d_qoff || !nq || (nb && !ref_bounds)) return set_error(HFM_E_ARG, "NULL argument or empty batch");
   if (x->kind != HFM_KIND_BIDIR) return set_error(HFM_E_ARG, "MEM/SMEM search needs a bidirectional index");
+  if (x->fwd.fmt != x->rev.fmt) return set_error(HFM_E_FORMAT, "the directions are of different texts: one holds ambiguity codes");
   if (mode > 1) return set_error(HFM_E_ARG, "mode must be 0 (SMEM) or 1 (MEM)");
   *out = nullptr;
   std::unique_lock<std::mutex> lk(x->mu);

@@ -149,3 +149,35 @@ def test_lookup_table_is_the_answer(oracle, change):
     for g, w in zip(h.locate_packed(flat, off, 64), o.locate_packed(flat, off, 64)):
         assert np.array_equal(g, w)
     assert np.array_equal(h.share().count_packed(flat, off), o.count_packed(flat, off))
+
+
+@pytest.mark.parametrize("wide_forward", [False, True])
+def test_directions_of_different_record_formats(oracle, wide_forward):
+    """One direction holds ambiguity codes, the other does not: their records have different sizes.
+    MEM searches, which read both, are refused; the forward index alone is searched as ever."""
+    import ctypes as C
+
+    import torch
+    from haystackfm_b200 import _lib as L
+    from haystackfm_b200.errors import FmIndexError
+    rng = np.random.default_rng(9)
+    a = rng.integers(1, 5, size=20_000).astype(np.uint8)
+    c = a.copy()
+    c[::50] = 5
+    if wide_forward:
+        a, c = c, a
+    fwd = _build([al.DnaSequence(a)], FmIndexConfig(sa_sample_rate=16, lookup_depth=4), 0, KIND_FM)
+    rev = _build([al.DnaSequence(c[::-1].copy())], FmIndexConfig(sa_sample_rate=16), 0, KIND_FM)
+    h = _Handle(struct.pack("<I", len(fwd)) + fwd + rev, KIND_BIDIR)
+    flat, off = pack_queries([a[k:k + 40].copy() for k in range(0, 19_000, 500)])
+    for variant, threads in ((3, 1), (2, 1), (4, 1), (3, 32)):
+        h.set_tuning(variant, 64, threads_per_read=threads)
+        with pytest.raises(FmIndexError):
+            h.mems_packed(flat, off, 19, 0, None, 64)
+    q, qo, g = torch.from_numpy(flat).cuda(), torch.from_numpy(off.astype(np.int64)).cuda(), C.c_void_p()
+    assert L.lib().hfm_mems_graph_create(h.h, q.data_ptr(), qo.data_ptr(), len(off) - 1, len(flat), 19, 0, None, 0, 64, 10_000,
+                                         C.byref(g)) != 0
+    o = oracle.OracleIndex(fwd, KIND_FM)
+    assert np.array_equal(h.count_packed(flat, off), o.count_packed(flat, off))
+    for g, w in zip(h.locate_packed(flat, off, 64), o.locate_packed(flat, off, 64)):
+        assert np.array_equal(g, w)
